@@ -132,7 +132,7 @@ static void preloadKernels(int dev) {
   done[dev] = true;
   cudaFuncAttributes attr;
   auto touch = [&](const void* fn) { if (fn && cudaFuncGetAttributes(&attr, fn) != cudaSuccess) (void)cudaGetLastError(); };
-  for (const void* fn : {p2pKernelFn(), copyKernelFn(), copyBulkKernelFn(), llCopyKernelFn(), localCopyKernelFn(4), localCopyKernelFn(8), localBulkCopyKernelFn(),
+  for (const void* fn : {p2pKernelFn(), copyKernelFn(), copyBulkKernelFn(), llCopyKernelFn(), localCopyKernelFn(4, nullptr, nullptr), localCopyKernelFn(8, nullptr, nullptr), localCopyKernelFn(4, nullptr, (const void*)1), localBulkCopyKernelFn(),
                          signalKernelFn(), waitSignalKernelFn()})
     touch(fn);
   for (int t = 0; t < ncclNumTypes; ++t) {
@@ -407,9 +407,10 @@ static ncclResult_t launchColl(ncclComm* comm, const void* fn, CollArgs* a, int 
 static ncclResult_t scaleCopy(ncclComm* comm, ncclDataType_t type, const void* src, void* dst, size_t count, const DevOp& op,
                               cudaStream_t stream) {
   ScaleArgs sa{src, dst, count, op.premulBits, op.premulPtr};
-  int ctas = (int)std::min<size_t>((count + 4095) / 4096, 1024);
+  const size_t perCta = 512 * 4 * 16;   // bytes that a CTA of the kernel moves in one tile
+  int ctas = (int)std::min<size_t>((count * typeSize(type) + perCta - 1) / perCta, (size_t)comm->devPlane->smCount * 16);
   comm->devPlane->launches++;
-  return launchKernel(scaleKernelFn(type), dim3(std::max(ctas, 1)), dim3(256), 0, &sa, stream, false);
+  return launchKernel(scaleKernelFn(type), dim3(std::max(ctas, 1)), dim3(512), 0, &sa, stream, false);
 }
 
 void sliceEven(size_t count, size_t es, int n, size_t* begin, size_t* cnt) {
@@ -930,7 +931,7 @@ static ncclResult_t runOneRank(ncclComm* comm, const Task& t) {
     size_t perCta = (size_t)threads * unroll * 16;
     int ctas = (int)std::min<size_t>((bytes + perCta - 1) / perCta, (size_t)comm->devPlane->smCount * paramCopyCtasPerSm());
     comm->devPlane->launches++;
-    NCCLCHECK(launchKernel(localCopyKernelFn(unroll), dim3(std::max(ctas, 1)), dim3(threads), 0, &ca, t.stream, false));
+    NCCLCHECK(launchKernel(localCopyKernelFn(unroll, src, dst), dim3(std::max(ctas, 1)), dim3(threads), 0, &ca, t.stream, false));
   }
   return ncclSuccess;
 }

@@ -28,7 +28,7 @@ ncclResult_t signalRun(ncclComm* comm, const Task& t) {
       size_t perCta = 512 * 4 * 16;
       int ctas = (int)std::min<size_t>((bytes + perCta - 1) / perCta, (size_t)dp->smCount * 2);
       dp->launches++;
-      NCCLCHECK(launchKernel(localCopyKernelFn(4), dim3(std::max(ctas, 1)), dim3(512), 0, &ca, t.stream, false));
+      NCCLCHECK(launchKernel(localCopyKernelFn(4, ca.src, ca.dst), dim3(std::max(ctas, 1)), dim3(512), 0, &ca, t.stream, false));
     }
     if (comm->nRanks == 1 && !dp->resWin) return ncclSuccess;
     OneSignalArgs sa{signalWord(comm, t.root, comm->rank, idx)};
