@@ -399,7 +399,11 @@ __global__ void __launch_bounds__(kEpThreads, 1) epDispatchKernel(const __grid_c
         const int j = pos - sCell[el * n + s];
         const char* slot = a.recvBuf[rank] + zoneOff + ((size_t)(el * n + s) * a.maxTokens + j) * slotBytes;
         const size_t o = (size_t)el * cap + pos;
-        if (lane == 0) a.srcInfo[rank][o] = make_int2(s, ((const int*)slot)[0]);
+        if (lane == 0) {
+          const int from = ((const int*)slot)[0];
+          a.srcInfo[rank][o] = make_int2(s, from);
+          if (a.rowOf) a.rowOf[from] = (int)o;
+        }
         char* dstTok = (char*)a.outTokens[rank] + o * rowBytes;
         {
           const size_t packs = rowBytes / 16;
@@ -654,7 +658,260 @@ __global__ void __launch_bounds__(kEpThreads, 1) epCombineKernel(const __grid_co
   }
 }
 
+// ---------------------------------------------------------------------------------------------- one rank
+// With one rank every row stays on this GPU and nobody has to be waited for. The local forms move each row once: dispatch
+// claims the rows of the output tensors and writes them straight from the input (the general kernel stores into a landing
+// zone and packs from there: written twice, read once more), combine reads the experts' rows where they lie. Both are bound
+// by memory: for 4096 tokens of 7168 bf16 channels and 8 of 32 experts dispatch went from 313 to 103 us and combine from 434 to
+// 81 us (5.1 and 6.5 TB/s).
+constexpr int kLocTokens = 64;    // tokens of a CTA whose rows are claimed (or looked up) together
+constexpr int kLocMaxK = 16;
+
+// Payload of the tokens t0 + j * tStep, j < batch, to the rows sRow[j * R .. j * R + R) (-1: none). A work item is one 16-byte
+// store per row: 8 channels of bf16, or 16 channels of e4m3, whose group of 128 is then shared by 8 lanes. The items of the
+// batch are dealt to the threads without regard to token borders, and the loads of a round are issued before the previous
+// round is stored. `claim` fills sRow between the first loads and the first stores.
+template <bool FP8, typename Claim>
+__device__ __forceinline__ void localPayload(const EpArgs& a, const __nv_bfloat16* x, int t0, int tStep, int batch, int R, const int* sRow, Claim claim) {
+  constexpr int U = FP8 ? 1 : 2;            // items of a thread per round
+  constexpr int kIn = FP8 ? 2 : 1;          // 16-byte loads of an item
+  const int H = a.hidden, C = H / (8 * kIn);
+  const int total = batch * C;              // a multiple of 8: the lanes of a group are in or out together
+  uint4 cur[U][kIn];
+  auto load = [&](int first) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = first + u * kEpLocalThreads;
+      const int j = i / C, c = i - j * C;
+#pragma unroll
+      for (int q = 0; q < kIn; ++q)
+        cur[u][q] = i < total ? ldStream16(x + (size_t)(t0 + j * tStep) * H + (size_t)(c * kIn + q) * 8) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  const size_t rowBytes = FP8 ? (size_t)H : (size_t)H * 2;
+  char* const out = (char*)a.outTokens[a.rank];
+  load(threadIdx.x);
+  claim();
+  for (int first = threadIdx.x; first - (int)(threadIdx.x & 31) < total; first += U * kEpLocalThreads) {
+    uint4 val[U];
+    float scale[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      scale[u] = 0.0f;
+      if (FP8) {
+        float v[16];
+        float amax = 0.0f;
+#pragma unroll
+        for (int q = 0; q < kIn; ++q) {
+          const __nv_bfloat162* p = (const __nv_bfloat162*)&cur[u][q];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            v[q * 8 + 2 * i] = __bfloat162float(p[i].x);
+            v[q * 8 + 2 * i + 1] = __bfloat162float(p[i].y);
+            amax = fmaxf(amax, fmaxf(fabsf(v[q * 8 + 2 * i]), fabsf(v[q * 8 + 2 * i + 1])));
+          }
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        amax = fmaxf(amax, 1e-4f);
+        scale[u] = amax * (1.0f / 448.0f);
+        const float inv = 448.0f / amax;
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          w[i] = (uint32_t)__nv_cvt_float_to_fp8(v[4 * i] * inv, __NV_SATFINITE, __NV_E4M3) |
+                 ((uint32_t)__nv_cvt_float_to_fp8(v[4 * i + 1] * inv, __NV_SATFINITE, __NV_E4M3) << 8) |
+                 ((uint32_t)__nv_cvt_float_to_fp8(v[4 * i + 2] * inv, __NV_SATFINITE, __NV_E4M3) << 16) |
+                 ((uint32_t)__nv_cvt_float_to_fp8(v[4 * i + 3] * inv, __NV_SATFINITE, __NV_E4M3) << 24);
+        val[u] = make_uint4(w[0], w[1], w[2], w[3]);
+      } else {
+        val[u] = cur[u][0];
+      }
+    }
+    load(first + U * kEpLocalThreads);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = first + u * kEpLocalThreads;
+      if (i >= total) continue;
+      const int j = i / C, c = i - j * C;
+      for (int r = 0; r < R; ++r) {
+        const int row = sRow[j * R + r];
+        if (row < 0) continue;
+        st16(out + (size_t)row * rowBytes + (size_t)c * 16, val[u]);
+        if (FP8 && (c & 7) == 0) a.outScales[a.rank][(size_t)row * (H / 128) + (c >> 3)] = scale[u];
+      }
+    }
+  }
+}
+
+template <bool FP8>
+__global__ void __launch_bounds__(kEpLocalThreads, 2) epDispatchLocalKernel(const __grid_constant__ EpArgs a) {
+  __shared__ int sRow[kLocTokens * kLocMaxK];
+  __shared__ int sHist[kEpMaxLocalExperts];
+  __shared__ int sIsLast;
+  const int me = a.rank, K = a.topk, E = a.numExperts, T = a.numTokens[me], cap = a.maxTokens;
+  const int b = blockIdx.x, grid = gridDim.x;
+  uint32_t* st = a.state[me];
+  const int64_t* idx = a.topkIdx[me];
+  const int mine = T > b ? (T - b + grid - 1) / grid : 0;   // tokens b, b + grid, ...
+  const bool rankMajor = a.layout == EP_RANK_MAJOR;
+  const int R = rankMajor ? 1 : K;
+  if (rankMajor) {
+    for (int e = threadIdx.x; e < E; e += kEpLocalThreads) sHist[e] = 0;
+    __syncthreads();
+    // routing rows of all slots, used or not, and the count of every expert
+    for (int t = b * kEpLocalThreads + threadIdx.x; t < cap; t += grid * kEpLocalThreads) {
+      bool any = false;
+      for (int k = 0; t < T && k < K; ++k) {
+        const int64_t e = idx[(size_t)t * K + k];
+        if (e >= 0 && e < E) {
+          any = true;
+          atomicAdd(&sHist[e], 1);
+        }
+      }
+      a.srcInfo[me][t] = any ? make_int2(me, t) : make_int2(-1, 0);
+      for (int k = 0; k < K; ++k) {
+        const size_t o = (size_t)t * K + k;
+        const int64_t e = any ? idx[o] : -1;
+        if (a.outTopkIdx[me]) a.outTopkIdx[me][o] = e >= 0 && e < E ? e : -1;
+        if (a.outTopkW[me]) a.outTopkW[me][o] = any && a.topkW[me] ? a.topkW[me][o] : 0.0f;
+      }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += kEpLocalThreads)
+      if (sHist[e]) atomicAdd(&st[kStCounters + e], (uint32_t)sHist[e]);
+  }
+  for (int base = 0; base < mine; base += kLocTokens) {
+    const int batch = mine - base < kLocTokens ? mine - base : kLocTokens;
+    const int t0 = b + base * grid;
+    localPayload<FP8>(a, a.x[me], t0, grid, batch, R, sRow, [&] {
+      __syncthreads();   // the previous batch is stored
+      for (int i = threadIdx.x; i < batch * R; i += kEpLocalThreads) {
+        const int t = t0 + i / R * grid;
+        int row = -1;
+        if (rankMajor) {
+          for (int k = 0; k < K && row < 0; ++k) {
+            const int64_t e = idx[(size_t)t * K + k];
+            if (e >= 0 && e < E) row = t;
+          }
+        } else {
+          const size_t o = (size_t)t * K + i % R;
+          const int64_t e = idx[o];
+          if (e >= 0 && e < E) {
+            const int s = (int)atomicAdd(&st[kStCounters + e], 1u);
+            if (s < cap) {   // always, unless a token names an expert twice
+              row = (int)e * cap + s;
+              a.srcInfo[me][row] = make_int2(me, (int)o);
+              a.rowOf[o] = row;
+            }
+          }
+        }
+        sRow[i] = row;
+      }
+      __syncthreads();
+    });
+  }
+  // the last CTA publishes the counts and leaves the counters at zero
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    sIsLast = atomicAdd(&st[2], 1u) == (uint32_t)grid - 1;
+  }
+  __syncthreads();
+  if (!sIsLast) return;
+  __threadfence();
+  for (int e = threadIdx.x; e < E; e += kEpLocalThreads) {
+    const uint32_t c = __ldcg(&st[kStCounters + e]);
+    const int n = rankMajor || c < (uint32_t)cap ? (int)c : cap;
+    a.expertCount[me][e] = n;
+    if (a.userCount) a.userCount[e] = n;
+    st[kStCounters + e] = 0;
+  }
+  if (threadIdx.x == 0) st[2] = 0;
+}
+
+// out[t] = sum over the token's selected experts of w * row, in fp32, in slot order. The (token, 8 channels) items are dealt to
+// the CTAs as contiguous ranges; where the rows lie and their weights is looked up once per token and CTA.
+__global__ void __launch_bounds__(kEpLocalThreads, 2) epCombineLocalKernel(const __grid_constant__ EpArgs a) {
+  __shared__ int sRow[kLocTokens * kLocMaxK];
+  __shared__ float sW[kLocTokens * kLocMaxK];
+  const int me = a.rank, H = a.hidden, K = a.topk, E = a.numExperts, T = a.numTokens[me];
+  const bool rankMajor = a.layout == EP_RANK_MAJOR;
+  const int R = rankMajor ? 1 : K;
+  const int64_t* idx = a.topkIdx[me];
+  const __nv_bfloat16* y = a.x[me];
+  __nv_bfloat16* out = (__nv_bfloat16*)a.outTokens[me];
+  const int C = H / 8;
+  const size_t items = (size_t)T * C;
+  const size_t lo = items * blockIdx.x / gridDim.x, hi = items * (blockIdx.x + 1) / gridDim.x;
+  if (lo >= hi) return;
+  const int tLast = (int)((hi - 1) / C);
+  for (int tb = (int)(lo / C); tb <= tLast; tb += kLocTokens) {
+    const int batch = tLast - tb + 1 < kLocTokens ? tLast - tb + 1 : kLocTokens;
+    __syncthreads();
+    for (int i = threadIdx.x; i < batch * R; i += kEpLocalThreads) {
+      const int t = tb + i / R;
+      int row = -1;
+      float w = 0.0f;
+      if (rankMajor) {
+        for (int k = 0; k < K && row < 0; ++k) {
+          const int64_t e = idx[(size_t)t * K + k];
+          if (e >= 0 && e < E) row = t;
+        }
+        w = 1.0f;   // the caller has weighted the rows
+      } else {
+        const size_t o = (size_t)t * K + i % R;
+        const int64_t e = idx[o];
+        if (e >= 0 && e < E) {
+          row = a.rowOf[o];
+          w = a.topkW[me][o];
+        }
+      }
+      sRow[i] = row;
+      sW[i] = w;
+    }
+    __syncthreads();
+    const size_t first = (size_t)tb * C > lo ? (size_t)tb * C : lo;
+    const size_t end = (size_t)(tb + batch) * C < hi ? (size_t)(tb + batch) * C : hi;
+    const int nItems = (int)(end - first), shift = (int)(first - (size_t)tb * C);
+    for (int i = threadIdx.x; i < nItems; i += kEpLocalThreads) {
+      const int j = (i + shift) / C, c = i + shift - j * C;
+      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      for (int r0 = 0; r0 < R; r0 += 8) {
+        uint4 v[8];
+        float wk[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int row = r0 + u < R ? sRow[j * R + r0 + u] : -1;
+          v[u] = make_uint4(0, 0, 0, 0);
+          wk[u] = 0.0f;
+          if (row >= 0) {
+            wk[u] = sW[j * R + r0 + u];
+            v[u] = ldStream16(y + (size_t)row * H + (size_t)c * 8);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const __nv_bfloat162* p = (const __nv_bfloat162*)&v[u];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            acc[2 * q] += wk[u] * __bfloat162float(p[q].x);
+            acc[2 * q + 1] += wk[u] * __bfloat162float(p[q].y);
+          }
+        }
+      }
+      uint4 o;
+      __nv_bfloat162* q = (__nv_bfloat162*)&o;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) q[k] = __floats2bfloat162_rn(acc[2 * k], acc[2 * k + 1]);
+      st16(out + (size_t)(tb + j) * H + (size_t)c * 8, o);
+    }
+  }
+}
+
 const void* epDispatchKernelFn() { return (const void*)epDispatchKernel; }
 const void* epCombineKernelFn() { return (const void*)epCombineKernel; }
+const void* epDispatchLocalKernelFn(int fp8) { return fp8 ? (const void*)epDispatchLocalKernel<true> : (const void*)epDispatchLocalKernel<false>; }
+const void* epCombineLocalKernelFn() { return (const void*)epCombineLocalKernel; }
 
 }  // namespace b200

@@ -36,6 +36,10 @@ struct EpArgs {
   long long* outTopkIdx[kMaxRanks];            // rank-major / flat: [slots, topk] expert ids of the token that are local to this rank, else -1
   float* outTopkW[kMaxRanks];                  // rank-major / flat: [slots, topk] the token's weights (may be null)
   int* recvTotal[kMaxRanks];                   // flat: number of tokens received (may be null)
+  // one-rank groups (null otherwise)
+  int* rowOf;                                  // expert-major: [numTokens, topk] row of the dispatched tensor that holds (token, k); written by
+                                               // every dispatch, read by the local combine
+  int* userCount;                              // local dispatch: the caller's copy of expertCount (may be null)
   // split-phase calls and rank masks
   int phases;                                  // bit 0: sending half of the kernel, bit 1: receiving half (send_only + ncclEpComplete run them apart)
   int enableMask;                              // a wait on a rank that runs out leaves that rank out from then on instead of failing the call
@@ -70,5 +74,9 @@ __host__ __device__ inline size_t epStageBytes(int hidden, int fp8) { return (ep
 
 const void* epDispatchKernelFn();
 const void* epCombineKernelFn();
+// A group of one rank, both halves in one call, expert-major or rank-major: no landing zones, no flags. kEpLocalThreads threads.
+constexpr int kEpLocalThreads = 512;
+const void* epDispatchLocalKernelFn(int fp8);
+const void* epCombineLocalKernelFn();
 
 }  // namespace b200

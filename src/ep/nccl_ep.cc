@@ -49,6 +49,7 @@ struct ncclEpHandle {
   const int64_t* topkIdx = nullptr;
   const float* topkW = nullptr;
   int2* srcInfo = nullptr;
+  int* rowOf = nullptr;               // one-rank groups, expert-major: where (token, k) went
   int* expertCount = nullptr;
   ncclEpAllocConfig_t alloc = {};     // the group's hooks, kept here so that a handle can outlive its group's record
   // a send_only call leaves its receiving half to ncclEpComplete
@@ -99,6 +100,17 @@ static ncclResult_t launchEp(const void* fn, EpArgs* a, int ctas, int ranksY, si
   // the attribute is per device and cheap to set: no process-wide "done once" flag
   if (smem > 40000) CUDACHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   return launchKernel(fn, dim3(ctas, ranksY), dim3(512), smem, a, stream, coop);
+}
+
+// Calls that the local kernels serve: one rank, both halves at once, rows whose places do not depend on one another. The flat
+// layout packs in arrival order and a split call must hold the rows between its halves: both take the general kernels.
+static bool localForm(const ncclEpGroup* g, int layout, bool sendOnly) { return g->n == 1 && !sendOnly && layout != EP_FLAT; }
+
+// `want`: CTAs that have something to do. Two CTAs per SM, or the caller's number of SMs with one each.
+static ncclResult_t launchEpLocal(ncclEpGroup* g, const void* fn, EpArgs* a, size_t want, cudaStream_t stream) {
+  const size_t most = g->cfg.max_num_sms ? std::min<size_t>(g->cfg.max_num_sms, g->smCount) : (size_t)2 * g->smCount;
+  if (g->comm->devPlane) g->comm->devPlane->launches++;
+  return launchKernel(fn, dim3((unsigned)std::max<size_t>(std::min(want, most), 1)), dim3(kEpLocalThreads), 0, a, stream, false);
 }
 
 B200_PARAM(EpBulk, "B200_EP_BULK", 1, "Expert-parallel dispatch hands the packed tokens to the bulk-copy engines (a ring of shared-memory stages per CTA) instead of storing them with the warps: 0 never, 1 for the expert-major layout, 2 for every layout")
@@ -220,7 +232,7 @@ ncclResult_t ncclEpGroupDestroy(ncclEpGroup_t g) {
 
 ncclResult_t ncclEpHandleMemSize(ncclEpGroup_t g, ncclEpLayout_t, const ncclEpHandleConfig_t*, size_t* size_out, int) {
   if (!g || !size_out) return ncclInvalidArgument;
-  *size_out = (size_t)g->El * g->n * g->maxTokens * sizeof(int2) + (size_t)g->El * sizeof(int);
+  *size_out = (size_t)g->El * g->n * g->maxTokens * sizeof(int2) + (size_t)g->El * sizeof(int) + (g->n == 1 ? (size_t)g->maxTokens * 16 * sizeof(int) : 0);
   return ncclSuccess;
 }
 
@@ -258,9 +270,13 @@ ncclResult_t ncclEpInitHandle(ncclEpHandle_t* out, ncclEpGroup_t g, ncclEpLayout
   h->K = num_topk;
   h->alloc = g->cfg.alloc;
   const size_t cap = (size_t)g->n * g->maxTokens;
-  CUDACHECK(epAlloc(h->alloc, (void**)&h->srcInfo, (size_t)g->El * cap * sizeof(int2)));
-  CUDACHECK(epAlloc(h->alloc, (void**)&h->expertCount, (size_t)g->El * sizeof(int)));
-  CUDACHECK(cudaMemset(h->expertCount, 0, (size_t)g->El * sizeof(int)));
+  // one allocation: srcInfo | expertCount | rowOf. The last two start at zero (whatever is read from rowOf is then a row of the
+  // dispatched tensor).
+  const size_t infoBytes = (size_t)g->El * cap * sizeof(int2), rows = g->n == 1 && layout == NCCL_EP_LAYOUT_EXPERT_MAJOR ? (size_t)g->maxTokens * num_topk : 0;
+  CUDACHECK(epAlloc(h->alloc, (void**)&h->srcInfo, infoBytes + (g->El + rows) * sizeof(int)));
+  h->expertCount = (int*)((char*)h->srcInfo + infoBytes);
+  if (rows) h->rowOf = h->expertCount + g->El;
+  CUDACHECK(cudaMemset(h->expertCount, 0, (g->El + rows) * sizeof(int)));
   *out = h;
   return ncclSuccess;
 }
@@ -286,7 +302,6 @@ ncclResult_t ncclEpHandleDestroy(ncclEpHandle_t h) {
   if (!h) return ncclSuccess;
   cudaDeviceSynchronize();
   epFree(h->alloc, h->srcInfo);
-  epFree(h->alloc, h->expertCount);
   delete h;
   return ncclSuccess;
 }
@@ -357,6 +372,7 @@ ncclResult_t ncclEpDispatch(ncclEpHandle_t h, const ncclEpDispatchInputs_t* in, 
   a.outScales[me] = fp8 ? (float*)out->scales->data : nullptr;
   a.expertCount[me] = h->expertCount;
   a.srcInfo[me] = h->srcInfo;
+  a.rowOf = h->rowOf;
   a.layout = h->layout == NCCL_EP_LAYOUT_RANK_MAJOR ? EP_RANK_MAJOR : h->layout == NCCL_EP_LAYOUT_FLAT ? EP_FLAT : EP_EXPERT_MAJOR;
   // the rank-major / flat forms measured slower through the bulk engines (one lane per destination writes the routing rows)
   a.bulkStages = (paramEpBulk() == 1 && a.layout == EP_EXPERT_MAJOR) || paramEpBulk() == 2 ? kEpBulkStages : 0;
@@ -369,11 +385,15 @@ ncclResult_t ncclEpDispatch(ncclEpHandle_t h, const ncclEpDispatchInputs_t* in, 
   if (h->pending) { WARN("ncclEpDispatch: a send_only call on this handle is still waiting for ncclEpComplete"); return ncclInvalidUsage; }
   const bool sendOnly = config && config->send_only;
   if (sendOnly) a.phases = 1;
+  void* counters = (li && li->expert_counters && li->expert_counters->data) ? li->expert_counters->data : nullptr;
+  if (localForm(g, a.layout, sendOnly) && (uintptr_t)in->tokens->data % 16 == 0) {   // the general kernel quantises from 8-byte loads
+    a.userCount = (int*)counters;
+    return launchEpLocal(g, epDispatchLocalKernelFn(fp8), &a, std::max(h->T, a.layout == EP_RANK_MAJOR ? (g->maxTokens + kEpLocalThreads - 1) / kEpLocalThreads : 1), stream);
+  }
   // the per-rank layouts count the tokens of every local expert with atomics while they unpack: start from zero
   if (a.layout != EP_EXPERT_MAJOR && !sendOnly) CUDACHECK(cudaMemsetAsync(h->expertCount, 0, (size_t)g->El * sizeof(int), stream));
   NCCLCHECK(launchEp(epDispatchKernelFn(), &a, ctas, 1, dispatchSmem(g->H, fp8, a.bulkStages), stream, false));
   if (g->comm->devPlane) g->comm->devPlane->launches++;
-  void* counters = (li && li->expert_counters && li->expert_counters->data) ? li->expert_counters->data : nullptr;
   if (sendOnly) {
     // tokens and counts are on their way; the receiving half (wait, pack) runs when ncclEpComplete is called
     h->pending = 1;
@@ -435,6 +455,10 @@ ncclResult_t ncclEpCombine(ncclEpHandle_t h, const ncclEpCombineInputs_t* in, co
   if (h->pending) { WARN("ncclEpCombine: a send_only call on this handle is still waiting for ncclEpComplete"); return ncclInvalidUsage; }
   const bool sendOnly = config && config->send_only;
   if (sendOnly) a.phases = 1;
+  if (localForm(g, a.layout, sendOnly)) {
+    a.rowOf = h->rowOf;
+    return h->T ? launchEpLocal(g, epCombineLocalKernelFn(), &a, ((size_t)h->T * (g->H / 8) + kEpLocalThreads - 1) / kEpLocalThreads, stream) : ncclSuccess;
+  }
   NCCLCHECK(launchEp(epCombineKernelFn(), &a, ctas, 1, 0, stream, false));
   if (g->comm->devPlane) g->comm->devPlane->launches++;
   if (sendOnly) {

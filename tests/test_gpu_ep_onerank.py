@@ -1,0 +1,91 @@
+"""Expert-parallel groups of one rank: the local dispatch / combine kernels against PyTorch and against the general kernels
+(which a split-phase call of the same group takes)."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def comm():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from nccl_b200 import Communicator, get_unique_id
+    torch.cuda.set_device(0)
+    c = Communicator(1, 0, get_unique_id())
+    yield c
+    c.destroy()
+
+
+def _batch(T, E, K, H, seed, drop):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    idx = torch.rand(T, E, device="cuda", generator=g).topk(K, dim=1).indices
+    if drop:
+        idx = torch.where(torch.rand(T, K, device="cuda", generator=g) < drop, torch.full_like(idx, -1), idx)
+    return x, idx.contiguous(), torch.rand(T, K, device="cuda", generator=g)
+
+
+# max_sms 1 makes one CTA serve several batches of 64 tokens; 256 experts and top-16 are the limits
+@pytest.mark.parametrize("T,cap,E,K,H,max_sms,drop", [(1, 1, 1, 1, 128, 0, 0.0), (5, 9, 256, 8, 640, 0, 0.2), (64, 64, 32, 16, 1024, 0, 0.0),
+                                                      (131, 140, 8, 3, 384, 1, 0.1), (700, 700, 16, 9, 7168, 0, 0.0), (2000, 2048, 8, 2, 128, 3, 0.3)])
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("layout", ["expert_major", "rank_major"])
+def test_local_kernels_match_the_general_ones(comm, T, cap, E, K, H, max_sms, drop, fp8, layout):
+    from nccl_b200.ops.ep import ExpertParallel
+    ep = ExpertParallel(comm, E, cap, H, max_sms=max_sms, layout=layout)
+    got = {}
+    for split in (False, True, False):   # the general kernels in between: the handle's records serve both
+        x, idx, w = _batch(T, E, K, H, 7, drop)
+        lead = (E, cap) if layout == "expert_major" else (1, cap)
+        toks = torch.zeros(*lead, H, dtype=torch.uint8 if fp8 else torch.bfloat16, device="cuda")
+        scales = torch.zeros(*lead, H // 128, device="cuda") if fp8 else None
+        toks, scales, counts = ep.dispatch(x, idx, w, fp8=fp8, toks=toks, scales=scales, send_only=split)
+        if split:
+            ep.complete()
+        y = toks
+        if fp8:
+            y = (toks.view(torch.float8_e4m3fn).float().view(*lead, H // 128, 128) * scales.unsqueeze(-1)).view(*lead, H).bfloat16()
+        out = ep.combine(y, send_only=split)
+        if split:
+            ep.complete()
+        mixed = ep.combine(y)   # a whole combine after a split dispatch as well
+        torch.cuda.synchronize()
+        assert torch.equal(out, mixed)
+        rows = [out, counts] + ([toks, ep.recv_topk_idx, ep.recv_topk_weights] + ([scales] if fp8 else []) if layout == "rank_major" else [])
+        if got:
+            assert all(torch.equal(a, b) for a, b in zip(rows, got["rows"]))   # bit for bit: same arithmetic in the same order
+        got["rows"] = rows
+        valid = (idx >= 0)
+        assert torch.equal(counts.long(), torch.bincount(idx[valid], minlength=E))
+        if layout == "expert_major":
+            ref = x.float() * (w * valid).sum(1, keepdim=True)
+        else:
+            ref = x.float() * valid.any(1, keepdim=True)
+        # e4m3 keeps 3 mantissa bits (2^-4 of the value), or 2^-9 of the block's scale among the subnormals; bf16 rounds twice
+        tol = (2 ** -4 if fp8 else 2 ** -7) * ref.abs() + (2 ** -8 * x.float().abs().amax() * (1 + w.sum(1).max()) if fp8 else 1e-6)
+        assert ((out.float() - ref).abs() <= tol).all()
+    assert comm.async_error() == 0
+    ep.destroy()
+
+
+def test_expert_named_twice_and_tokens_at_eight_bytes(comm):
+    from nccl_b200.ops.ep import ExpertParallel
+    ep = ExpertParallel(comm, 4, 16, 256)
+    x, idx, w = _batch(16, 4, 2, 256, 3, 0.0)
+    raw = torch.zeros(16 * 256 + 4, dtype=torch.bfloat16, device="cuda")
+    shifted = raw[4:].view(16, 256).copy_(x)   # 8-byte aligned: stays with the general kernel
+    a = ep.dispatch(x, idx, w, fp8=True)[2].clone()
+    b = ep.dispatch(shifted, idx, w, fp8=True)[2].clone()
+    assert torch.equal(a, b)
+    idx[:] = 1   # 32 claims for 16 rows: what does not fit is left out, nothing is written outside
+    toks, _, counts = ep.dispatch(x, idx, w, fp8=False)
+    torch.cuda.synchronize()
+    assert counts.tolist() == [0, 16, 0, 0]
+    idx.copy_(_batch(16, 4, 2, 256, 3, 0.0)[1])
+    toks, _, counts = ep.dispatch(x, idx, w, fp8=False)
+    out = ep.combine(toks)
+    torch.cuda.synchronize()
+    torch.testing.assert_close(out.float(), x.float() * w.sum(1, keepdim=True), rtol=2 ** -7, atol=1e-6)
+    ep.destroy()
