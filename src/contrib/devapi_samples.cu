@@ -12,7 +12,10 @@
 // contrib/nccl_ubx allreduce_2shot_* with residual and RMSNorm epilogue.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "nccl_device.h"
+#include "../tp/gemm_sm100.cuh"
 
 namespace {
 
@@ -141,6 +144,150 @@ __global__ void __launch_bounds__(kThreads) devApiArRmsNormKernel(ncclDevComm_t 
   bar.finish();
 }
 
+// One rank: x = partial + residual, residual <- x, out <- rmsnorm(x) * weight, as above without the sources to wait for.
+// Bound by memory on the SMs that the caller grants, so what counts is how much each of them has in flight: a producer warp
+// streams chunks of R neighbouring rows (partial and residual) into a ring of shared memory with bulk copies, groups of G
+// threads take one row each from there. 2048 rows of 8192 take 47 us on 64 CTAs; with a CTA to a row, its loads waiting for the
+// previous row's stores, they took 125.
+constexpr int kRowPacks = 8;          // 16-byte packs of a row per thread, at most
+constexpr int kRowStages = 16;        // chunks in the ring, at most
+constexpr size_t kRowRing = 200 << 10;
+constexpr int kRowThreads = kThreads + 32;
+
+struct RowArgs {
+  const char* partial;
+  char* residual;
+  char* out;
+  const char* weight;
+  float eps;
+  int tokens, hidden, chunkRows, stages;
+  int* status;
+};
+
+template <int G>
+__global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid_constant__ RowArgs a) {
+  using namespace b200::sm100;
+  using V = nccl_device::Vec16<__nv_bfloat16>;
+  constexpr int kGroups = kThreads / G, kWarps = G / 32;
+  extern __shared__ uint8_t ringRaw[];
+  uint8_t* ring = (uint8_t*)(((uintptr_t)ringRaw + 127) & ~(uintptr_t)127);
+  __shared__ float red[2][kThreads / 32];
+  __shared__ uint64_t fullBar[kRowStages], emptyBar[kRowStages];
+  __shared__ volatile int gaveUp;
+  const int R = a.chunkRows, chunks = (a.tokens + R - 1) / R;
+  const size_t rowBytes = (size_t)a.hidden * 2;
+  const uint32_t half = (uint32_t)(R * rowBytes);   // partial rows, then residual rows
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < a.stages; ++s) {
+      mbarInit(smemAddr(&fullBar[s]), 1);
+      mbarInit(smemAddr(&emptyBar[s]), R);   // one arrival per row
+    }
+    gaveUp = 0;
+    mbarInitFence();
+  }
+  __syncthreads();
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    if (gaveUp || mbarWait(smemAddr(bar), parity)) return;
+    gaveUp = 1;   // nobody waits any longer; the copies still under way are waited for below
+    atomicExch(a.status, 1);
+  };
+  if (threadIdx.x >= kThreads) {
+    if (threadIdx.x == kThreads) {
+      int i = 0;
+      for (int c = blockIdx.x; c < chunks && !gaveUp; c += gridDim.x, ++i) {
+        const int s = i % a.stages;
+        const uint32_t ph = (i / a.stages) & 1;
+        wait(&emptyBar[s], ph ^ 1);
+        const int rows = a.tokens - c * R < R ? a.tokens - c * R : R;
+        const uint32_t bytes = (uint32_t)(rows * rowBytes);
+        const size_t off = (size_t)c * R * rowBytes;
+        const uint32_t dst = smemAddr(ring) + (uint32_t)s * 2 * half, fb = smemAddr(&fullBar[s]);
+        mbarExpectTx(fb, 2 * bytes);
+        bulkLoad(dst, a.partial + off, bytes, fb);
+        bulkLoad(dst + half, a.residual + off, bytes, fb);
+      }
+      if (gaveUp)
+        for (int j = i > a.stages ? i - a.stages : 0; j < i; ++j) mbarWait(smemAddr(&fullBar[j % a.stages]), (j / a.stages) & 1, 1u << 20);
+    }
+  } else {
+    const int grp = threadIdx.x / G, tid = threadIdx.x % G;
+    const int packs = a.hidden / 8;
+    int parity = 0;
+    // row n of this CTA: row n % R of its chunk n / R
+    for (int n = grp;; n += kGroups, parity ^= 1) {
+      const int i = n / R, c = (int)blockIdx.x + i * (int)gridDim.x, r = n - i * R;
+      if (c >= chunks) break;
+      const int t = c * R + r;
+      if (t >= a.tokens) break;
+      const int s = i % a.stages;
+      wait(&fullBar[s], (i / a.stages) & 1);
+      const uint8_t* part = ring + (size_t)s * 2 * half + r * rowBytes;
+      char* res = a.residual + t * rowBytes;
+      uint4 sum[kRowPacks];
+      float ss = 0.0f;
+#pragma unroll
+      for (int k = 0; k < kRowPacks; ++k) {
+        const int pk = tid + k * G;
+        if (pk < packs) {
+          float x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+          V::add(x, *(const uint4*)(part + (size_t)pk * 16));
+          V::add(x, *(const uint4*)(part + half + (size_t)pk * 16));
+          // the residual stream is kept in bf16: normalise exactly what is stored
+          sum[k] = V::pack(x);
+          *(uint4*)(res + (size_t)pk * 16) = sum[k];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) x[j] = 0.0f;
+          V::add(x, sum[k]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) ss += x[j] * x[j];
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (kWarps > 1) {
+        // one word per warp, two sets by parity: a warp reaches the set again only after the group has met once more
+        if ((threadIdx.x & 31) == 0) red[parity][threadIdx.x >> 5] = ss;
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(G) : "memory");
+        ss = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) ss += red[parity][grp * kWarps + w];
+      }
+      if (tid == 0) mbarArrive(smemAddr(&emptyBar[s]));   // the whole group has read the row
+      const float inv = rsqrtf(ss / (float)a.hidden + a.eps);
+      char* out = a.out + t * rowBytes;
+#pragma unroll
+      for (int k = 0; k < kRowPacks; ++k) {
+        const int pk = tid + k * G;
+        if (pk < packs) {
+          float w[8] = {0, 0, 0, 0, 0, 0, 0, 0}, x[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+          V::add(w, *(const uint4*)(a.weight + (size_t)pk * 16));
+          V::add(x, sum[k]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) w[j] *= x[j] * inv;
+          *(uint4*)(out + (size_t)pk * 16) = V::pack(w);
+        }
+      }
+    }
+  }
+  __syncthreads();   // no thread leaves while a copy into this CTA's shared memory is under way
+}
+
+ncclResult_t launchRmsNormRows(RowArgs a, int nCtas, cudaStream_t stream) {
+  const size_t rowBytes = (size_t)a.hidden * 2;
+  // chunks of about 8 KiB (a copy below that costs more to issue than to move), while every CTA still gets several
+  a.chunkRows = std::max(1, std::min((int)(8192 / rowBytes), a.tokens / (4 * nCtas)));
+  a.stages = (int)std::min<size_t>(kRowStages, kRowRing / (2 * a.chunkRows * rowBytes));
+  const size_t smem = 128 + 2 * a.chunkRows * rowBytes * a.stages;
+  // the fewest threads to a row that hold it, more where there are not enough rows for that many groups
+  int g = 32;
+  while (g < kThreads && (g * kRowPacks < a.hidden / 8 || (long long)nCtas * (kThreads / g) > a.tokens)) g *= 2;
+  const void* fn = g == 32 ? (const void*)rmsNormRowsKernel<32> : g == 64 ? (const void*)rmsNormRowsKernel<64> : g == 128 ? (const void*)rmsNormRowsKernel<128> :
+                   g == 256 ? (const void*)rmsNormRowsKernel<256> : (const void*)rmsNormRowsKernel<512>;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return ncclUnhandledCudaError;
+  void* args[1] = {&a};
+  return cudaLaunchKernel(fn, dim3(nCtas), dim3(kRowThreads), args, smem, stream) == cudaSuccess ? ncclSuccess : ncclUnhandledCudaError;
+}
+
 // Exercises ncclLLA2ASession: every rank contributes two floats per slot; each rank receives the sum.
 __global__ void __launch_bounds__(256) devApiLLSumKernel(ncclDevComm_t dc, const float2* in, float2* out, int slots, int* status) {
   ncclCoopCta cta;
@@ -215,6 +362,10 @@ ncclResult_t b200DevApiArRmsNorm(const ncclDevComm_t* dc, ncclWindow_t inWin, si
   if (mode == 1 && !inWin->mcPtr) return ncclInvalidUsage;
   int* st = statusWord();
   if (!st) return ncclUnhandledCudaError;
+  if (dc->lsaSize == 1 && mode != 1) {
+    RowArgs a = {(const char*)inWin->peerPtr[inWin->rank] + inOff, (char*)resWin->peerPtr[resWin->rank] + resOff, (char*)outWin->peerPtr[outWin->rank] + outOff, (const char*)weight, eps, tokens, hidden, 0, 0, st};
+    return launchRmsNormRows(a, nCtas, stream);
+  }
   devApiArRmsNormKernel<<<nCtas, kThreads, 0, stream>>>(*dc, inWin->devSelf, inOff, resWin->devSelf, resOff, outWin->devSelf, outOff,
                                                         (const __nv_bfloat16*)weight, eps, tokens, hidden, mode, st);
   return cudaGetLastError() == cudaSuccess ? ncclSuccess : ncclUnhandledCudaError;

@@ -1,0 +1,37 @@
+"""The fused all-reduce + residual + RMSNorm kernel on one rank: row lengths around the limits of a group of threads, fewer
+and more rows than groups, against fp32 PyTorch."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("hidden", [8, 1016, 1024, 1032, 2048, 4096, 4104, 8192, 8200, 16384])
+@pytest.mark.parametrize("tokens,ctas", [(1, 64), (7, 3), (65, 1), (200, 5), (300, 64)])
+def test_rows(hidden, tokens, ctas):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from nccl_b200 import Communicator, get_unique_id
+    from nccl_b200.ops.devapi import DeviceComm
+    torch.cuda.set_device(0)
+    comm = Communicator(1, 0, get_unique_id())
+    dc = DeviceComm(comm)
+    part, resid, out = (dc.symmetric((tokens + 1) * hidden, torch.bfloat16).view(tokens + 1, hidden) for _ in range(3))
+    g = torch.Generator(device="cuda").manual_seed(hidden + tokens)
+    w = (1 + 0.1 * torch.randn(hidden, device="cuda", generator=g)).bfloat16()
+    for mode in (0, 2):
+        part.copy_(torch.randn(tokens + 1, hidden, device="cuda", generator=g))
+        resid.copy_(torch.randn(tokens + 1, hidden, device="cuda", generator=g))
+        out.fill_(9)
+        x = (part.float() + resid.float()).bfloat16()
+        ref = x.float() * torch.rsqrt(x.float().square().mean(1, keepdim=True) + 1e-5) * w.float()
+        guard = resid[tokens].clone()
+        torch.cuda.synchronize()
+        dc.ar_rmsnorm(part[:tokens], resid[:tokens], out[:tokens], w, eps=1e-5, mode=mode, ctas=ctas)
+        assert dc.status() == 0
+        assert torch.equal(resid[:tokens], x[:tokens]) and torch.equal(resid[tokens], guard) and (out[tokens] == 9).all()
+        # one bf16 rounding (2^-9) of a value that fp32 has to about 1e-6
+        torch.testing.assert_close(out[:tokens].float(), ref[:tokens], rtol=2 ** -8, atol=1e-6)
+    dc.destroy()
+    comm.destroy()
