@@ -13,6 +13,7 @@ using namespace b200;
 
 namespace b200 {
 B200_PARAM(TpCommCtas, "B200_TP_COMM_CTAS", 0, "CTAs that gather remote rows in all-gather -> GEMM (0: 4 for two ranks, 8 up to four, 16 beyond)")
+B200_PARAM(TpSplit, "B200_TP_SPLIT", 8, "Largest cluster of CTAs that shares the K dimension of a tile in plain bf16 GEMMs with few tiles (1: never, at most 8)")
 B200_PARAM(TpPair, "B200_TP_PAIR", 1, "bf16 GEMM on CTA pairs (256 x 256 tiles, tcgen05 cta_group::2) when the row count allows")
 }
 
@@ -20,6 +21,7 @@ struct ncclTpContext {
   ncclComm* comm = nullptr;
   int smCount = 0;
   int pairClusters = 0;   // clusters of the CTA-pair GEMM kernel that can be resident at once (0: unavailable)
+  int splitClusters[kTpMaxSplit + 1] = {};   // clusters of each size of the split kernel that can be resident at once
   void* accum = nullptr;           // symmetric staging window: bf16 [n sources][maxRows / n][maxCols]
   size_t accumBytes = 0;
   SymWindow* accumWin = nullptr;
@@ -63,6 +65,12 @@ static ncclResult_t makeMap(CUtensorMap* map, const void* base, int rows, int K,
   return ncclSuccess;
 }
 
+static void clusterAttribute(cudaLaunchAttribute* attr, int ctas) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = ctas;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+}
+
 static int tpCommCtas(const ncclTpContext* tp, int nRanks) {
   int64_t want = paramTpCommCtas();
   if (want <= 0) want = nRanks <= 2 ? 4 : nRanks <= 4 ? 8 : 16;
@@ -89,6 +97,37 @@ static void fillSyncTp(ncclComm* comm, SyncArgs* s) {
   s->timeoutNs = dp ? dp->timeoutNs : 5000000000ull;
 }
 
+// CTAs that share the K blocks of a tile in a plain bf16 GEMM, 1 for none: as many as leave every cluster resident at once,
+// when the 128 x 256 tiles alone would leave half of the SMs idle, and each CTA keeps kSplitMinBlocks K blocks (below that the
+// exchange of the partial sums costs more than the shorter loop saves).
+constexpr int kSplitMinBlocks = 8;
+static int splitOf(const ncclTpContext* tp, const TpGemmArgs* a) {
+  const int tiles = (a->M / 128) * (a->N / 256);
+  int s = std::min(std::min(std::min((int)paramTpSplit(), kTpMaxSplit), tp->smCount / tiles), a->K / 64 / kSplitMinBlocks);
+  while (s > 1 && tiles > tp->splitClusters[s]) --s;
+  return std::max(s, 1);
+}
+
+static ncclResult_t launchGemmSplit(ncclTpContext* tp, const void* A, const void* W, TpGemmArgs* a, cudaStream_t stream) {
+  CUtensorMap tmA, tmB;
+  NCCLCHECK(makeMap(&tmA, A, a->M, a->K, 128));
+  NCCLCHECK(makeMap(&tmB, W, a->N, a->K, 256));
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute cluster;
+  clusterAttribute(&cluster, a->splitK);
+  cfg.gridDim = dim3((a->M / 128) * (a->N / 256) * a->splitK);
+  cfg.blockDim = dim3(tpGemmSplitThreads());
+  cfg.dynamicSmemBytes = tpGemmSplitSmemBytes();
+  cfg.stream = stream;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = 1;
+  void* args[3] = {&tmA, &tmB, a};
+  cudaError_t e = cudaLaunchKernelExC(&cfg, tpGemmSplitKernelFn(), args);
+  if (e != cudaSuccess) { WARN("tensor-parallel GEMM launch failed: %s", cudaGetErrorString(e)); (void)cudaGetLastError(); return ncclUnhandledCudaError; }
+  if (tp->comm->devPlane) tp->comm->devPlane->launches++;
+  return ncclSuccess;
+}
+
 // Launches the bf16 GEMM kernel in the mode of `a`. Grid: one CTA per SM (fewer when there are fewer
 // tiles); in all-gather mode the last CTAs are the comm CTAs. The CTA-pair kernel runs when enabled,
 // when its clusters fit and when every rank's rows split into 256-row tiles.
@@ -96,6 +135,7 @@ static ncclResult_t launchGemm(ncclTpContext* tp, const void* A, const void* W, 
   const int n = a->nRanks;
   const bool fused = n > 1 && a->mode != TP_MODE_STORE;
   const bool gather = fused && a->mode == TP_MODE_GATHER;
+  if (!fused && (a->splitK = splitOf(tp, a)) > 1) return launchGemmSplit(tp, A, W, a, stream);
   const bool pair = paramTpPair() != 0 && tp->pairClusters > 0 && a->M % (256 * (fused ? n : 1)) == 0;
   int commCtas = gather ? tpCommCtas(tp, n) : 0;
   int grid;
@@ -275,6 +315,7 @@ ncclResult_t ncclTpCreate(ncclComm_t comm, size_t maxRows, size_t maxCols, ncclT
   CUDACHECK(cudaDeviceGetAttribute(&tp->smCount, cudaDevAttrMultiProcessorCount, comm->cudaDev));
   // function attributes are per device: set them here, with this context's device current, not once per process
   CUDACHECK(cudaFuncSetAttribute(tpGemmKernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmSmemBytes()));
+  CUDACHECK(cudaFuncSetAttribute(tpGemmSplitKernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmSplitSmemBytes()));
   CUDACHECK(cudaFuncSetAttribute(tpGemmFp8KernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmFp8SmemBytes()));
   {
     // how many clusters of two CTAs of the pair kernel the device can hold at once: the grid never exceeds it,
@@ -289,6 +330,17 @@ ncclResult_t ncclTpCreate(ncclComm_t comm, size_t maxRows, size_t maxCols, ncclT
       tp->pairClusters = std::min(clusters, tp->smCount / 2);
     else
       (void)cudaGetLastError();
+    cudaLaunchAttribute cluster;
+    cfg.attrs = &cluster;
+    cfg.numAttrs = 1;
+    cfg.blockDim = dim3(tpGemmSplitThreads());
+    cfg.dynamicSmemBytes = tpGemmSplitSmemBytes();
+    for (int size = 2; size <= kTpMaxSplit; ++size) {
+      clusterAttribute(&cluster, size);
+      cfg.gridDim = dim3(tp->smCount / size * size);
+      if (cudaOccupancyMaxActiveClusters(&clusters, tpGemmSplitKernelFn(), &cfg) == cudaSuccess) tp->splitClusters[size] = clusters;
+      else (void)cudaGetLastError();
+    }
     INFO(SUB_INIT, "tensor-parallel GEMM: %d SMs, %d resident CTA pairs", tp->smCount, tp->pairClusters);
   }
   const int n = comm->nRanks;

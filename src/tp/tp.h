@@ -20,6 +20,7 @@ struct TpGemmArgs {
   int M, N, K;
   int mode;
   int rank, nRanks;
+  int splitK;                     // split kernel: CTAs of a cluster that share the K blocks of a tile
   int gemmCtas;                   // GATHER: CTAs [0, gemmCtas) compute, the rest gather
   SyncArgs sync;
   // block-scaled fp8 (e4m3) operands: A scaled per row and 128 columns, W per 128 x 128 block
@@ -27,6 +28,8 @@ struct TpGemmArgs {
   const float* scaleW;            // [K/128][N/128]
   size_t scaleOffset;             // GATHER, fp8: byte offset of the scales inside every rank's activation window
 };
+
+constexpr int kTpMaxSplit = 8;     // largest cluster of the split kernel
 
 #if defined(__CUDACC__)
 constexpr int kTpBM = 128, kTpBN = 256;
@@ -78,6 +81,9 @@ __device__ __forceinline__ TileCoord tileOf(const TpGemmArgs& a, int t, int bm =
 
 const void* tpGemmKernelFn();
 const void* tpGemmPairKernelFn();      // CTA-pair variant (cluster of two, 256 x 256 tiles): same arguments, W map with 128-row boxes
+const void* tpGemmSplitKernelFn();     // plain C = A * W^T, one 128 x 256 tile per cluster of splitK CTAs
+size_t tpGemmSplitSmemBytes();
+int tpGemmSplitThreads();
 const void* tpGemmFp8KernelFn();
 const void* tpQuantRowsKernelFn();     // (const bf16* x, uint8_t* q, float* scales, int rows, int K): 1 x 128 blocks, scales [K/128][rows]
 const void* tpQuantBlocksKernelFn();   // same arguments: 128 x 128 blocks, scales [K/128][rows/128]
