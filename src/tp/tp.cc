@@ -196,7 +196,11 @@ ncclResult_t ncclTpQuantizeFp8(ncclTp_t tp, const void* x, void* q, float* scale
   if (blockRows == 128 && rows % 128) return ncclInvalidArgument;
   if (((uintptr_t)x & 7) || ((uintptr_t)q & 3)) return ncclInvalidArgument;
   void* args[5] = {(void*)&x, &q, &scales, &rows, &K};
-  if (blockRows == 1) {
+  int gx = 0, gy = 0;
+  tpQuantRowsWideGrid(rows, K, &gx, &gy);
+  if (blockRows == 1 && !(((uintptr_t)x | (uintptr_t)q) & 15) && gy <= 65535) {
+    CUDACHECK(cudaLaunchKernel(tpQuantRowsWideKernelFn(), dim3(gx, gy), dim3(256), args, 0, stream));
+  } else if (blockRows == 1) {
     size_t warps = (size_t)rows * (K / 128);
     int ctas = (int)std::min<size_t>((warps + 7) / 8, (size_t)tp->smCount * 16);
     CUDACHECK(cudaLaunchKernel(tpQuantRowsKernelFn(), dim3(std::max(ctas, 1)), dim3(256), args, 0, stream));

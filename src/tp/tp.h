@@ -85,6 +85,8 @@ const void* tpGemmSplitKernelFn();     // plain C = A * W^T, one 128 x 256 tile 
 size_t tpGemmSplitSmemBytes();
 int tpGemmSplitThreads();
 const void* tpGemmFp8KernelFn();
+const void* tpQuantRowsWideKernelFn(); // as the next one, for 16-byte aligned x and q, on the grid below
+void tpQuantRowsWideGrid(int rows, int K, int* x, int* y);
 const void* tpQuantRowsKernelFn();     // (const bf16* x, uint8_t* q, float* scales, int rows, int K): 1 x 128 blocks, scales [K/128][rows]
 const void* tpQuantBlocksKernelFn();   // same arguments: 128 x 128 blocks, scales [K/128][rows/128]
 size_t tpGemmFp8SmemBytes();

@@ -1,0 +1,76 @@
+"""Block-scaled fp8 GEMM at the edges of its tiles: pairs of CTAs whose last row tile is half empty, one row block, fewer and
+more K blocks than the scale look-ahead, more tiles than CTAs, with both kernel forms, against a 64-bit product."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(128, 256, 128), (256, 256, 128), (384, 512, 256), (640, 256, 640), (1920, 1024, 384), (4224, 2304, 1152)]
+
+
+def _run():
+    sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    from nccl_b200 import Communicator, get_unique_id
+    from nccl_b200.ops.tp import TensorParallel
+    torch.cuda.set_device(0)
+    comm = Communicator(1, 0, get_unique_id())
+    tp = TensorParallel(comm, 4096, 4096)
+    for M, N, K in SHAPES:
+        g = torch.Generator(device="cuda").manual_seed(M + N + K)
+        xq, xs = tp.quantize_fp8((torch.randn(M, K, device="cuda", generator=g) * torch.rand(M, 1, device="cuda", generator=g) * 4).bfloat16())
+        wq, ws = tp.quantize_fp8((torch.randn(N, K, device="cuda", generator=g) * 0.05).bfloat16(), 128)
+        xd = (xq.double().view(M, -1, 128) * xs.t().double().unsqueeze(-1)).view(M, K)
+        wd = (wq.double().view(N // 128, 128, -1, 128) * ws.t().double()[:, None, :, None]).view(N, K)
+        ref = xd @ wd.t()
+        out = torch.full((M + 1, N), 9.0, dtype=torch.bfloat16, device="cuda")
+        for _ in range(2):
+            tp.gemm_fp8(xq, xs, wq, ws, out=out[:M])
+            torch.cuda.synchronize()
+            # bf16 rounds to 2^-9 of the value; the sums are fp32 over K terms of at most the row's and column's size
+            bound = 2 ** -8 * ref.abs() + 2 ** -20 * (xd.abs() @ wd.abs().t())
+            assert ((out[:M].double() - ref).abs() <= bound).all(), (M, N, K)
+            assert (out[M] == 9).all()
+    assert comm.async_error() == 0
+    tp.destroy()
+    comm.destroy()
+    print("tiles ok")
+
+
+@pytest.mark.parametrize("pair", ["1", "0"])
+def test_fp8_tiles(pair):
+    if not torch.cuda.is_available() or torch.cuda.get_device_capability()[0] < 10:
+        pytest.skip("needs sm_100")
+    r = subprocess.run([sys.executable, os.path.abspath(__file__)], env=dict(os.environ, NCCL_B200_TP_PAIR=pair), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "tiles ok" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("rows,K", [(1, 128), (3, 2048), (4, 2176), (5, 896), (129, 4224)])
+@pytest.mark.parametrize("off", [0, 4])   # 4 elements: too little alignment for the wide loads
+def test_quantise_rows(rows, K, off):
+    if not torch.cuda.is_available() or torch.cuda.get_device_capability()[0] < 10:
+        pytest.skip("needs sm_100")
+    from nccl_b200 import Communicator, get_unique_id
+    from nccl_b200.ops.tp import TensorParallel
+    comm = Communicator(1, 0, get_unique_id())
+    tp = TensorParallel(comm, 256, 256)
+    x = torch.empty(rows * K + off, dtype=torch.bfloat16, device="cuda")[off:].view(rows, K)
+    x.copy_(torch.randn(rows, K, device="cuda") * torch.rand(rows, 1, device="cuda"))
+    x[0, :128] = 0
+    q = torch.full((rows + 1, K), 1.0, device="cuda").to(torch.float8_e4m3fn)
+    q, s = tp.quantize_fp8(x, q=q)
+    amax = x.float().view(rows, -1, 128).abs().amax(-1).clamp_min(1e-10)
+    scale = (amax.double() / 448).float()
+    want = (x.float().view(rows, -1, 128) * (1 / scale.double()).float().unsqueeze(-1)).view(rows, K).to(torch.float8_e4m3fn)
+    assert torch.equal(s.t(), scale)
+    assert torch.equal(q[:rows].view(torch.uint8), want.view(torch.uint8)) and (q[rows].float() == 1).all()
+    tp.destroy()
+    comm.destroy()
+
+
+if __name__ == "__main__":
+    _run()
