@@ -6,6 +6,7 @@ return immediately (stream-ordered).
 """
 import contextlib
 import ctypes
+import functools
 
 import numpy as np
 
@@ -28,6 +29,7 @@ def _torch():
     return torch
 
 
+@functools.lru_cache(maxsize=None)
 def _torch_types():
     torch = _torch()
     m = {torch.int8: INT8, torch.uint8: UINT8, torch.int32: INT32, torch.int64: INT64, torch.float16: FP16,
@@ -42,23 +44,32 @@ def describe(buf):
     """(pointer, element count, ncclDataType_t, is_cuda) of a tensor / array; None -> null pointer."""
     if buf is None:
         return 0, 0, None, False
-    if isinstance(buf, np.ndarray):
-        if not buf.flags["C_CONTIGUOUS"]:
-            raise ValueError("numpy buffers must be C-contiguous")
-        return buf.ctypes.data, buf.size, _NP_TYPES[buf.dtype], False
     if hasattr(buf, "data_ptr"):
         if not buf.is_contiguous():
             raise ValueError("tensors must be contiguous")
         return buf.data_ptr(), buf.numel(), _torch_types()[buf.dtype], buf.is_cuda
+    if isinstance(buf, np.ndarray):
+        if not buf.flags["C_CONTIGUOUS"]:
+            raise ValueError("numpy buffers must be C-contiguous")
+        return buf.ctypes.data, buf.size, _NP_TYPES[buf.dtype], False
     raise TypeError("unsupported buffer type %r" % type(buf))
 
 
 def _stream_of(buf, stream):
     if stream is not None:
         return stream if isinstance(stream, int) else stream.cuda_stream
-    if buf is not None and hasattr(buf, "is_cuda") and buf.is_cuda:
-        return _torch().cuda.current_stream(buf.device).cuda_stream
+    if buf is not None and getattr(buf, "is_cuda", False):
+        return current_stream(buf.device.index)
     return 0
+
+
+def current_stream(device=None):
+    """Handle of torch's current stream on a device (default: the current one)."""
+    torch = _torch()
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)   # without a Stream object around it
+    if raw is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return raw(torch.cuda.current_device() if device is None else device)
 
 
 def get_unique_id(lib=None):

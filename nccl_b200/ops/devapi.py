@@ -11,7 +11,7 @@ examples/06_device_api, contrib/nccl_ubx fused all-reduce + RMSNorm.
 import ctypes
 
 from .. import _lib
-from ..core import mem_alloc, mem_free
+from ..core import current_stream, mem_alloc, mem_free
 from ..utils.perf import tensor_at
 
 
@@ -84,12 +84,12 @@ class DeviceComm:
         self.dc = _DevComm()
         _lib.check(L.ncclDevCommCreate(comm.handle, ctypes.byref(req), ctypes.byref(self.dc)), "ncclDevCommCreate", L)
         self.barriers = barriers
-        self._wins = []      # (start, end, window pointer, raw allocation)
+        self._wins = []      # (start, end, window handle, raw allocation, typed window pointer)
 
     def destroy(self):
         if self.dc is not None:
             _torch().cuda.synchronize()
-            for _, _, win, ptr in self._wins:
+            for _, _, win, ptr, _ in self._wins:
                 self.comm.deregister_window(win)
                 mem_free(ptr, self.lib)
             self._wins = []
@@ -104,18 +104,18 @@ class DeviceComm:
         ptr = mem_alloc(nbytes, self.lib)
         raw = tensor_at(ptr, nbytes)
         win = self.comm.register_window(raw)
-        self._wins.append((ptr, ptr + nbytes, win, ptr))
+        self._wins.append((ptr, ptr + nbytes, win, ptr, ctypes.cast(win, ctypes.POINTER(_Window))))
         return raw[:numel * es].view(dtype)
 
     def _locate(self, t):
         a = t.data_ptr()
-        for lo, hi, win, _ in self._wins:
+        for lo, hi, _, _, win in self._wins:
             if lo <= a and a + t.numel() * t.element_size() <= hi:
-                return ctypes.cast(win, ctypes.POINTER(_Window)), a - lo
+                return win, a - lo
         raise ValueError("tensor does not live in a symmetric buffer of this device communicator")
 
     def _stream(self, stream):
-        return (stream or _torch().cuda.current_stream()).cuda_stream
+        return stream.cuda_stream if stream else current_stream()
 
     def all_reduce(self, send, recv, multimem=False, ctas=32, stream=None):
         torch = _torch()

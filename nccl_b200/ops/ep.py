@@ -15,7 +15,7 @@ applies its local experts and the weights and gives one pre-reduced row per rece
 import ctypes
 
 from .. import _lib
-from ..core import BF16, FP32, FP8_E4M3, INT32, INT64
+from ..core import INT64, current_stream
 
 EP_MAGIC = 0xC00FFFEE
 TENSOR_MAGIC = 0xCAFECAFE
@@ -102,6 +102,9 @@ class ExpertParallel:
         L.ncclEpDispatch.argtypes = [vp, ctypes.POINTER(DispIn), ctypes.POINTER(DispOut), ctypes.POINTER(LayoutInfo), ctypes.POINTER(DispCfg), vp]
         L.ncclEpCombine.argtypes = [vp, ctypes.POINTER(CombIO), ctypes.POINTER(CombIO), ctypes.POINTER(CombCfg), vp]
         L.ncclEpComplete.argtypes = [vp, vp, vp]
+        dims = [ctypes.c_int, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_size_t]
+        L.b200EpDispatch.argtypes = [vp] + ([vp] + dims) * 4 + [vp] * 5 + [ctypes.c_int, vp]
+        L.b200EpCombine.argtypes = [vp] + ([vp] + dims) * 2 + [ctypes.c_int, vp]
         L.ncclEpMaskQuery.argtypes = [vp, ctypes.POINTER(ctypes.c_int), vp]
         L.ncclEpMaskUpdate.argtypes = [vp, ctypes.POINTER(ctypes.c_int), vp]
         L.ncclEpMaskClean.argtypes = [vp, vp]
@@ -118,6 +121,7 @@ class ExpertParallel:
         self.group = g
         self.handle = None
         self._keep = None
+        self.recv_total = None
 
     def destroy(self):
         if self.handle:
@@ -128,7 +132,7 @@ class ExpertParallel:
             self.group = None
 
     def _stream(self):
-        return self.torch.cuda.current_stream().cuda_stream
+        return current_stream()
 
     def complete(self):
         """Runs the receiving half of the last ``send_only`` dispatch / combine."""
@@ -147,17 +151,22 @@ class ExpertParallel:
     def clear_mask(self):
         _lib.check(self.lib.ncclEpMaskClean(self.group, self._stream()), "ncclEpMaskClean", self.lib)
 
+    @staticmethod
+    def _dims(t):
+        """Dimensions and their sizes as the flat entry points take them."""
+        d = t.shape
+        return (3, d[0], d[1], d[2]) if len(d) == 3 else (2, d[0], d[1], 0) if len(d) == 2 else (len(d), 0, 0, 0)
+
     def dispatch(self, x, topk_idx, topk_weights, fp8=True, toks=None, scales=None, counts=None, send_only=False):
         """``send_only``: only queue the sends; ``complete()`` then waits for the peers' tokens and packs them
         (work queued in between overlaps the transfer)."""
         torch, L = self.torch, self.lib
-        idx_t = _tensor(topk_idx, INT64)
+        stream = self._stream()
         if self.handle is None:
+            idx_t = _tensor(topk_idx, INT64)
             h = ctypes.c_void_p()
-            _lib.check(L.ncclEpCreateHandle(ctypes.byref(h), self.group, self.layout_code, ctypes.byref(idx_t), None, None, self._stream()), "ncclEpCreateHandle", L)
+            _lib.check(L.ncclEpCreateHandle(ctypes.byref(h), self.group, self.layout_code, ctypes.byref(idx_t), None, None, stream), "ncclEpCreateHandle", L)
             self.handle = h
-        else:
-            _lib.check(L.ncclEpUpdateHandle(self.handle, ctypes.byref(idx_t), None, self._stream()), "ncclEpUpdateHandle", L)
         lead = {"expert_major": (self.El, self.cap), "rank_major": (self.n, self.max_tokens), "flat": (self.cap,)}[self.layout]
         if toks is None:
             toks = torch.empty(*lead, self.H, dtype=torch.uint8 if fp8 else torch.bfloat16, device=x.device)
@@ -165,42 +174,24 @@ class ExpertParallel:
             scales = torch.empty(*lead, self.H // 128, dtype=torch.float32, device=x.device)
         if counts is None:
             counts = torch.zeros(self.El, dtype=torch.int32, device=x.device)
-        xin, win = _tensor(x, BF16), _tensor(topk_weights, FP32)
-        tout, cnt_t = _tensor(toks, FP8_E4M3 if fp8 else BF16), _tensor(counts, INT32)
-        sout = _tensor(scales, FP32) if fp8 else None
-        din = _hdr(DispIn())
-        din.tokens, din.topk_weights = ctypes.pointer(xin), ctypes.pointer(win)
-        dout = _hdr(DispOut())
-        dout.tokens = ctypes.pointer(tout)
-        if fp8:
-            dout.scales = ctypes.pointer(sout)
-        li = _hdr(LayoutInfo())
-        li.expert_counters = ctypes.pointer(cnt_t)
-        extra = None
+        recv = (None, None, None)
         if self.layout != "expert_major":
             K = topk_idx.shape[1]
             self.recv_topk_idx = torch.empty(*lead, K, dtype=torch.int64, device=x.device)
             self.recv_topk_weights = torch.empty(*lead, K, dtype=torch.float32, device=x.device)
-            self.recv_total = torch.zeros(1, dtype=torch.int32, device=x.device)
-            extra = (_tensor(self.recv_topk_idx, INT64), _tensor(self.recv_topk_weights, FP32), _tensor(self.recv_total, INT32))
-            dout.topk_idx, dout.topk_weights = ctypes.pointer(extra[0]), ctypes.pointer(extra[1])
-            if self.layout == "flat":
-                li.recv_total_counter = ctypes.pointer(extra[2])
-        dcfg = _hdr(DispCfg())
-        dcfg.send_only = 1 if send_only else 0
-        _lib.check(L.ncclEpDispatch(self.handle, ctypes.byref(din), ctypes.byref(dout), ctypes.byref(li), ctypes.byref(dcfg), self._stream()), "ncclEpDispatch", L)
-        self._keep = (topk_idx, topk_weights, idx_t, xin, win, tout, cnt_t, sout, extra)
+            if self.layout == "flat" or self.recv_total is None:   # nothing writes the rank-major one: it stays zero
+                self.recv_total = torch.zeros(1, dtype=torch.int32, device=x.device)
+            recv = (self.recv_topk_idx.data_ptr(), self.recv_topk_weights.data_ptr(), self.recv_total.data_ptr() if self.layout == "flat" else None)
+        _lib.check(L.b200EpDispatch(self.handle, x.data_ptr(), *self._dims(x), topk_idx.data_ptr(), *self._dims(topk_idx), topk_weights.data_ptr(),
+                                    *self._dims(topk_weights), toks.data_ptr(), *self._dims(toks), scales.data_ptr() if fp8 else None, counts.data_ptr(),
+                                    *recv, int(send_only), stream), "ncclEpDispatch", L)
+        self._keep = (x, topk_idx, topk_weights, toks, scales, counts)
         self.T = x.shape[0]
         return toks, scales, counts
 
     def combine(self, y, out=None, send_only=False):
         torch, L = self.torch, self.lib
         out = out if out is not None else torch.empty(self.T, self.H, dtype=torch.bfloat16, device=y.device)
-        yin, oout = _tensor(y, BF16), _tensor(out, BF16)
-        cin, cout = _hdr(CombIO()), _hdr(CombIO())
-        cin.tokens, cout.tokens = ctypes.pointer(yin), ctypes.pointer(oout)
-        ccfg = _hdr(CombCfg())
-        ccfg.send_only = 1 if send_only else 0
-        _lib.check(L.ncclEpCombine(self.handle, ctypes.byref(cin), ctypes.byref(cout), ctypes.byref(ccfg), self._stream()), "ncclEpCombine", L)
-        self._keep_c = (yin, oout, y, out)
+        _lib.check(L.b200EpCombine(self.handle, y.data_ptr(), *self._dims(y), out.data_ptr(), *self._dims(out), int(send_only), self._stream()), "ncclEpCombine", L)
+        self._keep_c = (y, out)
         return out

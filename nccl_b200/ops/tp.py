@@ -9,6 +9,7 @@
 import ctypes
 
 from .. import _lib
+from ..core import current_stream
 
 
 def _torch():
@@ -40,8 +41,7 @@ class TensorParallel:
             self.handle = None
 
     def _stream(self, stream):
-        torch = _torch()
-        return (stream or torch.cuda.current_stream()).cuda_stream
+        return stream.cuda_stream if stream else current_stream()
 
     @staticmethod
     def _check(x, w):

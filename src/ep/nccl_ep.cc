@@ -490,6 +490,56 @@ ncclResult_t ncclEpComplete(ncclEpHandle_t h, const ncclEpCompleteConfig_t* conf
   return ncclSuccess;
 }
 
+// The calls above with every tensor given as pointer, number of dimensions and sizes, for callers to whom building the
+// structures costs more than the call (the Python wrapper). x: bf16; topkIdx: int64; topkW: fp32; toks: e4m3 when scales
+// are given, else bf16; recvIdx / recvW: rows of toks x top-k (per-rank layouts, else null).
+#define B200_EP_DIMS(t) int t##Nd, size_t t##0, size_t t##1, size_t t##2
+ncclResult_t b200EpDispatch(ncclEpHandle_t h, void* x, B200_EP_DIMS(xd), void* topkIdx, B200_EP_DIMS(id), void* topkW, B200_EP_DIMS(wd), void* toks,
+                            B200_EP_DIMS(td), void* scales, void* counts, void* recvIdx, void* recvW, void* recvTotal, int sendOnly, cudaStream_t stream) {
+  if (!h) return ncclInvalidArgument;
+  size_t xs[3] = {xd0, xd1, xd2}, is[3] = {id0, id1, id2}, ws[3] = {wd0, wd1, wd2}, ts[3] = {td0, td1, td2}, one = 1;
+  size_t rs[3] = {td0, tdNd == 3 ? td1 : (size_t)h->K, (size_t)h->K};   // the rows of toks, one routing row each
+  auto tensor = [](void* data, int nd, ncclDataType_t type, size_t* sizes) {
+    return ncclEpTensor_t{sizeof(ncclEpTensor_t), NCCL_EP_TENSOR_MAGIC, (unsigned)nd, type, data, nullptr, 0, sizes};
+  };
+  ncclEpTensor_t xT = tensor(x, xdNd, ncclBfloat16, xs), iT = tensor(topkIdx, idNd, ncclInt64, is), wT = tensor(topkW, wdNd, ncclFloat32, ws);
+  ncclEpTensor_t tT = tensor(toks, tdNd, scales ? ncclFloat8e4m3 : ncclBfloat16, ts), sT = tensor(scales, 1, ncclFloat32, &one), cT = tensor(counts, 1, ncclInt32, &one);
+  ncclEpTensor_t riT = tensor(recvIdx, tdNd, ncclInt64, rs), rwT = tensor(recvW, tdNd, ncclFloat32, rs), rtT = tensor(recvTotal, 1, ncclInt32, &one);
+  NCCLCHECK(ncclEpUpdateHandle(h, &iT, nullptr, stream));
+  ncclEpDispatchInputs_t in = {};
+  ncclEpDispatchOutputs_t out = {};
+  ncclEpLayoutInfo_t li = {};
+  ncclEpDispatchConfig_t cfg = {};
+  in.size = sizeof(in); out.size = sizeof(out); li.size = sizeof(li); cfg.size = sizeof(cfg);
+  in.magic = out.magic = li.magic = cfg.magic = NCCL_EP_MAGIC;
+  in.tokens = &xT;
+  in.topk_weights = &wT;
+  out.tokens = &tT;
+  out.scales = scales ? &sT : nullptr;
+  out.topk_idx = recvIdx ? &riT : nullptr;
+  out.topk_weights = recvW ? &rwT : nullptr;
+  li.expert_counters = counts ? &cT : nullptr;
+  li.recv_total_counter = recvTotal ? &rtT : nullptr;
+  cfg.send_only = sendOnly ? 1 : 0;
+  return ncclEpDispatch(h, &in, &out, &li, &cfg, stream);
+}
+
+ncclResult_t b200EpCombine(ncclEpHandle_t h, void* y, B200_EP_DIMS(yd), void* out, B200_EP_DIMS(od), int sendOnly, cudaStream_t stream) {
+  size_t ys[3] = {yd0, yd1, yd2}, os[3] = {od0, od1, od2};
+  ncclEpTensor_t yT = {sizeof(ncclEpTensor_t), NCCL_EP_TENSOR_MAGIC, (unsigned)ydNd, ncclBfloat16, y, nullptr, 0, ys};
+  ncclEpTensor_t oT = {sizeof(ncclEpTensor_t), NCCL_EP_TENSOR_MAGIC, (unsigned)odNd, ncclBfloat16, out, nullptr, 0, os};
+  ncclEpCombineInputs_t ci = {};
+  ncclEpCombineOutputs_t co = {};
+  ncclEpCombineConfig_t cfg = {};
+  ci.size = sizeof(ci); co.size = sizeof(co); cfg.size = sizeof(cfg);
+  ci.magic = co.magic = cfg.magic = NCCL_EP_MAGIC;
+  ci.tokens = &yT;
+  co.tokens = &oT;
+  cfg.send_only = sendOnly ? 1 : 0;
+  return ncclEpCombine(h, &ci, &co, &cfg, stream);
+}
+#undef B200_EP_DIMS
+
 // Rank masks: a masked rank receives nothing and nobody waits for it. With enable_mask in the group
 // configuration a wait on a rank that runs out (timeout_ns) sets that rank's mask word on the waiting rank
 // instead of failing the call; ncclEpMaskQuery shows the words, ncclEpMaskUpdate sets them (for example after a
