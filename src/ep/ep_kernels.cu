@@ -673,7 +673,7 @@ constexpr int kLocMaxK = 16;
 // round is stored. `claim` fills sRow between the first loads and the first stores.
 template <bool FP8, typename Claim>
 __device__ __forceinline__ void localPayload(const EpArgs& a, const __nv_bfloat16* x, int t0, int tStep, int batch, int R, const int* sRow, Claim claim) {
-  constexpr int U = FP8 ? 1 : 2;            // items of a thread per round
+  constexpr int U = 2;                      // items of a thread per round
   constexpr int kIn = FP8 ? 2 : 1;          // 16-byte loads of an item
   const int H = a.hidden, C = H / (8 * kIn);
   const int total = batch * C;              // a multiple of 8: the lanes of a group are in or out together
@@ -758,45 +758,45 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epDispatchLocalKernel(cons
   const int R = rankMajor ? 1 : K;
   if (rankMajor) {
     for (int e = threadIdx.x; e < E; e += kEpLocalThreads) sHist[e] = 0;
-    __syncthreads();
-    // routing rows of all slots, used or not, and the count of every expert
-    for (int t = b * kEpLocalThreads + threadIdx.x; t < cap; t += grid * kEpLocalThreads) {
-      bool any = false;
-      for (int k = 0; t < T && k < K; ++k) {
-        const int64_t e = idx[(size_t)t * K + k];
-        if (e >= 0 && e < E) {
-          any = true;
-          atomicAdd(&sHist[e], 1);
-        }
-      }
-      a.srcInfo[me][t] = any ? make_int2(me, t) : make_int2(-1, 0);
-      for (int k = 0; k < K; ++k) {
-        const size_t o = (size_t)t * K + k;
-        const int64_t e = any ? idx[o] : -1;
-        if (a.outTopkIdx[me]) a.outTopkIdx[me][o] = e >= 0 && e < E ? e : -1;
-        if (a.outTopkW[me]) a.outTopkW[me][o] = any && a.topkW[me] ? a.topkW[me][o] : 0.0f;
-      }
+    // slots behind the last token
+    for (int i = T * K + b * kEpLocalThreads + (int)threadIdx.x; i < cap * K; i += grid * kEpLocalThreads) {
+      if (i % K == 0) a.srcInfo[me][i / K] = make_int2(-1, 0);
+      if (a.outTopkIdx[me]) a.outTopkIdx[me][i] = -1;
+      if (a.outTopkW[me]) a.outTopkW[me][i] = 0.0f;
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < E; e += kEpLocalThreads)
-      if (sHist[e]) atomicAdd(&st[kStCounters + e], (uint32_t)sHist[e]);
   }
   for (int base = 0; base < mine; base += kLocTokens) {
     const int batch = mine - base < kLocTokens ? mine - base : kLocTokens;
     const int t0 = b + base * grid;
     localPayload<FP8>(a, a.x[me], t0, grid, batch, R, sRow, [&] {
       __syncthreads();   // the previous batch is stored
-      for (int i = threadIdx.x; i < batch * R; i += kEpLocalThreads) {
-        const int t = t0 + i / R * grid;
-        int row = -1;
-        if (rankMajor) {
-          for (int k = 0; k < K && row < 0; ++k) {
-            const int64_t e = idx[(size_t)t * K + k];
-            if (e >= 0 && e < E) row = t;
+      if (rankMajor) {
+        for (int j = threadIdx.x; j < batch; j += kEpLocalThreads) sRow[j] = -1;
+        __syncthreads();
+        for (int i = threadIdx.x; i < batch * K; i += kEpLocalThreads) {
+          const int t = t0 + i / K * grid;
+          const int64_t e = idx[(size_t)t * K + i % K];
+          if (e >= 0 && e < E) {
+            sRow[i / K] = t;   // any of the token's entries: the same value
+            atomicAdd(&sHist[e], 1);
           }
-        } else {
-          const size_t o = (size_t)t * K + i % R;
+        }
+        __syncthreads();
+        // the routing row goes with the token; a token without experts leaves its slot unused
+        for (int i = threadIdx.x; i < batch * K; i += kEpLocalThreads) {
+          const int t = t0 + i / K * grid;
+          const size_t o = (size_t)t * K + i % K;
+          const bool any = sRow[i / K] >= 0;
           const int64_t e = idx[o];
+          if (i % K == 0) a.srcInfo[me][t] = any ? make_int2(me, t) : make_int2(-1, 0);
+          if (a.outTopkIdx[me]) a.outTopkIdx[me][o] = e >= 0 && e < E ? e : -1;
+          if (a.outTopkW[me]) a.outTopkW[me][o] = any && a.topkW[me] ? a.topkW[me][o] : 0.0f;
+        }
+      } else {
+        for (int i = threadIdx.x; i < batch * K; i += kEpLocalThreads) {
+          const size_t o = (size_t)(t0 + i / K * grid) * K + i % K;
+          const int64_t e = idx[o];
+          int row = -1;
           if (e >= 0 && e < E) {
             const int s = (int)atomicAdd(&st[kStCounters + e], 1u);
             if (s < cap) {   // always, unless a token names an expert twice
@@ -805,11 +805,16 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epDispatchLocalKernel(cons
               a.rowOf[o] = row;
             }
           }
+          sRow[i] = row;
         }
-        sRow[i] = row;
+        __syncthreads();
       }
-      __syncthreads();
     });
+  }
+  if (rankMajor) {
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += kEpLocalThreads)
+      if (sHist[e]) atomicAdd(&st[kStCounters + e], (uint32_t)sHist[e]);
   }
   // the last CTA publishes the counts and leaves the counters at zero
   __syncthreads();
@@ -828,6 +833,56 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epDispatchLocalKernel(cons
     st[kStCounters + e] = 0;
   }
   if (threadIdx.x == 0) st[2] = 0;
+}
+
+// Items first, first + kEpLocalThreads, ... of a batch of tokens: KR rows of U items are fetched together, so that several loads
+// are in flight whatever the number of experts (one row per item ran at 1.8 TB/s). `store` takes token, channels and sums.
+template <int KR, typename Store>
+__device__ __forceinline__ void localSums(const __nv_bfloat16* y, int H, int C, int nItems, int shift, int R, const int* sRow, const float* sW, Store store) {
+  constexpr int U = KR == 1 ? 4 : 8 / KR;
+  for (int first = threadIdx.x; first < nItems; first += U * kEpLocalThreads) {
+    float acc[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[u][q] = 0.0f;
+    for (int r0 = 0; r0 < R; r0 += KR) {
+      uint4 v[U][KR];
+      float wk[U][KR];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = first + u * kEpLocalThreads + shift;
+        const int j = i / C, c = i - j * C;
+#pragma unroll
+        for (int r = 0; r < KR; ++r) {
+          const int row = i - shift < nItems && r0 + r < R ? sRow[j * R + r0 + r] : -1;
+          v[u][r] = make_uint4(0, 0, 0, 0);
+          wk[u][r] = 0.0f;
+          if (row >= 0) {
+            wk[u][r] = sW[j * R + r0 + r];
+            v[u][r] = ldStream16(y + (size_t)row * H + (size_t)c * 8);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int r = 0; r < KR; ++r) {
+          const __nv_bfloat162* p = (const __nv_bfloat162*)&v[u][r];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            acc[u][2 * q] += wk[u][r] * __bfloat162float(p[q].x);
+            acc[u][2 * q + 1] += wk[u][r] * __bfloat162float(p[q].y);
+          }
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = first + u * kEpLocalThreads + shift;
+      if (i - shift >= nItems) continue;
+      store(i / C, i % C, acc[u]);
+    }
+  }
 }
 
 // out[t] = sum over the token's selected experts of w * row, in fp32, in slot order. The (token, 8 channels) items are dealt to
@@ -874,38 +929,17 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epCombineLocalKernel(const
     const size_t first = (size_t)tb * C > lo ? (size_t)tb * C : lo;
     const size_t end = (size_t)(tb + batch) * C < hi ? (size_t)(tb + batch) * C : hi;
     const int nItems = (int)(end - first), shift = (int)(first - (size_t)tb * C);
-    for (int i = threadIdx.x; i < nItems; i += kEpLocalThreads) {
-      const int j = (i + shift) / C, c = i + shift - j * C;
-      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      for (int r0 = 0; r0 < R; r0 += 8) {
-        uint4 v[8];
-        float wk[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int row = r0 + u < R ? sRow[j * R + r0 + u] : -1;
-          v[u] = make_uint4(0, 0, 0, 0);
-          wk[u] = 0.0f;
-          if (row >= 0) {
-            wk[u] = sW[j * R + r0 + u];
-            v[u] = ldStream16(y + (size_t)row * H + (size_t)c * 8);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const __nv_bfloat162* p = (const __nv_bfloat162*)&v[u];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            acc[2 * q] += wk[u] * __bfloat162float(p[q].x);
-            acc[2 * q + 1] += wk[u] * __bfloat162float(p[q].y);
-          }
-        }
-      }
+    auto store = [&](int j, int c, const float (&acc)[8]) {
       uint4 o;
       __nv_bfloat162* q = (__nv_bfloat162*)&o;
 #pragma unroll
       for (int k = 0; k < 4; ++k) q[k] = __floats2bfloat162_rn(acc[2 * k], acc[2 * k + 1]);
       st16(out + (size_t)(tb + j) * H + (size_t)c * 8, o);
-    }
+    };
+    if (R == 1) localSums<1>(y, H, C, nItems, shift, R, sRow, sW, store);
+    else if (R == 2) localSums<2>(y, H, C, nItems, shift, R, sRow, sW, store);
+    else if (R <= 4) localSums<4>(y, H, C, nItems, shift, R, sRow, sW, store);
+    else localSums<8>(y, H, C, nItems, shift, R, sRow, sW, store);
   }
 }
 
