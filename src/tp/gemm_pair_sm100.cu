@@ -98,7 +98,7 @@ tpGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (!ok && threadIdx.x == 0) stSharedCluster(mapaShared(smemAddr((const void*)abortFlag), cr ^ 1), 1u);
 
   const int tilesN = a.N / BN;
-  const int nTiles = (a.M / PM) * tilesN;
+  const int nTiles = (a.M + PM - 1) / PM * tilesN;   // plain GEMMs: the last row tile may be half empty (its loads are filled with zeros)
   const int kBlocks = a.K / BK;
   const int pairIdx = blockIdx.x >> 1;
   const int nPairs = (gather ? a.gemmCtas : (int)gridDim.x) >> 1;
@@ -176,7 +176,7 @@ tpGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       tcFenceAfter();
       const int row0 = tc.mBlk * PM + (int)cr * 128 + q * 32;
       const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * BN;
-      tpStoreAccum(a, tBase, row0, tc.nBlk, tc.owner, wbuf, lane);
+      if (row0 < a.M) tpStoreAccum(a, tBase, row0, tc.nBlk, tc.owner, wbuf, lane);
       tcFenceBefore();
       __syncwarp();
       if (lane == 0) mbarArriveCluster(mapaShared(smemAddr(&accEmpty[buf]), 0));

@@ -129,19 +129,26 @@ static ncclResult_t launchGemmSplit(ncclTpContext* tp, const void* A, const void
 }
 
 // Launches the bf16 GEMM kernel in the mode of `a`. Grid: one CTA per SM (fewer when there are fewer
-// tiles); in all-gather mode the last CTAs are the comm CTAs. The CTA-pair kernel runs when enabled,
-// when its clusters fit and when every rank's rows split into 256-row tiles.
+// tiles); in all-gather mode the last CTAs are the comm CTAs. The CTA-pair kernel runs when enabled, when its clusters
+// fit and, in the fused modes, when every rank's rows split into 256-row tiles.
 static ncclResult_t launchGemm(ncclTpContext* tp, const void* A, const void* W, TpGemmArgs* a, cudaStream_t stream) {
   const int n = a->nRanks;
   const bool fused = n > 1 && a->mode != TP_MODE_STORE;
   const bool gather = fused && a->mode == TP_MODE_GATHER;
   if (!fused && (a->splitK = splitOf(tp, a)) > 1) return launchGemmSplit(tp, A, W, a, stream);
-  const bool pair = paramTpPair() != 0 && tp->pairClusters > 0 && a->M % (256 * (fused ? n : 1)) == 0;
+  bool pair = paramTpPair() != 0 && tp->pairClusters > 0 && (!fused || a->M % (256 * n) == 0);
+  if (pair && a->M % 256) {
+    // Plain GEMMs: pairs leave half of the last row tile empty. A K step of a pair tile takes 2/3 of the time of one of a
+    // 128 x 256 tile (both are bound by the operand traffic from L2: 32 KiB against 48 KiB per SM).
+    const int tilesN = a->N / 256, one = a->M / 128 * tilesN, two = (a->M / 128 + 1) / 2 * tilesN;
+    const int wavesOne = (one + tp->smCount - 1) / tp->smCount, wavesTwo = (two + tp->pairClusters - 1) / tp->pairClusters;
+    pair = 2 * wavesTwo < 3 * wavesOne;
+  }
   int commCtas = gather ? tpCommCtas(tp, n) : 0;
   int grid;
   if (pair) {
     commCtas = (commCtas + 1) & ~1;   // both CTAs of a cluster have the same role
-    const int tiles = (a->M / 256) * (a->N / 256);
+    const int tiles = (a->M + 255) / 256 * (a->N / 256);
     const int pairs = std::max(1, std::min(tp->pairClusters - commCtas / 2, tiles));
     a->gemmCtas = 2 * pairs;
     grid = 2 * pairs + commCtas;

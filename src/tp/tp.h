@@ -56,7 +56,7 @@ __device__ __forceinline__ TileCoord tileOf(const TpGemmArgs& a, int t, int bm =
   const int tilesN = a.N / kTpBN;
   TileCoord c;
   if (a.mode == TP_MODE_STORE || a.nRanks == 1) {
-    panelOrder(t, a.M / bm, tilesN, &c.mBlk, &c.nBlk);
+    panelOrder(t, (a.M + bm - 1) / bm, tilesN, &c.mBlk, &c.nBlk);
     c.owner = a.rank;
     if (a.mode == TP_MODE_REDUCE) c.owner = 0;
     return c;
