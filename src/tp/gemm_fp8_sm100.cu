@@ -8,9 +8,14 @@
 //   level 2  the epilogue warps read each finished block from TMEM (tcgen05.ld), multiply by
 //            scaleA[row] * scaleW[block] and add into fp32 registers, while the tensor cores
 //            already work on the next K block in the other accumulator.
-// Persistent CTAs of 320 threads: warp 0 TMA producer (128x128-byte A tiles, 256x128-byte W tiles,
-// 128-byte swizzle, 4-stage ring), warp 1 MMA issuer, warps 2-9 epilogue (each warp owns 32 TMEM
-// lanes and one 128-column half of the tile: 128 fp32 accumulators per thread).
+// 1920 x 4096 x 7168: 107 -> 78 us, 4096 x 9472 x 4096: 262 -> 198 us (1.21 -> 1.61 PFLOP/s) against a level 2 that waited for each
+// 32 columns in turn. What bounds the kernel is the round trip of an accumulator (MMAs, level 2, release) and behind that the operand traffic
+// from L2 (48 KiB per K block and SM). So level 2 is a pipeline of its own: 32 columns are fetched while the 32 before them are
+// multiplied (packed fp32 pairs), across K blocks too, and an accumulator is given back as soon as it is read.
+// Persistent CTAs of three warpgroups: warp 0 TMA producer (128x128-byte A tiles, 256x128-byte W tiles,
+// 128-byte swizzle, 4-stage ring), warp 1 MMA issuer, warps 4-11 epilogue (each warp owns 32 TMEM
+// lanes and one 128-column half of the tile: 128 fp32 accumulators per thread, for which the first warpgroup hands over its
+// registers).
 // The fused modes work as in the bf16 kernel (gemm_sm100.cu): REDUCE stores the scaled tile as bf16
 // into this rank's slot of the owning rank's staging buffer over NVLink (summed afterwards);
 // GATHER has comm CTAs pull remote row blocks with bulk copies and their scales with plain peer
@@ -31,15 +36,20 @@ using namespace sm100;
 
 namespace {
 constexpr int BM = kTpBM, BN = kTpBN, BK = 128, STAGES = 4, UMMA_K = 32;
-constexpr int kThreads = 320, kEpiWarps = 8;
+constexpr int kThreads = 384, kEpiWarps = 8;
 constexpr uint32_t kStageABytes = BM * BK, kStageBBytes = BN * BK;
 constexpr uint32_t kStageBytes = kStageABytes + kStageBBytes;
 constexpr uint32_t kTmemCols = 512;
 constexpr size_t kEpiBufBytes = kEpiWarps * 4096;   // one 32 x 128-byte transpose buffer per epilogue warp
 constexpr size_t kSmemBytes = 1024 + (size_t)STAGES * kStageBytes + 256 + kEpiBufBytes;
-constexpr int kPrefetch = 4;   // K blocks of scale look-ahead
+constexpr int kPrefetch = 1;   // K blocks of scale look-ahead: with more the accumulators spill
+// registers per thread: 168 at launch; the producer warpgroup keeps 56, the two epilogue warpgroups take 224
+constexpr int kRegsLaunch = 168, kRegsProducer = 56, kRegsEpilogue = 224;
+static_assert(128 * kRegsProducer + 256 * kRegsEpilogue <= kThreads * kRegsLaunch, "register shares exceed the launch");
 }  // namespace
 
+// FUSED: the modes with a collective. The plain form is compiled without what they keep in registers across the tile loop.
+template <bool FUSED>
 __global__ void __launch_bounds__(kThreads, 1)
 tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ TpGemmArgs a) {
   extern __shared__ uint8_t smemRaw[];
@@ -55,13 +65,13 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = a.rank, n = a.nRanks;
-  const bool multi = n > 1 && a.mode != TP_MODE_STORE;
-  const bool commCta = a.mode == TP_MODE_GATHER && n > 1 && (int)blockIdx.x >= a.gemmCtas;
+  const bool gather = FUSED && a.mode == TP_MODE_GATHER;
+  const bool commCta = gather && (int)blockIdx.x >= a.gemmCtas;
   const int kBlocks = a.K / BK;
 
   CtaBarrier bar;
   bool ok = true;
-  if (multi) {
+  if (FUSED) {
     bar.init(a.sync, rank, n, blockIdx.x);
     ok = bar.sync(false, false);
   }
@@ -139,7 +149,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
   const int tilesN = a.N / BN;
   const int nTiles = (a.M / BM) * tilesN;
-  const int gemmCtas = (a.mode == TP_MODE_GATHER && n > 1) ? a.gemmCtas : gridDim.x;
+  const int gemmCtas = gather ? a.gemmCtas : gridDim.x;
   const uint32_t smemA0 = smemAddr(smem), smemB0 = smemA0 + STAGES * kStageABytes;
   auto fail = [&](uint32_t kind, uint32_t what) {
     *abortFlag = 1;
@@ -152,14 +162,14 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
   };
 
-  if (warp == 0) {
-    if (electOne()) {
+  if (warp < 4) {
+    regsGive<kRegsProducer>();
+    if (warp == 0 && electOne()) {
       uint32_t kc = 0;
-      int armedStage[STAGES];
-      for (int s = 0; s < STAGES; ++s) armedStage[s] = -1;
+      uint32_t armed = 0, armedPhase = 0;   // per stage: a copy was issued, and for which phase of its barrier
       for (int t = blockIdx.x; t < nTiles && !*abortFlag; t += gemmCtas) {
         const TileCoord tc = tileOf(a, t);
-        if (a.mode == TP_MODE_GATHER && n > 1 && tc.owner != rank) {
+        if (gather && tc.owner != rank) {
           const uint32_t* f = a.blockFlags + tc.mBlk;
           bool got = false;
           for (uint32_t spin = 0; spin < (1u << 26); ++spin) {
@@ -179,16 +189,16 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           mbarExpectTx(fb, kStageBytes);
           tmaLoad2d(smemA0 + s * kStageABytes, &tmA, kb * BK, tc.mBlk * BM, fb);
           tmaLoad2d(smemB0 + s * kStageBBytes, &tmB, kb * BK, tc.nBlk * BN, fb);
-          armedStage[s] = (int)ph;
+          armed |= 1u << s;
+          armedPhase = (armedPhase & ~(1u << s)) | (ph << s);
         }
       }
       if (*abortFlag) {
+        // copies already issued still write into shared memory: wait for them (bounded)
         for (int s = 0; s < STAGES; ++s)
-          if (armedStage[s] >= 0) mbarWait(smemAddr(&fullBar[s]), (uint32_t)armedStage[s], 1u << 20);
+          if ((armed >> s) & 1u) mbarWait(smemAddr(&fullBar[s]), (armedPhase >> s) & 1u, 1u << 20);
       }
-    }
-  } else if (warp == 1) {
-    if (electOne()) {
+    } else if (warp == 1 && electOne()) {
       const uint32_t idesc = umInstrE4m3(BM, BN);
       uint32_t kc = 0;
       for (int t = blockIdx.x; t < nTiles && !*abortFlag; t += gemmCtas) {
@@ -213,19 +223,21 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       }
     }
   } else {
+    regsTake<kRegsEpilogue>();
     // ---- epilogue warps: TMEM lanes [32q, 32q+32), columns [128h, 128h+128)
     const int q = warp & 3;
-    const int h = (warp - 2) >> 2;
-    const float* scaleA = a.mode == TP_MODE_GATHER && n > 1 ? (const float*)((const char*)a.peerA[rank] + a.scaleOffset) : a.scaleA;
+    const int h = (warp - 4) >> 2;
+    const float* scaleA = gather ? (const float*)((const char*)a.peerA[rank] + a.scaleOffset) : a.scaleA;
     const int wBlocksN = a.N / 128;
     uint32_t kc = 0;
     for (int t = blockIdx.x; t < nTiles && !*abortFlag; t += gemmCtas) {
       const TileCoord tc = tileOf(a, t);
-      const int row = tc.mBlk * BM + q * 32 + lane;
+      const int row0 = tc.mBlk * BM + q * 32;
+      const int row = row0 + lane;
       const int wCol = tc.nBlk * 2 + h;
-      float acc[128];
+      uint64_t acc[64];   // fp32 pairs
 #pragma unroll
-      for (int j = 0; j < 128; ++j) acc[j] = 0.0f;
+      for (int j = 0; j < 64; ++j) acc[j] = 0;
       // Scales of the next kPrefetch K blocks travel ahead of the accumulators that need them.
       // In GATHER mode the scales of remote rows land together with the rows: the flag the TMA
       // producer waited for covers them, and accFull orders this warp after the producer.
@@ -236,11 +248,10 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       // Rows gathered from a peer arrive during this kernel: their scales may be read only after
       // the tile's first accumulator is published (the producer saw the block's flag before it
       // issued the TMA loads that fed it), and never through the read-only cache path.
-      const bool gathered = a.mode == TP_MODE_GATHER && n > 1;
-      const bool remoteRows = gathered && tc.owner != rank;
+      const bool remoteRows = gather && tc.owner != rank;
       auto scaleOf = [&](int kb) -> float {
         const float* pa = scaleA + (size_t)kb * a.M + row;
-        const float sa = gathered ? *(const volatile float*)pa : __ldg(pa);
+        const float sa = gather ? *(const volatile float*)pa : __ldg(pa);
         return sa * __ldg(a.scaleW + (size_t)kb * wBlocksN + wCol);
       };
       bool primed = false;
@@ -250,6 +261,16 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           if (u < kBlocks) sc[u] = scaleOf(u);
         primed = true;
       }
+      // two sets of 32 columns: one is fetched while the other is multiplied, across K blocks too
+      uint32_t even[32], odd[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) odd[j] = 0;
+      float sPrev = 0.0f;
+      auto madd = [&](int first, const uint32_t (&r)[32], float s) {
+        const uint64_t s2 = packF32x2(__float_as_uint(s), __float_as_uint(s));
+#pragma unroll
+        for (int j = 0; j < 16; ++j) fmaF32x2(acc[first / 2 + j], packF32x2(r[2 * j], r[2 * j + 1]), s2);
+      };
       for (int kb0 = 0; kb0 < kBlocks && !bad; kb0 += kPrefetch) {
 #pragma unroll
         for (int u = 0; u < kPrefetch; ++u) {
@@ -265,31 +286,36 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
               if (v < kBlocks) sc[v] = scaleOf(v);
             primed = true;
           }
+          const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * BN + h * 128;
           const float s = sc[u];
           if (kb + kPrefetch < kBlocks) sc[u] = scaleOf(kb + kPrefetch);
-          const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * BN + h * 128;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            uint32_t r[32];
-            tmemLd32(tBase + c * 32, r);
-            tmemLdWait();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) acc[c * 32 + j] = fmaf(__uint_as_float(r[j]), s, acc[c * 32 + j]);
-          }
+          tmemLd32(tBase, even);
+          madd(96, odd, sPrev);   // the last columns of the block before this one
+          tmemLdWait32(even);
+          tmemLd32(tBase + 32, odd);
+          madd(0, even, s);
+          tmemLdWait32(odd);
+          tmemLd32(tBase + 64, even);
+          madd(32, odd, s);
+          tmemLdWait32(even);
+          tmemLd32(tBase + 96, odd);
+          madd(64, even, s);
+          tmemLdWait32(odd);
           tcFenceBefore();
           __syncwarp();
           if (lane == 0) mbarArrive(smemAddr(&accEmpty[buf]));
+          sPrev = s;
           ++kc;
         }
       }
       if (bad) break;
+      madd(96, odd, sPrev);
       // final tile: bf16, transposed through shared memory so that every store instruction writes
       // whole 128-byte row segments (see the bf16 kernel); REDUCE targets the owner's staging slot
       {
-        const int row0 = tc.mBlk * BM + q * 32;
         __nv_bfloat16* dstBase;
         size_t ld;
-        if (a.mode == TP_MODE_REDUCE && n > 1) {
+        if (FUSED && a.mode == TP_MODE_REDUCE) {
           const int rowsPerRank = a.M / n;
           dstBase = (__nv_bfloat16*)a.partial[tc.owner] + ((size_t)rank * rowsPerRank + (row0 - tc.owner * rowsPerRank)) * a.N + (size_t)tc.nBlk * BN + h * 128;
           ld = (size_t)a.N;
@@ -297,18 +323,17 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           dstBase = (__nv_bfloat16*)a.C + (size_t)row0 * a.ldc + (size_t)tc.nBlk * BN + h * 128;
           ld = (size_t)a.ldc;
         }
-        uint8_t* wbuf = epiBuf + (size_t)(warp - 2) * 4096;
+        uint8_t* wbuf = epiBuf + (size_t)(warp - 4) * 4096;
+        auto bf16Pair = [&](int i) -> uint32_t {
+          const __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float((uint32_t)acc[i]), __uint_as_float((uint32_t)(acc[i] >> 32)));
+          return *(const uint32_t*)&p;
+        };
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            uint4 o;
-            const int b0 = cc * 64 + j * 8;
-            __nv_bfloat162 p0 = __floats2bfloat162_rn(acc[b0], acc[b0 + 1]);
-            __nv_bfloat162 p1 = __floats2bfloat162_rn(acc[b0 + 2], acc[b0 + 3]);
-            __nv_bfloat162 p2 = __floats2bfloat162_rn(acc[b0 + 4], acc[b0 + 5]);
-            __nv_bfloat162 p3 = __floats2bfloat162_rn(acc[b0 + 6], acc[b0 + 7]);
-            o.x = *(uint32_t*)&p0; o.y = *(uint32_t*)&p1; o.z = *(uint32_t*)&p2; o.w = *(uint32_t*)&p3;
+            const int b0 = cc * 32 + j * 4;
+            const uint4 o = make_uint4(bf16Pair(b0), bf16Pair(b0 + 1), bf16Pair(b0 + 2), bf16Pair(b0 + 3));
             *(uint4*)(wbuf + lane * 128 + ((j ^ (lane & 7)) * 16)) = o;
           }
           __syncwarp();
@@ -330,7 +355,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     tcFenceAfter();
     tmemDealloc(tmemBase, kTmemCols);
   }
-  if (multi) {
+  if (FUSED) {
     bar.sync(true, false);
     bar.finish();
   }
@@ -453,7 +478,7 @@ __global__ void __launch_bounds__(256) tpQuantBlocksKernel(const __nv_bfloat16* 
   }
 }
 
-const void* tpGemmFp8KernelFn() { return (const void*)tpGemmFp8Kernel; }
+const void* tpGemmFp8KernelFn(bool fused) { return fused ? (const void*)tpGemmFp8Kernel<true> : (const void*)tpGemmFp8Kernel<false>; }
 const void* tpQuantRowsWideKernelFn() { return (const void*)tpQuantRowsWideKernel; }
 void tpQuantRowsWideGrid(int rows, int K, int* x, int* y) {
   *x = (rows + kQuantRows - 1) / kQuantRows;

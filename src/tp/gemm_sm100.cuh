@@ -233,6 +233,19 @@ __device__ __forceinline__ void tmemLdWait32(uint32_t (&r)[32]) {
                  "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
                :: "memory");
 }
+// Two fp32 fused multiply-adds in one instruction, each rounded like fmaf.
+__device__ __forceinline__ uint64_t packF32x2(uint32_t lo, uint32_t hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+  return v;
+}
+__device__ __forceinline__ void fmaF32x2(uint64_t& acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+// Moves registers between the warpgroups of a CTA: all warps of a warpgroup execute it, and the shares of the warpgroups add
+// up to what the CTA was launched with.
+template <int N> __device__ __forceinline__ void regsGive() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regsTake() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 __device__ __forceinline__ void tmemLdWait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ bool electOne() {

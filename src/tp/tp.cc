@@ -182,7 +182,7 @@ static ncclResult_t launchGemmFp8(ncclTpContext* tp, const void* A, const void* 
   cfg.dynamicSmemBytes = tpGemmFp8SmemBytes();
   cfg.stream = stream;
   void* args[3] = {&tmA, &tmB, a};
-  cudaError_t e = cudaLaunchKernelExC(&cfg, tpGemmFp8KernelFn(), args);
+  cudaError_t e = cudaLaunchKernelExC(&cfg, tpGemmFp8KernelFn(a->nRanks > 1 && a->mode != TP_MODE_STORE), args);
   if (e != cudaSuccess) { WARN("fp8 tensor-parallel GEMM launch failed: %s", cudaGetErrorString(e)); (void)cudaGetLastError(); return ncclUnhandledCudaError; }
   if (tp->comm->devPlane) tp->comm->devPlane->launches++;
   return ncclSuccess;
@@ -327,7 +327,7 @@ ncclResult_t ncclTpCreate(ncclComm_t comm, size_t maxRows, size_t maxCols, ncclT
   // function attributes are per device: set them here, with this context's device current, not once per process
   CUDACHECK(cudaFuncSetAttribute(tpGemmKernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmSmemBytes()));
   CUDACHECK(cudaFuncSetAttribute(tpGemmSplitKernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmSplitSmemBytes()));
-  CUDACHECK(cudaFuncSetAttribute(tpGemmFp8KernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmFp8SmemBytes()));
+  for (bool fused : {false, true}) CUDACHECK(cudaFuncSetAttribute(tpGemmFp8KernelFn(fused), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmFp8SmemBytes()));
   {
     // how many clusters of two CTAs of the pair kernel the device can hold at once: the grid never exceeds it,
     // because its CTAs wait for one another (comm CTAs, cross-GPU barriers)

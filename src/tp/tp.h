@@ -84,7 +84,7 @@ const void* tpGemmPairKernelFn();      // CTA-pair variant (cluster of two, 256 
 const void* tpGemmSplitKernelFn();     // plain C = A * W^T, one 128 x 256 tile per cluster of splitK CTAs
 size_t tpGemmSplitSmemBytes();
 int tpGemmSplitThreads();
-const void* tpGemmFp8KernelFn();
+const void* tpGemmFp8KernelFn(bool fused);   // fused: REDUCE and GATHER with more than one rank
 const void* tpQuantRowsWideKernelFn(); // as the next one, for 16-byte aligned x and q, on the grid below
 void tpQuantRowsWideGrid(int rows, int K, int* x, int* y);
 const void* tpQuantRowsKernelFn();     // (const bf16* x, uint8_t* q, float* scales, int rows, int K): 1 x 128 blocks, scales [K/128][rows]

@@ -1,9 +1,5 @@
-"""Block-scaled fp8 GEMM at the edges of its tiles: pairs of CTAs whose last row tile is half empty, one row block, fewer and
-more K blocks than the scale look-ahead, more tiles than CTAs, with both kernel forms, against a 64-bit product."""
-import os
-import subprocess
-import sys
-
+"""Block-scaled fp8: the GEMM at the edges of its pipeline (one K block, odd and even numbers of them, one tile, more tiles than
+CTAs) against a 64-bit product, and the quantiser of activations at the edges of its tiles."""
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -13,8 +9,9 @@ pytestmark = pytest.mark.gpu
 SHAPES = [(128, 256, 128), (256, 256, 128), (384, 512, 256), (640, 256, 640), (1920, 1024, 384), (4224, 2304, 1152)]
 
 
-def _run():
-    sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+def test_fp8_tiles():
+    if not torch.cuda.is_available() or torch.cuda.get_device_capability()[0] < 10:
+        pytest.skip("needs sm_100")
     from nccl_b200 import Communicator, get_unique_id
     from nccl_b200.ops.tp import TensorParallel
     torch.cuda.set_device(0)
@@ -38,15 +35,6 @@ def _run():
     assert comm.async_error() == 0
     tp.destroy()
     comm.destroy()
-    print("tiles ok")
-
-
-@pytest.mark.parametrize("pair", ["1", "0"])
-def test_fp8_tiles(pair):
-    if not torch.cuda.is_available() or torch.cuda.get_device_capability()[0] < 10:
-        pytest.skip("needs sm_100")
-    r = subprocess.run([sys.executable, os.path.abspath(__file__)], env=dict(os.environ, NCCL_B200_TP_PAIR=pair), capture_output=True, text=True, timeout=300)
-    assert r.returncode == 0 and "tiles ok" in r.stdout, r.stdout + r.stderr
 
 
 @pytest.mark.parametrize("rows,K", [(1, 128), (3, 2048), (4, 2176), (5, 896), (129, 4224)])
@@ -70,7 +58,3 @@ def test_quantise_rows(rows, K, off):
     assert torch.equal(q[:rows].view(torch.uint8), want.view(torch.uint8)) and (q[rows].float() == 1).all()
     tp.destroy()
     comm.destroy()
-
-
-if __name__ == "__main__":
-    _run()
