@@ -98,8 +98,9 @@ static void fillSyncTp(ncclComm* comm, SyncArgs* s) {
 }
 
 // CTAs that share the K blocks of a tile in a plain bf16 GEMM, 1 for none: as many as leave every cluster resident at once,
-// when the 128 x 256 tiles alone would leave half of the SMs idle, and each CTA keeps kSplitMinBlocks K blocks (below that the
-// exchange of the partial sums costs more than the shorter loop saves).
+// when the 128 x 256 tiles alone would leave half of the SMs idle, and each CTA keeps kSplitMinBlocks K blocks. At that line two
+// CTAs still give 5 % (128 x 2048 x 1024: 9.7 instead of 10.2 us; twice the K 12.0 instead of 14.6, four CTAs 11.0), and at 64 tiles two
+// are even with CTA pairs for K = 1024 (1024 x 2048: 10.6 us both) and ahead beyond (512 x 4096 x 4096: 20.2 instead of 24.6).
 constexpr int kSplitMinBlocks = 8;
 static int splitOf(const ncclTpContext* tp, const TpGemmArgs* a) {
   const int tiles = (a->M / 128) * (a->N / 256);
@@ -139,7 +140,8 @@ static ncclResult_t launchGemm(ncclTpContext* tp, const void* A, const void* W, 
   bool pair = paramTpPair() != 0 && tp->pairClusters > 0 && (!fused || a->M % (256 * n) == 0);
   if (pair && a->M % 256) {
     // Plain GEMMs: pairs leave half of the last row tile empty. A K step of a pair tile takes 2/3 of the time of one of a
-    // 128 x 256 tile (both are bound by the operand traffic from L2: 32 KiB against 48 KiB per SM).
+    // 128 x 256 tile (both are bound by the operand traffic from L2: 32 KiB against 48 KiB per SM). Measured on either kernel:
+    // 4224 x 8192 x 2048 99.6 against 106.5 us, 3200 x 2304 x 4096 47.0 against 50.2.
     const int tilesN = a->N / 256, one = a->M / 128 * tilesN, two = (a->M / 128 + 1) / 2 * tilesN;
     const int wavesOne = (one + tp->smCount - 1) / tp->smCount, wavesTwo = (two + tp->pairClusters - 1) / tp->pairClusters;
     pair = 2 * wavesTwo < 3 * wavesOne;
