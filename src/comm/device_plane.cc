@@ -132,7 +132,7 @@ static void preloadKernels(int dev) {
   done[dev] = true;
   cudaFuncAttributes attr;
   auto touch = [&](const void* fn) { if (fn && cudaFuncGetAttributes(&attr, fn) != cudaSuccess) (void)cudaGetLastError(); };
-  for (const void* fn : {p2pKernelFn(), copyKernelFn(), copyBulkKernelFn(), llCopyKernelFn(), localCopyKernelFn(4, nullptr, nullptr), localCopyKernelFn(8, nullptr, nullptr), localCopyKernelFn(4, nullptr, (const void*)1), localBulkCopyKernelFn(),
+  for (const void* fn : {p2pKernelFn(), copyKernelFn(), copyBulkKernelFn(), llCopyKernelFn(), localCopyKernelFn(4, nullptr, nullptr), localCopyKernelFn(8, nullptr, nullptr), localCopyKernelFn(4, nullptr, (const void*)1), localCopyKernelFn(4, (const void*)1, (const void*)1), localBulkCopyKernelFn(),
                          signalKernelFn(), waitSignalKernelFn()})
     touch(fn);
   for (int t = 0; t < ncclNumTypes; ++t) {

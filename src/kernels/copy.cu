@@ -629,18 +629,42 @@ const void* scaleKernelFn(ncclDataType_t type) {
   }
 }
 
-// Local copy of `count` bytes: the data movement of a single-rank communicator (out-of-place
-// collectives reduce to dst = src) and of staged transfers.
-// A kernel of its own for sources that lie at another offset inside 16 bytes than the destination: putting packs together takes
-// registers that would cost the plain form its second CTA per SM (178 instead of 166 us for 512 MiB when both shared a kernel).
-// 32 MiB at odd offsets take 13 us; byte by byte they took 120.
-template <int U, bool SHIFTED>
-__global__ void __launch_bounds__(512, 2) localCopyKernel(ScaleArgs a) {
+// Local copy of `count` bytes between 16-byte aligned buffers: the data movement of a single-rank communicator
+// (out-of-place collectives reduce to dst = src) and of staged transfers. A CTA moves contiguous tiles of
+// U x blockDim x 16 bytes (all loads of a tile issued before its stores), and CTAs stride over
+// tiles, so that each DRAM page is opened once and enough bytes are in flight for HBM speed.
+template <int U>
+__global__ void __launch_bounds__(512) localCopyKernel(ScaleArgs a) {
+  const char* src = (const char*)a.src;
+  char* dst = (char*)a.dst;
+  const size_t bytes = a.count;
+  const size_t packs = bytes / 16;
+  const size_t tilePacks = (size_t)U * blockDim.x;
+  const size_t fullTiles = packs / tilePacks;
+  for (size_t t = blockIdx.x; t < fullTiles; t += gridDim.x) {
+    const size_t base = t * tilePacks + threadIdx.x;
+    uint4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = ldStream16(src + (base + (size_t)u * blockDim.x) * 16);
+#pragma unroll
+    for (int u = 0; u < U; ++u) st16(dst + (base + (size_t)u * blockDim.x) * 16, v[u]);
+  }
+  // remainder: packs past the last full tile, then loose bytes
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (size_t i = fullTiles * tilePacks + tid; i < packs; i += stride) st16(dst + i * 16, ldStream16(src + i * 16));
+  for (size_t j = packs * 16 + tid; j < bytes; j += stride) dst[j] = src[j];
+}
+// The same at any alignment. A kernel of its own: putting packs together takes registers that the aligned form needs for its second
+// CTA per SM (178 instead of 166 us for 512 MiB when both shared a kernel) and for what runs beside it. 32 MiB at odd offsets take
+// 13 us; byte by byte they took 120.
+template <bool SHIFTED>
+__global__ void __launch_bounds__(512, 2) localCopyUnalignedKernel(ScaleArgs a) {
   const char* src = (const char*)a.src;
   char* dst = (char*)a.dst;
   const PackSpan sp = packSpan(src, dst, a.count);
   auto same = [](uint4 v) { return v; };
-  streamPacks<U, SHIFTED>(src + sp.head, dst + sp.head, sp.packs, sp.shift, same);
+  streamPacks<4, SHIFTED>(src + sp.head, dst + sp.head, sp.packs, sp.shift, same);
   const size_t behind = sp.head + sp.packs * 16, loose = sp.head + (a.count - behind);
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < loose; i += (size_t)gridDim.x * blockDim.x) {
     const size_t j = i < sp.head ? i : behind + (i - sp.head);
@@ -678,8 +702,9 @@ const void* localBulkCopyKernelFn() { return (const void*)localBulkCopyKernel; }
 size_t localBulkCopySmemBytes() { return 128 + (size_t)kBulkStages * kBulkChunk + kBulkStages * 8; }
 
 const void* localCopyKernelFn(int unroll, const void* src, const void* dst) {
-  if (((uintptr_t)src ^ (uintptr_t)dst) & 15) return (const void*)localCopyKernel<4, true>;
-  return unroll >= 8 ? (const void*)localCopyKernel<8, false> : (const void*)localCopyKernel<4, false>;
+  if (((uintptr_t)src ^ (uintptr_t)dst) & 15) return (const void*)localCopyUnalignedKernel<true>;
+  if ((uintptr_t)src & 15) return (const void*)localCopyUnalignedKernel<false>;
+  return unroll >= 8 ? (const void*)localCopyKernel<8> : (const void*)localCopyKernel<4>;
 }
 
 // ------------------------------------------------------------------------- signals
