@@ -656,8 +656,8 @@ __global__ void __launch_bounds__(512) localCopyKernel(ScaleArgs a) {
   for (size_t j = packs * 16 + tid; j < bytes; j += stride) dst[j] = src[j];
 }
 // The same at any alignment. A kernel of its own: putting packs together takes registers that the aligned form needs for its second
-// CTA per SM (178 instead of 166 us for 512 MiB when both shared a kernel) and for what runs beside it. 32 MiB at odd offsets take
-// 13 us; byte by byte they took 120.
+// CTA per SM (178 instead of 166 us for 512 MiB when both shared a kernel). 32 MiB at odd offsets take 13 us; byte by byte they
+// took 120.
 template <bool SHIFTED>
 __global__ void __launch_bounds__(512, 2) localCopyUnalignedKernel(ScaleArgs a) {
   const char* src = (const char*)a.src;
