@@ -147,8 +147,8 @@ __global__ void __launch_bounds__(kThreads) devApiArRmsNormKernel(ncclDevComm_t 
 // One rank: x = partial + residual, residual <- x, out <- rmsnorm(x) * weight, as above without the sources to wait for.
 // Bound by memory on the SMs that the caller grants, so what counts is how much each of them has in flight: a producer warp
 // streams chunks of R neighbouring rows (partial and residual) into a ring of shared memory with bulk copies, groups of G
-// threads take one row each from there. 2048 rows of 8192 take 39 us on 64 CTAs; with a CTA to a row, its loads waiting for the
-// previous row's stores, they took 125.
+// threads take one row each from there. 2048 rows of 8192 take 36 us a call on 64 CTAs; with a CTA to a row, its loads waiting for
+// the previous row's stores, they took 127.
 constexpr int kRowPacks = 8;          // 16-byte packs of a row per thread, at most
 constexpr int kRowStages = 16;        // chunks in the ring, at most
 constexpr size_t kRowRing = 200 << 10;
@@ -282,17 +282,40 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
   __syncthreads();   // no thread leaves while a copy into this CTA's shared memory is under way
 }
 
-ncclResult_t launchRmsNormRows(RowArgs a, int nCtas, cudaStream_t stream) {
-  const size_t rowBytes = (size_t)a.hidden * 2;
-  // chunks of about 8 KiB (a copy below that costs more to issue than to move), while every CTA still gets several
-  a.chunkRows = std::max(1, std::min((int)(8192 / rowBytes), a.tokens / (4 * nCtas)));
-  a.stages = (int)std::min<size_t>(kRowStages, kRowRing / (2 * a.chunkRows * rowBytes));
-  const size_t smem = 128 + 2 * a.chunkRows * rowBytes * a.stages;
+// How the kernel above splits a call: threads to a row, rows of a chunk, chunks in the ring.
+//
+// A wait on a slot's barrier tells two uses of the slot apart by the parity of their phases, so a group may wait for a use only
+// when it has seen the one before: nothing orders the copies of two chunks, and a wait that skips a use would take a slot whose
+// copy of the lap before is still under way for loaded. Group g takes rows g, g + groups, ... of its CTA, so it sees every use of
+// the slots that it reads when a lap of the ring (stages x chunkRows rows) is a whole number of its steps. Both are kept to
+// multiples that see to it: 8192 channels get 4 stages where the ring would hold 6.
+struct RowPlan {
+  int group, chunkRows, stages;
+};
+
+RowPlan rowPlan(int tokens, int hidden, int nCtas) {
+  const size_t rowBytes = (size_t)hidden * 2;
+  RowPlan p;
   // the fewest threads to a row that hold it, more where there are not enough rows for that many groups
-  int g = 32;
-  while (g < kThreads && (g * kRowPacks < a.hidden / 8 || (long long)nCtas * (kThreads / g) > a.tokens)) g *= 2;
-  const void* fn = g == 32 ? (const void*)rmsNormRowsKernel<32> : g == 64 ? (const void*)rmsNormRowsKernel<64> : g == 128 ? (const void*)rmsNormRowsKernel<128> :
-                   g == 256 ? (const void*)rmsNormRowsKernel<256> : (const void*)rmsNormRowsKernel<512>;
+  p.group = 32;
+  while (p.group < kThreads && (p.group * kRowPacks < hidden / 8 || (long long)nCtas * (kThreads / p.group) > tokens)) p.group *= 2;
+  // chunks of about 8 KiB (a copy below that costs more to issue than to move), while every CTA still gets several; a power of
+  // two, like the number of groups
+  const int rows = std::min((int)(8192 / rowBytes), tokens / (4 * nCtas));
+  p.chunkRows = 1;
+  while (2 * p.chunkRows <= rows) p.chunkRows *= 2;
+  const int step = std::max(1, kThreads / p.group / p.chunkRows);
+  p.stages = (int)std::min<size_t>(kRowStages, kRowRing / (2 * p.chunkRows * rowBytes)) / step * step;
+  return p;
+}
+
+ncclResult_t launchRmsNormRows(RowArgs a, int nCtas, cudaStream_t stream) {
+  const RowPlan p = rowPlan(a.tokens, a.hidden, nCtas);
+  a.chunkRows = p.chunkRows;
+  a.stages = p.stages;
+  const size_t smem = 128 + (size_t)a.hidden * 4 * a.chunkRows * a.stages;
+  const void* fn = p.group == 32 ? (const void*)rmsNormRowsKernel<32> : p.group == 64 ? (const void*)rmsNormRowsKernel<64> : p.group == 128 ? (const void*)rmsNormRowsKernel<128> :
+                   p.group == 256 ? (const void*)rmsNormRowsKernel<256> : (const void*)rmsNormRowsKernel<512>;
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return ncclUnhandledCudaError;
   void* args[1] = {&a};
   return cudaLaunchKernel(fn, dim3(nCtas), dim3(kRowThreads), args, smem, stream) == cudaSuccess ? ncclSuccess : ncclUnhandledCudaError;
@@ -379,6 +402,17 @@ ncclResult_t b200DevApiArRmsNorm(const ncclDevComm_t* dc, ncclWindow_t inWin, si
   devApiArRmsNormKernel<<<nCtas, kThreads, 0, stream>>>(*dc, inWin->devSelf, inOff, resWin->devSelf, resOff, outWin->devSelf, outOff,
                                                         (const __nv_bfloat16*)weight, eps, tokens, hidden, mode, st);
   return cudaGetLastError() == cudaSuccess ? ncclSuccess : ncclUnhandledCudaError;
+}
+
+// The split of a one-rank call, for tests: threads to a row, threads of all groups, rows of a chunk, chunks in the ring.
+ncclResult_t b200DevApiArRmsNormPlan(int tokens, int hidden, int nCtas, int plan[4]) {
+  if (!plan || tokens < 0 || hidden < 8 || hidden % 8 || hidden > 8 * kThreads * 4 || nCtas < 1) return ncclInvalidArgument;
+  const RowPlan p = rowPlan(tokens, hidden, nCtas);
+  plan[0] = p.group;
+  plan[1] = kThreads;
+  plan[2] = p.chunkRows;
+  plan[3] = p.stages;
+  return ncclSuccess;
 }
 
 ncclResult_t b200DevApiLLSum(const ncclDevComm_t* dc, const void* in, void* out, int slots, int nCtas, cudaStream_t stream) {
