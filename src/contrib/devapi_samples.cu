@@ -396,6 +396,7 @@ ncclResult_t b200DevApiArRmsNorm(const ncclDevComm_t* dc, ncclWindow_t inWin, si
   int* st = statusWord();
   if (!st) return ncclUnhandledCudaError;
   if (dc->lsaSize == 1 && mode != 1) {
+    if (tokens == 0 || hidden <= 0) return ncclSuccess;   // no rows, or rows without channels: nothing to read or write
     RowArgs a = {(const char*)inWin->peerPtr[inWin->rank] + inOff, (char*)resWin->peerPtr[resWin->rank] + resOff, (char*)outWin->peerPtr[outWin->rank] + outOff, (const char*)weight, eps, tokens, hidden, 0, 0, st};
     return launchRmsNormRows(a, nCtas, stream);
   }

@@ -1,5 +1,7 @@
 """The fused all-reduce + residual + RMSNorm kernel on one rank: row lengths around the limits of a group of threads, fewer
 and more rows than groups, against fp32 PyTorch."""
+import ctypes
+
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -33,5 +35,27 @@ def test_rows(hidden, tokens, ctas):
         assert torch.equal(resid[:tokens], x[:tokens]) and torch.equal(resid[tokens], guard) and (out[tokens] == 9).all()
         # one bf16 rounding (2^-9) of a value that fp32 has to about 1e-6
         torch.testing.assert_close(out[:tokens].float(), ref[:tokens], rtol=2 ** -8, atol=1e-6)
+    dc.destroy()
+    comm.destroy()
+
+
+@pytest.mark.parametrize("tokens,hidden", [(5, 0), (5, -8), (0, 1024)])
+def test_empty_calls(tokens, hidden):
+    """No rows, or rows without channels, are an empty call of the C entry point: nothing is divided by their size, nothing is
+    launched or written."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from nccl_b200 import Communicator, get_unique_id
+    from nccl_b200.ops.devapi import DeviceComm
+    torch.cuda.set_device(0)
+    comm = Communicator(1, 0, get_unique_id())
+    dc = DeviceComm(comm)
+    bufs = [dc.symmetric(1024, torch.bfloat16).fill_(9) for _ in range(3)]
+    w = torch.ones(1024, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    for mode in (0, 2):
+        places = [v for b in bufs for v in dc._locate(b)]
+        assert dc.lib.b200DevApiArRmsNorm(ctypes.byref(dc.dc), *places, w.data_ptr(), 1e-6, tokens, hidden, mode, 4, 0) == 0
+    assert dc.status() == 0 and all((b == 9).all() for b in bufs)
     dc.destroy()
     comm.destroy()
