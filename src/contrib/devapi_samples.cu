@@ -316,9 +316,14 @@ ncclResult_t launchRmsNormRows(RowArgs a, int nCtas, cudaStream_t stream) {
   const size_t smem = 128 + (size_t)a.hidden * 4 * a.chunkRows * a.stages;
   const void* fn = p.group == 32 ? (const void*)rmsNormRowsKernel<32> : p.group == 64 ? (const void*)rmsNormRowsKernel<64> : p.group == 128 ? (const void*)rmsNormRowsKernel<128> :
                    p.group == 256 ? (const void*)rmsNormRowsKernel<256> : (const void*)rmsNormRowsKernel<512>;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return ncclUnhandledCudaError;
+  // The limit belongs to the function, which threads with other shapes launch at the same time: every call sets the same value, the
+  // largest ring, and never one below what another is about to launch with.
   void* args[1] = {&a};
-  return cudaLaunchKernel(fn, dim3(nCtas), dim3(kRowThreads), args, smem, stream) == cudaSuccess ? ncclSuccess : ncclUnhandledCudaError;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(128 + kRowRing)) == cudaSuccess &&
+      cudaLaunchKernel(fn, dim3(nCtas), dim3(kRowThreads), args, smem, stream) == cudaSuccess)
+    return ncclSuccess;
+  (void)cudaGetLastError();   // the call reports it: later checks do not find it again
+  return ncclUnhandledCudaError;
 }
 
 // Exercises ncclLLA2ASession: every rank contributes two floats per slot; each rank receives the sum.

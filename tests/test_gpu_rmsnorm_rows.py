@@ -1,6 +1,8 @@
 """The fused all-reduce + residual + RMSNorm kernel on one rank: row lengths around the limits of a group of threads, fewer
 and more rows than groups, against fp32 PyTorch."""
 import ctypes
+import sys
+import threading
 
 import pytest
 
@@ -59,3 +61,41 @@ def test_empty_calls(tokens, hidden):
     assert dc.status() == 0 and all((b == 9).all() for b in bufs)
     dc.destroy()
     comm.destroy()
+
+
+def test_threads_with_rings_of_different_sizes():
+    """Threads launch the same kernel (32 threads to a row) with rings of 32 KiB and of 128 KiB: none takes the limit of shared
+    memory away from another."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from nccl_b200 import Communicator, get_unique_id
+    from nccl_b200.ops.devapi import DeviceComm
+    torch.cuda.set_device(0)
+    failed, work = [], []
+    for tokens, hidden in ((40, 64), (16, 2048)) * 2:
+        comm = Communicator(1, 0, get_unique_id())
+        dc = DeviceComm(comm)
+        bufs = [dc.symmetric(tokens * hidden, torch.bfloat16).view(tokens, hidden).zero_() for _ in range(3)]
+        work.append((comm, dc, bufs, torch.ones(hidden, dtype=torch.bfloat16, device="cuda"), torch.cuda.Stream()))
+    torch.cuda.synchronize()
+
+    def calls(dc, bufs, w, stream):
+        torch.cuda.set_device(0)
+        places = [v for b in bufs for v in dc._locate(b)]
+        args = (ctypes.byref(dc.dc), *places, w.data_ptr(), 1e-6, *bufs[0].shape, 0, 1, stream.cuda_stream)
+        call = dc.lib.b200DevApiArRmsNorm   # without the interpreter's lock
+        failed.extend(r for r in (call(*args) for _ in range(20000)) if r)
+
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    threads = [threading.Thread(target=calls, args=w[1:]) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    sys.setswitchinterval(interval)
+    torch.cuda.synchronize()
+    assert not failed
+    for comm, dc, *_ in work:
+        dc.destroy()
+        comm.destroy()
