@@ -153,6 +153,7 @@ constexpr int kRowPacks = 8;          // 16-byte packs of a row per thread, at m
 constexpr int kRowStages = 16;        // chunks in the ring, at most
 constexpr size_t kRowRing = 200 << 10;
 constexpr int kRowThreads = kThreads + 32;
+constexpr int kStatusRing = 6;        // status word: a wait on the ring ran out
 
 // bf16 is the upper half of fp32
 __device__ __forceinline__ void unpackBf16(float (&x)[8], uint4 v) {
@@ -196,10 +197,13 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
     mbarInitFence();
   }
   __syncthreads();
-  auto wait = [&](uint64_t* bar, uint32_t parity) {
-    if (gaveUp || mbarWait(smemAddr(bar), parity)) return;
-    gaveUp = 1;   // nobody waits any longer; the copies still under way are waited for below
-    atomicExch(a.status, 1);
+  // false: this wait or one of another thread ran out. Nobody waits, copies or stores any longer; the copies still under way are
+  // waited for below
+  auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+    if (!gaveUp && mbarWait(smemAddr(bar), parity)) return true;
+    gaveUp = 1;
+    atomicExch(a.status, kStatusRing);
+    return false;
   };
   if (threadIdx.x >= kThreads) {
     if (threadIdx.x == kThreads) {
@@ -207,7 +211,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
       for (int c = blockIdx.x; c < chunks && !gaveUp; c += gridDim.x, ++i) {
         const int s = i % a.stages;
         const uint32_t ph = (i / a.stages) & 1;
-        wait(&emptyBar[s], ph ^ 1);
+        if (!wait(&emptyBar[s], ph ^ 1)) break;   // the slot is still being read
         const int rows = a.tokens - c * R < R ? a.tokens - c * R : R;
         const uint32_t bytes = (uint32_t)(rows * rowBytes);
         const size_t off = (size_t)c * R * rowBytes;
@@ -230,7 +234,9 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
       const int t = c * R + r;
       if (t >= a.tokens) break;
       const int s = i % a.stages;
-      wait(&fullBar[s], (i / a.stages) & 1);
+      // a row that did not arrive is left alone: neither read, stored nor released; its group still meets at the barrier
+      const bool ok = wait(&fullBar[s], (i / a.stages) & 1);
+      const int rowPacks = ok ? packs : 0;
       const uint8_t* part = ring + (size_t)s * 2 * half + r * rowBytes;
       char* res = a.residual + t * rowBytes;
       uint4 sum[kRowPacks];
@@ -238,7 +244,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
 #pragma unroll
       for (int k = 0; k < kRowPacks; ++k) {
         const int pk = tid + k * G;
-        if (pk < packs) {
+        if (pk < rowPacks) {
           float x[8], y[8];
           unpackBf16(x, *(const uint4*)(part + (size_t)pk * 16));
           unpackBf16(y, *(const uint4*)(part + half + (size_t)pk * 16));
@@ -262,13 +268,13 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) ss += red[parity][grp * kWarps + w];
       }
-      if (tid == 0) mbarArrive(smemAddr(&emptyBar[s]));   // the whole group has read the row
+      if (tid == 0 && ok) mbarArrive(smemAddr(&emptyBar[s]));   // the whole group has read the row
       const float inv = rsqrtf(ss / (float)a.hidden + a.eps);
       char* out = a.out + t * rowBytes;
 #pragma unroll
       for (int k = 0; k < kRowPacks; ++k) {
         const int pk = tid + k * G;
-        if (pk < packs) {
+        if (pk < rowPacks) {
           float w[8], x[8];
           unpackBf16(w, *(const uint4*)(a.weight + (size_t)pk * 16));
           unpackBf16(x, sum[k]);
@@ -440,7 +446,8 @@ ncclResult_t b200DevApiGinRing(const ncclDevComm_t* dc, ncclWindow_t win, size_t
 }
 
 // 0 when no device-API kernel launched by this thread on the current device gave up a wait,
-// otherwise the code of the wait (1 entry barrier, 2 exit barrier, 3 low-latency receive).
+// otherwise the code of the wait (1 entry barrier, 2 exit barrier, 3 low-latency receive, 4 put, 5 signal, 6 a row copied
+// into shared memory by the one-rank RMSNorm kernel).
 // Synchronises the device and clears the word.
 int b200DevApiStatus(void) {
   int* st = statusWord();
