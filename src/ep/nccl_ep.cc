@@ -103,8 +103,21 @@ static ncclResult_t launchEp(const void* fn, EpArgs* a, int ctas, int ranksY, si
 }
 
 // Calls that the local kernels serve: one rank, both halves at once, rows whose places do not depend on one another. The flat
-// layout packs in arrival order and a split call must hold the rows between its halves: both take the general kernels.
+// layout packs in arrival order and a split call must hold the rows between its halves: both take the general kernels. So do calls
+// whose outputs share memory with their inputs: the general kernels have every input row in a landing zone before they store a
+// result, the local ones read and store at once.
 static bool localForm(const ncclEpGroup* g, int layout, bool sendOnly) { return g->n == 1 && !sendOnly && layout != EP_FLAT; }
+
+struct Span {
+  const void* data;
+  size_t bytes;
+};
+static bool overlap(std::initializer_list<Span> outputs, std::initializer_list<Span> inputs) {
+  for (const Span& o : outputs)
+    for (const Span& i : inputs)
+      if (o.data && i.data && (const char*)o.data < (const char*)i.data + i.bytes && (const char*)i.data < (const char*)o.data + o.bytes) return true;
+  return false;
+}
 
 // `want`: CTAs that have something to do. Two CTAs per SM, or the caller's number of SMs with one each.
 static ncclResult_t launchEpLocal(ncclEpGroup* g, const void* fn, EpArgs* a, size_t want, cudaStream_t stream) {
@@ -386,7 +399,11 @@ ncclResult_t ncclEpDispatch(ncclEpHandle_t h, const ncclEpDispatchInputs_t* in, 
   const bool sendOnly = config && config->send_only;
   if (sendOnly) a.phases = 1;
   void* counters = (li && li->expert_counters && li->expert_counters->data) ? li->expert_counters->data : nullptr;
-  if (localForm(g, a.layout, sendOnly) && (uintptr_t)in->tokens->data % 16 == 0) {   // the general kernel quantises from 8-byte loads
+  const size_t T = (size_t)h->T, K = (size_t)h->K, rows = a.layout == EP_EXPERT_MAJOR ? g->El * cap : cap;
+  if (localForm(g, a.layout, sendOnly) && (uintptr_t)in->tokens->data % 16 == 0 &&   // the general kernel quantises from 8-byte loads
+      !overlap({{a.outTokens[me], rows * g->H * (fp8 ? 1 : 2)}, {a.outScales[me], rows * (g->H / 128) * sizeof(float)}, {outIdx, rows * K * sizeof(int64_t)},
+                {outW, rows * K * sizeof(float)}, {counters, g->El * sizeof(int)}},
+               {{a.x[me], T * g->H * 2}, {a.topkIdx[me], T * K * sizeof(int64_t)}, {a.topkW[me], T * K * sizeof(float)}})) {
     a.userCount = (int*)counters;
     return launchEpLocal(g, epDispatchLocalKernelFn(fp8), &a, std::max(h->T, a.layout == EP_RANK_MAJOR ? (g->maxTokens + kEpLocalThreads - 1) / kEpLocalThreads : 1), stream);
   }
@@ -455,7 +472,12 @@ ncclResult_t ncclEpCombine(ncclEpHandle_t h, const ncclEpCombineInputs_t* in, co
   if (h->pending) { WARN("ncclEpCombine: a send_only call on this handle is still waiting for ncclEpComplete"); return ncclInvalidUsage; }
   const bool sendOnly = config && config->send_only;
   if (sendOnly) a.phases = 1;
-  if (localForm(g, a.layout, sendOnly)) {
+  // rank-major: row t of the result is made from row t of the input by the same threads, so it may take its very place
+  const size_t T = (size_t)h->T, rowBytes = (size_t)g->H * 2;
+  const bool inPlace = a.layout == EP_RANK_MAJOR && a.outTokens[me] == (const void*)a.x[me];
+  if (localForm(g, a.layout, sendOnly) && !overlap({{a.outTokens[me], T * rowBytes}},
+                                                   {{inPlace ? nullptr : a.x[me], (a.layout == EP_EXPERT_MAJOR ? g->El * cap : cap) * rowBytes},
+                                                    {a.topkIdx[me], T * h->K * sizeof(int64_t)}, {weights, T * h->K * sizeof(float)}})) {
     a.rowOf = h->rowOf;
     return h->T ? launchEpLocal(g, epCombineLocalKernelFn(), &a, ((size_t)h->T * (g->H / 8) + kEpLocalThreads - 1) / kEpLocalThreads, stream) : ncclSuccess;
   }

@@ -89,3 +89,32 @@ def test_expert_named_twice_and_tokens_at_eight_bytes(comm):
     torch.cuda.synchronize()
     torch.testing.assert_close(out.float(), x.float() * w.sum(1, keepdim=True), rtol=2 ** -7, atol=1e-6)
     ep.destroy()
+
+
+@pytest.mark.parametrize("layout", ["expert_major", "rank_major"])
+def test_outputs_over_inputs(comm, layout):
+    """A result may lie in the memory of what it is made from: the rows are read before any result is stored."""
+    from nccl_b200.ops.ep import ExpertParallel
+    T, E, K, H = 600, 4, 2, 1024
+    ep = ExpertParallel(comm, E, T, H, layout=layout)
+    x, idx, w = _batch(T, E, K, H, 11, 0.1)
+    valid = idx >= 0
+    y = ep.dispatch(x, idx, w, fp8=False)[0].clone()
+    want = ep.combine(y).clone()
+    scale = (w * valid).sum(1, keepdim=True) if layout == "expert_major" else valid.any(1, keepdim=True)
+    torch.testing.assert_close(want.float(), x.float() * scale, rtol=2 ** -7, atol=1e-6)
+    for shift in (0, 1, 5):   # rows of the input that the first row of the result lies behind its start
+        z = torch.empty(y.numel() + shift * H, dtype=y.dtype, device="cuda")
+        z[:y.numel()] = y.view(-1)
+        out = z[shift * H:(shift + T) * H].view(T, H)
+        assert torch.equal(ep.combine(z[:y.numel()].view(y.shape), out=out), want)
+    for shift in (0, 3):      # the tokens lie in the tensor that they are dispatched to
+        toks = torch.zeros_like(y)
+        inside = toks.view(-1, H)[shift:shift + T] if shift + T <= toks.numel() // H else toks.view(-1, H)[:T]
+        inside.copy_(x)
+        got, _, counts = ep.dispatch(inside, idx, w, fp8=False, toks=toks)
+        assert torch.equal(counts.long(), torch.bincount(idx[valid], minlength=E))
+        assert torch.equal(ep.combine(got), want)
+    torch.cuda.synchronize()
+    assert comm.async_error() == 0
+    ep.destroy()
