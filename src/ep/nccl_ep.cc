@@ -108,6 +108,14 @@ static ncclResult_t launchEp(const void* fn, EpArgs* a, int ctas, int ranksY, si
 // result, the local ones read and store at once.
 static bool localForm(const ncclEpGroup* g, int layout, bool sendOnly) { return g->n == 1 && !sendOnly && layout != EP_FLAT; }
 
+// Memory that a kernel of this GPU may write. Counts that lie elsewhere (pinned host memory, another GPU) are copied there by the
+// general path, and the copy refuses what it cannot reach.
+static bool onThisGpu(const void* p, int dev) {
+  cudaPointerAttributes attr;
+  if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+  return attr.type == cudaMemoryTypeDevice && attr.device == dev;
+}
+
 struct Span {
   const void* data;
   size_t bytes;
@@ -401,6 +409,7 @@ ncclResult_t ncclEpDispatch(ncclEpHandle_t h, const ncclEpDispatchInputs_t* in, 
   void* counters = (li && li->expert_counters && li->expert_counters->data) ? li->expert_counters->data : nullptr;
   const size_t T = (size_t)h->T, K = (size_t)h->K, rows = a.layout == EP_EXPERT_MAJOR ? g->El * cap : cap;
   if (localForm(g, a.layout, sendOnly) && (uintptr_t)in->tokens->data % 16 == 0 &&   // the general kernel quantises from 8-byte loads
+      (!counters || onThisGpu(counters, g->comm->cudaDev)) &&
       !overlap({{a.outTokens[me], rows * g->H * (fp8 ? 1 : 2)}, {a.outScales[me], rows * (g->H / 128) * sizeof(float)}, {outIdx, rows * K * sizeof(int64_t)},
                 {outW, rows * K * sizeof(float)}, {counters, g->El * sizeof(int)}},
                {{a.x[me], T * g->H * 2}, {a.topkIdx[me], T * K * sizeof(int64_t)}, {a.topkW[me], T * K * sizeof(float)}})) {

@@ -118,3 +118,23 @@ def test_outputs_over_inputs(comm, layout):
     torch.cuda.synchronize()
     assert comm.async_error() == 0
     ep.destroy()
+
+
+@pytest.mark.parametrize("layout", ["expert_major", "rank_major"])
+def test_counts_outside_the_gpu(comm, layout):
+    """Expert counts may be asked for in pinned host memory; memory that the GPU cannot reach is refused with an error."""
+    from nccl_b200.ops.ep import ExpertParallel
+    ep = ExpertParallel(comm, 8, 32, 256, layout=layout)
+    x, idx, w = _batch(32, 8, 2, 256, 5, 0.2)
+    want = torch.bincount(idx[idx >= 0], minlength=8).cpu()
+    pinned = torch.zeros(8, dtype=torch.int32).pin_memory()
+    ep.dispatch(x, idx, w, fp8=False, counts=pinned)
+    torch.cuda.synchronize()
+    assert torch.equal(pinned.long(), want)
+    with pytest.raises(Exception):
+        ep.dispatch(x, idx, w, fp8=False, counts=torch.zeros(8, dtype=torch.int32))
+    torch.cuda.synchronize()
+    assert torch.equal(ep.dispatch(x, idx, w, fp8=False)[2].long().cpu(), want)
+    torch.cuda.synchronize()
+    assert comm.async_error() == 0
+    ep.destroy()
