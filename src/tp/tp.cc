@@ -139,12 +139,15 @@ static ncclResult_t launchGemm(ncclTpContext* tp, const void* A, const void* W, 
   if (!fused && (a->splitK = splitOf(tp, a)) > 1) return launchGemmSplit(tp, A, W, a, stream);
   bool pair = paramTpPair() != 0 && tp->pairClusters > 0 && (!fused || a->M % (256 * n) == 0);
   if (pair && a->M % 256) {
-    // Plain GEMMs: pairs leave half of the last row tile empty. A K step of a pair tile takes 2/3 of the time of one of a
-    // 128 x 256 tile (both are bound by the operand traffic from L2: 32 KiB against 48 KiB per SM). Measured on either kernel:
-    // 4224 x 8192 x 2048 99.6 against 106.5 us, 3200 x 2304 x 4096 47.0 against 50.2.
+    // Plain GEMMs: pairs leave half of the last row tile empty. A K step of a pair tile takes 0.92 to 0.97 of the time of one of two
+    // 128 x 256 tiles (32 KiB of operands from L2 per SM against 48), but a launch of pairs takes about 1.5 us longer, so they pay
+    // when they need no more waves and have enough steps. Kernel times of pairs over one-CTA tiles, weights from memory and from
+    // L2: one wave 1.2 at K = 512, 1.08 at 1536, 1.04 at 3584, 0.91-1.04 at 7168; two waves 0.97-1.02 at 1024, 0.96-1.01 at 1536,
+    // 0.91-1.01 at 4096; three and more 0.91-0.98 from 1024 on, about 1.0 at 512; four waves where one-CTA
+    // tiles need three 1.1.
     const int tilesN = a->N / 256, one = a->M / 128 * tilesN, two = (a->M / 128 + 1) / 2 * tilesN;
     const int wavesOne = (one + tp->smCount - 1) / tp->smCount, wavesTwo = (two + tp->pairClusters - 1) / tp->pairClusters;
-    pair = 2 * wavesTwo < 3 * wavesOne;
+    pair = wavesOne > 1 && wavesTwo <= wavesOne && a->K >= (wavesOne > 2 ? 1024 : 1536);
   }
   int commCtas = gather ? tpCommCtas(tp, n) : 0;
   int grid;
