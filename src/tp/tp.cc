@@ -98,13 +98,15 @@ static void fillSyncTp(ncclComm* comm, SyncArgs* s) {
 }
 
 // CTAs that share the K blocks of a tile in a plain bf16 GEMM, 1 for none: as many as leave every cluster resident at once,
-// when the 128 x 256 tiles alone would leave half of the SMs idle, and each CTA keeps kSplitMinBlocks K blocks. At that line two
-// CTAs still give 5 % (128 x 2048 x 1024: 9.7 instead of 10.2 us; twice the K 12.0 instead of 14.6, four CTAs 11.0), and at 64 tiles two
-// are even with CTA pairs for K = 1024 (1024 x 2048: 10.6 us both) and ahead beyond (512 x 4096 x 4096: 20.2 instead of 24.6).
-constexpr int kSplitMinBlocks = 8;
-static int splitOf(const ncclTpContext* tp, const TpGemmArgs* a) {
-  const int tiles = (a->M / 128) * (a->N / 256);
-  int s = std::min(std::min(std::min((int)paramTpSplit(), kTpMaxSplit), tp->smCount / tiles), a->K / 64 / kSplitMinBlocks);
+// when the 128 x 256 tiles alone would leave half of the SMs idle, and each CTA keeps kSplitMinBlocks K blocks. Where short loops save
+// no more than the exchange of the partial sums costs, a CTA keeps its tile. Kernel times against the kernel that the call would
+// take instead, weights from memory and from L2, 4 to 72 tiles. One CTA to a tile: K = 1024 1.01-1.10, 1280 0.94-1.05, 1536
+// 0.87-1.00, 1792 0.84-0.96, 2560 0.71-0.88. CTA pairs: K = 1024 0.95-1.03, 1280 0.92-1.00, 2560 0.80-0.90.
+constexpr int kSplitMinBlocks = 8, kSplitFromOne = 1536 / 64;
+static int splitOf(const ncclTpContext* tp, const TpGemmArgs* a, bool insteadOfPairs) {
+  const int tiles = (a->M / 128) * (a->N / 256), blocks = a->K / 64;
+  if (!insteadOfPairs && blocks < kSplitFromOne) return 1;
+  int s = std::min(std::min(std::min((int)paramTpSplit(), kTpMaxSplit), tp->smCount / tiles), blocks / kSplitMinBlocks);
   while (s > 1 && tiles > tp->splitClusters[s]) --s;
   return std::max(s, 1);
 }
@@ -136,8 +138,9 @@ static ncclResult_t launchGemm(ncclTpContext* tp, const void* A, const void* W, 
   const int n = a->nRanks;
   const bool fused = n > 1 && a->mode != TP_MODE_STORE;
   const bool gather = fused && a->mode == TP_MODE_GATHER;
-  if (!fused && (a->splitK = splitOf(tp, a)) > 1) return launchGemmSplit(tp, A, W, a, stream);
-  bool pair = paramTpPair() != 0 && tp->pairClusters > 0 && (!fused || a->M % (256 * n) == 0);
+  const bool pairs = paramTpPair() != 0 && tp->pairClusters > 0;
+  if (!fused && (a->splitK = splitOf(tp, a, pairs && a->M % 256 == 0)) > 1) return launchGemmSplit(tp, A, W, a, stream);
+  bool pair = pairs && (!fused || a->M % (256 * n) == 0);
   if (pair && a->M % 256) {
     // Plain GEMMs: pairs leave half of the last row tile empty. A K step of a pair tile takes 0.92 to 0.97 of the time of one of two
     // 128 x 256 tiles (32 KiB of operands from L2 per SM against 48), but a launch of pairs takes about 1.5 us longer, so they pay
