@@ -145,12 +145,13 @@ static ncclResult_t launchGemm(ncclTpContext* tp, const void* A, const void* W, 
     // Plain GEMMs: pairs leave half of the last row tile empty. A K step of a pair tile takes 0.92 to 0.97 of the time of one of two
     // 128 x 256 tiles (32 KiB of operands from L2 per SM against 48), but a launch of pairs takes about 1.5 us longer, so they pay
     // when they need no more waves and have enough steps. Kernel times of pairs over one-CTA tiles, weights from memory and from
-    // L2: one wave 1.2 at K = 512, 1.08 at 1536, 1.04 at 3584, 0.91-1.04 at 7168; two waves 0.97-1.02 at 1024, 0.96-1.01 at 1536,
-    // 0.91-1.01 at 4096; three and more 0.91-0.98 from 1024 on, about 1.0 at 512; four waves where one-CTA
-    // tiles need three 1.1.
+    // L2: two waves 0.97-1.02 at K = 1024, 0.96-1.01 at 1536, 0.91-1.01 at 4096; three and more 0.91-0.98 from 1024 on, about 1.0 at
+    // 512; four waves where one-CTA tiles need three 1.1. One wave 1.2 at 512, 1.08 at 1536; at 4096 to 7168 0.90-0.98 when
+    // the operands are more than 60 MiB or come from memory, 1.00-1.06 when they are fewer and in L2.
     const int tilesN = a->N / 256, one = a->M / 128 * tilesN, two = (a->M / 128 + 1) / 2 * tilesN;
     const int wavesOne = (one + tp->smCount - 1) / tp->smCount, wavesTwo = (two + tp->pairClusters - 1) / tp->pairClusters;
-    pair = wavesOne > 1 && wavesTwo <= wavesOne && a->K >= (wavesOne > 2 ? 1024 : 1536);
+    const bool enough = wavesOne > 2 ? a->K >= 1024 : wavesOne > 1 ? a->K >= 1536 : a->K >= 4096 && ((size_t)a->M + a->N) * a->K * 2 > (size_t)60 << 20;
+    pair = wavesTwo <= wavesOne && enough;
   }
   int commCtas = gather ? tpCommCtas(tp, n) : 0;
   int grid;

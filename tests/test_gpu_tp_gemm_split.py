@@ -12,10 +12,10 @@ pytestmark = pytest.mark.gpu
 
 # with the largest cluster: tiles x shares 2x8 (K 66 blocks), 1x7 (61 blocks), 5x3, 22x6, 29x5, 32x4, 40x3; where the split begins 1x1 (23
 # blocks) and 1x3 (24 blocks) instead of one CTA, 64x1 (15 blocks) and 64x2 (16 blocks) instead of pairs; 1x1 further below;
-# without clusters: the one-CTA and the pair kernel, the latter also where the rows end inside a tile (the last two)
+# without clusters: the one-CTA and the pair kernel, the latter also where the rows end inside a tile (the last three)
 SHAPES = [(256, 256, 4224), (128, 256, 3904), (128, 256, 960), (128, 256, 1024), (128, 256, 1472), (128, 256, 1536), (128, 1280, 1664), (128, 5632, 3200),
           (128, 7424, 2752), (128, 8192, 2048), (640, 2048, 1600), (256, 8192, 960), (256, 8192, 1024), (256, 8192, 1088), (1920, 5120, 320),
-          (4224, 4096, 192), (1920, 5120, 1536), (4224, 4096, 1024)]
+          (4224, 4096, 192), (1920, 5120, 1536), (4224, 4096, 1024), (384, 8192, 4096)]
 
 
 def _run():
