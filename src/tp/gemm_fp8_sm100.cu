@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(256) tpQuantRowsWideKernel(const __nv_bfloat16
   }
 }
 
-// The same from 8-byte aligned x into 4-byte aligned q. One warp per (row, K block).
+// The same from 8-byte aligned x into 4-byte aligned q, and for few K blocks. One warp per (row, K block).
 __global__ void __launch_bounds__(256) tpQuantRowsKernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scales,
                                                           int rows, int K) {
   const int kBlocks = K / 128;

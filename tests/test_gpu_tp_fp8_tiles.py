@@ -37,8 +37,8 @@ def test_fp8_tiles():
     comm.destroy()
 
 
-@pytest.mark.parametrize("rows,K", [(1, 128), (3, 2048), (4, 2176), (5, 896), (129, 4224)])
-@pytest.mark.parametrize("off", [0, 4])   # 4 elements: too little alignment for the wide loads
+@pytest.mark.parametrize("rows,K", [(1, 128), (7, 384), (9, 512), (3, 2048), (4, 2176), (5, 896), (129, 4224)])
+@pytest.mark.parametrize("off", [0, 4])   # 4 elements: too little alignment for the wide loads, which rows from 512 channels on take
 def test_quantise_rows(rows, K, off):
     if not torch.cuda.is_available() or torch.cuda.get_device_capability()[0] < 10:
         pytest.skip("needs sm_100")
