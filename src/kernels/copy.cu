@@ -535,6 +535,11 @@ const void* reshardKernelFn() { return (const void*)reshardKernel; }
 // How a byte range splits when dst is written in 16-byte packs and src may lie at any other alignment: `head` bytes before
 // the first pack, `packs` packs, the rest behind them. With shift != 0 a pack of dst straddles two aligned words of src and
 // is put together from both; head and packs are chosen so that neither word reaches outside the source range.
+//
+// Up to kLooseBytes the elements (bytes) are moved one by one: finding the packs takes longer than it saves. Kernel times of
+// packs over elements: copy of 100 bytes 1.9-2.1 / 1.5 us, 1025 1.7-2.1 / 1.3-1.9, 2000 1.8-2.1 / 1.6-2.0, 5000 1.8-2.1 / 2.5-2.8;
+// scale of 128 elements 1.6-2.1 / 1.2-1.5, 500 fp32 1.6-2.0 / 1.3-1.7, 1000 fp32 1.9-2.1 / 2.0.
+constexpr size_t kLooseBytes = 2048;
 struct PackSpan {
   size_t head, packs;
   int shift;
@@ -590,6 +595,11 @@ __global__ void __launch_bounds__(512, 2) scaleKernel(ScaleArgs a) {
   if (a.scalarPtr) s = *(const T*)a.scalarPtr;
   else memcpy(&s, &a.scalarBits, sizeof(T));
   const A sa = Elem<T>::ld(s);
+  const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  if (a.count * sizeof(T) <= kLooseBytes) {
+    for (size_t i = tid; i < a.count; i += stride) ((T*)a.dst)[i] = Elem<T>::st(Elem<T>::ld(((const T*)a.src)[i]) * sa);
+    return;
+  }
   const char* src = (const char*)a.src;
   char* dst = (char*)a.dst;
   const PackSpan sp = packSpan(src, dst, a.count * sizeof(T));
@@ -605,7 +615,7 @@ __global__ void __launch_bounds__(512, 2) scaleKernel(ScaleArgs a) {
   // elements before the first and behind the last pack
   const size_t before = sp.head / sizeof(T), behind = before + sp.packs * Pack16<T>::N;
   const size_t loose = before + (a.count - behind);
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < loose; i += (size_t)gridDim.x * blockDim.x) {
+  for (size_t i = tid; i < loose; i += stride) {
     const size_t e = i < before ? i : behind + (i - before);
     ((T*)dst)[e] = Elem<T>::st(Elem<T>::ld(((const T*)src)[e]) * sa);
   }
@@ -657,16 +667,21 @@ __global__ void __launch_bounds__(512) localCopyKernel(ScaleArgs a) {
 }
 // The same at any alignment. A kernel of its own: putting packs together takes registers that the aligned form needs for its second
 // CTA per SM (178 instead of 166 us for 512 MiB when both shared a kernel). 32 MiB at odd offsets take 13 us; byte by byte they
-// took 120.
+// took 120. The shifted form spills 12 bytes at the 64 registers that two CTAs per SM leave it.
 template <bool SHIFTED>
 __global__ void __launch_bounds__(512, 2) localCopyUnalignedKernel(ScaleArgs a) {
   const char* src = (const char*)a.src;
   char* dst = (char*)a.dst;
+  const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  if (a.count <= kLooseBytes) {
+    for (size_t i = tid; i < a.count; i += stride) dst[i] = src[i];
+    return;
+  }
   const PackSpan sp = packSpan(src, dst, a.count);
   auto same = [](uint4 v) { return v; };
   streamPacks<4, SHIFTED>(src + sp.head, dst + sp.head, sp.packs, sp.shift, same);
   const size_t behind = sp.head + sp.packs * 16, loose = sp.head + (a.count - behind);
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < loose; i += (size_t)gridDim.x * blockDim.x) {
+  for (size_t i = tid; i < loose; i += stride) {
     const size_t j = i < sp.head ? i : behind + (i - sp.head);
     dst[j] = src[j];
   }

@@ -23,8 +23,10 @@ def _between_bands(count, off, dtype):
     return raw, raw[off:off + count]
 
 
-# one below, at and above: a pack, the shortest span that is moved in packs, a tile (4 x 512 packs), several tiles
-@pytest.mark.parametrize("nbytes", [1, 15, 16, 17, 31, 32, 33, 47, 48, 49, 4095, 32767, 32768, 32769, 32768 * 3 + 21, (1 << 20) + 13])
+# one below, at and above: a pack, what is moved byte by byte (up to 2048), a tile (4 x 512 packs), several tiles; from 2049 on
+# with ends of 1, 8, 15 and 16 bytes behind the packs
+@pytest.mark.parametrize("nbytes", [1, 15, 16, 17, 31, 32, 33, 47, 48, 49, 2047, 2048, 2049, 2056, 2064, 2079, 2080, 2081, 4095, 32767, 32768, 32769,
+                                    32768 * 3 + 21, (1 << 20) + 13])
 @pytest.mark.parametrize("soff,doff", [(0, 0), (1, 1), (0, 1), (3, 0), (15, 14), (7, 9), (8, 4), (16, 5)])
 def test_copy_at_any_alignment(comm, nbytes, soff, doff):
     sraw, src = _between_bands(nbytes, soff, torch.uint8)
@@ -37,7 +39,7 @@ def test_copy_at_any_alignment(comm, nbytes, soff, doff):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16", "float16", "float64", "int32", "int64"])
-@pytest.mark.parametrize("count,soff,doff", [(1, 0, 0), (7, 0, 0), (9, 1, 0), (40, 1, 1), (2047, 0, 3), (16384, 0, 0), (16391, 3, 2), (100003, 1, 0)])
+@pytest.mark.parametrize("count,soff,doff", [(1, 0, 0), (7, 0, 0), (9, 1, 0), (40, 1, 1), (256, 1, 0), (257, 0, 1), (513, 1, 2), (1025, 3, 1), (2047, 0, 3), (16384, 0, 0), (16391, 3, 2), (100003, 1, 0)])
 def test_scale_at_any_element_offset(comm, dtype, count, soff, doff):
     from nccl_b200 import core
     dt = getattr(torch, dtype)
