@@ -49,6 +49,7 @@ static inline bool pdlFor(int ctas, bool shortKernel) {
   if (paramLaunchPdl() == 0) return false;
   return !shortKernel || ctas <= paramLaunchPdlMaxCtas();
 }
+bool devPlanePdl() { return paramLaunchPdl() != 0; }
 B200_PARAM(BarrierMulticast, "B200_BARRIER_MC_MIN_RANKS", -1, "Cross-GPU barriers arrive with one multimem.red on a multicast alias of the flag page from this many ranks on (0 = never, -1 = from the selection table)")
 
 // ------------------------------------------------------------------------------------ tuning
@@ -410,7 +411,7 @@ static ncclResult_t scaleCopy(ncclComm* comm, ncclDataType_t type, const void* s
   const size_t perCta = 512 * 4 * 16;   // bytes that a CTA of the kernel moves in one tile
   int ctas = (int)std::min<size_t>((count * typeSize(type) + perCta - 1) / perCta, (size_t)comm->devPlane->smCount * 16);
   comm->devPlane->launches++;
-  return launchKernel(scaleKernelFn(type), dim3(std::max(ctas, 1)), dim3(512), 0, &sa, stream, false);
+  return launchKernel(scaleKernelFn(type), dim3(std::max(ctas, 1)), dim3(512), 0, &sa, stream, false, pdlFor(ctas, false));
 }
 
 void sliceEven(size_t count, size_t es, int n, size_t* begin, size_t* cnt) {
@@ -931,7 +932,7 @@ static ncclResult_t runOneRank(ncclComm* comm, const Task& t) {
     size_t perCta = (size_t)threads * unroll * 16;
     int ctas = (int)std::min<size_t>((bytes + perCta - 1) / perCta, (size_t)comm->devPlane->smCount * paramCopyCtasPerSm());
     comm->devPlane->launches++;
-    NCCLCHECK(launchKernel(localCopyKernelFn(unroll, src, dst), dim3(std::max(ctas, 1)), dim3(threads), 0, &ca, t.stream, false));
+    NCCLCHECK(launchKernel(localCopyKernelFn(unroll, src, dst), dim3(std::max(ctas, 1)), dim3(threads), 0, &ca, t.stream, false, pdlFor(ctas, false)));
   }
   return ncclSuccess;
 }

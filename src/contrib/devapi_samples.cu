@@ -15,6 +15,8 @@
 #include <algorithm>
 
 #include "nccl_device.h"
+#include "../comm/device_plane.h"
+#include "../kernels/common.cuh"
 #include "../tp/gemm_sm100.cuh"
 
 namespace {
@@ -197,6 +199,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
     mbarInitFence();
   }
   __syncthreads();
+  b200::pdlEnter();   // the set-up above overlaps the end of the kernel before
   // false: this wait or one of another thread ran out. Nobody waits, copies or stores any longer; the copies still under way are
   // waited for below
   auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
@@ -325,8 +328,20 @@ ncclResult_t launchRmsNormRows(RowArgs a, int nCtas, cudaStream_t stream) {
   // The limit belongs to the function, which threads with other shapes launch at the same time: every call sets the same value, the
   // largest ring, and never one below what another is about to launch with.
   void* args[1] = {&a};
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute pdl;
+  cfg.gridDim = dim3(nCtas);
+  cfg.blockDim = dim3(kRowThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  if (b200::devPlanePdl()) {
+    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &pdl;
+    cfg.numAttrs = 1;
+  }
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(128 + kRowRing)) == cudaSuccess &&
-      cudaLaunchKernel(fn, dim3(nCtas), dim3(kRowThreads), args, smem, stream) == cudaSuccess)
+      cudaLaunchKernelExC(&cfg, fn, args) == cudaSuccess)
     return ncclSuccess;
   (void)cudaGetLastError();   // the call reports it: later checks do not find it again
   return ncclUnhandledCudaError;

@@ -746,6 +746,7 @@ __device__ __forceinline__ void localPayload(const EpArgs& a, const __nv_bfloat1
 
 template <bool FP8>
 __global__ void __launch_bounds__(kEpLocalThreads, 2) epDispatchLocalKernel(const __grid_constant__ EpArgs a) {
+  pdlEnter();
   __shared__ int sRow[kLocTokens * kLocMaxK];
   __shared__ int sHist[kEpMaxLocalExperts];
   __shared__ int sIsLast;
@@ -888,6 +889,7 @@ __device__ __forceinline__ void localSums(const __nv_bfloat16* y, int H, int C, 
 // out[t] = sum over the token's selected experts of w * row, in fp32, in slot order. The (token, 8 channels) items are dealt to
 // the CTAs as contiguous ranges; where the rows lie and their weights is looked up once per token and CTA.
 __global__ void __launch_bounds__(kEpLocalThreads, 2) epCombineLocalKernel(const __grid_constant__ EpArgs a) {
+  pdlEnter();
   __shared__ int sRow[kLocTokens * kLocMaxK];
   __shared__ float sW[kLocTokens * kLocMaxK];
   const int me = a.rank, H = a.hidden, K = a.topk, E = a.numExperts, T = a.numTokens[me];

@@ -131,7 +131,7 @@ static bool overlap(std::initializer_list<Span> outputs, std::initializer_list<S
 static ncclResult_t launchEpLocal(ncclEpGroup* g, const void* fn, EpArgs* a, size_t want, cudaStream_t stream) {
   const size_t most = g->cfg.max_num_sms ? std::min<size_t>(g->cfg.max_num_sms, g->smCount) : (size_t)2 * g->smCount;
   if (g->comm->devPlane) g->comm->devPlane->launches++;
-  return launchKernel(fn, dim3((unsigned)std::max<size_t>(std::min(want, most), 1)), dim3(kEpLocalThreads), 0, a, stream, false);
+  return launchKernel(fn, dim3((unsigned)std::max<size_t>(std::min(want, most), 1)), dim3(kEpLocalThreads), 0, a, stream, false, devPlanePdl());
 }
 
 B200_PARAM(EpBulk, "B200_EP_BULK", 1, "Expert-parallel dispatch hands the packed tokens to the bulk-copy engines (a ring of shared-memory stages per CTA) instead of storing them with the warps: 0 never, 1 for the expert-major layout, 2 for every layout")

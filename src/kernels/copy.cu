@@ -590,6 +590,7 @@ __device__ __forceinline__ void streamPacks(const char* src, char* dst, size_t p
 // element they took 25.
 template <typename T>
 __global__ void __launch_bounds__(512, 2) scaleKernel(ScaleArgs a) {
+  pdlEnter();
   using A = typename Elem<T>::Acc;
   T s;
   if (a.scalarPtr) s = *(const T*)a.scalarPtr;
@@ -645,6 +646,7 @@ const void* scaleKernelFn(ncclDataType_t type) {
 // tiles, so that each DRAM page is opened once and enough bytes are in flight for HBM speed.
 template <int U>
 __global__ void __launch_bounds__(512) localCopyKernel(ScaleArgs a) {
+  pdlEnter();
   const char* src = (const char*)a.src;
   char* dst = (char*)a.dst;
   const size_t bytes = a.count;
@@ -670,6 +672,7 @@ __global__ void __launch_bounds__(512) localCopyKernel(ScaleArgs a) {
 // took 120. The shifted form spills 12 bytes at the 64 registers that two CTAs per SM leave it.
 template <bool SHIFTED>
 __global__ void __launch_bounds__(512, 2) localCopyUnalignedKernel(ScaleArgs a) {
+  pdlEnter();
   const char* src = (const char*)a.src;
   char* dst = (char*)a.dst;
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;

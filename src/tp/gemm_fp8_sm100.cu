@@ -146,6 +146,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   __syncthreads();
   tcFenceAfter();
   const uint32_t tmemBase = *tmemSlot;
+  pdlEnter();   // the set-up above overlaps the end of the kernel before; operands and results are touched behind it
 
   const int tilesN = a.N / BN;
   const int nTiles = (a.M / BM) * tilesN;
@@ -251,8 +252,8 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       const bool remoteRows = gather && tc.owner != rank;
       auto scaleOf = [&](int kb) -> float {
         const float* pa = scaleA + (size_t)kb * a.M + row;
-        const float sa = gather ? *(const volatile float*)pa : __ldg(pa);
-        return sa * __ldg(a.scaleW + (size_t)kb * wBlocksN + wCol);
+        const float sa = *(const volatile float*)pa;
+        return sa * *(const volatile float*)(a.scaleW + (size_t)kb * wBlocksN + wCol);
       };
       bool primed = false;
       if (!remoteRows) {
@@ -374,8 +375,9 @@ __device__ __forceinline__ uint32_t packE4m3x4(float a, float b, float c, float 
 // warp and 8-byte accesses per group they took 18.
 // Needs 16-byte aligned x and q.
 constexpr int kQuantRows = 4, kQuantBlocks = 16;
-__global__ void __launch_bounds__(256) tpQuantRowsWideKernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scales,
+__global__ void __launch_bounds__(256) tpQuantRowsWideKernel(const __nv_bfloat16* x, uint8_t* q, float* scales,
                                                              int rows, int K) {
+  pdlEnter();
   const int kBlocks = K / 128;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = (int)blockIdx.x * kQuantRows + (lane >> 3);
@@ -385,8 +387,8 @@ __global__ void __launch_bounds__(256) tpQuantRowsWideKernel(const __nv_bfloat16
     const int kb = (int)blockIdx.y * kQuantBlocks + u * 8 + warp;
     const bool in = row < rows && kb < kBlocks;
     const uint4* p = (const uint4*)(x + (size_t)row * K + (size_t)kb * 128 + (lane & 7) * 16);
-    raw[u][0] = in ? __ldg(p) : make_uint4(0, 0, 0, 0);
-    raw[u][1] = in ? __ldg(p + 1) : make_uint4(0, 0, 0, 0);
+    raw[u][0] = in ? ldStream16(p) : make_uint4(0, 0, 0, 0);
+    raw[u][1] = in ? ldStream16(p + 1) : make_uint4(0, 0, 0, 0);
   }
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
@@ -419,8 +421,9 @@ __global__ void __launch_bounds__(256) tpQuantRowsWideKernel(const __nv_bfloat16
 }
 
 // The same from 8-byte aligned x into 4-byte aligned q, and for few K blocks. One warp per (row, K block).
-__global__ void __launch_bounds__(256) tpQuantRowsKernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scales,
+__global__ void __launch_bounds__(256) tpQuantRowsKernel(const __nv_bfloat16* x, uint8_t* q, float* scales,
                                                           int rows, int K) {
+  pdlEnter();
   const int kBlocks = K / 128;
   const size_t warpId = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const size_t nWarps = ((size_t)gridDim.x * blockDim.x) >> 5;
@@ -442,8 +445,9 @@ __global__ void __launch_bounds__(256) tpQuantRowsKernel(const __nv_bfloat16* __
 }
 
 // Weights: one scale per 128 x 128 block. One CTA of 256 threads per block; scales[kb][rows/128].
-__global__ void __launch_bounds__(256) tpQuantBlocksKernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scales,
+__global__ void __launch_bounds__(256) tpQuantBlocksKernel(const __nv_bfloat16* x, uint8_t* q, float* scales,
                                                             int rows, int K) {
+  pdlEnter();
   __shared__ float red[8];
   const int kBlocks = K / 128, rBlocks = rows / 128;
   for (int blk = blockIdx.x; blk < kBlocks * rBlocks; blk += gridDim.x) {

@@ -95,6 +95,7 @@ tpGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   clusterSync();   // both CTAs' barriers are initialised before either signals the other's
   tcFenceAfter();
   const uint32_t tmemBase = *tmemSlot;
+  pdlEnter();   // the set-up above overlaps the end of the kernel before; operands and results are touched behind it
   if (!ok && threadIdx.x == 0) stSharedCluster(mapaShared(smemAddr((const void*)abortFlag), cr ^ 1), 1u);
 
   const int tilesN = a.N / BN;

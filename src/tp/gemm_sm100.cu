@@ -93,6 +93,7 @@ tpGemmKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   __syncthreads();
   tcFenceAfter();
   const uint32_t tmemBase = *tmemSlot;
+  pdlEnter();   // the set-up above overlaps the end of the kernel before; operands and results are touched behind it
 
   const int tilesN = a.N / BN;
   const int nTiles = (a.M / BM) * tilesN;

@@ -65,6 +65,7 @@ tpGemmSplitKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   tcFenceAfter();
   const uint32_t tmemBase = *tmemSlot;
+  pdlEnter();   // the set-up above overlaps the end of the kernel before; operands and results are touched behind it
   const uint32_t ring = smemAddr(smem);
 
   const int tilesN = a.N / BN;

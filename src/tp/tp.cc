@@ -71,6 +71,27 @@ static void clusterAttribute(cudaLaunchAttribute* attr, int ctas) {
   attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
 }
 
+// Launches with programmatic stream serialisation when `pdl`: the kernel's set-up overlaps the end of the kernel before it. Plain
+// calls only: the fused kernels meet their partners on other GPUs before they would wait.
+static ncclResult_t launchTp(ncclTpContext* tp, const void* fn, dim3 grid, int threads, size_t smem, void** args, bool pdl, int cluster, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attrs[2];
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attrs;
+  if (cluster > 1) clusterAttribute(&attrs[cfg.numAttrs++], cluster);
+  if (pdl && devPlanePdl()) {
+    attrs[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
+  if (e != cudaSuccess) { WARN("tensor-parallel kernel launch failed: %s", cudaGetErrorString(e)); (void)cudaGetLastError(); return ncclUnhandledCudaError; }
+  if (tp->comm->devPlane) tp->comm->devPlane->launches++;
+  return ncclSuccess;
+}
+
 static int tpCommCtas(const ncclTpContext* tp, int nRanks) {
   int64_t want = paramTpCommCtas();
   if (want <= 0) want = nRanks <= 2 ? 4 : nRanks <= 4 ? 8 : 16;
@@ -115,20 +136,8 @@ static ncclResult_t launchGemmSplit(ncclTpContext* tp, const void* A, const void
   CUtensorMap tmA, tmB;
   NCCLCHECK(makeMap(&tmA, A, a->M, a->K, 128));
   NCCLCHECK(makeMap(&tmB, W, a->N, a->K, 256));
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute cluster;
-  clusterAttribute(&cluster, a->splitK);
-  cfg.gridDim = dim3((a->M / 128) * (a->N / 256) * a->splitK);
-  cfg.blockDim = dim3(tpGemmSplitThreads());
-  cfg.dynamicSmemBytes = tpGemmSplitSmemBytes();
-  cfg.stream = stream;
-  cfg.attrs = &cluster;
-  cfg.numAttrs = 1;
   void* args[3] = {&tmA, &tmB, a};
-  cudaError_t e = cudaLaunchKernelExC(&cfg, tpGemmSplitKernelFn(), args);
-  if (e != cudaSuccess) { WARN("tensor-parallel GEMM launch failed: %s", cudaGetErrorString(e)); (void)cudaGetLastError(); return ncclUnhandledCudaError; }
-  if (tp->comm->devPlane) tp->comm->devPlane->launches++;
-  return ncclSuccess;
+  return launchTp(tp, tpGemmSplitKernelFn(), dim3((a->M / 128) * (a->N / 256) * a->splitK), tpGemmSplitThreads(), tpGemmSplitSmemBytes(), args, true, a->splitK, stream);
 }
 
 // Launches the bf16 GEMM kernel in the mode of `a`. Grid: one CTA per SM (fewer when there are fewer
@@ -169,32 +178,18 @@ static ncclResult_t launchGemm(ncclTpContext* tp, const void* A, const void* W, 
   CUtensorMap tmA, tmB;
   NCCLCHECK(makeMap(&tmA, A, a->M, a->K, 128));
   NCCLCHECK(makeMap(&tmB, W, a->N, a->K, pair ? 128 : 256));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(pair ? tpGemmPairThreads() : tpGemmThreads());
-  cfg.dynamicSmemBytes = pair ? tpGemmPairSmemBytes() : tpGemmSmemBytes();
-  cfg.stream = stream;
   void* args[3] = {&tmA, &tmB, a};
-  cudaError_t e = cudaLaunchKernelExC(&cfg, pair ? tpGemmPairKernelFn() : tpGemmKernelFn(), args);
-  if (e != cudaSuccess) { WARN("tensor-parallel GEMM launch failed: %s", cudaGetErrorString(e)); (void)cudaGetLastError(); return ncclUnhandledCudaError; }
-  if (tp->comm->devPlane) tp->comm->devPlane->launches++;
-  return ncclSuccess;
+  return launchTp(tp, pair ? tpGemmPairKernelFn() : tpGemmKernelFn(), dim3(grid), pair ? tpGemmPairThreads() : tpGemmThreads(),
+                  pair ? tpGemmPairSmemBytes() : tpGemmSmemBytes(), args, !fused, 1, stream);
 }
 
 static ncclResult_t launchGemmFp8(ncclTpContext* tp, const void* A, const void* W, TpGemmArgs* a, int grid, cudaStream_t stream) {
   CUtensorMap tmA, tmB;
   NCCLCHECK(makeMap(&tmA, A, a->M, a->K, 128, 1));
   NCCLCHECK(makeMap(&tmB, W, a->N, a->K, 256, 1));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(tpGemmFp8Threads());
-  cfg.dynamicSmemBytes = tpGemmFp8SmemBytes();
-  cfg.stream = stream;
   void* args[3] = {&tmA, &tmB, a};
-  cudaError_t e = cudaLaunchKernelExC(&cfg, tpGemmFp8KernelFn(a->nRanks > 1 && a->mode != TP_MODE_STORE), args);
-  if (e != cudaSuccess) { WARN("fp8 tensor-parallel GEMM launch failed: %s", cudaGetErrorString(e)); (void)cudaGetLastError(); return ncclUnhandledCudaError; }
-  if (tp->comm->devPlane) tp->comm->devPlane->launches++;
-  return ncclSuccess;
+  const bool fused = a->nRanks > 1 && a->mode != TP_MODE_STORE;
+  return launchTp(tp, tpGemmFp8KernelFn(fused), dim3(grid), tpGemmFp8Threads(), tpGemmFp8SmemBytes(), args, !fused, 1, stream);
 }
 
 static ncclResult_t checkShapeFp8(int M, int N, int K, int n) {
@@ -218,17 +213,15 @@ ncclResult_t ncclTpQuantizeFp8(ncclTp_t tp, const void* x, void* q, float* scale
   // over the other: 8192 rows K = 128 4.5 / 2.8 us, 256 4.7 / 4.0, 384 4.8 / 5.2, 512 5.0 / 6.1; 32768 rows 13.5 / 6.1, 14.1 / 10.4,
   // 14.6 / 14.3, 15.0 / 17.9.
   if (blockRows == 1 && K >= 512 && !(((uintptr_t)x | (uintptr_t)q) & 15) && gy <= 65535) {
-    CUDACHECK(cudaLaunchKernel(tpQuantRowsWideKernelFn(), dim3(gx, gy), dim3(256), args, 0, stream));
+    return launchTp(tp, tpQuantRowsWideKernelFn(), dim3(gx, gy), 256, 0, args, true, 1, stream);
   } else if (blockRows == 1) {
     size_t warps = (size_t)rows * (K / 128);
     int ctas = (int)std::min<size_t>((warps + 7) / 8, (size_t)tp->smCount * 16);
-    CUDACHECK(cudaLaunchKernel(tpQuantRowsKernelFn(), dim3(std::max(ctas, 1)), dim3(256), args, 0, stream));
+    return launchTp(tp, tpQuantRowsKernelFn(), dim3(std::max(ctas, 1)), 256, 0, args, true, 1, stream);
   } else {
     int blocks = (rows / 128) * (K / 128);
-    CUDACHECK(cudaLaunchKernel(tpQuantBlocksKernelFn(), dim3(std::min(blocks, tp->smCount * 8)), dim3(256), args, 0, stream));
+    return launchTp(tp, tpQuantBlocksKernelFn(), dim3(std::min(blocks, tp->smCount * 8)), 256, 0, args, true, 1, stream);
   }
-  if (tp->comm->devPlane) tp->comm->devPlane->launches++;
-  return ncclSuccess;
 }
 
 ncclResult_t ncclTpGemmFp8(ncclTp_t tp, const void* A, const float* scaleA, const void* W, const float* scaleW, void* C, int M, int N, int K, cudaStream_t stream) {
