@@ -1,0 +1,170 @@
+"""Forward and backward of the decoder's units with this package's own row kernels, for the sharded engine on a GPU.
+
+The functions do what `llama.decoder_layer` and `llama.head_loss` do under autograd with checkpointing, over the same flat
+buffers, with the backward written out:
+
+  * RMSNorm (with the residual addition before it), rotary embedding, SwiGLU and cross entropy are one kernel each way
+    (src/contrib/train_ops.cu) in place of chains of framework operations;
+  * wq | wk | wv and w_gate | w_up lie next to each other in the flat buffer and are one matrix each;
+  * weight gradients are written where the reduce-scatter reads them, and the recomputation leaves out the last product,
+    whose result no gradient needs.
+
+Between kernels everything is bf16 as before; sums, exponentials and rotations are held in fp32 and rounded once.
+"""
+import ctypes
+
+import torch
+import torch.nn.functional as F
+
+from .. import _lib
+from . import llama as M
+
+_P, _I = ctypes.c_void_p, ctypes.c_int
+_ENTRIES = {
+    "b200RmsNorm": [_P] * 6 + [_I, _I, ctypes.c_float, _P],
+    "b200RmsNormBackward": [_P] * 8 + [_I, _I, _P],
+    "b200RmsNormBackwardCtas": [_I],
+    "b200Rope": [_P] * 3 + [_I] * 5 + [_P],
+    "b200RopeBackward": [_P] * 7 + [_I] * 5 + [_P],
+    "b200SwiGlu": [_P] * 2 + [_I, _I, _P],
+    "b200SwiGluBackward": [_P] * 2 + [_I, _I, _P],
+    "b200CrossEntropy": [_P] * 5 + [_I, _I, _P],
+}
+
+
+def applies(cfg, tokens, targets):
+    """Whether a step on a GPU takes this path: shapes that the kernels' 16-byte accesses fit, and no mode of the framework that
+    looks into, or changes, the single operations. Everything else goes through `llama` and autograd."""
+    h, d = cfg.hidden, cfg.head_dim
+    return (h % 8 == 0 and h <= 16384 and d > 0 and d % 16 == 0 and d * cfg.heads == h and cfg.heads % cfg.kv_heads == 0 and cfg.ffn % 8 == 0 and
+            cfg.vocab % 8 == 0 and tokens.dim() == 2 and tokens.numel() > 0 and targets.dtype == torch.int64 and targets.numel() == tokens.numel() and
+            torch.is_grad_enabled() and not torch.is_anomaly_enabled() and not torch.is_autocast_enabled("cuda"))
+
+
+class FusedUnits:
+    """The units of one configuration; `lib` is this package's library."""
+
+    def __init__(self, cfg, lib):
+        self.cfg, self.lib = cfg, lib
+        self._call = {}
+        for name, types in _ENTRIES.items():
+            fn = getattr(lib, name)
+            fn.argtypes = types
+            fn.restype = ctypes.c_int
+            self._call[name] = fn
+
+    def _run(self, name, *args):
+        rc = self._call[name](*args, torch.cuda.current_stream().cuda_stream)
+        if rc:
+            _lib.check(rc, name, self.lib)
+
+    # ------------------------------------------------------------------ kernels
+    def norm(self, x, gain, add=None, need_rstd=False):
+        """(x + add, its RMSNorm, 1 / rms per row or None)."""
+        h = torch.empty_like(x)
+        total = x if add is None else torch.empty_like(x)
+        rstd = torch.empty(x.shape[0], dtype=torch.float32, device=x.device) if need_rstd else None
+        self._run("b200RmsNorm", x.data_ptr(), None if add is None else add.data_ptr(), gain.data_ptr(), total.data_ptr(), h.data_ptr(),
+                  rstd.data_ptr() if need_rstd else None, x.shape[0], x.shape[1], self.cfg.eps)
+        return total, h, rstd
+
+    def norm_backward(self, x, gain, rstd, dh, res, dgain):
+        """Gradient of x (plus `res`); the gain's goes into dgain."""
+        rows, hidden = x.shape
+        dx = torch.empty_like(x)
+        partial = torch.empty(self._call["b200RmsNormBackwardCtas"](rows), hidden, dtype=torch.float32, device=x.device)
+        self._run("b200RmsNormBackward", x.data_ptr(), gain.data_ptr(), rstd.data_ptr(), dh.data_ptr(), None if res is None else res.data_ptr(),
+                  dx.data_ptr(), dgain.data_ptr(), partial.data_ptr(), rows, hidden)
+        return dx
+
+    def rope(self, qkv, rope, seq):
+        c = self.cfg
+        self._run("b200Rope", qkv.data_ptr(), rope[0].data_ptr(), rope[1].data_ptr(), qkv.shape[0], seq, c.heads, c.kv_heads, c.head_dim)
+
+    def rope_backward(self, dq, dk, dv, rope, tokens, seq):
+        """[tokens, (heads + 2 kv_heads) * head_dim] from the gradients [B, heads, S, head_dim] of attention's inputs."""
+        c = self.cfg
+        out = torch.empty(tokens, (c.heads + 2 * c.kv_heads) * c.head_dim, dtype=dq.dtype, device=dq.device)
+        parts = [t if t.stride(3) == 1 and not any(s % 8 for s in t.stride()[:3]) and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+                 for t in (dq, dk, dv)]
+        strides = (ctypes.c_longlong * 9)(*[s for t in parts for s in t.stride()[:3]])
+        self._run("b200RopeBackward", *[t.data_ptr() for t in parts], strides, out.data_ptr(), rope[0].data_ptr(), rope[1].data_ptr(),
+                  tokens, seq, c.heads, c.kv_heads, c.head_dim)
+        return out
+
+    def swiglu(self, gu):
+        act = torch.empty(gu.shape[0], gu.shape[1] // 2, dtype=gu.dtype, device=gu.device)
+        self._run("b200SwiGlu", gu.data_ptr(), act.data_ptr(), act.shape[0], act.shape[1])
+        return act
+
+    def swiglu_backward(self, gu, dact):
+        """In place: gu becomes the gradients of gate and up, dact becomes silu(gate) * up."""
+        self._run("b200SwiGluBackward", gu.data_ptr(), dact.data_ptr(), dact.shape[0], dact.shape[1])
+
+    def cross_entropy(self, logits, targets):
+        """Mean loss; logits become their gradient."""
+        rows, vocab = logits.shape
+        loss = torch.empty((), dtype=torch.float32, device=logits.device)
+        work = torch.empty(rows + 1, dtype=torch.float32, device=logits.device)
+        ok = torch.empty((), dtype=torch.bool, device=logits.device)
+        self._run("b200CrossEntropy", logits.data_ptr(), targets.data_ptr(), loss.data_ptr(), work.data_ptr(), ok.data_ptr(), rows, vocab)
+        torch._assert_async(ok, "a target is no class of the vocabulary")
+        return loss
+
+    # ------------------------------------------------------------------ units
+    def _layer_views(self, flat):
+        c = self.cfg
+        h, qkv, f = c.hidden, (c.heads + 2 * c.kv_heads) * c.head_dim, c.ffn
+        return M.views(flat, [("norm1", (h,)), ("wqkv", (qkv, h)), ("wo", (h, h)), ("norm2", (h,)), ("w_gu", (2 * f, h)), ("w_down", (h, f))])
+
+    def _up_to_attention(self, x, p, rope, shape, backward):
+        """(norm1's output and 1 / rms, q, k, v as attention takes them, its output [B, heads, S, head_dim])."""
+        c, (B, S) = self.cfg, shape
+        _, h, rstd = self.norm(x, p["norm1"], need_rstd=backward)
+        qkv = torch.mm(h, p["wqkv"].t())
+        self.rope(qkv, rope, S)
+        q, k, v = (t.transpose(1, 2) for t in qkv.view(B, S, c.heads + 2 * c.kv_heads, c.head_dim).split((c.heads, c.kv_heads, c.kv_heads), dim=2))
+        if backward:
+            q, k, v = (t.detach().requires_grad_(True) for t in (q, k, v))
+        return h, rstd, (q, k, v), F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
+
+    def layer(self, x, flat, rope, shape):
+        """x [B * S, hidden] -> [B * S, hidden]; shape = (B, S)."""
+        p = self._layer_views(flat)
+        _, _, _, a = self._up_to_attention(x, p, rope, shape, False)
+        y, h, _ = self.norm(x, p["norm2"], add=torch.mm(a.transpose(1, 2).reshape(x.shape), p["wo"].t()))
+        return y.addmm_(self.swiglu(torch.mm(h, p["w_gu"].t())), p["w_down"].t())
+
+    def layer_backward(self, x, flat, gflat, rope, shape, gy):
+        """Gradient of the layer's input; the weights' gradients go into gflat (laid out like flat)."""
+        p, g = self._layer_views(flat), self._layer_views(gflat)
+        h1, rstd1, qkv, a = self._up_to_attention(x, p, rope, shape, True)
+        o = a.detach().transpose(1, 2).reshape(x.shape)
+        x2, h2, rstd2 = self.norm(x, p["norm2"], add=torch.mm(o, p["wo"].t()), need_rstd=True)
+        gu = torch.mm(h2, p["w_gu"].t())
+        act = torch.mm(gy, p["w_down"])
+        self.swiglu_backward(gu, act)
+        torch.mm(gy.t(), act, out=g["w_down"])
+        del act
+        dh = torch.mm(gu, p["w_gu"])
+        torch.mm(gu.t(), h2, out=g["w_gu"])
+        del gu, h2
+        g2 = self.norm_backward(x2, p["norm2"], rstd2, dh, gy, g["norm2"])
+        torch.mm(g2.t(), o, out=g["wo"])
+        do = torch.mm(g2, p["wo"]).view(shape[0], shape[1], self.cfg.heads, self.cfg.head_dim).transpose(1, 2)
+        dqkv = self.rope_backward(*torch.autograd.grad(a, qkv, do), rope, x.shape[0], shape[1])
+        del a, qkv, o, do
+        dh = torch.mm(dqkv, p["wqkv"])
+        torch.mm(dqkv.t(), h1, out=g["wqkv"])
+        return self.norm_backward(x, p["norm1"], rstd1, dh, g2, g["norm1"])
+
+    def head(self, x, flat, gflat, targets):
+        """(mean loss, gradient of the hidden states); the weights' gradients go into gflat."""
+        shapes = M.head_shapes(self.cfg)
+        p, g = M.views(flat, shapes), M.views(gflat, shapes)
+        _, h, rstd = self.norm(x, p["norm"], need_rstd=True)
+        logits = torch.mm(h, p["out"].t())
+        loss = self.cross_entropy(logits, targets)
+        dh = torch.mm(logits, p["out"])
+        torch.mm(logits.t(), h, out=g["out"])
+        return loss, self.norm_backward(x, p["norm"], rstd, dh, None, g["norm"])

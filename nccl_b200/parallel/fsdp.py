@@ -24,6 +24,7 @@ import torch
 from .. import _lib
 from ..core import mem_alloc, mem_free
 from ..models import llama as M
+from ..models import llama_fused
 
 
 def _align(n, a):
@@ -48,6 +49,7 @@ class FSDPEngine:
         self.own = _lib.load()         # the optimizer kernel always comes from this package's library
         if self.cuda:
             self.own.b200FusedAdamW.argtypes = [ctypes.c_void_p] * 5 + [ctypes.c_size_t] + [ctypes.c_float] * 6 + [ctypes.c_int, ctypes.c_void_p]
+            self.fused = llama_fused.FusedUnits(cfg, self.own)
         specs = M.unit_specs(cfg)
         self.units = []
         gen = torch.Generator().manual_seed(seed)
@@ -173,17 +175,22 @@ class FSDPEngine:
         u.master.mul_(1 - self.lr * self.wd).addcdiv_(mhat, denom, value=-self.lr)
         u.param.copy_(u.master.to(torch.bfloat16))
 
-    def _write_grads(self, idx, gslot, grads):
+    def _grad_flat(self, idx, gslot):
+        """The unit's flat gradient buffer, once the reduce-scatter that read it last is through; its padding is zero."""
         u = self.units[idx]
         if self.cuda:
             torch.cuda.current_stream().wait_event(self.ev_grad_free[gslot])
         flat = self.ggrad[gslot]
+        if u.padded > u.numel:
+            flat[u.numel:u.padded].zero_()
+        return flat[:u.numel]
+
+    def _write_grads(self, idx, gslot, grads):
+        flat = self._grad_flat(idx, gslot)
         off = 0
         for g in grads:
             flat[off:off + g.numel()].copy_(g.reshape(-1))
             off += g.numel()
-        if u.padded > off:
-            flat[off:u.padded].zero_()
 
     # ------------------------------------------------------------------ one training step
     def step(self, tokens, targets):
@@ -210,6 +217,13 @@ class FSDPEngine:
                 return M.head_loss(x, vs, cfg, targets)
             return M.decoder_layer(x, vs, cfg, rope)
 
+        # shapes and modes that the row kernels fit: the layers and the head have their backward written out
+        fused = self.fused if self.cuda and llama_fused.applies(cfg, tokens, targets) else None
+        shape = tuple(tokens.shape)
+
+        def weights(idx, slot):
+            return self.gbuf[slot][:self.units[idx].numel]
+
         # forward (the head is differentiated at once: its recompute would be wasted work)
         self._gather(0, 0)
         x = None
@@ -218,31 +232,48 @@ class FSDPEngine:
             self._wait_gathered(idx % 2)
             saved[idx] = x
             with torch.no_grad():
-                x = run(idx, params(idx, idx % 2, False), x)
+                if fused and idx:
+                    x = fused.layer(x, weights(idx, idx % 2), rope, shape)
+                else:
+                    x = run(idx, params(idx, idx % 2, False), x)
+                    x = x.view(-1, cfg.hidden) if fused else x
             self._release(idx % 2)
         # head: forward + backward
         idx = U - 1
         slot = idx % 2
         self._wait_gathered(slot)
-        vs = params(idx, slot, True)
-        xin = x.detach().requires_grad_(True)
-        loss = run(idx, vs, xin)
-        names = [n for n, _ in self.units[idx].shapes]
-        grads = torch.autograd.grad(loss, [xin] + [vs[n] for n in names])
-        self._gather(idx - 1, (idx - 1) % 2)
-        self._release(slot)
-        self._write_grads(idx, idx % 2, grads[1:])
-        self._reduce_and_update(idx, idx % 2)
-        gx = grads[0]
-        del grads, vs, xin, x
+        if fused:
+            loss, gx = fused.head(x, weights(idx, slot), self._grad_flat(idx, slot), targets.reshape(-1).contiguous())
+            self._gather(idx - 1, (idx - 1) % 2)
+            self._release(slot)
+        else:
+            vs = params(idx, slot, True)
+            xin = x.detach().requires_grad_(True)
+            loss = run(idx, vs, xin)
+            names = [n for n, _ in self.units[idx].shapes]
+            grads = torch.autograd.grad(loss, [xin] + [vs[n] for n in names])
+            self._gather(idx - 1, (idx - 1) % 2)
+            self._release(slot)
+            self._write_grads(idx, slot, grads[1:])
+            gx = grads[0]
+            del grads, vs, xin
+        self._reduce_and_update(idx, slot)
+        del x
         # backward through the layers and the embedding
         for idx in range(U - 2, -1, -1):
             slot = idx % 2
             if idx - 1 >= 0:
                 self._gather(idx - 1, (idx - 1) % 2)
             self._wait_gathered(slot)
+            if fused and idx:
+                gx = fused.layer_backward(saved[idx], weights(idx, slot), self._grad_flat(idx, slot), rope, shape, gx)
+                self._release(slot)
+                self._reduce_and_update(idx, slot)
+                saved[idx] = None
+                continue
             vs = params(idx, slot, True)
             names = [n for n, _ in self.units[idx].shapes]
+            gx = gx.view(*shape, cfg.hidden) if fused else gx
             with torch.enable_grad():
                 if idx == 0:
                     out = run(idx, vs, None)

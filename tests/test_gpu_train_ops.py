@@ -1,0 +1,218 @@
+"""Row kernels of the training step (src/contrib/train_ops.cu) against the same formulas in 64 bits on the same bf16 inputs, and the
+units built from them against autograd.
+
+A result that is rounded once to bf16 is off by at most 2**-9 of its value; twice that is allowed, and for results that are
+sums an absolute part: 2**-20 of the sum of the magnitudes (fp32 sums of up to 16384 terms in a tree)."""
+import math
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from nccl_b200.models import llama as M  # noqa: E402
+from nccl_b200.models import llama_fused  # noqa: E402
+
+gpu = pytest.mark.gpu
+ROUND = 2.0 ** -8
+
+
+def _units(**kw):
+    from nccl_b200 import _lib
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    return llama_fused.FusedUnits(M.LlamaConfig(**kw), _lib.load())
+
+
+def _rand(*shape, seed, scale=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(*shape, device="cuda", generator=g) * scale).bfloat16()
+
+
+def _close(got, ref, spread=0.0):
+    err = (got.double() - ref).abs() - (ROUND * ref.abs() + 2.0 ** -20 * spread + 1e-30)
+    assert bool(torch.isfinite(got.double()).all()) and float(err.max()) <= 0, float(err.max())
+
+
+@gpu
+@pytest.mark.parametrize("rows,hidden", [(1, 8), (3, 264), (301, 512), (2, 4096), (5, 4104), (700, 8192), (3, 8200), (2, 16384)])
+@pytest.mark.parametrize("with_add", [False, True])
+def test_norm_both_ways(rows, hidden, with_add):
+    u = _units(eps=1e-5)
+    x, add, gain = _rand(rows, hidden, seed=1), _rand(rows, hidden, seed=2, scale=0.3), (1 + 0.1 * _rand(hidden, seed=3).float()).bfloat16()
+    dh, res, dgain = _rand(rows, hidden, seed=4), _rand(rows, hidden, seed=5), torch.empty(hidden, dtype=torch.bfloat16, device="cuda")
+    total, h, rstd = u.norm(x, gain, add=add if with_add else None, need_rstd=True)
+    if with_add:
+        assert torch.equal(total, x + add)
+    xd = total.double().requires_grad_(True)
+    gd = gain.double().requires_grad_(True)
+    ref = xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-5) * gd
+    _close(h, ref.detach(), spread=ref.detach().abs())
+    dx = u.norm_backward(total, gain, rstd, dh, res if with_add else None, dgain)
+    gx, gg = torch.autograd.grad(ref, (xd, gd), dh.double())
+    xn = (xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-5)).detach()
+    r = res.double() if with_add else torch.zeros_like(gx)
+    scale = torch.rsqrt(xd.detach().square().mean(-1, keepdim=True) + 1e-5)
+    dn = (dh.double() * gain.double())
+    _close(dx, gx + r, spread=r.abs() + scale * (dn.abs() + xn.abs() * (dn * xn).abs().mean(-1, keepdim=True)))
+    _close(dgain, gg, spread=(dh.double() * xn).abs().sum(0))
+
+
+@gpu
+@pytest.mark.parametrize("B,S,heads,kv,d", [(1, 1, 1, 1, 16), (2, 65, 4, 2, 64), (1, 7, 3, 1, 48), (2, 33, 16, 8, 128), (1, 5, 2, 2, 256)])
+def test_rope_both_ways(B, S, heads, kv, d):
+    u = _units(hidden=heads * d, heads=heads, kv_heads=kv)
+    rope = M.rope_tables(u.cfg, S, "cuda")
+    qkv = _rand(B * S, (heads + 2 * kv) * d, seed=1)
+    src = qkv.clone().view(B, S, heads + 2 * kv, d)
+    u.rope(qkv, rope, S)
+    out = qkv.view(B, S, heads + 2 * kv, d)
+    c, s = (t.double()[None, :, None, :] for t in rope)
+
+    def turned(x, sign):
+        a, b = x[..., :d // 2].double(), x[..., d // 2:].double()
+        return torch.cat([a * c - sign * b * s, b * c + sign * a * s], -1), torch.cat([(a * c).abs() + (b * s).abs(), (b * c).abs() + (a * s).abs()], -1)
+
+    assert torch.equal(out[:, :, heads + kv:], src[:, :, heads + kv:])
+    _close(out[:, :, :heads + kv], *turned(src[:, :, :heads + kv], 1))
+    # gradients as [B, heads, S, D] in memory, as [B, S, heads, D], and at an odd offset
+    grads = [_rand(B, n, S, d, seed=2 + i) for i, n in enumerate((heads, kv, kv))]
+    for form in ("heads", "tokens", "offset"):
+        if form == "tokens":
+            got = [t.transpose(1, 2).contiguous().transpose(1, 2) for t in grads]
+        elif form == "offset":
+            got = [torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t) for t in grads]
+        else:
+            got = grads
+        back = u.rope_backward(*got, rope, B * S, S).view(B, S, heads + 2 * kv, d)
+        for t, at in zip(grads[:2], (slice(0, heads), slice(heads, heads + kv))):
+            _close(back[:, :, at], *turned(t.transpose(1, 2), -1))
+        assert torch.equal(back[:, :, heads + kv:], grads[2].transpose(1, 2))
+
+
+@gpu
+@pytest.mark.parametrize("rows,ffn", [(1, 8), (3, 2040), (17, 2056), (260, 14336)])
+def test_swiglu_both_ways(rows, ffn):
+    u = _units()
+    gu = _rand(rows, 2 * ffn, seed=1, scale=4.0)
+    gu[0, :4] = torch.tensor([-80.0, 300.0, 0.0, -30.0], device="cuda")
+    gate, up = (t.double() for t in gu.split(ffn, 1))
+    sig = torch.sigmoid(gate)
+    act = u.swiglu(gu)
+    _close(act, gate * sig * up)
+    dact = _rand(rows, ffn, seed=2)
+    d = dact.double()
+    u.swiglu_backward(gu, dact)
+    assert torch.equal(dact, act)
+    dgate, dup = gu.split(ffn, 1)
+    _close(dgate, d * up * sig * (1 + gate * (1 - sig)), spread=(d * up).abs() * (1 + gate.abs()))
+    _close(dup, d * gate * sig)
+
+
+@gpu
+@pytest.mark.parametrize("rows,vocab", [(1, 8), (3, 264), (65, 1024), (130, 16384), (2, 128256)])
+def test_cross_entropy(rows, vocab):
+    u = _units()
+    logits = _rand(rows, vocab, seed=1, scale=5.0)
+    logits[0, 1:4] = -math.inf
+    targets = torch.randint(0, vocab, (rows,), generator=torch.Generator().manual_seed(1)).cuda()
+    targets[0] = vocab - 1
+    if rows > 2:
+        targets[rows // 2] = -100
+    x = logits.double().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(x, targets)
+    g, = torch.autograd.grad(ref, x)
+    loss = u.cross_entropy(logits, targets)
+    assert abs(float(loss) - float(ref)) <= 2e-6 * abs(float(ref)) + 1e-6
+    # the exponent, a difference of numbers up to about 50, is off by a few 2**-24 of that: 1e-5 of the softmax (at the target, where 1
+    # is taken off, of 1)
+    soft = torch.softmax(x.detach(), -1) / max(int((targets != -100).sum()), 1)
+    _close(logits, g, spread=2.0 ** 20 * 1e-5 * soft)
+
+
+@gpu
+def test_cross_entropy_without_a_row_that_counts():
+    u = _units()
+    logits = _rand(3, 64, seed=1)
+    loss = u.cross_entropy(logits, torch.full((3,), -100, device="cuda"))
+    assert math.isnan(float(loss)) and not logits.any()   # as the framework's own
+
+
+@gpu
+def test_cross_entropy_of_infinite_and_nan_logits():
+    u = _units()
+    logits = _rand(4, 64, seed=1)
+    logits[0], logits[1, 5], logits[2, 7] = -math.inf, math.inf, math.nan
+    targets = torch.tensor([0, 1, 2, 3], device="cuda")
+    x = logits.double().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(x, targets, reduction="none")
+    g, = torch.autograd.grad(ref.sum() / 4, x)
+    u.cross_entropy(logits, targets)
+    assert torch.equal(logits.isnan(), g.isnan())
+    _close(logits[3:], g[3:], spread=2.0 ** 20 * 1e-5)
+
+
+@gpu
+@pytest.mark.parametrize("B,S,hidden,heads,kv,ffn,vocab", [(1, 65, 128, 8, 2, 264, 512), (2, 130, 512, 4, 2, 1024, 1032), (1, 1, 64, 1, 1, 8, 8), (2, 257, 1024, 8, 8, 2816, 2048)])
+def test_units_are_as_close_to_64_bits_as_autograd_in_bf16(B, S, hidden, heads, kv, ffn, vocab):
+    u = _units(layers=1, hidden=hidden, heads=heads, kv_heads=kv, ffn=ffn, vocab=vocab)
+    cfg = u.cfg
+    rope = M.rope_tables(cfg, S, "cuda")
+    gen = torch.Generator().manual_seed(0)
+    layer, head = (M.init_flat(s, gen, std=0.05).cuda() for s in (M.layer_shapes(cfg), M.head_shapes(cfg)))
+    x, gy = _rand(B, S, hidden, seed=1), _rand(B, S, hidden, seed=2)
+    targets = torch.randint(0, vocab, (B, S), generator=gen).cuda()
+
+    def by_autograd(dtype):
+        xs, fl, fh = (t.to(dtype).requires_grad_(True) for t in (x, layer, head))
+        p = M.views(fl, M.layer_shapes(cfg))
+        if dtype == torch.float64:
+            def norm(v, gain):
+                return v * torch.rsqrt(v.square().mean(-1, keepdim=True) + cfg.eps) * gain
+            c, s = (t.double()[None, :, None, :] for t in rope)
+
+            def turn(v):
+                a, b = v.chunk(2, -1)
+                return torch.cat([a * c - b * s, b * c + a * s], -1)
+            h = norm(xs, p["norm1"])
+            q, k, v = ((h @ p[n].T).view(B, S, -1, cfg.head_dim) for n in ("wq", "wk", "wv"))
+            q, k, v = (t.transpose(1, 2) for t in (turn(q), turn(k).repeat_interleave(heads // kv, 2), v.repeat_interleave(heads // kv, 2)))
+            mask = torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1)
+            a = (q @ k.transpose(-1, -2) / math.sqrt(cfg.head_dim)).masked_fill(mask, -math.inf).softmax(-1) @ v
+            y = xs + a.transpose(1, 2).reshape(B, S, -1) @ p["wo"].T
+            h = norm(y, p["norm2"])
+            gate = h @ p["w_gate"].T
+            y = y + (gate * torch.sigmoid(gate) * (h @ p["w_up"].T)) @ p["w_down"].T
+            ph = M.views(fh, M.head_shapes(cfg))
+            loss = torch.nn.functional.cross_entropy((norm(xs, ph["norm"]) @ ph["out"].T).view(-1, vocab), targets.view(-1))
+        else:
+            y = M.decoder_layer(xs, p, cfg, rope)
+            loss = M.head_loss(xs, M.views(fh, M.head_shapes(cfg)), cfg, targets)
+        return [y.detach(), *torch.autograd.grad(y, (xs, fl), gy.to(dtype)), loss.detach(), *torch.autograd.grad(loss, (xs, fh))]
+
+    exact, general = by_autograd(torch.float64), by_autograd(torch.bfloat16)
+    glayer, ghead = torch.full_like(layer, 7.0), torch.full_like(head, 7.0)
+    flat = x.view(-1, hidden)
+    with torch.no_grad():
+        y = u.layer(flat, layer, rope, (B, S))
+    got = [y, u.layer_backward(flat, layer, glayer, rope, (B, S), gy.view(-1, hidden)), glayer]
+    loss, gx = u.head(flat, head, ghead, targets.view(-1))
+    got += [loss, gx, ghead]
+    for name, e, a, b in zip(("y", "dx", "dw", "loss", "head dx", "head dw"), exact, general, got):
+        scale = float(e.norm()) + 1e-30
+        old, new = float((a.double() - e).norm()) / scale, float((b.double().view(e.shape) - e).norm()) / scale
+        # the loss is one number, whose error is the luck of the logits' rounding: two roundings to bf16 at most
+        assert new <= (2 ** -8 if name == "loss" else 1.05 * old + 1e-5), (name, old, new)
+
+
+def test_what_stays_with_autograd():
+    tok = torch.zeros(2, 8, dtype=torch.int64)
+    good = dict(hidden=256, heads=4, kv_heads=2, ffn=512, vocab=1024)
+    assert llama_fused.applies(M.LlamaConfig(**good), tok, tok)
+    for change in ({"heads": 32}, {"hidden": 260}, {"ffn": 516}, {"vocab": 1001}, {"hidden": 32768}, {"kv_heads": 3}):
+        assert not llama_fused.applies(M.LlamaConfig(**{**good, **change}), tok, tok)
+    cfg = M.LlamaConfig(**good)
+    assert not llama_fused.applies(cfg, tok, tok[:1]) and not llama_fused.applies(cfg, tok, tok.int()) and not llama_fused.applies(cfg, tok[:, :0], tok[:, :0])
+    with torch.no_grad():
+        assert not llama_fused.applies(cfg, tok, tok)
+    with torch.autograd.detect_anomaly(check_nan=False):
+        assert not llama_fused.applies(cfg, tok, tok)
