@@ -35,26 +35,43 @@ namespace b200 {
 using namespace sm100;
 
 namespace {
-constexpr int BM = kTpBM, BN = kTpBN, BK = 128, STAGES = 4, UMMA_K = 32;
+constexpr int BM = kTpBM, BK = 128, UMMA_K = 32;
 constexpr int kThreads = 384, kEpiWarps = 8;
-constexpr uint32_t kStageABytes = BM * BK, kStageBBytes = BN * BK;
-constexpr uint32_t kStageBytes = kStageABytes + kStageBBytes;
-constexpr uint32_t kTmemCols = 512;
-constexpr size_t kEpiBufBytes = kEpiWarps * 4096;   // one 32 x 128-byte transpose buffer per epilogue warp
-constexpr size_t kSmemBytes = 1024 + (size_t)STAGES * kStageBytes + 256 + kEpiBufBytes;
-constexpr int kPrefetch = 1;   // K blocks of scale look-ahead: with more the accumulators spill
+constexpr uint32_t kTmemCols = 512, kAccCols = 256;   // two accumulators, at fixed columns
+constexpr size_t kEpiBufBytes = kEpiWarps * 4096;     // one 32 x 128-byte transpose buffer per epilogue warp
+constexpr size_t kRingBytes = 4 * (BM + 256) * BK;    // operand ring: as many stages as fit
+constexpr size_t kSmemBytes = 1024 + kRingBytes + 256 + kEpiBufBytes;
+constexpr uint32_t kChunkBytes = BM * 32 * 4;         // fp32 partial sums of 32 columns
+// partial sums of one owner's chunks from the other shares, for every width and cluster size
+constexpr bool exchangeFits() {
+  for (int w : kTpWidths)
+    for (int s = 2; s <= kTpMaxSplit; ++s)
+      if ((size_t)((w / 32 + s - 1) / s) * (s - 1) * kChunkBytes > kRingBytes) return false;
+  return true;
+}
+static_assert(exchangeFits(), "partial sums must fit the operand ring");
 // registers per thread: 168 at launch; the producer warpgroup keeps 56, the two epilogue warpgroups take 224
 constexpr int kRegsLaunch = 168, kRegsProducer = 56, kRegsEpilogue = 224;
 static_assert(128 * kRegsProducer + 256 * kRegsEpilogue <= kThreads * kRegsLaunch, "register shares exceed the launch");
+__device__ __forceinline__ void stSharedCluster16(uint32_t clusterAddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(clusterAddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 }  // namespace
 
 // FUSED: the modes with a collective. The plain form is compiled without what they keep in registers across the tile loop.
-template <bool FUSED>
+// BN: columns of a tile, a multiple of 32; the last tile of a row may hang over N (zeros from the tensor map, nothing stored).
+// SPLIT: one tile per cluster of a.splitK CTAs that share its K blocks (see the end of the kernel).
+template <bool FUSED, int BN, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ TpGemmArgs a) {
+  constexpr uint32_t kStageABytes = BM * BK, kStageBBytes = BN * BK, kStageBytes = kStageABytes + kStageBBytes;
+  constexpr int STAGES = kRingBytes / kStageBytes;
+  // chunks of 32 columns: the first warpgroup of the epilogue takes kChunks of them, the second as many or one fewer
+  constexpr int kAll = BN / 32, kChunks = (kAll + 1) / 2, kSets = kChunks % 2 ? 3 : 2;
+  static_assert(!(FUSED && (SPLIT || BN != kTpBN)), "the fused modes use whole tiles");
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
-  uint8_t* ctrl = smem + (size_t)STAGES * kStageBytes;
+  uint8_t* ctrl = smem + kRingBytes;
   uint64_t* fullBar = (uint64_t*)ctrl;
   uint64_t* emptyBar = fullBar + STAGES;
   uint64_t* accFull = emptyBar + STAGES;
@@ -67,7 +84,9 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   const int rank = a.rank, n = a.nRanks;
   const bool gather = FUSED && a.mode == TP_MODE_GATHER;
   const bool commCta = gather && (int)blockIdx.x >= a.gemmCtas;
-  const int kBlocks = a.K / BK;
+  const int share = SPLIT ? (int)clusterCtaRank() : 0, S = SPLIT ? a.splitK : 1;
+  const int kBegin = SPLIT ? a.K / BK * share / S : 0;                          // the host keeps S <= K blocks: never empty
+  const int kBlocks = (SPLIT ? a.K / BK * (share + 1) / S : a.K / BK) - kBegin;   // of this CTA
 
   CtaBarrier bar;
   bool ok = true;
@@ -83,7 +102,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int commIdx = blockIdx.x - a.gemmCtas, commN = gridDim.x - a.gemmCtas;
     constexpr int kPipeStages = 6;
     constexpr uint32_t kPipeChunk = 32768;
-    static_assert((size_t)kPipeStages * kPipeChunk <= (size_t)STAGES * kStageBytes, "copy ring must fit the operand ring");
+    static_assert((size_t)kPipeStages * kPipeChunk <= kRingBytes, "copy ring must fit the operand ring");
     uint64_t* pipeBars = fullBar;
     if (threadIdx.x == 0) {
       for (int s = 0; s < kPipeStages; ++s) mbarInit(smemAddr(&pipeBars[s]), 1);
@@ -148,9 +167,10 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   const uint32_t tmemBase = *tmemSlot;
   pdlEnter();   // the set-up above overlaps the end of the kernel before; operands and results are touched behind it
 
-  const int tilesN = a.N / BN;
+  const int tilesN = (a.N + BN - 1) / BN;
   const int nTiles = (a.M / BM) * tilesN;
-  const int gemmCtas = gather ? a.gemmCtas : gridDim.x;
+  const int gemmCtas = gather ? a.gemmCtas : gridDim.x / S;
+  const int tile0 = blockIdx.x / S;
   const uint32_t smemA0 = smemAddr(smem), smemB0 = smemA0 + STAGES * kStageABytes;
   auto fail = [&](uint32_t kind, uint32_t what) {
     *abortFlag = 1;
@@ -168,8 +188,8 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (warp == 0 && electOne()) {
       uint32_t kc = 0;
       uint32_t armed = 0, armedPhase = 0;   // per stage: a copy was issued, and for which phase of its barrier
-      for (int t = blockIdx.x; t < nTiles && !*abortFlag; t += gemmCtas) {
-        const TileCoord tc = tileOf(a, t);
+      for (int t = tile0; t < nTiles && !*abortFlag; t += gemmCtas) {
+        const TileCoord tc = tileOf(a, t, BM, BN);
         if (gather && tc.owner != rank) {
           const uint32_t* f = a.blockFlags + tc.mBlk;
           bool got = false;
@@ -188,8 +208,8 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           if (!mbarWait(smemAddr(&emptyBar[s]), ph ^ 1)) { fail(WAIT_TILE, 1000 + s); break; }
           const uint32_t fb = smemAddr(&fullBar[s]);
           mbarExpectTx(fb, kStageBytes);
-          tmaLoad2d(smemA0 + s * kStageABytes, &tmA, kb * BK, tc.mBlk * BM, fb);
-          tmaLoad2d(smemB0 + s * kStageBBytes, &tmB, kb * BK, tc.nBlk * BN, fb);
+          tmaLoad2d(smemA0 + s * kStageABytes, &tmA, (kBegin + kb) * BK, tc.mBlk * BM, fb);
+          tmaLoad2d(smemB0 + s * kStageBBytes, &tmB, (kBegin + kb) * BK, tc.nBlk * BN, fb);
           armed |= 1u << s;
           armedPhase = (armedPhase & ~(1u << s)) | (ph << s);
         }
@@ -202,7 +222,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     } else if (warp == 1 && electOne()) {
       const uint32_t idesc = umInstrE4m3(BM, BN);
       uint32_t kc = 0;
-      for (int t = blockIdx.x; t < nTiles && !*abortFlag; t += gemmCtas) {
+      for (int t = tile0; t < nTiles && !*abortFlag; t += gemmCtas) {
         bool bad = false;
         for (int kb = 0; kb < kBlocks; ++kb, ++kc) {
           const int buf = kc & 1;
@@ -212,7 +232,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           const uint32_t ph = (kc / STAGES) & 1;
           if (!mbarWait(smemAddr(&fullBar[s]), ph)) { fail(WAIT_TILE, 3000 + s); bad = true; break; }
           tcFenceAfter();
-          const uint32_t dT = tmemBase + buf * BN;
+          const uint32_t dT = tmemBase + buf * kAccCols;
           const uint32_t aAddr = smemA0 + s * kStageABytes, bAddr = smemB0 + s * kStageBBytes;
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k)
@@ -225,103 +245,94 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
   } else {
     regsTake<kRegsEpilogue>();
-    // ---- epilogue warps: TMEM lanes [32q, 32q+32), columns [128h, 128h+128)
+    // ---- epilogue warps: TMEM lanes [32q, 32q+32), columns [c0, c0 + 32 * mine) of the tile
     const int q = warp & 3;
     const int h = (warp - 4) >> 2;
+    const int c0 = h * kChunks * 32;
+    const bool full = h == 0 || kAll % 2 == 0;   // the last of kChunks chunks is this warpgroup's too
+    const int mine = full ? kChunks : kChunks - 1;
     const float* scaleA = gather ? (const float*)((const char*)a.peerA[rank] + a.scaleOffset) : a.scaleA;
     const int wBlocksN = a.N / 128;
     uint32_t kc = 0;
-    for (int t = blockIdx.x; t < nTiles && !*abortFlag; t += gemmCtas) {
-      const TileCoord tc = tileOf(a, t);
+    uint64_t acc[kChunks * 16];   // fp32 pairs
+    for (int t = tile0; t < nTiles && !*abortFlag; t += gemmCtas) {
+      const TileCoord tc = tileOf(a, t, BM, BN);
       const int row0 = tc.mBlk * BM + q * 32;
       const int row = row0 + lane;
-      const int wCol = tc.nBlk * 2 + h;
-      uint64_t acc[64];   // fp32 pairs
+      // W has a scale per 128 columns: within this warp's columns it changes once at most, and never where tiles and halves do not
+      // cross a multiple of 128. Columns behind N get the last block's (their sums are zero).
+      const int col = tc.nBlk * BN + c0;
+      const int wCol = min(col >> 7, wBlocksN - 1), wNext = min(wCol + 1, wBlocksN - 1);
+      constexpr bool kTwo = BN % 128 != 0;
+      const int turn = kTwo ? (128 - (col & 127)) / 32 : kChunks;   // first chunk that lies in the second block
 #pragma unroll
-      for (int j = 0; j < 64; ++j) acc[j] = 0;
-      // Scales of the next kPrefetch K blocks travel ahead of the accumulators that need them.
+      for (int j = 0; j < kChunks * 16; ++j) acc[j] = 0;
+      // The scales of the next K block travel ahead of the accumulator that needs them.
       // In GATHER mode the scales of remote rows land together with the rows: the flag the TMA
       // producer waited for covers them, and accFull orders this warp after the producer.
-      float sc[kPrefetch];
-#pragma unroll
-      for (int u = 0; u < kPrefetch; ++u) sc[u] = 0.0f;
       bool bad = false;
       // Rows gathered from a peer arrive during this kernel: their scales may be read only after
       // the tile's first accumulator is published (the producer saw the block's flag before it
       // issued the TMA loads that fed it), and never through the read-only cache path.
       const bool remoteRows = gather && tc.owner != rank;
-      auto scaleOf = [&](int kb) -> float {
-        const float* pa = scaleA + (size_t)kb * a.M + row;
-        const float sa = *(const volatile float*)pa;
-        return sa * *(const volatile float*)(a.scaleW + (size_t)kb * wBlocksN + wCol);
+      float nextA = 0.0f, nextW[2] = {0.0f, 0.0f};
+      auto fetchScales = [&](int kb) {
+        nextA = *(const volatile float*)(scaleA + (size_t)(kBegin + kb) * a.M + row);
+        const float* w = a.scaleW + (size_t)(kBegin + kb) * wBlocksN;
+        nextW[0] = *(const volatile float*)(w + wCol);
+        if (kTwo) nextW[1] = *(const volatile float*)(w + wNext);
       };
-      bool primed = false;
-      if (!remoteRows) {
+      if (!remoteRows) fetchScales(0);
+      // sets of 32 columns: one is fetched while the one before is multiplied, across K blocks too
+      uint32_t set[kSets][32];
 #pragma unroll
-        for (int u = 0; u < kPrefetch; ++u)
-          if (u < kBlocks) sc[u] = scaleOf(u);
-        primed = true;
-      }
-      // two sets of 32 columns: one is fetched while the other is multiplied, across K blocks too
-      uint32_t even[32], odd[32];
+      for (int j = 0; j < 32; ++j) set[(kChunks - 1) % kSets][j] = 0;
+      float s[2] = {0.0f, 0.0f};
+      auto madd = [&](int c, const uint32_t (&r)[32], float by) {
+        const uint64_t s2 = packF32x2(__float_as_uint(by), __float_as_uint(by));
 #pragma unroll
-      for (int j = 0; j < 32; ++j) odd[j] = 0;
-      float sPrev = 0.0f;
-      auto madd = [&](int first, const uint32_t (&r)[32], float s) {
-        const uint64_t s2 = packF32x2(__float_as_uint(s), __float_as_uint(s));
-#pragma unroll
-        for (int j = 0; j < 16; ++j) fmaF32x2(acc[first / 2 + j], packF32x2(r[2 * j], r[2 * j + 1]), s2);
+        for (int j = 0; j < 16; ++j) fmaF32x2(acc[c * 16 + j], packF32x2(r[2 * j], r[2 * j + 1]), s2);
       };
-      for (int kb0 = 0; kb0 < kBlocks && !bad; kb0 += kPrefetch) {
+      auto scaleFor = [&](int c) { return kTwo && c >= turn ? s[1] : s[0]; };
+      for (int kb = 0; kb < kBlocks; ++kb, ++kc) {
+        const int buf = kc & 1;
+        const uint32_t aph = (kc >> 1) & 1;
+        if (!mbarWait(smemAddr(&accFull[buf]), aph)) { if (lane == 0) fail(WAIT_TILE, 4000 + buf); bad = true; break; }
+        tcFenceAfter();
+        if (remoteRows && kb == 0) fetchScales(0);
+        const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * kAccCols + c0;
+        const float next0 = nextA * nextW[0], next1 = nextA * nextW[1];
+        if (kb + 1 < kBlocks) fetchScales(kb + 1);
+        tmemLd32(tBase, set[0]);
+        if (full) madd(kChunks - 1, set[(kChunks - 1) % kSets], scaleFor(kChunks - 1));   // the last columns of the block before this one
+        tmemLdWait32(set[0]);
+        s[0] = next0;
+        s[1] = next1;
 #pragma unroll
-        for (int u = 0; u < kPrefetch; ++u) {
-          const int kb = kb0 + u;
-          if (kb >= kBlocks || bad) continue;
-          const int buf = kc & 1;
-          const uint32_t aph = (kc >> 1) & 1;
-          if (!mbarWait(smemAddr(&accFull[buf]), aph)) { if (lane == 0) fail(WAIT_TILE, 4000 + buf); bad = true; continue; }
-          tcFenceAfter();
-          if (!primed) {
-#pragma unroll
-            for (int v = 0; v < kPrefetch; ++v)
-              if (v < kBlocks) sc[v] = scaleOf(v);
-            primed = true;
-          }
-          const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * BN + h * 128;
-          const float s = sc[u];
-          if (kb + kPrefetch < kBlocks) sc[u] = scaleOf(kb + kPrefetch);
-          tmemLd32(tBase, even);
-          madd(96, odd, sPrev);   // the last columns of the block before this one
-          tmemLdWait32(even);
-          tmemLd32(tBase + 32, odd);
-          madd(0, even, s);
-          tmemLdWait32(odd);
-          tmemLd32(tBase + 64, even);
-          madd(32, odd, s);
-          tmemLdWait32(even);
-          tmemLd32(tBase + 96, odd);
-          madd(64, even, s);
-          tmemLdWait32(odd);
-          tcFenceBefore();
-          __syncwarp();
-          if (lane == 0) mbarArrive(smemAddr(&accEmpty[buf]));
-          sPrev = s;
-          ++kc;
+        for (int c = 1; c < kChunks; ++c) {
+          if (c < kChunks - 1 || full) tmemLd32(tBase + c * 32, set[c % kSets]);
+          madd(c - 1, set[(c - 1) % kSets], scaleFor(c - 1));
+          tmemLdWait32(set[c % kSets]);
         }
+        tcFenceBefore();
+        __syncwarp();
+        if (lane == 0) mbarArrive(smemAddr(&accEmpty[buf]));
       }
       if (bad) break;
-      madd(96, odd, sPrev);
+      if (full) madd(kChunks - 1, set[(kChunks - 1) % kSets], scaleFor(kChunks - 1));
+      if (SPLIT) break;   // one tile, finished with the other shares below
       // final tile: bf16, transposed through shared memory so that every store instruction writes
-      // whole 128-byte row segments (see the bf16 kernel); REDUCE targets the owner's staging slot
+      // whole row segments of 128 bytes (see the bf16 kernel; 64 where the columns are no multiple of 64); REDUCE targets the
+      // owner's staging slot
       {
         __nv_bfloat16* dstBase;
         size_t ld;
         if (FUSED && a.mode == TP_MODE_REDUCE) {
           const int rowsPerRank = a.M / n;
-          dstBase = (__nv_bfloat16*)a.partial[tc.owner] + ((size_t)rank * rowsPerRank + (row0 - tc.owner * rowsPerRank)) * a.N + (size_t)tc.nBlk * BN + h * 128;
+          dstBase = (__nv_bfloat16*)a.partial[tc.owner] + ((size_t)rank * rowsPerRank + (row0 - tc.owner * rowsPerRank)) * a.N + (size_t)tc.nBlk * BN + c0;
           ld = (size_t)a.N;
         } else {
-          dstBase = (__nv_bfloat16*)a.C + (size_t)row0 * a.ldc + (size_t)tc.nBlk * BN + h * 128;
+          dstBase = (__nv_bfloat16*)a.C + (size_t)row0 * a.ldc + (size_t)tc.nBlk * BN + c0;
           ld = (size_t)a.ldc;
         }
         uint8_t* wbuf = epiBuf + (size_t)(warp - 4) * 4096;
@@ -329,25 +340,92 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           const __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float((uint32_t)acc[i]), __uint_as_float((uint32_t)(acc[i] >> 32)));
           return *(const uint32_t*)&p;
         };
+        constexpr int kSeg = kChunks % 2 || kAll % 2 ? 1 : 2, kParts = kSeg * 4;   // chunks, 16-byte parts of a row segment
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
+        for (int cc = 0; cc < kChunks; cc += kSeg) {
+          if (BN != kTpBN && (cc >= mine || col + cc * 32 >= a.N)) break;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int b0 = cc * 32 + j * 4;
+          for (int j = 0; j < kParts; ++j) {
+            const int b0 = cc * 16 + j * 4;
             const uint4 o = make_uint4(bf16Pair(b0), bf16Pair(b0 + 1), bf16Pair(b0 + 2), bf16Pair(b0 + 3));
-            *(uint4*)(wbuf + lane * 128 + ((j ^ (lane & 7)) * 16)) = o;
+            *(uint4*)(wbuf + lane * (kParts * 16) + ((j ^ (lane & (kParts - 1))) * 16)) = o;
           }
           __syncwarp();
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int rr = k * 4 + (lane >> 3), j = lane & 7;
-            const uint4 o = *(const uint4*)(wbuf + rr * 128 + ((j ^ (rr & 7)) * 16));
-            *(uint4*)((char*)(dstBase + (size_t)rr * ld) + cc * 128 + j * 16) = o;
+          for (int k = 0; k < kParts; ++k) {
+            const int rr = k * (32 / kParts) + lane / kParts, j = lane & (kParts - 1);
+            const uint4 o = *(const uint4*)(wbuf + rr * (kParts * 16) + ((j ^ (rr & (kParts - 1))) * 16));
+            *(uint4*)((char*)(dstBase + (size_t)rr * ld) + cc * 64 + j * 16) = o;
           }
           __syncwarp();
         }
       }
     }
+    if (SPLIT) {
+      // Every CTA holds the scaled fp32 sums of its share of the K blocks in registers. Chunk g of 32 columns belongs to CTA g % S: the
+      // others put their sums into its operand ring (free: all MMAs of the cluster are behind the first barrier), and the owner
+      // adds them in the order of the shares, rounds once and stores. The result does not depend on the schedule.
+      const int rowInTile = q * 32 + lane;
+      auto slotOf = [&](int g, int from, int owner) {
+        const int others = from < owner ? from : from - 1;
+        return (uint32_t)((g / S) * (S - 1) + others) * kChunkBytes + (uint32_t)rowInTile * 16;
+      };
+      __syncwarp();
+      clusterSync();
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c) {
+        const int g = h * kChunks + c, owner = g % S;
+        if (c >= mine || owner == share) continue;
+        const uint32_t dst = mapaShared(smemA0 + slotOf(g, share, owner), (uint32_t)owner);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          stSharedCluster16(dst + j * (BM * 16), (uint32_t)acc[c * 16 + 2 * j], (uint32_t)(acc[c * 16 + 2 * j] >> 32), (uint32_t)acc[c * 16 + 2 * j + 1],
+                            (uint32_t)(acc[c * 16 + 2 * j + 1] >> 32));
+      }
+      clusterSync();
+      const TileCoord tc = tileOf(a, tile0, BM, BN);
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c) {
+        const int g = h * kChunks + c, col = tc.nBlk * BN + g * 32;
+        if (c >= mine || g % S != share || col >= a.N) continue;
+        float sum[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) sum[j] = 0.0f;
+        for (int from = 0; from < S; ++from) {
+          if (from == share) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              sum[2 * j] += __uint_as_float((uint32_t)acc[c * 16 + j]);
+              sum[2 * j + 1] += __uint_as_float((uint32_t)(acc[c * 16 + j] >> 32));
+            }
+          } else {
+            const uint8_t* src = smem + slotOf(g, from, share);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float4 v = *(const float4*)(src + j * (BM * 16));
+              sum[4 * j] += v.x;
+              sum[4 * j + 1] += v.y;
+              sum[4 * j + 2] += v.z;
+              sum[4 * j + 3] += v.w;
+            }
+          }
+        }
+        __nv_bfloat16* out = (__nv_bfloat16*)a.C + (size_t)(tc.mBlk * BM + rowInTile) * a.ldc + col;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint4 o;
+          __nv_bfloat162* p = (__nv_bfloat162*)&o;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) p[k] = __floats2bfloat162_rn(sum[8 * j + 2 * k], sum[8 * j + 2 * k + 1]);
+          *(uint4*)(out + j * 8) = o;
+        }
+      }
+    }
+  }
+  if (SPLIT && warp < 4) {
+    __syncwarp();
+    clusterSync();
+    clusterSync();
   }
 
   tcFenceBefore();
@@ -482,7 +560,19 @@ __global__ void __launch_bounds__(256) tpQuantBlocksKernel(const __nv_bfloat16* 
   }
 }
 
-const void* tpGemmFp8KernelFn(bool fused) { return fused ? (const void*)tpGemmFp8Kernel<true> : (const void*)tpGemmFp8Kernel<false>; }
+template <bool SPLIT>
+static const void* plainFp8(int width) {
+  switch (width) {
+    case 128: return (const void*)tpGemmFp8Kernel<false, 128, SPLIT>;
+    case 160: return (const void*)tpGemmFp8Kernel<false, 160, SPLIT>;
+    case 192: return (const void*)tpGemmFp8Kernel<false, 192, SPLIT>;
+    case 224: return (const void*)tpGemmFp8Kernel<false, 224, SPLIT>;
+    default: return (const void*)tpGemmFp8Kernel<false, 256, SPLIT>;
+  }
+}
+const void* tpGemmFp8KernelFn(bool fused, int width, bool split) {
+  return fused ? (const void*)tpGemmFp8Kernel<true, kTpBN, false> : split ? plainFp8<true>(width) : plainFp8<false>(width);
+}
 const void* tpQuantRowsWideKernelFn() { return (const void*)tpQuantRowsWideKernel; }
 void tpQuantRowsWideGrid(int rows, int K, int* x, int* y) {
   *x = (rows + kQuantRows - 1) / kQuantRows;

@@ -14,6 +14,8 @@ using namespace b200;
 namespace b200 {
 B200_PARAM(TpCommCtas, "B200_TP_COMM_CTAS", 0, "CTAs that gather remote rows in all-gather -> GEMM (0: 4 for two ranks, 8 up to four, 16 beyond)")
 B200_PARAM(TpSplit, "B200_TP_SPLIT", 8, "Largest cluster of CTAs that shares the K dimension of a tile in plain bf16 GEMMs with few tiles (1: never, at most 8)")
+B200_PARAM(TpFp8Width, "B200_TP_FP8_WIDTH", 0, "Tile width of plain block-scaled fp8 GEMMs: 128, 160, 192, 224 or 256 (0: by shape)")
+B200_PARAM(TpFp8Split, "B200_TP_FP8_SPLIT", 0, "CTAs that share the K blocks of a tile in plain block-scaled fp8 GEMMs: 1 to 8 (0: by shape)")
 B200_PARAM(TpPair, "B200_TP_PAIR", 1, "bf16 GEMM on CTA pairs (256 x 256 tiles, tcgen05 cta_group::2) when the row count allows")
 }
 
@@ -183,13 +185,23 @@ static ncclResult_t launchGemm(ncclTpContext* tp, const void* A, const void* W, 
                   pair ? tpGemmPairSmemBytes() : tpGemmSmemBytes(), args, !fused, 1, stream);
 }
 
-static ncclResult_t launchGemmFp8(ncclTpContext* tp, const void* A, const void* W, TpGemmArgs* a, int grid, cudaStream_t stream) {
+static ncclResult_t launchGemmFp8(ncclTpContext* tp, const void* A, const void* W, TpGemmArgs* a, int grid, cudaStream_t stream, int width = 256) {
   CUtensorMap tmA, tmB;
   NCCLCHECK(makeMap(&tmA, A, a->M, a->K, 128, 1));
-  NCCLCHECK(makeMap(&tmB, W, a->N, a->K, 256, 1));
+  NCCLCHECK(makeMap(&tmB, W, a->N, a->K, width, 1));
   void* args[3] = {&tmA, &tmB, a};
   const bool fused = a->nRanks > 1 && a->mode != TP_MODE_STORE;
-  return launchTp(tp, tpGemmFp8KernelFn(fused), dim3(grid), tpGemmFp8Threads(), tpGemmFp8SmemBytes(), args, !fused, 1, stream);
+  return launchTp(tp, tpGemmFp8KernelFn(fused, width, a->splitK > 1), dim3(grid), tpGemmFp8Threads(), tpGemmFp8SmemBytes(), args, !fused, std::max(a->splitK, 1), stream);
+}
+
+// Tile width, CTAs that share the K blocks of a tile (1: none), and grid of a plain fp8 GEMM.
+static void planFp8(const ncclTpContext* tp, TpGemmArgs* a, int* width, int* grid) {
+  *width = 256;
+  for (int w : kTpWidths)
+    if (w == paramTpFp8Width()) *width = w;
+  a->splitK = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(paramTpFp8Split(), kTpMaxSplit), a->K / 128));
+  const int tiles = a->M / 128 * ((a->N + *width - 1) / *width);
+  *grid = a->splitK > 1 ? tiles * a->splitK : std::min(tp->smCount, tiles);
 }
 
 static ncclResult_t checkShapeFp8(int M, int N, int K, int n) {
@@ -234,8 +246,9 @@ ncclResult_t ncclTpGemmFp8(ncclTp_t tp, const void* A, const float* scaleA, cons
   a.rank = tp->comm->rank; a.nRanks = tp->comm->nRanks;
   a.scaleA = scaleA; a.scaleW = scaleW;
   fillSyncTp(tp->comm, &a.sync);
-  int tiles = (M / 128) * (N / 256);
-  return launchGemmFp8(tp, A, W, &a, std::min(tp->smCount, tiles), stream);
+  int width, grid;
+  planFp8(tp, &a, &width, &grid);
+  return launchGemmFp8(tp, A, W, &a, grid, stream, width);
 }
 
 ncclResult_t ncclTpGemmReduceScatterFp8(ncclTp_t tp, const void* A, const float* scaleA, const void* W, const float* scaleW, void* out, int M, int N, int K,
@@ -332,7 +345,10 @@ ncclResult_t ncclTpCreate(ncclComm_t comm, size_t maxRows, size_t maxCols, ncclT
   // function attributes are per device: set them here, with this context's device current, not once per process
   CUDACHECK(cudaFuncSetAttribute(tpGemmKernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmSmemBytes()));
   CUDACHECK(cudaFuncSetAttribute(tpGemmSplitKernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmSplitSmemBytes()));
-  for (bool fused : {false, true}) CUDACHECK(cudaFuncSetAttribute(tpGemmFp8KernelFn(fused), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmFp8SmemBytes()));
+  CUDACHECK(cudaFuncSetAttribute(tpGemmFp8KernelFn(true, 256, false), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmFp8SmemBytes()));
+  for (int width : kTpWidths)
+    for (bool split : {false, true})
+      CUDACHECK(cudaFuncSetAttribute(tpGemmFp8KernelFn(false, width, split), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmFp8SmemBytes()));
   {
     // how many clusters of two CTAs of the pair kernel the device can hold at once: the grid never exceeds it,
     // because its CTAs wait for one another (comm CTAs, cross-GPU barriers)

@@ -29,7 +29,8 @@ struct TpGemmArgs {
   size_t scaleOffset;             // GATHER, fp8: byte offset of the scales inside every rank's activation window
 };
 
-constexpr int kTpMaxSplit = 8;     // largest cluster of the split kernel
+constexpr int kTpMaxSplit = 8;     // largest cluster of CTAs that share the K blocks of a tile
+constexpr int kTpWidths[] = {256, 224, 192, 160, 128};   // tile widths of plain GEMMs; the fused modes use the first
 
 #if defined(__CUDACC__)
 constexpr int kTpBM = 128, kTpBN = 256;
@@ -51,9 +52,10 @@ __device__ __forceinline__ void panelOrder(int j, int rows, int tilesN, int* r, 
 // Tile t of this CTA's walk: the whole output for plain GEMMs; owner by owner for the fused modes
 // (REDUCE starts with the next rank so that every step each GPU receives from one peer; GATHER
 // starts with the rows that are already local), panel order inside each block of rows.
-// `bm` is the tile height in rows (128 for one CTA, 256 for a CTA pair); mBlk counts tiles of that height.
-__device__ __forceinline__ TileCoord tileOf(const TpGemmArgs& a, int t, int bm = kTpBM) {
-  const int tilesN = a.N / kTpBN;
+// `bm` is the tile height in rows (128 for one CTA, 256 for a CTA pair), `bn` its width; mBlk and nBlk count tiles of that size. Only
+// plain GEMMs have tiles narrower than kTpBN.
+__device__ __forceinline__ TileCoord tileOf(const TpGemmArgs& a, int t, int bm = kTpBM, int bn = kTpBN) {
+  const int tilesN = (a.N + bn - 1) / bn;
   TileCoord c;
   if (a.mode == TP_MODE_STORE || a.nRanks == 1) {
     panelOrder(t, (a.M + bm - 1) / bm, tilesN, &c.mBlk, &c.nBlk);
@@ -84,7 +86,9 @@ const void* tpGemmPairKernelFn();      // CTA-pair variant (cluster of two, 256 
 const void* tpGemmSplitKernelFn();     // plain C = A * W^T, one 128 x 256 tile per cluster of splitK CTAs
 size_t tpGemmSplitSmemBytes();
 int tpGemmSplitThreads();
-const void* tpGemmFp8KernelFn(bool fused);   // fused: REDUCE and GATHER with more than one rank
+// fused: REDUCE and GATHER with more than one rank, tiles of 128 x 256. Others: tiles of 128 x width (one of kTpWidths); split: one tile
+// per cluster of splitK CTAs that share its K blocks
+const void* tpGemmFp8KernelFn(bool fused, int width, bool split);
 const void* tpQuantRowsWideKernelFn(); // as the next one, for 16-byte aligned x and q, on the grid below
 void tpQuantRowsWideGrid(int rows, int K, int* x, int* y);
 const void* tpQuantRowsKernelFn();     // (const bf16* x, uint8_t* q, float* scales, int rows, int K): 1 x 128 blocks, scales [K/128][rows]
