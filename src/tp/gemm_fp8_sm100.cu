@@ -8,10 +8,14 @@
 //   level 2  the epilogue warps read each finished block from TMEM (tcgen05.ld), multiply by
 //            scaleA[row] * scaleW[block] and add into fp32 registers, while the tensor cores
 //            already work on the next K block in the other accumulator.
-// 1920 x 4096 x 7168: 107 -> 78 us, 4096 x 9472 x 4096: 262 -> 198 us (1.21 -> 1.61 PFLOP/s) against a level 2 that waited for each
-// 32 columns in turn. What bounds the kernel is the round trip of an accumulator (MMAs, level 2, release) and behind that the operand traffic
+// 1920 x 4096 x 7168 67 us, 8192 x 8192 x 7168 496 us (1.94 PFLOP/s), against 107 us and 1.2 PFLOP/s of a level 2 that waited for each 32
+// columns in turn. What bounds the kernel is the round trip of an accumulator (MMAs, level 2, release) and behind that the operand traffic
 // from L2 (48 KiB per K block and SM). So level 2 is a pipeline of its own: 32 columns are fetched while the 32 before them are
-// multiplied (packed fp32 pairs), across K blocks too, and an accumulator is given back as soon as it is read.
+// multiplied (packed fp32 pairs), across K blocks too, an accumulator is given back as soon as it is read, and the two scales of the
+// next K block are multiplied only when it is there (as one product fetched ahead they held up the block before: 78 us for the first
+// shape).
+// Plain calls with few tiles take tiles of 128 columns, or a cluster of CTAs to a tile, each with its share of the K blocks, so that
+// more SMs work (the rule and its figures are in tp.cc).
 // Persistent CTAs of three warpgroups: warp 0 TMA producer (128x128-byte A tiles, 256x128-byte W tiles,
 // 128-byte swizzle, 4-stage ring), warp 1 MMA issuer, warps 4-11 epilogue (each warp owns 32 TMEM
 // lanes and one 128-column half of the tile: 128 fp32 accumulators per thread, for which the first warpgroup hands over its
@@ -44,7 +48,7 @@ constexpr size_t kSmemBytes = 1024 + kRingBytes + 256 + kEpiBufBytes;
 constexpr uint32_t kChunkBytes = BM * 32 * 4;         // fp32 partial sums of 32 columns
 // partial sums of one owner's chunks from the other shares, for every width and cluster size
 constexpr bool exchangeFits() {
-  for (int w : kTpWidths)
+  for (int w : {128, 256})
     for (int s = 2; s <= kTpMaxSplit; ++s)
       if ((size_t)((w / 32 + s - 1) / s) * (s - 1) * kChunkBytes > kRingBytes) return false;
   return true;
@@ -59,15 +63,15 @@ __device__ __forceinline__ void stSharedCluster16(uint32_t clusterAddr, uint32_t
 }  // namespace
 
 // FUSED: the modes with a collective. The plain form is compiled without what they keep in registers across the tile loop.
-// BN: columns of a tile, a multiple of 32; the last tile of a row may hang over N (zeros from the tensor map, nothing stored).
+// BN: columns of a tile, 256 or (plain calls with few tiles) 128.
 // SPLIT: one tile per cluster of a.splitK CTAs that share its K blocks (see the end of the kernel).
 template <bool FUSED, int BN, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ TpGemmArgs a) {
   constexpr uint32_t kStageABytes = BM * BK, kStageBBytes = BN * BK, kStageBytes = kStageABytes + kStageBBytes;
   constexpr int STAGES = kRingBytes / kStageBytes;
-  // chunks of 32 columns: the first warpgroup of the epilogue takes kChunks of them, the second as many or one fewer
-  constexpr int kAll = BN / 32, kChunks = (kAll + 1) / 2, kSets = kChunks % 2 ? 3 : 2;
+  constexpr int kHalf = BN / 2, kChunks = kHalf / 32;   // columns and chunks of 32 columns of an epilogue warp
+  static_assert(BN == 256 || BN == 128, "a warp's columns lie in one block of W's scales");
   static_assert(!(FUSED && (SPLIT || BN != kTpBN)), "the fused modes use whole tiles");
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
@@ -167,7 +171,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   const uint32_t tmemBase = *tmemSlot;
   pdlEnter();   // the set-up above overlaps the end of the kernel before; operands and results are touched behind it
 
-  const int tilesN = (a.N + BN - 1) / BN;
+  const int tilesN = a.N / BN;
   const int nTiles = (a.M / BM) * tilesN;
   const int gemmCtas = gather ? a.gemmCtas : gridDim.x / S;
   const int tile0 = blockIdx.x / S;
@@ -245,12 +249,10 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
   } else {
     regsTake<kRegsEpilogue>();
-    // ---- epilogue warps: TMEM lanes [32q, 32q+32), columns [c0, c0 + 32 * mine) of the tile
+    // ---- epilogue warps: TMEM lanes [32q, 32q+32), columns [kHalf * h, kHalf * (h + 1))
     const int q = warp & 3;
     const int h = (warp - 4) >> 2;
-    const int c0 = h * kChunks * 32;
-    const bool full = h == 0 || kAll % 2 == 0;   // the last of kChunks chunks is this warpgroup's too
-    const int mine = full ? kChunks : kChunks - 1;
+    const int c0 = h * kHalf;
     const float* scaleA = gather ? (const float*)((const char*)a.peerA[rank] + a.scaleOffset) : a.scaleA;
     const int wBlocksN = a.N / 128;
     uint32_t kc = 0;
@@ -259,12 +261,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       const TileCoord tc = tileOf(a, t, BM, BN);
       const int row0 = tc.mBlk * BM + q * 32;
       const int row = row0 + lane;
-      // W has a scale per 128 columns: within this warp's columns it changes once at most, and never where tiles and halves do not
-      // cross a multiple of 128. Columns behind N get the last block's (their sums are zero).
-      const int col = tc.nBlk * BN + c0;
-      const int wCol = min(col >> 7, wBlocksN - 1), wNext = min(wCol + 1, wBlocksN - 1);
-      constexpr bool kTwo = BN % 128 != 0;
-      const int turn = kTwo ? (128 - (col & 127)) / 32 : kChunks;   // first chunk that lies in the second block
+      const int wCol = (tc.nBlk * BN + c0) / 128;
 #pragma unroll
       for (int j = 0; j < kChunks * 16; ++j) acc[j] = 0;
       // The scales of the next K block travel ahead of the accumulator that needs them.
@@ -275,25 +272,22 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       // the tile's first accumulator is published (the producer saw the block's flag before it
       // issued the TMA loads that fed it), and never through the read-only cache path.
       const bool remoteRows = gather && tc.owner != rank;
-      float nextA = 0.0f, nextW[2] = {0.0f, 0.0f};
+      float nextA = 0.0f, nextW = 0.0f;
       auto fetchScales = [&](int kb) {
         nextA = *(const volatile float*)(scaleA + (size_t)(kBegin + kb) * a.M + row);
-        const float* w = a.scaleW + (size_t)(kBegin + kb) * wBlocksN;
-        nextW[0] = *(const volatile float*)(w + wCol);
-        if (kTwo) nextW[1] = *(const volatile float*)(w + wNext);
+        nextW = *(const volatile float*)(a.scaleW + (size_t)(kBegin + kb) * wBlocksN + wCol);
       };
       if (!remoteRows) fetchScales(0);
       // sets of 32 columns: one is fetched while the one before is multiplied, across K blocks too
-      uint32_t set[kSets][32];
+      uint32_t set[2][32];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) set[(kChunks - 1) % kSets][j] = 0;
-      float s[2] = {0.0f, 0.0f};
+      for (int j = 0; j < 32; ++j) set[1][j] = 0;
+      float s = 0.0f;
       auto madd = [&](int c, const uint32_t (&r)[32], float by) {
         const uint64_t s2 = packF32x2(__float_as_uint(by), __float_as_uint(by));
 #pragma unroll
         for (int j = 0; j < 16; ++j) fmaF32x2(acc[c * 16 + j], packF32x2(r[2 * j], r[2 * j + 1]), s2);
       };
-      auto scaleFor = [&](int c) { return kTwo && c >= turn ? s[1] : s[0]; };
       for (int kb = 0; kb < kBlocks; ++kb, ++kc) {
         const int buf = kc & 1;
         const uint32_t aph = (kc >> 1) & 1;
@@ -301,29 +295,27 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         tcFenceAfter();
         if (remoteRows && kb == 0) fetchScales(0);
         const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * kAccCols + c0;
-        const float next0 = nextA * nextW[0], next1 = nextA * nextW[1];
+        const float next = nextA * nextW;
         if (kb + 1 < kBlocks) fetchScales(kb + 1);
         tmemLd32(tBase, set[0]);
-        if (full) madd(kChunks - 1, set[(kChunks - 1) % kSets], scaleFor(kChunks - 1));   // the last columns of the block before this one
+        madd(kChunks - 1, set[1], s);   // the last columns of the block before this one
         tmemLdWait32(set[0]);
-        s[0] = next0;
-        s[1] = next1;
+        s = next;
 #pragma unroll
         for (int c = 1; c < kChunks; ++c) {
-          if (c < kChunks - 1 || full) tmemLd32(tBase + c * 32, set[c % kSets]);
-          madd(c - 1, set[(c - 1) % kSets], scaleFor(c - 1));
-          tmemLdWait32(set[c % kSets]);
+          tmemLd32(tBase + c * 32, set[c & 1]);
+          madd(c - 1, set[(c - 1) & 1], s);
+          tmemLdWait32(set[c & 1]);
         }
         tcFenceBefore();
         __syncwarp();
         if (lane == 0) mbarArrive(smemAddr(&accEmpty[buf]));
       }
       if (bad) break;
-      if (full) madd(kChunks - 1, set[(kChunks - 1) % kSets], scaleFor(kChunks - 1));
+      madd(kChunks - 1, set[1], s);
       if (SPLIT) break;   // one tile, finished with the other shares below
       // final tile: bf16, transposed through shared memory so that every store instruction writes
-      // whole row segments of 128 bytes (see the bf16 kernel; 64 where the columns are no multiple of 64); REDUCE targets the
-      // owner's staging slot
+      // whole 128-byte row segments (see the bf16 kernel); REDUCE targets the owner's staging slot
       {
         __nv_bfloat16* dstBase;
         size_t ld;
@@ -340,22 +332,20 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           const __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float((uint32_t)acc[i]), __uint_as_float((uint32_t)(acc[i] >> 32)));
           return *(const uint32_t*)&p;
         };
-        constexpr int kSeg = kChunks % 2 || kAll % 2 ? 1 : 2, kParts = kSeg * 4;   // chunks, 16-byte parts of a row segment
 #pragma unroll
-        for (int cc = 0; cc < kChunks; cc += kSeg) {
-          if (BN != kTpBN && (cc >= mine || col + cc * 32 >= a.N)) break;
+        for (int cc = 0; cc < kChunks / 2; ++cc) {
 #pragma unroll
-          for (int j = 0; j < kParts; ++j) {
-            const int b0 = cc * 16 + j * 4;
+          for (int j = 0; j < 8; ++j) {
+            const int b0 = cc * 32 + j * 4;
             const uint4 o = make_uint4(bf16Pair(b0), bf16Pair(b0 + 1), bf16Pair(b0 + 2), bf16Pair(b0 + 3));
-            *(uint4*)(wbuf + lane * (kParts * 16) + ((j ^ (lane & (kParts - 1))) * 16)) = o;
+            *(uint4*)(wbuf + lane * 128 + ((j ^ (lane & 7)) * 16)) = o;
           }
           __syncwarp();
 #pragma unroll
-          for (int k = 0; k < kParts; ++k) {
-            const int rr = k * (32 / kParts) + lane / kParts, j = lane & (kParts - 1);
-            const uint4 o = *(const uint4*)(wbuf + rr * (kParts * 16) + ((j ^ (rr & (kParts - 1))) * 16));
-            *(uint4*)((char*)(dstBase + (size_t)rr * ld) + cc * 64 + j * 16) = o;
+          for (int k = 0; k < 8; ++k) {
+            const int rr = k * 4 + (lane >> 3), j = lane & 7;
+            const uint4 o = *(const uint4*)(wbuf + rr * 128 + ((j ^ (rr & 7)) * 16));
+            *(uint4*)((char*)(dstBase + (size_t)rr * ld) + cc * 128 + j * 16) = o;
           }
           __syncwarp();
         }
@@ -375,7 +365,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
       for (int c = 0; c < kChunks; ++c) {
         const int g = h * kChunks + c, owner = g % S;
-        if (c >= mine || owner == share) continue;
+        if (owner == share) continue;
         const uint32_t dst = mapaShared(smemA0 + slotOf(g, share, owner), (uint32_t)owner);
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -387,7 +377,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll
       for (int c = 0; c < kChunks; ++c) {
         const int g = h * kChunks + c, col = tc.nBlk * BN + g * 32;
-        if (c >= mine || g % S != share || col >= a.N) continue;
+        if (g % S != share) continue;
         float sum[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) sum[j] = 0.0f;
@@ -560,18 +550,10 @@ __global__ void __launch_bounds__(256) tpQuantBlocksKernel(const __nv_bfloat16* 
   }
 }
 
-template <bool SPLIT>
-static const void* plainFp8(int width) {
-  switch (width) {
-    case 128: return (const void*)tpGemmFp8Kernel<false, 128, SPLIT>;
-    case 160: return (const void*)tpGemmFp8Kernel<false, 160, SPLIT>;
-    case 192: return (const void*)tpGemmFp8Kernel<false, 192, SPLIT>;
-    case 224: return (const void*)tpGemmFp8Kernel<false, 224, SPLIT>;
-    default: return (const void*)tpGemmFp8Kernel<false, 256, SPLIT>;
-  }
-}
 const void* tpGemmFp8KernelFn(bool fused, int width, bool split) {
-  return fused ? (const void*)tpGemmFp8Kernel<true, kTpBN, false> : split ? plainFp8<true>(width) : plainFp8<false>(width);
+  if (fused) return (const void*)tpGemmFp8Kernel<true, 256, false>;
+  if (width == 256) return split ? (const void*)tpGemmFp8Kernel<false, 256, true> : (const void*)tpGemmFp8Kernel<false, 256, false>;
+  return split ? (const void*)tpGemmFp8Kernel<false, 128, true> : (const void*)tpGemmFp8Kernel<false, 128, false>;
 }
 const void* tpQuantRowsWideKernelFn() { return (const void*)tpQuantRowsWideKernel; }
 void tpQuantRowsWideGrid(int rows, int K, int* x, int* y) {

@@ -14,7 +14,7 @@ using namespace b200;
 namespace b200 {
 B200_PARAM(TpCommCtas, "B200_TP_COMM_CTAS", 0, "CTAs that gather remote rows in all-gather -> GEMM (0: 4 for two ranks, 8 up to four, 16 beyond)")
 B200_PARAM(TpSplit, "B200_TP_SPLIT", 8, "Largest cluster of CTAs that shares the K dimension of a tile in plain bf16 GEMMs with few tiles (1: never, at most 8)")
-B200_PARAM(TpFp8Width, "B200_TP_FP8_WIDTH", 0, "Tile width of plain block-scaled fp8 GEMMs: 128, 160, 192, 224 or 256 (0: by shape)")
+B200_PARAM(TpFp8Width, "B200_TP_FP8_WIDTH", 0, "Tile width of plain block-scaled fp8 GEMMs: 128 or 256 (0: by shape)")
 B200_PARAM(TpFp8Split, "B200_TP_FP8_SPLIT", 0, "CTAs that share the K blocks of a tile in plain block-scaled fp8 GEMMs: 1 to 8 (0: by shape)")
 B200_PARAM(TpPair, "B200_TP_PAIR", 1, "bf16 GEMM on CTA pairs (256 x 256 tiles, tcgen05 cta_group::2) when the row count allows")
 }
@@ -24,6 +24,7 @@ struct ncclTpContext {
   int smCount = 0;
   int pairClusters = 0;   // clusters of the CTA-pair GEMM kernel that can be resident at once (0: unavailable)
   int splitClusters[kTpMaxSplit + 1] = {};   // clusters of each size of the split kernel that can be resident at once
+  int fp8Clusters[kTpMaxSplit + 1] = {};     // the same for the fp8 kernel
   void* accum = nullptr;           // symmetric staging window: bf16 [n sources][maxRows / n][maxCols]
   size_t accumBytes = 0;
   SymWindow* accumWin = nullptr;
@@ -194,14 +195,34 @@ static ncclResult_t launchGemmFp8(ncclTpContext* tp, const void* A, const void* 
   return launchTp(tp, tpGemmFp8KernelFn(fused, width, a->splitK > 1), dim3(grid), tpGemmFp8Threads(), tpGemmFp8SmemBytes(), args, !fused, std::max(a->splitK, 1), stream);
 }
 
-// Tile width, CTAs that share the K blocks of a tile (1: none), and grid of a plain fp8 GEMM.
+// Tile width, CTAs that share the K blocks of a tile (1: none), and grid of a plain fp8 GEMM: the least expected time. A K block takes
+// 0.53 us in a tile of 256 columns and 0.38 us in one of 128 (the round trip of the accumulator bounds both), a wave of tiles about
+// 3.0 and 2.4 us besides (start, first operands, store), the exchange of a cluster 3.7 us (7 us for three CTAs and more on 256
+// columns, which are not used). Kernel times, whole 128 x 256 tiles / the choice: 128 x 1024 x 7168 33.8 / 12.0 us (128 columns, four
+// CTAs), 128 x 4096 x 4096 21.4 / 11.6 (the same), 512 x 2048 x 7168 33.9 / 17.6 (two CTAs), 1024 x 2048 x 7168 34.5 / 23.2 (256 columns,
+// two CTAs), 512 x 4096 x 1024 8.9 / 7.4 (128 columns, whole), 896 x 2560 x 3584 20.0 / 15.3 (the same). The other side of the line:
+// 2560 x 3072 x 2048 in 128 columns 32.3 / 24.6, 256 x 4096 x 1536 with two CTAs 9.1 / 8.6. Six and eight CTAs to a tile gained nothing over
+// four; widths of 160 to 224, whose warps meet two scales of W, lost 5 to 50 %.
 static void planFp8(const ncclTpContext* tp, TpGemmArgs* a, int* width, int* grid) {
-  *width = 256;
-  for (int w : kTpWidths)
-    if (w == paramTpFp8Width()) *width = w;
-  a->splitK = (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(paramTpFp8Split(), kTpMaxSplit), a->K / 128));
-  const int tiles = a->M / 128 * ((a->N + *width - 1) / *width);
-  *grid = a->splitK > 1 ? tiles * a->splitK : std::min(tp->smCount, tiles);
+  const int blocks = a->K / 128;
+  const int only = paramTpFp8Width() == 128 || paramTpFp8Width() == 256 ? (int)paramTpFp8Width() : 0;
+  float best = 0.0f;
+  *width = 0;
+  for (int w : {256, 128}) {
+    const int tiles = a->M / 128 * (a->N / w);
+    const int forced = (int)std::max<int64_t>(0, std::min<int64_t>(paramTpFp8Split(), kTpMaxSplit)), most = forced ? forced : w == 256 ? 2 : 4;
+    if (only && only != w) continue;
+    for (int s = forced ? std::max(1, std::min(most, blocks)) : 1; s <= std::min(most, blocks); ++s) {
+      if (s > 1 && !forced && tiles > tp->fp8Clusters[s]) break;
+      const int waves = (tiles + tp->smCount - 1) / tp->smCount, share = (blocks + s - 1) / s;
+      const float us = waves * (w == 256 ? 3.0f + 0.53f * share : 2.4f + 0.38f * share) + (s > 1 ? 3.7f : 0.0f);
+      if (*width && us > 0.97f * best) continue;   // what is simpler stays where the others are hardly faster
+      best = us;
+      *width = w;
+      a->splitK = s;
+      *grid = s > 1 ? tiles * s : std::min(tp->smCount, tiles);
+    }
+  }
 }
 
 static ncclResult_t checkShapeFp8(int M, int N, int K, int n) {
@@ -346,7 +367,7 @@ ncclResult_t ncclTpCreate(ncclComm_t comm, size_t maxRows, size_t maxCols, ncclT
   CUDACHECK(cudaFuncSetAttribute(tpGemmKernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmSmemBytes()));
   CUDACHECK(cudaFuncSetAttribute(tpGemmSplitKernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmSplitSmemBytes()));
   CUDACHECK(cudaFuncSetAttribute(tpGemmFp8KernelFn(true, 256, false), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmFp8SmemBytes()));
-  for (int width : kTpWidths)
+  for (int width : {128, 256})
     for (bool split : {false, true})
       CUDACHECK(cudaFuncSetAttribute(tpGemmFp8KernelFn(false, width, split), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmFp8SmemBytes()));
   {
@@ -365,12 +386,17 @@ ncclResult_t ncclTpCreate(ncclComm_t comm, size_t maxRows, size_t maxCols, ncclT
     cudaLaunchAttribute cluster;
     cfg.attrs = &cluster;
     cfg.numAttrs = 1;
-    cfg.blockDim = dim3(tpGemmSplitThreads());
-    cfg.dynamicSmemBytes = tpGemmSplitSmemBytes();
     for (int size = 2; size <= kTpMaxSplit; ++size) {
       clusterAttribute(&cluster, size);
       cfg.gridDim = dim3(tp->smCount / size * size);
+      cfg.blockDim = dim3(tpGemmSplitThreads());
+      cfg.dynamicSmemBytes = tpGemmSplitSmemBytes();
       if (cudaOccupancyMaxActiveClusters(&clusters, tpGemmSplitKernelFn(), &cfg) == cudaSuccess) tp->splitClusters[size] = clusters;
+      else (void)cudaGetLastError();
+      // both widths have the same threads, registers and shared memory
+      cfg.blockDim = dim3(tpGemmFp8Threads());
+      cfg.dynamicSmemBytes = tpGemmFp8SmemBytes();
+      if (cudaOccupancyMaxActiveClusters(&clusters, tpGemmFp8KernelFn(false, 256, true), &cfg) == cudaSuccess) tp->fp8Clusters[size] = clusters;
       else (void)cudaGetLastError();
     }
     INFO(SUB_INIT, "tensor-parallel GEMM: %d SMs, %d resident CTA pairs", tp->smCount, tp->pairClusters);

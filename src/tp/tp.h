@@ -30,7 +30,6 @@ struct TpGemmArgs {
 };
 
 constexpr int kTpMaxSplit = 8;     // largest cluster of CTAs that share the K blocks of a tile
-constexpr int kTpWidths[] = {256, 224, 192, 160, 128};   // tile widths of plain GEMMs; the fused modes use the first
 
 #if defined(__CUDACC__)
 constexpr int kTpBM = 128, kTpBN = 256;
@@ -86,7 +85,7 @@ const void* tpGemmPairKernelFn();      // CTA-pair variant (cluster of two, 256 
 const void* tpGemmSplitKernelFn();     // plain C = A * W^T, one 128 x 256 tile per cluster of splitK CTAs
 size_t tpGemmSplitSmemBytes();
 int tpGemmSplitThreads();
-// fused: REDUCE and GATHER with more than one rank, tiles of 128 x 256. Others: tiles of 128 x width (one of kTpWidths); split: one tile
+// fused: REDUCE and GATHER with more than one rank, tiles of 128 x 256. Others: tiles of 128 x width (256 or 128), split: one tile
 // per cluster of splitK CTAs that share its K blocks
 const void* tpGemmFp8KernelFn(bool fused, int width, bool split);
 const void* tpQuantRowsWideKernelFn(); // as the next one, for 16-byte aligned x and q, on the grid below

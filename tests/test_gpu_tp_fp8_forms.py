@@ -1,5 +1,5 @@
-"""Block-scaled fp8 GEMM in every tile width and with the K blocks shared by clusters of 2 to 8 CTAs, against a 64-bit product: last tiles
-that hang over N, scales of W that change inside a warp's columns, uneven shares, more tiles than CTAs."""
+"""Block-scaled fp8 GEMM in both tile widths and with the K blocks shared by clusters of 2 to 8 CTAs, against a 64-bit product: uneven
+shares, fewer K blocks than CTAs, more tiles than CTAs."""
 import os
 import subprocess
 import sys
@@ -47,7 +47,7 @@ def _run(width, split):
 
 
 # width 0 and split 0: what the rule takes
-@pytest.mark.parametrize("width,split", [(0, 0), (256, 1), (224, 1), (192, 1), (160, 1), (128, 1), (256, 8), (224, 5), (192, 3), (160, 7), (128, 8), (128, 2)])
+@pytest.mark.parametrize("width,split", [(0, 0), (256, 1), (128, 1), (256, 2), (256, 8), (128, 2), (128, 3), (128, 4), (128, 7)])
 def test_fp8_forms(width, split):
     if not torch.cuda.is_available() or torch.cuda.get_device_capability()[0] < 10:
         pytest.skip("needs sm_100")
