@@ -29,6 +29,7 @@ _ENTRIES = {
     "b200SwiGlu": [_P] * 2 + [_I, _I, _P],
     "b200SwiGluBackward": [_P] * 2 + [_I, _I, _P],
     "b200CrossEntropy": [_P] * 5 + [_I, _I, _P],
+    "b200EmbeddingBackward": [_P] * 3 + [_I] * 3 + [_P],
 }
 
 
@@ -39,6 +40,11 @@ def applies(cfg, tokens, targets):
     return (h % 8 == 0 and h <= 16384 and d > 0 and d % 16 == 0 and d * cfg.heads == h and cfg.heads % cfg.kv_heads == 0 and cfg.ffn % 8 == 0 and
             cfg.vocab % 8 == 0 and tokens.dim() == 2 and tokens.numel() > 0 and targets.dtype == torch.int64 and targets.numel() == tokens.numel() and
             torch.is_grad_enabled() and not torch.is_anomaly_enabled() and not torch.is_autocast_enabled("cuda"))
+
+
+def embedding_applies(tokens):
+    """Every id looks through all others: 64-bit ids, and few enough of them."""
+    return tokens.dtype == torch.int64 and tokens.numel() <= 8192
 
 
 class FusedUnits:
@@ -157,6 +163,11 @@ class FusedUnits:
         dh = torch.mm(dqkv, p["wqkv"])
         torch.mm(dqkv.t(), h1, out=g["wqkv"])
         return self.norm_backward(x, p["norm1"], rstd1, dh, g2, g["norm1"])
+
+    def embedding_backward(self, tokens, gx, gflat):
+        """The gradient of the table, into gflat."""
+        c, ids = self.cfg, tokens.reshape(-1).contiguous()
+        self._run("b200EmbeddingBackward", ids.data_ptr(), gx.data_ptr(), gflat.data_ptr(), ids.numel(), c.vocab, c.hidden)
 
     def head(self, x, flat, gflat, targets):
         """(mean loss, gradient of the hidden states); the weights' gradients go into gflat."""

@@ -271,6 +271,11 @@ class FSDPEngine:
                 self._reduce_and_update(idx, slot)
                 saved[idx] = None
                 continue
+            if fused and llama_fused.embedding_applies(tokens):
+                fused.embedding_backward(tokens, gx, self._grad_flat(idx, slot))
+                self._release(slot)
+                self._reduce_and_update(idx, slot)
+                continue
             vs = params(idx, slot, True)
             names = [n for n, _ in self.units[idx].shapes]
             gx = gx.view(*shape, cfg.hidden) if fused else gx

@@ -216,3 +216,15 @@ def test_what_stays_with_autograd():
         assert not llama_fused.applies(cfg, tok, tok)
     with torch.autograd.detect_anomaly(check_nan=False):
         assert not llama_fused.applies(cfg, tok, tok)
+
+
+@gpu
+@pytest.mark.parametrize("shape,hidden,vocab", [((1, 1), 8, 8), ((2, 65), 64, 16), ((1, 700), 2056, 1000), ((3, 257), 4096, 5), ((2, 1024), 128, 50000)])
+def test_embedding_backward(shape, hidden, vocab):
+    u = _units(hidden=hidden, vocab=vocab)
+    tokens = torch.randint(0, vocab, shape, generator=torch.Generator().manual_seed(2)).cuda()
+    gx = _rand(*shape, hidden, seed=1)
+    out = torch.full((vocab * hidden,), 7.0, dtype=torch.bfloat16, device="cuda")
+    u.embedding_backward(tokens, gx, out)
+    ref, spread = (torch.zeros(vocab, hidden, dtype=torch.float64, device="cuda").index_add_(0, tokens.view(-1), t.view(-1, hidden)) for t in (gx.double(), gx.double().abs()))
+    _close(out.view(vocab, hidden), ref, spread)
