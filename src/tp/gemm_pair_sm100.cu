@@ -27,25 +27,29 @@ using namespace sm100;
 
 namespace {
 constexpr int PM = 256;                         // rows of a pair tile
-constexpr int BN = kTpBN, BK = kTpBK, UMMA_K = 16;
-constexpr int P_STAGES = 6;
+constexpr int BK = kTpBK, UMMA_K = 16;
 constexpr int kThreads = 192;
-constexpr uint32_t kHalfBytes = 128 * BK * 2;   // 128 rows x 64 bf16: A half and W half are the same size
-constexpr uint32_t kStageBytes = 2 * kHalfBytes;
+constexpr uint32_t kHalfABytes = 128 * BK * 2;          // this CTA's 128 rows of A x 64 bf16
+constexpr size_t kRingBytes = 6 * 2 * kHalfABytes;      // operand ring: as many stages as fit
 constexpr int kAccBufs = 2;                     // accumulators of 256 columns in tensor memory: the epilogue of one tile overlaps the MMAs of the next
 constexpr uint32_t kTmemCols = kAccBufs * 256;
 constexpr size_t kEpiBufBytes = 4 * 4096;
-constexpr size_t kSmemBytes = 1024 + (size_t)P_STAGES * kStageBytes + 256 + kEpiBufBytes;
-static_assert(kTpPipeBytes <= (size_t)P_STAGES * kStageBytes, "copy ring must fit the operand ring");
-static_assert(kTpPipeStages <= 2 * P_STAGES, "not enough barriers for the copy ring");
-static_assert((2 * P_STAGES + 4) * 8 + 8 <= 256, "control block too small");
+constexpr size_t kSmemBytes = 1024 + kRingBytes + 256 + kEpiBufBytes;
+static_assert(kTpPipeBytes <= kRingBytes, "copy ring must fit the operand ring");
 }  // namespace
 
+// BN: width of the tiles, kTpBN in the modes with a collective; each CTA stages BN / 2 rows of W. The last tile of a row may hang over
+// N (zeros from the tensor map, nothing stored).
+template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 tpGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ TpGemmArgs a) {
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
-  uint8_t* ctrl = smem + (size_t)P_STAGES * kStageBytes;
+  constexpr uint32_t kHalfBBytes = BN / 2 * BK * 2, kStageBytes = kHalfABytes + kHalfBBytes;
+  constexpr int P_STAGES = kRingBytes / kStageBytes;
+  static_assert(kTpPipeStages <= 2 * P_STAGES, "not enough barriers for the copy ring");
+  static_assert((2 * P_STAGES + 4) * 8 + 8 <= 256, "control block too small");
+  uint8_t* ctrl = smem + kRingBytes;
   uint64_t* fullBar = (uint64_t*)ctrl;            // [P_STAGES]
   uint64_t* emptyBar = fullBar + P_STAGES;        // [P_STAGES]
   uint64_t* accFull = emptyBar + P_STAGES;        // [2]
@@ -98,12 +102,12 @@ tpGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   pdlEnter();   // the set-up above overlaps the end of the kernel before; operands and results are touched behind it
   if (!ok && threadIdx.x == 0) stSharedCluster(mapaShared(smemAddr((const void*)abortFlag), cr ^ 1), 1u);
 
-  const int tilesN = a.N / BN;
+  const int tilesN = (a.N + BN - 1) / BN;
   const int nTiles = (a.M + PM - 1) / PM * tilesN;   // plain GEMMs: the last row tile may be half empty (its loads are filled with zeros)
   const int kBlocks = a.K / BK;
   const int pairIdx = blockIdx.x >> 1;
   const int nPairs = (gather ? a.gemmCtas : (int)gridDim.x) >> 1;
-  const uint32_t smemA0 = smemAddr(smem), smemB0 = smemA0 + P_STAGES * kHalfBytes;
+  const uint32_t smemA0 = smemAddr(smem), smemB0 = smemA0 + P_STAGES * kHalfABytes;
   auto fail = [&](uint32_t kind, uint32_t what) {
     *abortFlag = 1;
     stSharedCluster(mapaShared(smemAddr((const void*)abortFlag), cr ^ 1), 1u);   // the partner gives up too
@@ -116,7 +120,7 @@ tpGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int armedStage[P_STAGES];
       for (int s = 0; s < P_STAGES; ++s) armedStage[s] = -1;
       for (int t = pairIdx; t < nTiles && !*abortFlag; t += nPairs) {
-        const TileCoord tc = tileOf(a, t, PM);
+        const TileCoord tc = tileOf(a, t, PM, BN);
         const int myBlk = tc.mBlk * 2 + (int)cr;   // this CTA's 128-row block of A
         if (gather && tc.owner != rank && !tpWaitBlock(a, myBlk, abortFlag)) { fail(WAIT_TILE, (uint32_t)myBlk); break; }
         for (int kb = 0; kb < kBlocks; ++kb, ++kc) {
@@ -126,8 +130,8 @@ tpGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           if (*abortFlag) break;
           if (leader) mbarExpectTx(smemAddr(&fullBar[s]), 2 * kStageBytes);   // the bytes of both CTAs
           const uint32_t fb = mapaShared(smemAddr(&fullBar[s]), 0);
-          tmaLoad2dPair(smemA0 + s * kHalfBytes, &tmA, kb * BK, myBlk * 128, fb);
-          tmaLoad2dPair(smemB0 + s * kHalfBytes, &tmB, kb * BK, tc.nBlk * BN + (int)cr * 128, fb);
+          tmaLoad2dPair(smemA0 + s * kHalfABytes, &tmA, kb * BK, myBlk * 128, fb);
+          tmaLoad2dPair(smemB0 + s * kHalfBBytes, &tmB, kb * BK, tc.nBlk * BN + (int)cr * (BN / 2), fb);
           armedStage[s] = (int)ph;
         }
       }
@@ -147,14 +151,14 @@ tpGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const uint32_t aph = (it / kAccBufs) & 1;
         if (!mbarWait(smemAddr(&accEmpty[buf]), aph ^ 1)) { fail(WAIT_TILE, 2000 + buf); break; }
         tcFenceAfter();
-        const uint32_t dT = tmemBase + buf * BN;
+        const uint32_t dT = tmemBase + buf * 256;
         bool bad = false;
         for (int kb = 0; kb < kBlocks; ++kb, ++kc) {
           const int s = kc % P_STAGES;
           const uint32_t ph = (kc / P_STAGES) & 1;
           if (!mbarWait(smemAddr(&fullBar[s]), ph)) { fail(WAIT_TILE, 3000 + s); bad = true; break; }
           tcFenceAfter();
-          const uint32_t aAddr = smemA0 + s * kHalfBytes, bAddr = smemB0 + s * kHalfBytes;
+          const uint32_t aAddr = smemA0 + s * kHalfABytes, bAddr = smemB0 + s * kHalfBBytes;
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k)
             ummaBf16Pair(dT, umDescK128(aAddr + k * UMMA_K * 2), umDescK128(bAddr + k * UMMA_K * 2), idesc, (kb | k) != 0);
@@ -170,14 +174,14 @@ tpGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint8_t* wbuf = epiBuf + (size_t)(warp - 2) * 4096;
     int it = 0;
     for (int t = pairIdx; t < nTiles && !*abortFlag; t += nPairs, ++it) {
-      const TileCoord tc = tileOf(a, t, PM);
+      const TileCoord tc = tileOf(a, t, PM, BN);
       const int buf = it % kAccBufs;
       const uint32_t aph = (it / kAccBufs) & 1;
       if (!mbarWait(smemAddr(&accFull[buf]), aph)) { if (lane == 0) fail(WAIT_TILE, 4000 + buf); break; }
       tcFenceAfter();
       const int row0 = tc.mBlk * PM + (int)cr * 128 + q * 32;
-      const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * BN;
-      if (row0 < a.M) tpStoreAccum(a, tBase, row0, tc.nBlk, tc.owner, wbuf, lane);
+      const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * 256;
+      if (row0 < a.M) tpStoreAccum<BN>(a, tBase, row0, tc.nBlk, tc.owner, wbuf, lane);
       tcFenceBefore();
       __syncwarp();
       if (lane == 0) mbarArriveCluster(mapaShared(smemAddr(&accEmpty[buf]), 0));
@@ -200,7 +204,15 @@ tpGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
-const void* tpGemmPairKernelFn() { return (const void*)tpGemmPairKernel; }
+const void* tpGemmPairKernelFn(int width) {
+  switch (width) {
+    case 128: return (const void*)tpGemmPairKernel<128>;
+    case 160: return (const void*)tpGemmPairKernel<160>;
+    case 192: return (const void*)tpGemmPairKernel<192>;
+    case 224: return (const void*)tpGemmPairKernel<224>;
+    default: return (const void*)tpGemmPairKernel<256>;
+  }
+}
 size_t tpGemmPairSmemBytes() { return kSmemBytes; }
 int tpGemmPairThreads() { return kThreads; }
 

@@ -79,21 +79,26 @@ __device__ __forceinline__ bool tpWaitBlock(const TpGemmArgs& a, int mb, volatil
 // transposes 64 columns at a time through 4 KiB of shared memory (16-byte chunks XOR-swizzled by
 // row against bank conflicts) and writes 128 contiguous bytes per row, four rows per instruction:
 // whole lines for HBM and NVLink.
+// W is the width of the tile: the columns behind it, and those behind the last of C, are left out (both in steps of 32).
+template <int W>
 __device__ __forceinline__ void tpStoreAccum(const TpGemmArgs& a, uint32_t tBase, int row0, int nBlk, int owner, uint8_t* wbuf, int lane) {
   using namespace sm100;
   __nv_bfloat16* dstBase;
   size_t ld;
   if (a.mode == TP_MODE_REDUCE && a.nRanks > 1) {
     const int rowsPerRank = a.M / a.nRanks;
-    dstBase = (__nv_bfloat16*)a.partial[owner] + ((size_t)a.rank * rowsPerRank + (row0 - owner * rowsPerRank)) * a.N + (size_t)nBlk * kTpBN;
+    dstBase = (__nv_bfloat16*)a.partial[owner] + ((size_t)a.rank * rowsPerRank + (row0 - owner * rowsPerRank)) * a.N + (size_t)nBlk * W;
     ld = (size_t)a.N;
   } else {
-    dstBase = (__nv_bfloat16*)a.C + (size_t)row0 * a.ldc + (size_t)nBlk * kTpBN;
+    dstBase = (__nv_bfloat16*)a.C + (size_t)row0 * a.ldc + (size_t)nBlk * W;
     ld = (size_t)a.ldc;
   }
-  for (int cc = 0; cc < kTpBN / 64; ++cc) {
+  const int cols = W == kTpBN ? W : min(W, a.N - nBlk * W);
+  for (int cc = 0; cc * 64 < cols; ++cc) {
+    const bool both = W == kTpBN || cc * 64 + 32 < cols;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
+      if (half && !both) break;
       uint32_t r[32];
       tmemLd32(tBase + (cc * 2 + half) * 32, r);
       tmemLdWait();
@@ -114,7 +119,7 @@ __device__ __forceinline__ void tpStoreAccum(const TpGemmArgs& a, uint32_t tBase
     for (int k = 0; k < 8; ++k) {
       const int rr = k * 4 + (lane >> 3), j = lane & 7;
       const uint4 o = *(const uint4*)(wbuf + rr * 128 + ((j ^ (rr & 7)) * 16));
-      *(uint4*)((char*)(dstBase + (size_t)rr * ld) + cc * 128 + j * 16) = o;
+      if (both || j < 4) *(uint4*)((char*)(dstBase + (size_t)rr * ld) + cc * 128 + j * 16) = o;
     }
     __syncwarp();
   }

@@ -33,19 +33,23 @@ namespace b200 {
 
 using namespace sm100;
 
-constexpr int BM = kTpBM, BN = kTpBN, BK = kTpBK, STAGES = 4, UMMA_K = 16;
+constexpr int BM = kTpBM, BK = kTpBK, UMMA_K = 16;
 constexpr int kTpThreads = 192;
-constexpr uint32_t kStageABytes = BM * BK * 2, kStageBBytes = BN * BK * 2;
-constexpr uint32_t kStageBytes = kStageABytes + kStageBBytes;
-constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kTmemCols = 512, kAccCols = 256;      // two accumulators, at fixed columns
 constexpr size_t kEpiBufBytes = 4 * 4096;   // one 32 x 128-byte transpose buffer per epilogue warp
-constexpr size_t kTpSmemBytes = 1024 + (size_t)STAGES * kStageBytes + 256 + kEpiBufBytes;
+constexpr size_t kRingBytes = 4 * (BM + 256) * BK * 2;   // operand ring: as many stages as fit
+constexpr size_t kTpSmemBytes = 1024 + kRingBytes + 256 + kEpiBufBytes;
 
+// BN: width of the tiles, kTpBN in the modes with a collective. The last tile of a row may hang over N (zeros from the tensor map,
+// nothing stored).
+template <int BN>
 __global__ void __launch_bounds__(kTpThreads, 1)
 tpGemmKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ TpGemmArgs a) {
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
-  uint8_t* ctrl = smem + (size_t)STAGES * kStageBytes;
+  constexpr uint32_t kStageABytes = BM * BK * 2, kStageBBytes = BN * BK * 2, kStageBytes = kStageABytes + kStageBBytes;
+  constexpr int STAGES = kRingBytes / kStageBytes;
+  uint8_t* ctrl = smem + kRingBytes;
   uint64_t* fullBar = (uint64_t*)ctrl;            // [STAGES]
   uint64_t* emptyBar = fullBar + STAGES;          // [STAGES]
   uint64_t* accFull = emptyBar + STAGES;          // [2]
@@ -68,7 +72,7 @@ tpGemmKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
 
   if (commCta) {
     // ---- all-gather role: pull the other ranks' row blocks in consumption order
-    static_assert(kTpPipeBytes <= (size_t)STAGES * kStageBytes, "copy ring must fit the operand ring");
+    static_assert(kTpPipeBytes <= kRingBytes, "copy ring must fit the operand ring");
     static_assert(kTpPipeStages <= 2 * STAGES, "not enough barriers");   // the operand barriers are unused by a comm CTA
     tpCommRole(a, blockIdx.x - a.gemmCtas, gridDim.x - a.gemmCtas, smem, fullBar, ok);
     bar.sync(true, false);   // nobody reads my rows any more
@@ -95,7 +99,7 @@ tpGemmKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
   const uint32_t tmemBase = *tmemSlot;
   pdlEnter();   // the set-up above overlaps the end of the kernel before; operands and results are touched behind it
 
-  const int tilesN = a.N / BN;
+  const int tilesN = (a.N + BN - 1) / BN;
   const int nTiles = (a.M / BM) * tilesN;
   const int kBlocks = a.K / BK;
   const int gemmCtas = (a.mode == TP_MODE_GATHER && n > 1) ? a.gemmCtas : gridDim.x;
@@ -111,7 +115,7 @@ tpGemmKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       int armedStage[STAGES];
       for (int s = 0; s < STAGES; ++s) armedStage[s] = -1;
       for (int t = blockIdx.x; t < nTiles && !*abortFlag; t += gemmCtas) {
-        const TileCoord tc = tileOf(a, t);
+        const TileCoord tc = tileOf(a, t, BM, BN);
         if (a.mode == TP_MODE_GATHER && n > 1 && tc.owner != rank) {
           // wait until the comm CTAs have landed this block of rows
           if (!tpWaitBlock(a, tc.mBlk, abortFlag)) { fail(WAIT_TILE, (uint32_t)tc.mBlk); break; }
@@ -143,7 +147,7 @@ tpGemmKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
         const uint32_t aph = (it >> 1) & 1;
         if (!mbarWait(smemAddr(&accEmpty[buf]), aph ^ 1)) { fail(WAIT_TILE, 2000 + buf); break; }
         tcFenceAfter();
-        const uint32_t dT = tmemBase + buf * BN;
+        const uint32_t dT = tmemBase + buf * kAccCols;
         bool bad = false;
         for (int kb = 0; kb < kBlocks; ++kb, ++kc) {
           const int s = kc % STAGES;
@@ -165,14 +169,14 @@ tpGemmKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     const int q = warp & 3;
     int it = 0;
     for (int t = blockIdx.x; t < nTiles && !*abortFlag; t += gemmCtas, ++it) {
-      const TileCoord tc = tileOf(a, t);
+      const TileCoord tc = tileOf(a, t, BM, BN);
       const int buf = it & 1;
       const uint32_t aph = (it >> 1) & 1;
       if (!mbarWait(smemAddr(&accFull[buf]), aph)) { if (lane == 0) fail(WAIT_TILE, 4000 + buf); break; }
       tcFenceAfter();
       const int row0 = tc.mBlk * BM + q * 32;   // first of this warp's 32 rows
-      const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * BN;
-      tpStoreAccum(a, tBase, row0, tc.nBlk, tc.owner, epiBuf + (size_t)(warp - 2) * 4096, lane);
+      const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * kAccCols;
+      tpStoreAccum<BN>(a, tBase, row0, tc.nBlk, tc.owner, epiBuf + (size_t)(warp - 2) * 4096, lane);
       tcFenceBefore();
       __syncwarp();
       if (lane == 0) mbarArrive(smemAddr(&accEmpty[buf]));
@@ -213,7 +217,15 @@ __global__ void tpReduceKernel(const __nv_bfloat16* __restrict__ staged, __nv_bf
   }
 }
 
-const void* tpGemmKernelFn() { return (const void*)tpGemmKernel; }
+const void* tpGemmKernelFn(int width) {
+  switch (width) {
+    case 128: return (const void*)tpGemmKernel<128>;
+    case 160: return (const void*)tpGemmKernel<160>;
+    case 192: return (const void*)tpGemmKernel<192>;
+    case 224: return (const void*)tpGemmKernel<224>;
+    default: return (const void*)tpGemmKernel<256>;
+  }
+}
 const void* tpReduceKernelFn() { return (const void*)tpReduceKernel; }
 size_t tpGemmSmemBytes() { return kTpSmemBytes; }
 int tpGemmThreads() { return kTpThreads; }

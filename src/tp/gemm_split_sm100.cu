@@ -15,17 +15,18 @@ namespace b200 {
 using namespace sm100;
 
 namespace {
-constexpr int BM = kTpBM, BN = kTpBN, BK = kTpBK, STAGES = 4, UMMA_K = 16;
+constexpr int BM = kTpBM, BK = kTpBK, UMMA_K = 16;
 constexpr int kThreads = 192;
-constexpr uint32_t kStageABytes = BM * BK * 2, kStageBBytes = BN * BK * 2;
-constexpr uint32_t kStageBytes = kStageABytes + kStageBBytes;
-constexpr size_t kSmemBytes = 1024 + (size_t)STAGES * kStageBytes + 256;
-constexpr int kChunk = 32, kChunks = BN / kChunk;
+constexpr uint32_t kStageABytes = BM * BK * 2;
+constexpr size_t kRingBytes = 4 * (BM + 256) * BK * 2;   // operand ring: as many stages as fit
+constexpr size_t kSmemBytes = 1024 + kRingBytes + 256;
+constexpr int kChunk = 32;
 constexpr uint32_t kChunkBytes = BM * kChunk * 4;
-// chunks of one owner x shares of the others, for every cluster size
+// chunks of one owner x shares of the others, for every width and cluster size
 constexpr bool fits() {
-  for (int s = 2; s <= kTpMaxSplit; ++s)
-    if ((size_t)((kChunks + s - 1) / s) * (s - 1) * kChunkBytes > (size_t)STAGES * kStageBytes) return false;
+  for (int w : {128, 256})
+    for (int s = 2; s <= kTpMaxSplit; ++s)
+      if ((size_t)((w / kChunk + s - 1) / s) * (s - 1) * kChunkBytes > kRingBytes) return false;
   return true;
 }
 static_assert(fits(), "partial sums must fit the operand ring");
@@ -35,11 +36,15 @@ __device__ __forceinline__ void stSharedCluster16(uint32_t clusterAddr, uint32_t
 }
 }  // namespace
 
+// BN: width of the tiles, 256 or 128
+template <int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 tpGemmSplitKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ TpGemmArgs a) {
   extern __shared__ uint8_t smemRaw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
-  uint8_t* ctrl = smem + (size_t)STAGES * kStageBytes;
+  constexpr uint32_t kStageBBytes = BN * BK * 2, kStageBytes = kStageABytes + kStageBBytes;
+  constexpr int STAGES = kRingBytes / kStageBytes, kChunks = BN / kChunk;
+  uint8_t* ctrl = smem + kRingBytes;
   uint64_t* fullBar = (uint64_t*)ctrl;            // [STAGES]
   uint64_t* emptyBar = fullBar + STAGES;          // [STAGES]
   uint64_t* accFull = emptyBar + STAGES;
@@ -187,7 +192,7 @@ tpGemmSplitKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   }
 }
 
-const void* tpGemmSplitKernelFn() { return (const void*)tpGemmSplitKernel; }
+const void* tpGemmSplitKernelFn(int width) { return width == 128 ? (const void*)tpGemmSplitKernel<128> : (const void*)tpGemmSplitKernel<256>; }
 size_t tpGemmSplitSmemBytes() { return kSmemBytes; }
 int tpGemmSplitThreads() { return kThreads; }
 

@@ -14,6 +14,7 @@ using namespace b200;
 namespace b200 {
 B200_PARAM(TpCommCtas, "B200_TP_COMM_CTAS", 0, "CTAs that gather remote rows in all-gather -> GEMM (0: 4 for two ranks, 8 up to four, 16 beyond)")
 B200_PARAM(TpSplit, "B200_TP_SPLIT", 8, "Largest cluster of CTAs that shares the K dimension of a tile in plain bf16 GEMMs with few tiles (1: never, at most 8)")
+B200_PARAM(TpWidth, "B200_TP_WIDTH", 0, "Tile width of plain bf16 GEMMs whose tiles are not split: 128, 160, 192, 224 or 256 (0: by shape)")
 B200_PARAM(TpFp8Width, "B200_TP_FP8_WIDTH", 0, "Tile width of plain block-scaled fp8 GEMMs: 128 or 256 (0: by shape)")
 B200_PARAM(TpFp8Split, "B200_TP_FP8_SPLIT", 0, "CTAs that share the K blocks of a tile in plain block-scaled fp8 GEMMs: 1 to 8 (0: by shape)")
 B200_PARAM(TpPair, "B200_TP_PAIR", 1, "bf16 GEMM on CTA pairs (256 x 256 tiles, tcgen05 cta_group::2) when the row count allows")
@@ -126,7 +127,8 @@ static void fillSyncTp(ncclComm* comm, SyncArgs* s) {
 // no more than the exchange of the partial sums costs, a CTA keeps its tile. Kernel times against the kernel that the call would
 // take instead, weights from memory and from L2, 4 to 72 tiles. One CTA to a tile: K = 1024 1.01-1.10, 1280 0.94-1.05, 1536
 // 0.87-1.00, 1792 0.84-0.96, 2560 0.71-0.88. CTA pairs: K = 1024 0.95-1.03, 1280 0.92-1.00, 2560 0.80-0.90.
-constexpr int kSplitMinBlocks = 8, kSplitFromOne = 1536 / 64;
+constexpr int kSplitMinBlocks = 8, kSplitFromOne = 1536 / 64;   // clusters on tiles of 256 columns
+constexpr int kNarrowMaxSplit = 5;                              // clusters on tiles of 128 columns: six and eight CTAs gained nothing more
 static int splitOf(const ncclTpContext* tp, const TpGemmArgs* a, bool insteadOfPairs) {
   const int tiles = (a->M / 128) * (a->N / 256), blocks = a->K / 64;
   if (!insteadOfPairs && blocks < kSplitFromOne) return 1;
@@ -135,12 +137,89 @@ static int splitOf(const ncclTpContext* tp, const TpGemmArgs* a, bool insteadOfP
   return std::max(s, 1);
 }
 
-static ncclResult_t launchGemmSplit(ncclTpContext* tp, const void* A, const void* W, TpGemmArgs* a, cudaStream_t stream) {
+static ncclResult_t launchGemmSplit(ncclTpContext* tp, const void* A, const void* W, TpGemmArgs* a, int width, cudaStream_t stream) {
   CUtensorMap tmA, tmB;
   NCCLCHECK(makeMap(&tmA, A, a->M, a->K, 128));
-  NCCLCHECK(makeMap(&tmB, W, a->N, a->K, 256));
+  NCCLCHECK(makeMap(&tmB, W, a->N, a->K, width));
   void* args[3] = {&tmA, &tmB, a};
-  return launchTp(tp, tpGemmSplitKernelFn(), dim3((a->M / 128) * (a->N / 256) * a->splitK), tpGemmSplitThreads(), tpGemmSplitSmemBytes(), args, true, a->splitK, stream);
+  return launchTp(tp, tpGemmSplitKernelFn(width), dim3((a->M / 128) * (a->N / width) * a->splitK), tpGemmSplitThreads(), tpGemmSplitSmemBytes(), args, true, a->splitK, stream);
+}
+
+// How a plain bf16 GEMM runs: one-CTA tiles of 128 x width, CTA pairs (256 x width), or clusters of `split` CTAs that share the K steps of a
+// tile of 128 x width.
+struct GemmPlan {
+  bool pair = false;
+  int width = 256, split = 1;
+};
+
+// Tiles of 256 columns, by what the widths below do not change: clusters for few tiles, else pairs where they pay.
+static GemmPlan basePlan(const ncclTpContext* tp, const TpGemmArgs* a, bool pairs) {
+  GemmPlan p;
+  p.split = splitOf(tp, a, pairs && a->M % 256 == 0);
+  if (p.split > 1) return p;
+  p.pair = pairs;
+  if (p.pair && a->M % 256) {
+    // Pairs leave half of the last row tile empty. A K step of a pair tile takes 0.92 to 0.97 of the time of one of two
+    // 128 x 256 tiles (32 KiB of operands from L2 per SM against 48), but a launch of pairs takes about 1.5 us longer, so they pay
+    // when they need no more waves and have enough steps. Kernel times of pairs over one-CTA tiles, weights from memory and from
+    // L2: two waves 0.97-1.02 at K = 1024, 0.96-1.01 at 1536, 0.91-1.01 at 4096; three and more 0.91-0.98 from 1024 on, about 1.0 at
+    // 512; four waves where one-CTA tiles need three 1.1. One wave 1.2 at 512, 1.08 at 1536; at 4096 to 7168 0.90-0.98 when
+    // the operands are more than 60 MiB or come from memory, 1.00-1.06 when they are fewer and in L2.
+    const int tilesN = a->N / 256, one = a->M / 128 * tilesN, two = (a->M / 128 + 1) / 2 * tilesN;
+    const int wavesOne = (one + tp->smCount - 1) / tp->smCount, wavesTwo = (two + tp->pairClusters - 1) / tp->pairClusters;
+    const bool enough = wavesOne > 2 ? a->K >= 1024 : wavesOne > 1 ? a->K >= 1536 : a->K >= 4096 && ((size_t)a->M + a->N) * a->K * 2 > (size_t)60 << 20;
+    p.pair = wavesTwo <= wavesOne && enough;
+  }
+  return p;
+}
+
+static int wavesOf(const ncclTpContext* tp, const TpGemmArgs* a, const GemmPlan& p) {
+  const int tilesN = (a->N + p.width - 1) / p.width;
+  return p.pair ? ((a->M + 255) / 256 * tilesN + tp->pairClusters - 1) / tp->pairClusters : (a->M / 128 * tilesN + tp->smCount - 1) / tp->smCount;
+}
+
+// Expected time in us, operands in L2: start and last store, K steps of 64 with every SM at work, what a wave of tiles adds, and the
+// exchange of a cluster. Fitted to 31 shapes of 4 to 2048 tiles and 8 to 128 K steps; up to four waves it is within about 10 %.
+static float expectedUs(const ncclTpContext* tp, const TpGemmArgs* a, const GemmPlan& p) {
+  const int steps = a->K / 64, share = (steps + p.split - 1) / p.split, waves = p.split > 1 ? 1 : wavesOf(tp, a, p);
+  float step;
+  switch (p.width) {
+    case 128: step = p.pair ? 0.23f : 0.21f; break;
+    case 160: step = p.pair ? 0.25f : 0.255f; break;
+    case 192: step = p.pair ? 0.26f : 0.31f; break;
+    case 224: step = p.pair ? 0.315f : 0.38f; break;
+    default: step = p.pair ? 0.35f : 0.385f; break;
+  }
+  const float exchange = p.split == 1 ? 0.0f : p.width == 128 ? 2.0f + 0.4f * p.split : p.split == 2 ? 2.2f : 6.5f;
+  return (p.pair ? 4.1f : 3.3f) + waves * share * step + (waves - 1) * 0.8f + exchange;
+}
+
+// Narrower tiles, alone or shared by a cluster, where 256 columns leave the last wave (or all but a few SMs) empty: a step of 160 columns
+// takes 0.65 of the time of one of 256, so what counts is how the tiles fill the chip. Up to four waves of pair tiles: beyond, the
+// last wave matters less and the widest tiles have the best rate (8192 x 8192 x 3584: pairs of 256 303 us, 224 312, 192 349).
+// Kernel times with 256 columns / the choice, us: 128 x 1024 x 2048 10.3 / 7.3 (128 columns, four CTAs), 128 x 4096 x 4096 18.5 / 12.8,
+// 128 x 8192 x 8192 30.4 / 28.3 (two CTAs; memory), 512 x 4096 x 1024 10.6 / 7.7 (128 columns), 1152 x 2304 x 7168 40.6 / 31.8 (160),
+// 2048 x 2560 x 4096 46.1 / 35.4 (160), 1280 x 4096 x 3584 38.4 / 31.9 (pairs of 192), 2560 x 3072 x 2048 25.6 / 23.7 (pairs of 224).
+// The other side of the line: 1920 x 4096 x 7168 82.3 with pairs of 256, 91.7 of 192; 3328 x 4096 x 1536 29.5 / 31.7.
+static GemmPlan planGemm(const ncclTpContext* tp, const TpGemmArgs* a, bool pairs) {
+  GemmPlan best = basePlan(tp, a, pairs);
+  for (int w : kTpWidths)
+    if (w == paramTpWidth()) {
+      if (best.split == 1) best.width = w;
+      return best;
+    }
+  if (((a->M + 255) / 256 * (a->N / 256) + tp->smCount / 2 - 1) / (tp->smCount / 2) > 4) return best;
+  float us = 0.95f * expectedUs(tp, a, best);   // what is simpler stays where the others are hardly faster
+  auto consider = [&](const GemmPlan& p) {
+    const float t = expectedUs(tp, a, p);
+    if (t < us) { us = t; best = p; }
+  };
+  for (int w : kTpWidths)
+    for (bool pair : {false, true})
+      if (pairs || !pair) consider({pair, w, 1});
+  const int tiles = a->M / 128 * (a->N / 128), most = std::min(std::min((int)paramTpSplit(), kNarrowMaxSplit), a->K / 64);
+  for (int s = 2; s <= most && tiles <= tp->splitClusters[s]; ++s) consider({false, 128, s});
+  return best;
 }
 
 // Launches the bf16 GEMM kernel in the mode of `a`. Grid: one CTA per SM (fewer when there are fewer
@@ -151,38 +230,32 @@ static ncclResult_t launchGemm(ncclTpContext* tp, const void* A, const void* W, 
   const bool fused = n > 1 && a->mode != TP_MODE_STORE;
   const bool gather = fused && a->mode == TP_MODE_GATHER;
   const bool pairs = paramTpPair() != 0 && tp->pairClusters > 0;
-  if (!fused && (a->splitK = splitOf(tp, a, pairs && a->M % 256 == 0)) > 1) return launchGemmSplit(tp, A, W, a, stream);
-  bool pair = pairs && (!fused || a->M % (256 * n) == 0);
-  if (pair && a->M % 256) {
-    // Plain GEMMs: pairs leave half of the last row tile empty. A K step of a pair tile takes 0.92 to 0.97 of the time of one of two
-    // 128 x 256 tiles (32 KiB of operands from L2 per SM against 48), but a launch of pairs takes about 1.5 us longer, so they pay
-    // when they need no more waves and have enough steps. Kernel times of pairs over one-CTA tiles, weights from memory and from
-    // L2: two waves 0.97-1.02 at K = 1024, 0.96-1.01 at 1536, 0.91-1.01 at 4096; three and more 0.91-0.98 from 1024 on, about 1.0 at
-    // 512; four waves where one-CTA tiles need three 1.1. One wave 1.2 at 512, 1.08 at 1536; at 4096 to 7168 0.90-0.98 when
-    // the operands are more than 60 MiB or come from memory, 1.00-1.06 when they are fewer and in L2.
-    const int tilesN = a->N / 256, one = a->M / 128 * tilesN, two = (a->M / 128 + 1) / 2 * tilesN;
-    const int wavesOne = (one + tp->smCount - 1) / tp->smCount, wavesTwo = (two + tp->pairClusters - 1) / tp->pairClusters;
-    const bool enough = wavesOne > 2 ? a->K >= 1024 : wavesOne > 1 ? a->K >= 1536 : a->K >= 4096 && ((size_t)a->M + a->N) * a->K * 2 > (size_t)60 << 20;
-    pair = wavesTwo <= wavesOne && enough;
-  }
+  GemmPlan plan;
+  if (fused) plan.pair = pairs && a->M % (256 * n) == 0;
+  else plan = planGemm(tp, a, pairs);
+  a->splitK = plan.split;
+  if (plan.split > 1) return launchGemmSplit(tp, A, W, a, plan.width, stream);
+  const bool pair = plan.pair;
+  const int width = plan.width;
   int commCtas = gather ? tpCommCtas(tp, n) : 0;
   int grid;
+  const int tilesN = (a->N + width - 1) / width;
   if (pair) {
     commCtas = (commCtas + 1) & ~1;   // both CTAs of a cluster have the same role
-    const int tiles = (a->M + 255) / 256 * (a->N / 256);
+    const int tiles = (a->M + 255) / 256 * tilesN;
     const int pairs = std::max(1, std::min(tp->pairClusters - commCtas / 2, tiles));
     a->gemmCtas = 2 * pairs;
     grid = 2 * pairs + commCtas;
   } else {
-    const int tiles = (a->M / 128) * (a->N / 256);
+    const int tiles = (a->M / 128) * tilesN;
     grid = gather ? tp->smCount : std::min(tp->smCount, tiles);
     a->gemmCtas = grid - commCtas;
   }
   CUtensorMap tmA, tmB;
   NCCLCHECK(makeMap(&tmA, A, a->M, a->K, 128));
-  NCCLCHECK(makeMap(&tmB, W, a->N, a->K, pair ? 128 : 256));
+  NCCLCHECK(makeMap(&tmB, W, a->N, a->K, pair ? width / 2 : width));
   void* args[3] = {&tmA, &tmB, a};
-  return launchTp(tp, pair ? tpGemmPairKernelFn() : tpGemmKernelFn(), dim3(grid), pair ? tpGemmPairThreads() : tpGemmThreads(),
+  return launchTp(tp, pair ? tpGemmPairKernelFn(width) : tpGemmKernelFn(width), dim3(grid), pair ? tpGemmPairThreads() : tpGemmThreads(),
                   pair ? tpGemmPairSmemBytes() : tpGemmSmemBytes(), args, !fused, 1, stream);
 }
 
@@ -364,8 +437,8 @@ ncclResult_t ncclTpCreate(ncclComm_t comm, size_t maxRows, size_t maxCols, ncclT
   if (cur != comm->cudaDev) CUDACHECK(cudaSetDevice(comm->cudaDev));
   CUDACHECK(cudaDeviceGetAttribute(&tp->smCount, cudaDevAttrMultiProcessorCount, comm->cudaDev));
   // function attributes are per device: set them here, with this context's device current, not once per process
-  CUDACHECK(cudaFuncSetAttribute(tpGemmKernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmSmemBytes()));
-  CUDACHECK(cudaFuncSetAttribute(tpGemmSplitKernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmSplitSmemBytes()));
+  for (int width : kTpWidths) CUDACHECK(cudaFuncSetAttribute(tpGemmKernelFn(width), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmSmemBytes()));
+  for (int width : {128, 256}) CUDACHECK(cudaFuncSetAttribute(tpGemmSplitKernelFn(width), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmSplitSmemBytes()));
   CUDACHECK(cudaFuncSetAttribute(tpGemmFp8KernelFn(true, 256, false), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmFp8SmemBytes()));
   for (int width : {128, 256})
     for (bool split : {false, true})
@@ -378,8 +451,10 @@ ncclResult_t ncclTpCreate(ncclComm_t comm, size_t maxRows, size_t maxCols, ncclT
     cfg.blockDim = dim3(tpGemmPairThreads());
     cfg.dynamicSmemBytes = tpGemmPairSmemBytes();
     int clusters = 0;
-    if (cudaFuncSetAttribute(tpGemmPairKernelFn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmPairSmemBytes()) == cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&clusters, tpGemmPairKernelFn(), &cfg) == cudaSuccess)
+    bool pairsFit = true;
+    for (int width : kTpWidths)
+      pairsFit = pairsFit && cudaFuncSetAttribute(tpGemmPairKernelFn(width), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmPairSmemBytes()) == cudaSuccess;
+    if (pairsFit && cudaOccupancyMaxActiveClusters(&clusters, tpGemmPairKernelFn(256), &cfg) == cudaSuccess)
       tp->pairClusters = std::min(clusters, tp->smCount / 2);
     else
       (void)cudaGetLastError();
@@ -391,7 +466,7 @@ ncclResult_t ncclTpCreate(ncclComm_t comm, size_t maxRows, size_t maxCols, ncclT
       cfg.gridDim = dim3(tp->smCount / size * size);
       cfg.blockDim = dim3(tpGemmSplitThreads());
       cfg.dynamicSmemBytes = tpGemmSplitSmemBytes();
-      if (cudaOccupancyMaxActiveClusters(&clusters, tpGemmSplitKernelFn(), &cfg) == cudaSuccess) tp->splitClusters[size] = clusters;
+      if (cudaOccupancyMaxActiveClusters(&clusters, tpGemmSplitKernelFn(256), &cfg) == cudaSuccess) tp->splitClusters[size] = clusters;
       else (void)cudaGetLastError();
       // both widths have the same threads, registers and shared memory
       cfg.blockDim = dim3(tpGemmFp8Threads());

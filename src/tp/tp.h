@@ -30,6 +30,7 @@ struct TpGemmArgs {
 };
 
 constexpr int kTpMaxSplit = 8;     // largest cluster of CTAs that share the K blocks of a tile
+constexpr int kTpWidths[] = {256, 224, 192, 160, 128};   // tile widths of plain bf16 GEMMs; the fused modes use the first
 
 #if defined(__CUDACC__)
 constexpr int kTpBM = 128, kTpBN = 256;
@@ -80,9 +81,9 @@ __device__ __forceinline__ TileCoord tileOf(const TpGemmArgs& a, int t, int bm =
 }
 #endif
 
-const void* tpGemmKernelFn();
-const void* tpGemmPairKernelFn();      // CTA-pair variant (cluster of two, 256 x 256 tiles): same arguments, W map with 128-row boxes
-const void* tpGemmSplitKernelFn();     // plain C = A * W^T, one 128 x 256 tile per cluster of splitK CTAs
+const void* tpGemmKernelFn(int width);       // tiles of 128 x width (one of kTpWidths), W map with boxes of width rows
+const void* tpGemmPairKernelFn(int width);   // CTA-pair variant (cluster of two, tiles of 256 x width): same arguments, W map with boxes of width / 2 rows
+const void* tpGemmSplitKernelFn(int width);  // plain C = A * W^T, one tile of 128 x width (256 or 128) per cluster of splitK CTAs
 size_t tpGemmSplitSmemBytes();
 int tpGemmSplitThreads();
 // fused: REDUCE and GATHER with more than one rank, tiles of 128 x 256. Others: tiles of 128 x width (256 or 128), split: one tile
