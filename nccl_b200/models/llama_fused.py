@@ -141,9 +141,16 @@ class FusedUnits:
         y, h, _ = self.norm(x, p["norm2"], add=torch.mm(a.transpose(1, 2).reshape(x.shape), p["wo"].t()))
         return y.addmm_(self.swiglu(torch.mm(h, p["w_gu"].t())), p["w_down"].t())
 
-    def layer_backward(self, x, flat, gflat, rope, shape, gy):
-        """Gradient of the layer's input; the weights' gradients go into gflat (laid out like flat)."""
+    def layer_backward(self, x, flat, gflat, rope, shape, gy, ready=None):
+        """Gradient of the layer's input; the weights' gradients go into gflat (laid out like flat). ready(lo) is told that from element lo on
+        the gradients are written and the weights are read no more."""
         p, g = self._layer_views(flat), self._layer_views(gflat)
+        begin = flat.data_ptr()
+
+        def done(name):
+            if ready:
+                ready((p[name].data_ptr() - begin) // flat.element_size())
+
         h1, rstd1, qkv, a = self._up_to_attention(x, p, rope, shape, True)
         o = a.detach().transpose(1, 2).reshape(x.shape)
         x2, h2, rstd2 = self.norm(x, p["norm2"], add=torch.mm(o, p["wo"].t()), need_rstd=True)
@@ -151,13 +158,16 @@ class FusedUnits:
         act = torch.mm(gy, p["w_down"])
         self.swiglu_backward(gu, act)
         torch.mm(gy.t(), act, out=g["w_down"])
+        done("w_down")
         del act
         dh = torch.mm(gu, p["w_gu"])
         torch.mm(gu.t(), h2, out=g["w_gu"])
+        done("w_gu")
         del gu, h2
         g2 = self.norm_backward(x2, p["norm2"], rstd2, dh, gy, g["norm2"])
         torch.mm(g2.t(), o, out=g["wo"])
         do = torch.mm(g2, p["wo"]).view(shape[0], shape[1], self.cfg.heads, self.cfg.head_dim).transpose(1, 2)
+        done("wo")
         dqkv = self.rope_backward(*torch.autograd.grad(a, qkv, do), rope, x.shape[0], shape[1])
         del a, qkv, o, do
         dh = torch.mm(dqkv, p["wqkv"])

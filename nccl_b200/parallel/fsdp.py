@@ -31,6 +31,11 @@ def _align(n, a):
     return (n + a - 1) // a * a
 
 
+# elements of a unit from which one rank updates it in pieces: a piece's launch and event cost the host 15 us, its update at least as much
+# of the GPU's time
+kEarlyUpdate = 1 << 24
+
+
 class _Unit:
     pass
 
@@ -83,9 +88,10 @@ class FSDPEngine:
             u.m = torch.zeros(u.shard, dtype=torch.float32, device=self.device)
             u.v = torch.zeros(u.shard, dtype=torch.float32, device=self.device)
             self.units.append(u)
-        biggest = max(u.padded for u in self.units)
-        self.gbuf = [self._buffer(biggest, torch.bfloat16) for _ in range(2)]
-        self.ggrad = [self._buffer(biggest, torch.bfloat16) for _ in range(2)]
+        # One rank's shards are the whole units: they are gathered and reduced where they lie (nothing is copied).
+        biggest = max(u.padded for u in self.units) if self.n > 1 else 0
+        self.gbuf = [self._buffer(biggest, torch.bfloat16) for _ in range(2 if self.n > 1 else 0)]
+        self.ggrad = [self._buffer(biggest, torch.bfloat16) for _ in range(2 if self.n > 1 else 0)]
         if self.cuda:
             self.comm_stream = torch.cuda.Stream(device=self.device)
             ev = lambda: torch.cuda.Event()   # noqa: E731
@@ -93,6 +99,7 @@ class FSDPEngine:
             self.ev_free = [ev() for _ in range(2)]
             self.ev_grad_ready = [ev() for _ in range(2)]
             self.ev_grad_free = [ev() for _ in range(2)]
+            self.ev_ready = ev()
             for e in self.ev_free + self.ev_grad_free:
                 e.record()
         self.collectives = 0      # all-gathers + reduce-scatters issued (for reporting)
@@ -122,9 +129,18 @@ class FSDPEngine:
         self._wins, self._allocs = [], []
 
     # ------------------------------------------------------------------ communication
+    def _whole(self, idx, slot):
+        """Where all of the unit's parameters lie once they are gathered."""
+        u = self.units[idx]
+        return self.gbuf[slot][:u.padded] if self.n > 1 else u.param
+
+    def _whole_grad(self, idx, gslot):
+        u = self.units[idx]
+        return self.ggrad[gslot][:u.padded] if self.n > 1 else u.grad
+
     def _gather(self, idx, slot):
         u = self.units[idx]
-        dst = self.gbuf[slot][:u.padded]
+        dst = self._whole(idx, slot)
         if self.cuda:
             with torch.cuda.stream(self.comm_stream):
                 self.comm_stream.wait_event(self.ev_free[slot])
@@ -142,28 +158,34 @@ class FSDPEngine:
         if self.cuda:
             self.ev_free[slot].record(torch.cuda.current_stream())
 
-    def _reduce_and_update(self, idx, gslot):
-        """Reduce-scatter of ggrad[gslot] into the unit's gradient shard, then AdamW on the shard."""
+    def _update_early(self, idx, lo, hi):
+        """One rank: AdamW on elements [lo, hi) of the unit, whose gradients are final and whose weights this step reads no more."""
+        self.ev_ready.record(torch.cuda.current_stream())
+        self.comm_stream.wait_event(self.ev_ready)
+        self._adamw(self.units[idx], self.comm_stream, lo, hi)
+
+    def _reduce_and_update(self, idx, gslot, hi=None):
+        """Reduce-scatter of the unit's gradients into its gradient shard, then AdamW on the shard (its first `hi` elements, if the others are through)."""
         u = self.units[idx]
-        src = self.ggrad[gslot][:u.padded]
+        src = self._whole_grad(idx, gslot)
         if self.cuda:
             self.ev_grad_ready[gslot].record(torch.cuda.current_stream())
             with torch.cuda.stream(self.comm_stream):
                 self.comm_stream.wait_event(self.ev_grad_ready[gslot])
                 self.comm.reduce_scatter(src, u.grad, stream=self.comm_stream)
                 self.ev_grad_free[gslot].record(self.comm_stream)
-                self._adamw(u, self.comm_stream)
+                self._adamw(u, self.comm_stream, 0, hi)
         else:
             self.comm.reduce_scatter(src, u.grad)
             self._adamw(u, None)
         self.collectives += 1
 
-    def _adamw(self, u, stream):
+    def _adamw(self, u, stream, lo=0, hi=None):
         b1, b2 = self.betas
         step = self.step_count
         if self.cuda:
-            rc = self.own.b200FusedAdamW(u.master.data_ptr(), u.m.data_ptr(), u.v.data_ptr(), u.grad.data_ptr(), u.param.data_ptr(), u.shard,
-                                         self.lr, b1, b2, self.eps, self.wd, 1.0 / self.n, step, stream.cuda_stream)
+            rc = self.own.b200FusedAdamW(u.master.data_ptr() + 4 * lo, u.m.data_ptr() + 4 * lo, u.v.data_ptr() + 4 * lo, u.grad.data_ptr() + 2 * lo,
+                                         u.param.data_ptr() + 2 * lo, (u.shard if hi is None else hi) - lo, self.lr, b1, b2, self.eps, self.wd, 1.0 / self.n, step, stream.cuda_stream)
             _lib.check(rc, "b200FusedAdamW", self.own)
             self.kernels += 1
             return
@@ -178,9 +200,9 @@ class FSDPEngine:
     def _grad_flat(self, idx, gslot):
         """The unit's flat gradient buffer, once the reduce-scatter that read it last is through; its padding is zero."""
         u = self.units[idx]
-        if self.cuda:
+        if self.cuda and self.n > 1:
             torch.cuda.current_stream().wait_event(self.ev_grad_free[gslot])
-        flat = self.ggrad[gslot]
+        flat = self._whole_grad(idx, gslot)
         if u.padded > u.numel:
             flat[u.numel:u.padded].zero_()
         return flat[:u.numel]
@@ -204,8 +226,7 @@ class FSDPEngine:
 
         def params(idx, slot, need_grad):
             u = self.units[idx]
-            flat = self.gbuf[slot][:u.numel]
-            vs = M.views(flat, u.shapes)
+            vs = M.views(self._whole(idx, slot)[:u.numel], u.shapes)
             if need_grad:
                 vs = {k: t.detach().requires_grad_(True) for k, t in vs.items()}
             return vs
@@ -222,7 +243,7 @@ class FSDPEngine:
         shape = tuple(tokens.shape)
 
         def weights(idx, slot):
-            return self.gbuf[slot][:self.units[idx].numel]
+            return self._whole(idx, slot)[:self.units[idx].numel]
 
         # forward (the head is differentiated at once: its recompute would be wasted work)
         self._gather(0, 0)
@@ -244,7 +265,6 @@ class FSDPEngine:
         self._wait_gathered(slot)
         if fused:
             loss, gx = fused.head(x, weights(idx, slot), self._grad_flat(idx, slot), targets.reshape(-1).contiguous())
-            self._gather(idx - 1, (idx - 1) % 2)
             self._release(slot)
         else:
             vs = params(idx, slot, True)
@@ -252,23 +272,32 @@ class FSDPEngine:
             loss = run(idx, vs, xin)
             names = [n for n, _ in self.units[idx].shapes]
             grads = torch.autograd.grad(loss, [xin] + [vs[n] for n in names])
-            self._gather(idx - 1, (idx - 1) % 2)
             self._release(slot)
             self._write_grads(idx, slot, grads[1:])
             gx = grads[0]
             del grads, vs, xin
         self._reduce_and_update(idx, slot)
         del x
-        # backward through the layers and the embedding
+        # backward through the layers and the embedding; the last layer's parameters are still gathered from the forward
         for idx in range(U - 2, -1, -1):
             slot = idx % 2
+            u = self.units[idx]
             if idx - 1 >= 0:
                 self._gather(idx - 1, (idx - 1) % 2)
             self._wait_gathered(slot)
             if fused and idx:
-                gx = fused.layer_backward(saved[idx], weights(idx, slot), self._grad_flat(idx, slot), rope, shape, gx)
+                # one rank's large units: the optimizer takes the weights as their gradients come (it is bound by memory, the rest of the
+                # backward by the tensor cores), and little of it is left behind the last unit
+                done = [u.shard]
+                if self.n == 1 and u.numel >= kEarlyUpdate:
+                    def ready(lo):
+                        self._update_early(idx, lo, done[0])
+                        done[0] = lo
+                else:
+                    ready = None
+                gx = fused.layer_backward(saved[idx], weights(idx, slot), self._grad_flat(idx, slot), rope, shape, gx, ready)
                 self._release(slot)
-                self._reduce_and_update(idx, slot)
+                self._reduce_and_update(idx, slot, done[0])
                 saved[idx] = None
                 continue
             if fused and llama_fused.embedding_applies(tokens):
@@ -306,6 +335,6 @@ class FSDPEngine:
             self._wait_gathered(0)
             if self.cuda:
                 torch.cuda.synchronize()
-            out.append(self.gbuf[0][:u.numel].float().cpu().clone())
+            out.append(self._whole(idx, 0)[:u.numel].float().cpu().clone())
             self._release(0)
         return out
