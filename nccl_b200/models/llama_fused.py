@@ -9,7 +9,8 @@ buffers, with the backward written out:
   * weight gradients are written where the reduce-scatter reads them, and the recomputation leaves out the last product,
     whose result no gradient needs.
 
-Between kernels everything is bf16 as before; sums, exponentials and rotations are held in fp32 and rounded once.
+Between kernels everything is bf16 as before; sums, exponentials and rotations are held in fp32. The forward rounds where the
+operations of `llama` round, so that both give the same loss up to the order of sums; the backward rounds each result once.
 """
 import ctypes
 
@@ -123,23 +124,24 @@ class FusedUnits:
         h, qkv, f = c.hidden, (c.heads + 2 * c.kv_heads) * c.head_dim, c.ffn
         return M.views(flat, [("norm1", (h,)), ("wqkv", (qkv, h)), ("wo", (h, h)), ("norm2", (h,)), ("w_gu", (2 * f, h)), ("w_down", (h, f))])
 
-    def _up_to_attention(self, x, p, rope, shape, backward):
-        """(norm1's output and 1 / rms, q, k, v as attention takes them, its output [B, heads, S, head_dim])."""
+    def _up_to_attention(self, x, add, p, rope, shape, backward):
+        """(x + add, norm1's output and 1 / rms, q, k, v as attention takes them, its output [B, heads, S, head_dim])."""
         c, (B, S) = self.cfg, shape
-        _, h, rstd = self.norm(x, p["norm1"], need_rstd=backward)
+        x, h, rstd = self.norm(x, p["norm1"], add=add, need_rstd=backward)
         qkv = torch.mm(h, p["wqkv"].t())
         self.rope(qkv, rope, S)
         q, k, v = (t.transpose(1, 2) for t in qkv.view(B, S, c.heads + 2 * c.kv_heads, c.head_dim).split((c.heads, c.kv_heads, c.kv_heads), dim=2))
         if backward:
             q, k, v = (t.detach().requires_grad_(True) for t in (q, k, v))
-        return h, rstd, (q, k, v), F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
+        return x, h, rstd, (q, k, v), F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
 
-    def layer(self, x, flat, rope, shape):
-        """x [B * S, hidden] -> [B * S, hidden]; shape = (B, S)."""
+    def layer(self, x, add, flat, rope, shape):
+        """The layer of input x + add (add may be None), [B * S, hidden] with shape = (B, S): its input and its output, the latter as two terms
+        that the next unit's norm adds up."""
         p = self._layer_views(flat)
-        _, _, _, a = self._up_to_attention(x, p, rope, shape, False)
+        x, _, _, _, a = self._up_to_attention(x, add, p, rope, shape, False)
         y, h, _ = self.norm(x, p["norm2"], add=torch.mm(a.transpose(1, 2).reshape(x.shape), p["wo"].t()))
-        return y.addmm_(self.swiglu(torch.mm(h, p["w_gu"].t())), p["w_down"].t())
+        return x, y, torch.mm(self.swiglu(torch.mm(h, p["w_gu"].t())), p["w_down"].t())
 
     def layer_backward(self, x, flat, gflat, rope, shape, gy, ready=None):
         """Gradient of the layer's input; the weights' gradients go into gflat (laid out like flat). ready(lo) is told that from element lo on
@@ -151,7 +153,7 @@ class FusedUnits:
             if ready:
                 ready((p[name].data_ptr() - begin) // flat.element_size())
 
-        h1, rstd1, qkv, a = self._up_to_attention(x, p, rope, shape, True)
+        _, h1, rstd1, qkv, a = self._up_to_attention(x, None, p, rope, shape, True)
         o = a.detach().transpose(1, 2).reshape(x.shape)
         x2, h2, rstd2 = self.norm(x, p["norm2"], add=torch.mm(o, p["wo"].t()), need_rstd=True)
         gu = torch.mm(h2, p["w_gu"].t())
@@ -179,11 +181,11 @@ class FusedUnits:
         c, ids = self.cfg, tokens.reshape(-1).contiguous()
         self._run("b200EmbeddingBackward", ids.data_ptr(), gx.data_ptr(), gflat.data_ptr(), ids.numel(), c.vocab, c.hidden)
 
-    def head(self, x, flat, gflat, targets):
-        """(mean loss, gradient of the hidden states); the weights' gradients go into gflat."""
+    def head(self, x, add, flat, gflat, targets):
+        """(mean loss, gradient of the hidden states x + add); the weights' gradients go into gflat."""
         shapes = M.head_shapes(self.cfg)
         p, g = M.views(flat, shapes), M.views(gflat, shapes)
-        _, h, rstd = self.norm(x, p["norm"], need_rstd=True)
+        x, h, rstd = self.norm(x, p["norm"], add=add, need_rstd=True)
         logits = torch.mm(h, p["out"].t())
         loss = self.cross_entropy(logits, targets)
         dh = torch.mm(logits, p["out"])

@@ -247,15 +247,15 @@ class FSDPEngine:
 
         # forward (the head is differentiated at once: its recompute would be wasted work)
         self._gather(0, 0)
-        x = None
+        x = add = None   # a layer leaves its output as two terms
         for idx in range(U - 1):
             self._gather(idx + 1, (idx + 1) % 2)
             self._wait_gathered(idx % 2)
-            saved[idx] = x
             with torch.no_grad():
                 if fused and idx:
-                    x = fused.layer(x, weights(idx, idx % 2), rope, shape)
+                    saved[idx], x, add = fused.layer(x, add, weights(idx, idx % 2), rope, shape)
                 else:
+                    saved[idx] = x
                     x = run(idx, params(idx, idx % 2, False), x)
                     x = x.view(-1, cfg.hidden) if fused else x
             self._release(idx % 2)
@@ -264,7 +264,7 @@ class FSDPEngine:
         slot = idx % 2
         self._wait_gathered(slot)
         if fused:
-            loss, gx = fused.head(x, weights(idx, slot), self._grad_flat(idx, slot), targets.reshape(-1).contiguous())
+            loss, gx = fused.head(x, add, weights(idx, slot), self._grad_flat(idx, slot), targets.reshape(-1).contiguous())
             self._release(slot)
         else:
             vs = params(idx, slot, True)
@@ -277,7 +277,7 @@ class FSDPEngine:
             gx = grads[0]
             del grads, vs, xin
         self._reduce_and_update(idx, slot)
-        del x
+        del x, add
         # backward through the layers and the embedding; the last layer's parameters are still gathered from the forward
         for idx in range(U - 2, -1, -1):
             slot = idx % 2

@@ -37,6 +37,8 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
   return q;
 }
 
+__device__ __forceinline__ float toBf16(float f) { return __bfloat162float(__float2bfloat16_rn(f)); }
+
 // Sum over the block, the same value in every thread. `red` has 32 floats; two calls in a row need a different `red`.
 __device__ __forceinline__ float blockSum(float v, float* red) {
 #pragma unroll
@@ -52,7 +54,8 @@ __device__ __forceinline__ float blockSum(float v, float* red) {
 
 // ---------------------------------------------------------------------------------------------- RMSNorm
 // One CTA per row, V packs of 8 channels per thread kept in registers between the sum of squares and the scaling.
-// sum = x + add when `add` (rounded to bf16, and normalised as rounded), h = sum * rsqrt(mean(sum^2) + eps) * gain.
+// sum = x + add when `add` (rounded to bf16, and normalised as rounded), h = bf16(sum * rsqrt(mean(sum^2) + eps)) * gain: rounded where
+// the model's own operations round, like the activation below, so that the loss is theirs.
 template <int V>
 __global__ void __launch_bounds__(kMaxRowThreads) rmsNormKernel(const uint4* x, const uint4* add, const uint4* gain, uint4* sum, uint4* h, float* rstd,
                                                                int packs, float eps) {
@@ -87,7 +90,7 @@ __global__ void __launch_bounds__(kMaxRowThreads) rmsNormKernel(const uint4* x, 
       float g[8];
       unpack8(gain[p], g);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) g[i] *= f[v][i] * r;
+      for (int i = 0; i < 8; ++i) g[i] *= toBf16(f[v][i] * r);
       h[row + p] = pack8(g);
     }
   }
@@ -240,7 +243,7 @@ __global__ void __launch_bounds__(kMaxRowThreads) ropeBackwardKernel(HeadGrad dq
 }
 
 // ---------------------------------------------------------------------------------------------- SwiGLU
-// gu [rows][gate | up]; act = silu(gate) * up.
+// gu [rows][gate | up]; act = bf16(silu(gate)) * up.
 __global__ void __launch_bounds__(256) swigluKernel(const uint4* gu, uint4* act, int packs) {
   const size_t row = blockIdx.x;
   const int p = blockIdx.y * blockDim.x + threadIdx.x;
@@ -249,7 +252,7 @@ __global__ void __launch_bounds__(256) swigluKernel(const uint4* gu, uint4* act,
   unpack8(gu[row * 2 * packs + p], g);
   unpack8(gu[row * 2 * packs + packs + p], u);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) u[i] *= g[i] / (1.0f + expf(-g[i]));
+  for (int i = 0; i < 8; ++i) u[i] *= toBf16(g[i] / (1.0f + expf(-g[i])));
   act[row * packs + p] = pack8(u);
 }
 
