@@ -751,6 +751,7 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epDispatchLocalKernel(cons
   __shared__ int sHist[kEpMaxLocalExperts];
   __shared__ int sIsLast;
   const int me = a.rank, K = a.topk, E = a.numExperts, T = a.numTokens[me], cap = a.maxTokens;
+  constexpr int kTicketWarp = kEpLocalThreads / 32 - 1;
   const int b = blockIdx.x, grid = gridDim.x;
   uint32_t* st = a.state[me];
   const int64_t* idx = a.topkIdx[me];
@@ -766,9 +767,34 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epDispatchLocalKernel(cons
       if (a.outTopkW[me]) a.outTopkW[me][i] = 0.0f;
     }
   }
+  // One warp takes the CTA's ticket as soon as its last rows are claimed (behind a __syncthreads that follows the claims), while the
+  // others move the payload: at the end of the kernel the counters, a fence and the ticket were trips to memory behind each other.
+  // Rank-major dispatch and combine of 2000 tokens 21.3 -> 20.1 us a pass, with the combine's rows fetched beside the routing.
+  auto takeTicket = [&] {
+    if ((int)threadIdx.x / 32 != kTicketWarp) return;
+    const int lane = threadIdx.x & 31;
+    if (rankMajor)
+      for (int e = lane; e < E; e += 32)
+        if (sHist[e]) atomicAdd(&st[kStCounters + e], (uint32_t)sHist[e]);
+    __syncwarp();
+    if (lane == 0) {
+      __threadfence();
+      sIsLast = atomicAdd(&st[2], 1u) == (uint32_t)grid - 1;
+    }
+  };
+  if (mine == 0) {
+    __syncthreads();
+    takeTicket();
+  }
   for (int base = 0; base < mine; base += kLocTokens) {
     const int batch = mine - base < kLocTokens ? mine - base : kLocTokens;
     const int t0 = b + base * grid;
+    const bool lastBatch = base + kLocTokens >= mine;
+    // the first entries of the batch's routing travel with the first loads of its payload
+    const size_t o0 = (size_t)(t0 + (int)threadIdx.x / K * grid) * K + threadIdx.x % K;
+    const bool has = (int)threadIdx.x < batch * K;
+    const int64_t e0 = has ? idx[o0] : -1;
+    const float w0 = has && rankMajor && a.outTopkW[me] && a.topkW[me] ? a.topkW[me][o0] : 0.0f;
     localPayload<FP8>(a, a.x[me], t0, grid, batch, R, sRow, [&] {
       __syncthreads();   // the previous batch is stored
       if (rankMajor) {
@@ -776,27 +802,28 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epDispatchLocalKernel(cons
         __syncthreads();
         for (int i = threadIdx.x; i < batch * K; i += kEpLocalThreads) {
           const int t = t0 + i / K * grid;
-          const int64_t e = idx[(size_t)t * K + i % K];
+          const int64_t e = i < kEpLocalThreads ? e0 : idx[(size_t)t * K + i % K];
           if (e >= 0 && e < E) {
             sRow[i / K] = t;   // any of the token's entries: the same value
             atomicAdd(&sHist[e], 1);
           }
         }
         __syncthreads();
+        if (lastBatch) takeTicket();
         // the routing row goes with the token; a token without experts leaves its slot unused
         for (int i = threadIdx.x; i < batch * K; i += kEpLocalThreads) {
           const int t = t0 + i / K * grid;
           const size_t o = (size_t)t * K + i % K;
-          const bool any = sRow[i / K] >= 0;
-          const int64_t e = idx[o];
+          const bool any = sRow[i / K] >= 0, early = i < kEpLocalThreads;
+          const int64_t e = early ? e0 : idx[o];
           if (i % K == 0) a.srcInfo[me][t] = any ? make_int2(me, t) : make_int2(-1, 0);
           if (a.outTopkIdx[me]) a.outTopkIdx[me][o] = e >= 0 && e < E ? e : -1;
-          if (a.outTopkW[me]) a.outTopkW[me][o] = any && a.topkW[me] ? a.topkW[me][o] : 0.0f;
+          if (a.outTopkW[me]) a.outTopkW[me][o] = any && a.topkW[me] ? (early ? w0 : a.topkW[me][o]) : 0.0f;
         }
       } else {
         for (int i = threadIdx.x; i < batch * K; i += kEpLocalThreads) {
           const size_t o = (size_t)(t0 + i / K * grid) * K + i % K;
-          const int64_t e = idx[o];
+          const int64_t e = i < kEpLocalThreads ? e0 : idx[o];
           int row = -1;
           if (e >= 0 && e < E) {
             const int s = (int)atomicAdd(&st[kStCounters + e], 1u);
@@ -809,20 +836,11 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epDispatchLocalKernel(cons
           sRow[i] = row;
         }
         __syncthreads();
+        if (lastBatch) takeTicket();
       }
     });
   }
-  if (rankMajor) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < E; e += kEpLocalThreads)
-      if (sHist[e]) atomicAdd(&st[kStCounters + e], (uint32_t)sHist[e]);
-  }
-  // the last CTA publishes the counts and leaves the counters at zero
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    sIsLast = atomicAdd(&st[2], 1u) == (uint32_t)grid - 1;
-  }
+  // the CTA with the last ticket publishes the counts and leaves the counters at zero
   __syncthreads();
   if (!sIsLast) return;
   __threadfence();
@@ -886,6 +904,42 @@ __device__ __forceinline__ void localSums(const __nv_bfloat16* y, int H, int C, 
   }
 }
 
+// The same where row t of y is all that goes into token t, if it has an expert at all: the first rows travel while `lookup` fills sRow.
+template <typename Lookup, typename Store>
+__device__ __forceinline__ void localRows(const __nv_bfloat16* y, int H, int C, int tb, int nItems, int shift, const int* sRow, Lookup lookup, Store store) {
+  constexpr int U = 4;
+  uint4 v[U];
+  auto load = [&](int first) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = first + u * kEpLocalThreads;
+      v[u] = make_uint4(0, 0, 0, 0);
+      if (i < nItems) v[u] = ldStream16(y + (size_t)tb * H + (size_t)(i + shift) * 8);
+    }
+  };
+  load(threadIdx.x);
+  lookup();
+  for (int first = threadIdx.x; first < nItems; first += U * kEpLocalThreads) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = first + u * kEpLocalThreads + shift;
+      if (i - shift >= nItems) continue;
+      const int j = i / C;
+      float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      if (sRow[j] >= 0) {
+        const __nv_bfloat162* p = (const __nv_bfloat162*)&v[u];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          acc[2 * q] += __bfloat162float(p[q].x);
+          acc[2 * q + 1] += __bfloat162float(p[q].y);
+        }
+      }
+      store(j, i - j * C, acc);
+    }
+    load(first + U * kEpLocalThreads);
+  }
+}
+
 // out[t] = sum over the token's selected experts of w * row, in fp32, in slot order. The (token, 8 channels) items are dealt to
 // the CTAs as contiguous ranges; where the rows lie and their weights is looked up once per token and CTA.
 __global__ void __launch_bounds__(kEpLocalThreads, 2) epCombineLocalKernel(const __grid_constant__ EpArgs a) {
@@ -905,29 +959,30 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epCombineLocalKernel(const
   const int tLast = (int)((hi - 1) / C);
   for (int tb = (int)(lo / C); tb <= tLast; tb += kLocTokens) {
     const int batch = tLast - tb + 1 < kLocTokens ? tLast - tb + 1 : kLocTokens;
-    __syncthreads();
-    for (int i = threadIdx.x; i < batch * R; i += kEpLocalThreads) {
-      const int t = tb + i / R;
-      int row = -1;
-      float w = 0.0f;
-      if (rankMajor) {
-        for (int k = 0; k < K && row < 0; ++k) {
-          const int64_t e = idx[(size_t)t * K + k];
-          if (e >= 0 && e < E) row = t;
+    auto lookup = [&] {
+      __syncthreads();
+      for (int i = threadIdx.x; i < batch * R; i += kEpLocalThreads) {
+        const int t = tb + i / R;
+        int row = -1;
+        float w = 0.0f;
+        if (rankMajor) {
+          for (int k = 0; k < K && row < 0; ++k) {
+            const int64_t e = idx[(size_t)t * K + k];
+            if (e >= 0 && e < E) row = t;
+          }
+        } else {
+          const size_t o = (size_t)t * K + i % R;
+          const int64_t e = idx[o];
+          if (e >= 0 && e < E) {
+            row = a.rowOf[o];
+            w = a.topkW[me][o];
+          }
         }
-        w = 1.0f;   // the caller has weighted the rows
-      } else {
-        const size_t o = (size_t)t * K + i % R;
-        const int64_t e = idx[o];
-        if (e >= 0 && e < E) {
-          row = a.rowOf[o];
-          w = a.topkW[me][o];
-        }
+        sRow[i] = row;
+        sW[i] = w;
       }
-      sRow[i] = row;
-      sW[i] = w;
-    }
-    __syncthreads();
+      __syncthreads();
+    };
     const size_t first = (size_t)tb * C > lo ? (size_t)tb * C : lo;
     const size_t end = (size_t)(tb + batch) * C < hi ? (size_t)(tb + batch) * C : hi;
     const int nItems = (int)(end - first), shift = (int)(first - (size_t)tb * C);
@@ -938,6 +993,11 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epCombineLocalKernel(const
       for (int k = 0; k < 4; ++k) q[k] = __floats2bfloat162_rn(acc[2 * k], acc[2 * k + 1]);
       st16(out + (size_t)(tb + j) * H + (size_t)c * 8, o);
     };
+    if (rankMajor) {   // the caller has weighted the rows
+      localRows(y, H, C, tb, nItems, shift, sRow, lookup, store);
+      continue;
+    }
+    lookup();
     if (R == 1) localSums<1>(y, H, C, nItems, shift, R, sRow, sW, store);
     else if (R == 2) localSums<2>(y, H, C, nItems, shift, R, sRow, sW, store);
     else if (R <= 4) localSums<4>(y, H, C, nItems, shift, R, sRow, sW, store);

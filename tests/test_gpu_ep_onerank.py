@@ -138,3 +138,26 @@ def test_counts_outside_the_gpu(comm, layout):
     torch.cuda.synchronize()
     assert comm.async_error() == 0
     ep.destroy()
+
+
+@pytest.mark.parametrize("layout", ["expert_major", "rank_major"])
+def test_calls_in_a_row_leave_no_counts_behind(comm, layout):
+    """Tickets are taken before the payload is through: calls behind each other without waiting, of changing sizes, none among them."""
+    from nccl_b200.ops.ep import ExpertParallel
+    E, K, H, cap = 64, 6, 2048, 900
+    ep = ExpertParallel(comm, E, cap, H, layout=layout)
+    got, want = [], []
+    for T in (900, 1, 513, 64, 899, 3):
+        x, idx, w = _batch(T, E, K, H, T, 0.2)
+        counts = torch.full((E,), 7, dtype=torch.int32, device="cuda")
+        toks = ep.dispatch(x, idx, w, fp8=False, counts=counts)[0].clone()
+        valid = idx >= 0
+        scale = (w * valid).sum(1, keepdim=True) if layout == "expert_major" else valid.any(1, keepdim=True)
+        got.append((counts, ep.combine(toks)[:T].clone()))
+        want.append((torch.bincount(idx[valid], minlength=E), x.float() * scale))
+    torch.cuda.synchronize()
+    for (c, out), (cr, ref) in zip(got, want):
+        assert torch.equal(c.long(), cr)
+        torch.testing.assert_close(out.float(), ref, rtol=2 ** -7, atol=1e-6)
+    assert comm.async_error() == 0
+    ep.destroy()
