@@ -149,22 +149,31 @@ __global__ void __launch_bounds__(kThreads) devApiArRmsNormKernel(ncclDevComm_t 
 // One rank: x = partial + residual, residual <- x, out <- rmsnorm(x) * weight, as above without the sources to wait for.
 // Bound by memory on the SMs that the caller grants, so what counts is how much each of them has in flight: a producer warp
 // streams chunks of R neighbouring rows (partial and residual) into a ring of shared memory with bulk copies, groups of G
-// threads take one row each from there. 2048 rows of 8192 take 36 us a call on 64 CTAs; with a CTA to a row, its loads waiting for
-// the previous row's stores, they took 127.
+// threads take one row each from there. 2048 rows of 8192 take 34 us a call on 64 CTAs; with a CTA to a row, its loads waiting for
+// the previous row's stores, they took 127. Values are added, squared and scaled in pairs, and the gains stay in registers from row to
+// row (40 % fewer instructions: 2048 rows of 4096 20.9 -> 19.1 us, 4096 of 8192 63.0 -> 61.8); 56 registers and 1024 threads spilled.
 constexpr int kRowPacks = 8;          // 16-byte packs of a row per thread, at most
 constexpr int kRowStages = 16;        // chunks in the ring, at most
 constexpr size_t kRowRing = 200 << 10;
 constexpr int kRowThreads = kThreads + 32;
 constexpr int kStatusRing = 6;        // status word: a wait on the ring ran out
 
-// bf16 is the upper half of fp32
-__device__ __forceinline__ void unpackBf16(float (&x)[8], uint4 v) {
-  const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+// Pairs of values: bf16 is the upper half of fp32.
+__device__ __forceinline__ uint64_t unpackBf16x2(uint32_t u) { return b200::sm100::packF32x2(u << 16, u & 0xffff0000u); }
+__device__ __forceinline__ uint64_t mulF32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// The exact sum rounded once, which is what fp32 gives too: where a sum of two bf16 numbers does not fit into fp32, the smaller one is
+// far below a tie of the larger.
+__device__ __forceinline__ uint4 addBf16(const uint4& a, const uint4& b) {
+  uint4 r;
+  const __nv_bfloat162 *x = (const __nv_bfloat162*)&a, *y = (const __nv_bfloat162*)&b;
+  __nv_bfloat162* z = (__nv_bfloat162*)&r;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    x[2 * i] = __uint_as_float(u[i] << 16);
-    x[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
-  }
+  for (int i = 0; i < 4; ++i) z[i] = __hadd2_rn(x[i], y[i]);
+  return r;
 }
 
 struct RowArgs {
@@ -180,7 +189,6 @@ struct RowArgs {
 template <int G>
 __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid_constant__ RowArgs a) {
   using namespace b200::sm100;
-  using V = nccl_device::Vec16<__nv_bfloat16>;
   constexpr int kGroups = kThreads / G, kWarps = G / 32;
   extern __shared__ uint8_t ringRaw[];
   uint8_t* ring = (uint8_t*)(((uintptr_t)ringRaw + 127) & ~(uintptr_t)127);
@@ -229,6 +237,10 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
   } else {
     const int grp = threadIdx.x / G, tid = threadIdx.x % G;
     const int packs = a.hidden / 8;
+    uint4 gain[kRowPacks];   // the same channels of every row
+#pragma unroll
+    for (int k = 0; k < kRowPacks; ++k)
+      if (tid + k * G < packs) gain[k] = *(const uint4*)(a.weight + (size_t)(tid + k * G) * 16);
     int parity = 0;
     // row n of this CTA: row n % R of its chunk n / R
     for (int n = grp;; n += kGroups, parity ^= 1) {
@@ -243,24 +255,23 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
       const uint8_t* part = ring + (size_t)s * 2 * half + r * rowBytes;
       char* res = a.residual + t * rowBytes;
       uint4 sum[kRowPacks];
-      float ss = 0.0f;
+      uint64_t squares = 0;   // two fp32 sums
 #pragma unroll
       for (int k = 0; k < kRowPacks; ++k) {
         const int pk = tid + k * G;
         if (pk < rowPacks) {
-          float x[8], y[8];
-          unpackBf16(x, *(const uint4*)(part + (size_t)pk * 16));
-          unpackBf16(y, *(const uint4*)(part + half + (size_t)pk * 16));
-#pragma unroll
-          for (int j = 0; j < 8; ++j) x[j] += y[j];
           // the residual stream is kept in bf16: normalise exactly what is stored
-          sum[k] = V::pack(x);
+          sum[k] = addBf16(*(const uint4*)(part + (size_t)pk * 16), *(const uint4*)(part + half + (size_t)pk * 16));
           *(uint4*)(res + (size_t)pk * 16) = sum[k];
-          unpackBf16(x, sum[k]);
+          const uint32_t u[4] = {sum[k].x, sum[k].y, sum[k].z, sum[k].w};
 #pragma unroll
-          for (int j = 0; j < 8; ++j) ss += x[j] * x[j];
+          for (int j = 0; j < 4; ++j) {
+            const uint64_t x = unpackBf16x2(u[j]);
+            fmaF32x2(squares, x, x);
+          }
         }
       }
+      float ss = __uint_as_float((uint32_t)squares) + __uint_as_float((uint32_t)(squares >> 32));
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
       if (kWarps > 1) {
@@ -273,17 +284,23 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
       }
       if (tid == 0 && ok) mbarArrive(smemAddr(&emptyBar[s]));   // the whole group has read the row
       const float inv = rsqrtf(ss / (float)a.hidden + a.eps);
+      const uint64_t inv2 = packF32x2(__float_as_uint(inv), __float_as_uint(inv));
       char* out = a.out + t * rowBytes;
 #pragma unroll
       for (int k = 0; k < kRowPacks; ++k) {
         const int pk = tid + k * G;
         if (pk < rowPacks) {
-          float w[8], x[8];
-          unpackBf16(w, *(const uint4*)(a.weight + (size_t)pk * 16));
-          unpackBf16(x, sum[k]);
+          const uint32_t u[4] = {sum[k].x, sum[k].y, sum[k].z, sum[k].w};
+          uint32_t g[4] = {gain[k].x, gain[k].y, gain[k].z, gain[k].w}, o[4];
+          // keeps the gains packed: unpacked ahead of the loop over the rows they would not fit
+          asm volatile("" : "+r"(g[0]), "+r"(g[1]), "+r"(g[2]), "+r"(g[3]));
 #pragma unroll
-          for (int j = 0; j < 8; ++j) w[j] *= x[j] * inv;
-          *(uint4*)(out + (size_t)pk * 16) = V::pack(w);
+          for (int j = 0; j < 4; ++j) {
+            const uint64_t y = mulF32x2(mulF32x2(unpackBf16x2(u[j]), inv2), unpackBf16x2(g[j]));
+            const __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float((uint32_t)y), __uint_as_float((uint32_t)(y >> 32)));
+            o[j] = *(const uint32_t*)&b;
+          }
+          *(uint4*)(out + (size_t)pk * 16) = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
     }
