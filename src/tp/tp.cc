@@ -122,13 +122,12 @@ static void fillSyncTp(ncclComm* comm, SyncArgs* s) {
   s->timeoutNs = dp ? dp->timeoutNs : 5000000000ull;
 }
 
-// CTAs that share the K blocks of a tile in a plain bf16 GEMM, 1 for none: as many as leave every cluster resident at once,
+// Parts of K that a plain bf16 GEMM sums by themselves, 1 for none, and the CTAs that share a tile of 256 columns: as many as leave every cluster resident at once,
 // when the 128 x 256 tiles alone would leave half of the SMs idle, and each CTA keeps kSplitMinBlocks K blocks. Where short loops save
 // no more than the exchange of the partial sums costs, a CTA keeps its tile. Kernel times against the kernel that the call would
 // take instead, weights from memory and from L2, 4 to 72 tiles. One CTA to a tile: K = 1024 1.01-1.10, 1280 0.94-1.05, 1536
 // 0.87-1.00, 1792 0.84-0.96, 2560 0.71-0.88. CTA pairs: K = 1024 0.95-1.03, 1280 0.92-1.00, 2560 0.80-0.90.
 constexpr int kSplitMinBlocks = 8, kSplitFromOne = 1536 / 64;   // clusters on tiles of 256 columns
-constexpr int kNarrowMaxSplit = 5;                              // clusters on tiles of 128 columns: six and eight CTAs gained nothing more
 static int splitOf(const ncclTpContext* tp, const TpGemmArgs* a, bool insteadOfPairs) {
   const int tiles = (a->M / 128) * (a->N / 256), blocks = a->K / 64;
   if (!insteadOfPairs && blocks < kSplitFromOne) return 1;
@@ -139,23 +138,24 @@ static int splitOf(const ncclTpContext* tp, const TpGemmArgs* a, bool insteadOfP
 
 static ncclResult_t launchGemmSplit(ncclTpContext* tp, const void* A, const void* W, TpGemmArgs* a, int width, cudaStream_t stream) {
   CUtensorMap tmA, tmB;
+  tpGemmSplitPlan(a, width);
   NCCLCHECK(makeMap(&tmA, A, a->M, a->K, 128));
   NCCLCHECK(makeMap(&tmB, W, a->N, a->K, width));
   void* args[3] = {&tmA, &tmB, a};
   return launchTp(tp, tpGemmSplitKernelFn(width), dim3((a->M / 128) * (a->N / width) * a->splitK), tpGemmSplitThreads(), tpGemmSplitSmemBytes(), args, true, a->splitK, stream);
 }
 
-// How a plain bf16 GEMM runs: one-CTA tiles of 128 x width, CTA pairs (256 x width), or clusters of `split` CTAs that share the K steps of a
-// tile of 128 x width.
+// How a plain bf16 GEMM runs: one-CTA tiles of 128 x width, CTA pairs (256 x width), or (shares > 1) clusters of `split` CTAs that share the K
+// steps of a tile of 128 x width.
 struct GemmPlan {
   bool pair = false;
-  int width = 256, split = 1;
+  int width = 256, split = 1, shares = 1;
 };
 
 // Tiles of 256 columns, by what the widths below do not change: clusters for few tiles, else pairs where they pay.
 static GemmPlan basePlan(const ncclTpContext* tp, const TpGemmArgs* a, bool pairs) {
   GemmPlan p;
-  p.split = splitOf(tp, a, pairs && a->M % 256 == 0);
+  p.split = p.shares = splitOf(tp, a, pairs && a->M % 256 == 0);
   if (p.split > 1) return p;
   p.pair = pairs;
   if (p.pair && a->M % 256) {
@@ -179,9 +179,11 @@ static int wavesOf(const ncclTpContext* tp, const TpGemmArgs* a, const GemmPlan&
 }
 
 // Expected time in us, operands in L2: start and last store, K steps of 64 with every SM at work, what a wave of tiles adds, and the
-// exchange of a cluster. Fitted to 31 shapes of 4 to 2048 tiles and 8 to 128 K steps; up to four waves it is within about 10 %.
+// exchange of a cluster. Fitted to 31 shapes of 4 to 2048 tiles and 8 to 128 K steps, the shared forms to 32; up to four waves it is
+// within about 10 %.
 static float expectedUs(const ncclTpContext* tp, const TpGemmArgs* a, const GemmPlan& p) {
-  const int steps = a->K / 64, share = (steps + p.split - 1) / p.split, waves = p.split > 1 ? 1 : wavesOf(tp, a, p);
+  const int steps = a->K / 64, own = (p.shares + p.split - 1) / p.split, waves = p.shares > 1 ? 1 : wavesOf(tp, a, p);
+  const int share = p.shares > 1 ? (steps * own + p.shares - 1) / p.shares : steps;   // K steps of a CTA
   float step;
   switch (p.width) {
     case 128: step = p.pair ? 0.23f : 0.21f; break;
@@ -190,35 +192,55 @@ static float expectedUs(const ncclTpContext* tp, const TpGemmArgs* a, const Gemm
     case 224: step = p.pair ? 0.315f : 0.38f; break;
     default: step = p.pair ? 0.35f : 0.385f; break;
   }
-  const float exchange = p.split == 1 ? 0.0f : p.width == 128 ? 2.0f + 0.4f * p.split : p.split == 2 ? 2.2f : 6.5f;
+  float exchange = 0.0f;
+  if (p.shares > 1 && p.split == 1) {   // nothing to exchange: the sums are in the CTA's own tensor memory
+    exchange = 0.6f;
+    step = 0.235f;
+  } else if (p.shares > 1) {
+    exchange = p.width == 256 ? (p.split == 2 ? 2.2f : p.split == 3 ? 4.0f : 5.5f) : 2.0f + 0.4f * p.split + (p.split == 3 ? 0.6f : 0.0f);   // three: one has two chunks
+  }
   return (p.pair ? 4.1f : 3.3f) + waves * share * step + (waves - 1) * 0.8f + exchange;
 }
 
 // Narrower tiles, alone or shared by a cluster, where 256 columns leave the last wave (or all but a few SMs) empty: a step of 160 columns
 // takes 0.65 of the time of one of 256, so what counts is how the tiles fill the chip. Up to four waves of pair tiles: beyond, the
 // last wave matters less and the widest tiles have the best rate (8192 x 8192 x 3584: pairs of 256 303 us, 224 312, 192 349).
-// Kernel times with 256 columns / the choice, us: 128 x 1024 x 2048 10.3 / 7.3 (128 columns, four CTAs), 128 x 4096 x 4096 18.5 / 12.8,
-// 128 x 8192 x 8192 30.4 / 28.3 (two CTAs; memory), 512 x 4096 x 1024 10.6 / 7.7 (128 columns), 1152 x 2304 x 7168 40.6 / 31.8 (160),
-// 2048 x 2560 x 4096 46.1 / 35.4 (160), 1280 x 4096 x 3584 38.4 / 31.9 (pairs of 192), 2560 x 3072 x 2048 25.6 / 23.7 (pairs of 224).
+// Kernel times with 256 columns / the choice, us: 1152 x 2304 x 7168 40.6 / 31.8 (160 columns), 2048 x 2560 x 4096 46.1 / 35.4 (160),
+// 1280 x 4096 x 3584 38.4 / 31.9 (pairs of 192), 2560 x 3072 x 2048 25.6 / 23.7 (pairs of 224).
 // The other side of the line: 1920 x 4096 x 7168 82.3 with pairs of 256, 91.7 of 192; 3328 x 4096 x 1536 29.5 / 31.7.
+// The width never changes the sums: where K is summed in shares it stays so, with an accumulator per share. Weights from memory: 128 x
+// 1024 x 2048 10.2 / 7.5 (128 columns, four CTAs), 128 x 4096 x 4096 17.5 / 14.3 (six shares on four CTAs), 128 x 8192 x 8192 29.7 / 29.3 (four on
+// two), 512 x 4096 x 1024 10.2 / 8.2 (two on one); 896 x 1536 x 3264 stays, 14.7 / 17.2 (three on one). Fewer shares would be faster by what their sums
+// cost to exchange (12.5, 28.3 and 7.5 us for the second to fourth shape), but twice as many results would not be the rounded product
+// (0.25 % for 0.12 % of the third).
 static GemmPlan planGemm(const ncclTpContext* tp, const TpGemmArgs* a, bool pairs) {
   GemmPlan best = basePlan(tp, a, pairs);
   for (int w : kTpWidths)
     if (w == paramTpWidth()) {
-      if (best.split == 1) best.width = w;
+      if (best.shares == 1) best.width = w;
       return best;
     }
   if (((a->M + 255) / 256 * (a->N / 256) + tp->smCount / 2 - 1) / (tp->smCount / 2) > 4) return best;
-  float us = 0.95f * expectedUs(tp, a, best);   // what is simpler stays where the others are hardly faster
+  float us = (best.shares > 1 ? 0.97f : 0.95f) * expectedUs(tp, a, best);   // what is simpler stays where the others are hardly faster
   auto consider = [&](const GemmPlan& p) {
     const float t = expectedUs(tp, a, p);
     if (t < us) { us = t; best = p; }
   };
+  auto earlySums = [](int split, int shares) {
+    TpGemmArgs form = {};
+    form.splitK = split;
+    form.shares = shares;
+    return tpGemmSplitPlan(&form, 128);
+  };
+  const int shares = best.shares, tiles = a->M / 128 * (a->N / 128);
+  if (shares > 1) {
+    for (int s = (shares + kTpMaxOwnShares - 1) / kTpMaxOwnShares; s <= shares && tiles <= (s > 1 ? tp->splitClusters[s] : tp->smCount); ++s)
+      if (earlySums(s, shares) <= kTpMaxEarly) consider({false, 128, s, shares});
+    return best;
+  }
   for (int w : kTpWidths)
     for (bool pair : {false, true})
-      if (pairs || !pair) consider({pair, w, 1});
-  const int tiles = a->M / 128 * (a->N / 128), most = std::min(std::min((int)paramTpSplit(), kNarrowMaxSplit), a->K / 64);
-  for (int s = 2; s <= most && tiles <= tp->splitClusters[s]; ++s) consider({false, 128, s});
+      if (pairs || !pair) consider({pair, w});
   return best;
 }
 
@@ -234,7 +256,8 @@ static ncclResult_t launchGemm(ncclTpContext* tp, const void* A, const void* W, 
   if (fused) plan.pair = pairs && a->M % (256 * n) == 0;
   else plan = planGemm(tp, a, pairs);
   a->splitK = plan.split;
-  if (plan.split > 1) return launchGemmSplit(tp, A, W, a, plan.width, stream);
+  a->shares = plan.shares;
+  if (plan.shares > 1) return launchGemmSplit(tp, A, W, a, plan.width, stream);
   const bool pair = plan.pair;
   const int width = plan.width;
   int commCtas = gather ? tpCommCtas(tp, n) : 0;

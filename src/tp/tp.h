@@ -10,6 +10,11 @@ enum TpMode : int {
   TP_MODE_GATHER = 2,   // all-gather -> GEMM: comm CTAs pull remote row blocks while the GEMM runs
 };
 
+constexpr int kTpMaxSplit = 8;     // largest cluster of CTAs that share the K blocks of a tile
+constexpr int kTpMaxOwnShares = 4; // of a CTA of the bf16 split kernel, on tiles of 128 columns
+constexpr int kTpMaxEarly = 4;     // sums of 32 columns behind the operand ring: four stages of operands stay
+constexpr int kTpWidths[] = {256, 224, 192, 160, 128};   // tile widths of plain bf16 GEMMs; the fused modes use the first
+
 struct TpGemmArgs {
   void* C;                        // bf16 output [M, ldc] (STORE / GATHER)
   int ldc;
@@ -20,7 +25,12 @@ struct TpGemmArgs {
   int M, N, K;
   int mode;
   int rank, nRanks;
-  int splitK;                     // split kernel: CTAs of a cluster that share the K blocks of a tile
+  int splitK;                     // CTAs of a cluster that share the K blocks of a tile
+  int shares;                     // bf16 split kernel: parts of K with a sum each, splitK or (tiles of 128 columns) up to four times as many
+  // bf16 split kernel, filled by tpGemmSplitPlan: first share of each CTA of a cluster, sums of a chunk that CTA c as their owner takes in
+  // while it still multiplies, and the most of them in one CTA
+  uint8_t firstShare[kTpMaxSplit + 1], earlySums[kTpMaxSplit];
+  int early;
   int gemmCtas;                   // GATHER: CTAs [0, gemmCtas) compute, the rest gather
   SyncArgs sync;
   // block-scaled fp8 (e4m3) operands: A scaled per row and 128 columns, W per 128 x 128 block
@@ -28,9 +38,6 @@ struct TpGemmArgs {
   const float* scaleW;            // [K/128][N/128]
   size_t scaleOffset;             // GATHER, fp8: byte offset of the scales inside every rank's activation window
 };
-
-constexpr int kTpMaxSplit = 8;     // largest cluster of CTAs that share the K blocks of a tile
-constexpr int kTpWidths[] = {256, 224, 192, 160, 128};   // tile widths of plain bf16 GEMMs; the fused modes use the first
 
 #if defined(__CUDACC__)
 constexpr int kTpBM = 128, kTpBN = 256;
@@ -83,7 +90,8 @@ __device__ __forceinline__ TileCoord tileOf(const TpGemmArgs& a, int t, int bm =
 
 const void* tpGemmKernelFn(int width);       // tiles of 128 x width (one of kTpWidths), W map with boxes of width rows
 const void* tpGemmPairKernelFn(int width);   // CTA-pair variant (cluster of two, tiles of 256 x width): same arguments, W map with boxes of width / 2 rows
-const void* tpGemmSplitKernelFn(int width);  // plain C = A * W^T, one tile of 128 x width (256 or 128) per cluster of splitK CTAs
+const void* tpGemmSplitKernelFn(int width);  // plain C = A * W^T, one tile of 128 x width (256 or 128) per cluster of splitK CTAs, K in `shares` sums
+int tpGemmSplitPlan(TpGemmArgs* a, int width);   // from splitK and shares; returns `early`, and above kTpMaxEarly there is no such form
 size_t tpGemmSplitSmemBytes();
 int tpGemmSplitThreads();
 // fused: REDUCE and GATHER with more than one rank, tiles of 128 x 256. Others: tiles of 128 x width (256 or 128), split: one tile

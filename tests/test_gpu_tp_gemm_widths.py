@@ -12,7 +12,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(128, 256, 64), (256, 256, 128), (384, 1280, 192), (512, 2304, 320), (2048, 4096, 64), (2176, 2304, 1024), (128, 512, 448),
-          # by rule: 128 columns with 4 CTAs, 5, 3, 2 and alone; 160; pairs of 192; pairs of 224; 192
+          # by rule: 128 columns with 4 shares of K on 4 CTAs, 8 on 8, 6 on 4, 4 on 2 and 2 on one; 160; pairs of 192; pairs of 224; 192
           (128, 1024, 2048), (128, 1024, 7168), (128, 4096, 4096), (128, 8192, 2112), (512, 4096, 1024), (2048, 2560, 1024), (768, 8192, 1024),
           (2560, 3072, 1024), (1792, 3328, 512), (1152, 2304, 1600)]
 
