@@ -153,6 +153,9 @@ inline bool flagSet(const volatile uint32_t* f) { return f && __atomic_load_n((c
 inline bool commValid(const ncclComm* c) { return c && c->startMagic == kCommMagic && c->endMagic == kCommMagic; }
 ncclResult_t commEnsureReady(ncclComm* c);  // waits for / reports the state of a non-blocking init
 
+// Communicators of this process with more than one rank, from their creation until they are gone: init.cc
+int peerComms();
+
 // process-wide checkpoint calls walk the live communicators: contrib/checkpoint.cc
 void checkpointCommAdd(ncclComm* comm);
 void checkpointCommRemove(ncclComm* comm);

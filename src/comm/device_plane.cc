@@ -39,7 +39,7 @@ B200_PARAM(StagePipeline, "B200_STAGE_PIPELINE", 1, "Reductions on unregistered 
 B200_PARAM(StagePipelineMin, "B200_STAGE_PIPELINE_MIN", 67108864, "Smallest message in bytes that is pipelined through the staging area")
 B200_PARAM(P2pDirect, "B200_P2P_DIRECT", 1, "Large sends write straight into a receive buffer that lies in a registered window (rendezvous) instead of going through the mailbox")
 B200_PARAM(LLCtas, "B200_LL_CTAS", 0, "CTAs of the flagged-line kernels (0: one per 512 lines, at most 64)")
-B200_PARAM(LaunchPdl, "B200_PDL", 1, "Programmatic stream serialisation of collective launches (a kernel is scheduled while the previous one of the stream drains): 0 never, 1 yes, but for the flagged-line kernels only up to NCCL_B200_PDL_MAX_CTAS CTAs, 2 always")
+B200_PARAM(LaunchPdl, "B200_PDL", 1, "Programmatic stream serialisation of launches (a kernel is scheduled while the previous one of the stream drains): 0 never, 1 yes, but for the flagged-line kernels only up to NCCL_B200_PDL_MAX_CTAS CTAs, and for kernels without a partner on another GPU (plain GEMMs, quantisers, one-rank copies, scaling, expert parallelism and RMSNorm) only while the process has no communicator of several ranks, 2 always")
 B200_PARAM(LaunchPdlMaxCtas, "B200_PDL_MAX_CTAS", 4, "Largest grid of a flagged-line kernel that is launched with programmatic stream serialisation: measured between two such kernels, the gap is 1.5 us against 2.4 us without it for one CTA, about equal at four CTAs, and 3 to 3.5 us from eight CTAs on")
 // Whether a launch of `ctas` CTAs asks for programmatic stream serialisation. The flagged-line kernels (`shortKernel`) last a few
 // microseconds, so the gap to the next kernel is a large part of a call: there the attribute is dropped for the grids where it
@@ -49,7 +49,11 @@ static inline bool pdlFor(int ctas, bool shortKernel) {
   if (paramLaunchPdl() == 0) return false;
   return !shortKernel || ctas <= paramLaunchPdlMaxCtas();
 }
-bool devPlanePdl() { return paramLaunchPdl() != 0; }
+// Kernels without a partner on another GPU. Collectives let their successors start as soon as they have started themselves, and then wait
+// for peers: a plain kernel behind one of them would hold SMs, shared and tensor memory all that time, which kernels on other streams (the
+// one that a peer waits for among them) may need. The predecessor on the stream may be a collective of any communicator, so
+// only a process without communicators of several ranks asks for the overlap; there it is worth 2 to 2.4 us a call.
+bool devPlanePdl() { return paramLaunchPdl() == 2 || (paramLaunchPdl() == 1 && peerComms() == 0); }
 B200_PARAM(BarrierMulticast, "B200_BARRIER_MC_MIN_RANKS", -1, "Cross-GPU barriers arrive with one multimem.red on a multicast alias of the flag page from this many ranks on (0 = never, -1 = from the selection table)")
 
 // ------------------------------------------------------------------------------------ tuning
@@ -411,7 +415,7 @@ static ncclResult_t scaleCopy(ncclComm* comm, ncclDataType_t type, const void* s
   const size_t perCta = 512 * 4 * 16;   // bytes that a CTA of the kernel moves in one tile
   int ctas = (int)std::min<size_t>((count * typeSize(type) + perCta - 1) / perCta, (size_t)comm->devPlane->smCount * 16);
   comm->devPlane->launches++;
-  return launchKernel(scaleKernelFn(type), dim3(std::max(ctas, 1)), dim3(512), 0, &sa, stream, false, pdlFor(ctas, false));
+  return launchKernel(scaleKernelFn(type), dim3(std::max(ctas, 1)), dim3(512), 0, &sa, stream, false, devPlanePdl());
 }
 
 void sliceEven(size_t count, size_t es, int n, size_t* begin, size_t* cnt) {
@@ -932,7 +936,7 @@ static ncclResult_t runOneRank(ncclComm* comm, const Task& t) {
     size_t perCta = (size_t)threads * unroll * 16;
     int ctas = (int)std::min<size_t>((bytes + perCta - 1) / perCta, (size_t)comm->devPlane->smCount * paramCopyCtasPerSm());
     comm->devPlane->launches++;
-    NCCLCHECK(launchKernel(localCopyKernelFn(unroll, src, dst), dim3(std::max(ctas, 1)), dim3(threads), 0, &ca, t.stream, false, pdlFor(ctas, false)));
+    NCCLCHECK(launchKernel(localCopyKernelFn(unroll, src, dst), dim3(std::max(ctas, 1)), dim3(threads), 0, &ca, t.stream, false, devPlanePdl()));
   }
   return ncclSuccess;
 }

@@ -78,7 +78,8 @@ ncclResult_t devPlaneRunReshard(ncclComm* comm, SymWindow* win, const ReshardRun
                                 size_t totalBytes, cudaStream_t stream);
 ncclResult_t devPlaneCheckStatus(ncclComm* comm);   // turns a kernel-side time-out into an async error
 void tuningDefaults(TuningTable* t);
-// Whether kernels without a partner on another GPU are launched with programmatic stream serialisation.
+// Whether kernels without a partner on another GPU are launched with programmatic stream serialisation: while no kernel of this process can
+// be waiting for a peer.
 bool devPlanePdl();
 ncclResult_t tuningLoadFile(TuningTable* t, const char* path);
 // Predicted duration (microseconds) of a task, used by ncclGroupSimulateEnd.

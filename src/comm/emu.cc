@@ -249,6 +249,8 @@ int b200EmuP2p(void* ctx, int nOps, const int* opRank, const int* peer, const in
 extern "C" unsigned long long b200CommLaunchCount(ncclComm_t comm) {
   return (commValid(comm) && comm->devPlane) ? comm->devPlane->launches : 0;
 }
+// whether a plain kernel launched now would overlap the end of the kernel before it
+extern "C" int b200PlainLaunchesOverlap() { return devPlanePdl() ? 1 : 0; }
 extern "C" int b200CommIsSymmetric(ncclComm_t comm) { return commValid(comm) && comm->lsaAll ? 1 : 0; }
 extern "C" int b200CommHasMulticast(ncclComm_t comm) { return commValid(comm) && comm->sym && comm->sym->mcUsable ? 1 : 0; }
 

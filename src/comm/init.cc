@@ -37,6 +37,9 @@ const char* algoName(int a) {
   return a >= 0 && a < ALGO_COUNT ? n[a] : "Auto";
 }
 
+static std::atomic<int> gPeerComms{0};
+int peerComms() { return gPeerComms.load(); }
+
 static std::mutex gInitLock;
 static bool gInitDone = false;
 static ncclResult_t libInit() {
@@ -206,6 +209,7 @@ static void freeComm(ncclComm* comm) {
   else if (comm->abortFlag) cudaFreeHost((void*)comm->abortFlag);
   (void)cudaGetLastError();
   comm->startMagic = comm->endMagic = 0;
+  if (comm->nRanks > 1) --gPeerComms;   // none of its kernels is left
   delete comm;
 }
 
@@ -256,6 +260,7 @@ static ncclResult_t commCreate(ncclComm** out, const InitArgs& ia, const ncclCon
     if (cudaGetDevice(&comm->cudaDev) != cudaSuccess) { (void)cudaGetLastError(); delete comm; return ncclUnhandledCudaError; }
     comm->nvmlDev = comm->cudaDev;
   }
+  if (comm->nRanks > 1) ++gPeerComms;   // freeComm takes it off
   *out = comm;
   if (comm->config.blocking) {
     ncclResult_t r = initBody(comm, ia);
