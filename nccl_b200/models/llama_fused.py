@@ -143,9 +143,9 @@ class FusedUnits:
         y, h, _ = self.norm(x, p["norm2"], add=torch.mm(a.transpose(1, 2).reshape(x.shape), p["wo"].t()))
         return x, y, torch.mm(self.swiglu(torch.mm(h, p["w_gu"].t())), p["w_down"].t())
 
-    def layer_backward(self, x, flat, gflat, rope, shape, gy, ready=None):
-        """Gradient of the layer's input; the weights' gradients go into gflat (laid out like flat). ready(lo) is told that from element lo on
-        the gradients are written and the weights are read no more."""
+    def layer_backward(self, x, flat, gflat, rope, shape, gy, ready=None, before=None):
+        """Gradient of the layer's input; the weights' gradients go into gflat (laid out like flat). before() is called ahead of the first
+        write into gflat, ready(lo) is told that from element lo on the gradients are written and the weights are read no more."""
         p, g = self._layer_views(flat), self._layer_views(gflat)
         begin = flat.data_ptr()
 
@@ -159,6 +159,8 @@ class FusedUnits:
         gu = torch.mm(h2, p["w_gu"].t())
         act = torch.mm(gy, p["w_down"])
         self.swiglu_backward(gu, act)
+        if before:
+            before()   # the recomputation does not wait for whoever still reads gflat
         torch.mm(gy.t(), act, out=g["w_down"])
         done("w_down")
         del act
@@ -181,13 +183,15 @@ class FusedUnits:
         c, ids = self.cfg, tokens.reshape(-1).contiguous()
         self._run("b200EmbeddingBackward", ids.data_ptr(), gx.data_ptr(), gflat.data_ptr(), ids.numel(), c.vocab, c.hidden)
 
-    def head(self, x, add, flat, gflat, targets):
-        """(mean loss, gradient of the hidden states x + add); the weights' gradients go into gflat."""
+    def head(self, x, add, flat, gflat, targets, before=None):
+        """(mean loss, gradient of the hidden states x + add); the weights' gradients go into gflat, before() ahead of them."""
         shapes = M.head_shapes(self.cfg)
         p, g = M.views(flat, shapes), M.views(gflat, shapes)
         x, h, rstd = self.norm(x, p["norm"], add=add, need_rstd=True)
         logits = torch.mm(h, p["out"].t())
         loss = self.cross_entropy(logits, targets)
         dh = torch.mm(logits, p["out"])
+        if before:
+            before()
         torch.mm(logits.t(), h, out=g["out"])
         return loss, self.norm_backward(x, p["norm"], rstd, dh, None, g["norm"])

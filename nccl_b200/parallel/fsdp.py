@@ -198,16 +198,19 @@ class FSDPEngine:
         u.param.copy_(u.master.to(torch.bfloat16))
 
     def _grad_flat(self, idx, gslot):
-        """The unit's flat gradient buffer, once the reduce-scatter that read it last is through; its padding is zero."""
+        """The unit's flat gradient buffer, to be written behind `_take_grads`."""
+        return self._whole_grad(idx, gslot)[:self.units[idx].numel]
+
+    def _take_grads(self, idx, gslot):
+        """What follows may write the unit's gradients: the reduce-scatter that read the buffer last is through, the padding is zero."""
         u = self.units[idx]
         if self.cuda and self.n > 1:
             torch.cuda.current_stream().wait_event(self.ev_grad_free[gslot])
-        flat = self._whole_grad(idx, gslot)
         if u.padded > u.numel:
-            flat[u.numel:u.padded].zero_()
-        return flat[:u.numel]
+            self._whole_grad(idx, gslot)[u.numel:u.padded].zero_()
 
     def _write_grads(self, idx, gslot, grads):
+        self._take_grads(idx, gslot)
         flat = self._grad_flat(idx, gslot)
         off = 0
         for g in grads:
@@ -264,7 +267,8 @@ class FSDPEngine:
         slot = idx % 2
         self._wait_gathered(slot)
         if fused:
-            loss, gx = fused.head(x, add, weights(idx, slot), self._grad_flat(idx, slot), targets.reshape(-1).contiguous())
+            loss, gx = fused.head(x, add, weights(idx, slot), self._grad_flat(idx, slot), targets.reshape(-1).contiguous(),
+                                  before=lambda: self._take_grads(idx, slot))
             self._release(slot)
         else:
             vs = params(idx, slot, True)
@@ -295,12 +299,14 @@ class FSDPEngine:
                         done[0] = lo
                 else:
                     ready = None
-                gx = fused.layer_backward(saved[idx], weights(idx, slot), self._grad_flat(idx, slot), rope, shape, gx, ready)
+                gx = fused.layer_backward(saved[idx], weights(idx, slot), self._grad_flat(idx, slot), rope, shape, gx, ready,
+                                          before=lambda: self._take_grads(idx, slot))
                 self._release(slot)
                 self._reduce_and_update(idx, slot, done[0])
                 saved[idx] = None
                 continue
             if fused and llama_fused.embedding_applies(tokens):
+                self._take_grads(idx, slot)
                 fused.embedding_backward(tokens, gx, self._grad_flat(idx, slot))
                 self._release(slot)
                 self._reduce_and_update(idx, slot)

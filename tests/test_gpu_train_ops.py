@@ -222,6 +222,39 @@ def test_what_stays_with_autograd():
         assert not llama_fused.applies(cfg, tok, tok)
 
 
+def test_gradient_buffers_are_waited_for_behind_the_recomputation():
+    """On the CPU, with kernels that do nothing: what is called before the first write stands right in front of that product."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from nccl_b200 import _lib
+
+    class NoKernels(llama_fused.FusedUnits):
+        def _run(self, name, *args):
+            log.append(name)
+
+    class Products(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            if func.overloadpacket == torch.ops.aten.mm:
+                log.append("into" if "out" in (kwargs or {}) else "mm")
+            return func(*args, **(kwargs or {}))
+
+    u = NoKernels(M.LlamaConfig(hidden=64, heads=4, kv_heads=2, ffn=128, vocab=64), _lib.load())
+    rope = M.rope_tables(u.cfg, 8, "cpu")
+    x, gy = (torch.zeros(16, 64, dtype=torch.bfloat16) for _ in range(2))
+    for unit in ("layer", "head"):
+        log = []
+        shapes = M.layer_shapes(u.cfg) if unit == "layer" else M.head_shapes(u.cfg)
+        flat, gflat = (torch.zeros(M.numel(shapes), dtype=torch.bfloat16) for _ in range(2))
+        with Products():
+            if unit == "layer":
+                u.layer_backward(x, flat, gflat, rope, (2, 8), gy, before=lambda: log.append("before"))
+            else:
+                u.cross_entropy = lambda logits, targets: log.append("loss")
+                u.head(x, None, flat, gflat, torch.zeros(16, dtype=torch.int64), before=lambda: log.append("before"))
+        at = log.index("before")
+        assert log.count("before") == 1 and log.index("into") == at + 1 and log[:at].count("mm") == (4 if unit == "layer" else 2)
+
+
 @gpu
 @pytest.mark.parametrize("shape,hidden,vocab", [((1, 1), 8, 8), ((2, 65), 64, 16), ((1, 700), 2056, 1000), ((3, 257), 4096, 5), ((2, 1024), 128, 50000)])
 def test_embedding_backward(shape, hidden, vocab):
