@@ -30,7 +30,8 @@ _ENTRIES = {
     "b200SwiGlu": [_P] * 2 + [_I, _I, _P],
     "b200SwiGluBackward": [_P] * 2 + [_I, _I, _P],
     "b200CrossEntropy": [_P] * 5 + [_I, _I, _P],
-    "b200EmbeddingBackward": [_P] * 3 + [_I] * 3 + [_P],
+    "b200EmbeddingBackward": [_P] * 4 + [_I] * 3 + [_P],
+    "b200EmbeddingBackwardWork": [_I, _I],
 }
 
 
@@ -44,7 +45,8 @@ def applies(cfg, tokens, targets):
 
 
 def embedding_applies(tokens):
-    """Every id looks through all others: 64-bit ids, and few enough of them."""
+    """64-bit ids, and no more of them than the kernel takes: each is compared with all others. 8192 uniform ids of 4096 channels 78 us against
+    762 by autograd, all of them the same id 90 against 471."""
     return tokens.dtype == torch.int64 and tokens.numel() <= 8192
 
 
@@ -57,7 +59,7 @@ class FusedUnits:
         for name, types in _ENTRIES.items():
             fn = getattr(lib, name)
             fn.argtypes = types
-            fn.restype = ctypes.c_int
+            fn.restype = ctypes.c_size_t if name.endswith("Work") else ctypes.c_int
             self._call[name] = fn
 
     def _run(self, name, *args):
@@ -181,7 +183,8 @@ class FusedUnits:
     def embedding_backward(self, tokens, gx, gflat):
         """The gradient of the table, into gflat."""
         c, ids = self.cfg, tokens.reshape(-1).contiguous()
-        self._run("b200EmbeddingBackward", ids.data_ptr(), gx.data_ptr(), gflat.data_ptr(), ids.numel(), c.vocab, c.hidden)
+        work = torch.empty(self._call["b200EmbeddingBackwardWork"](ids.numel(), c.hidden), dtype=torch.float32, device=ids.device)
+        self._run("b200EmbeddingBackward", ids.data_ptr(), gx.data_ptr(), gflat.data_ptr(), work.data_ptr(), ids.numel(), c.vocab, c.hidden)
 
     def head(self, x, add, flat, gflat, targets, before=None):
         """(mean loss, gradient of the hidden states x + add); the weights' gradients go into gflat, before() ahead of them."""

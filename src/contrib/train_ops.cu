@@ -376,39 +376,158 @@ __global__ void __launch_bounds__(1024) meanLossKernel(const float* rowLoss, con
 }
 
 // ---------------------------------------------------------------------------------------------- embedding
-// out[id] = sum over the tokens with that id of dx, in fp32 in the order of the tokens, rounded once; rows of other ids are not
-// touched. The CTA of an id's first token adds up: it looks through all ids, which stay in L2 (so the work grows with the square of
-// the tokens; the engine takes this kernel up to 8192 of them). 2048 tokens of 4096 channels 33 us behind a 23 us memset of a table of
-// 16384 rows; filling, adding and copying into the flat buffer took 311.
-__global__ void __launch_bounds__(256) embeddingBackwardKernel(const long long* ids, const uint4* dx, uint4* out, int tokens, int vocab, int packs) {
-  __shared__ uint32_t hit[2][8];
-  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long id = ids[t];
-  if (id < 0 || id >= vocab) return;
-  bool earlier = false;
-  for (int j = threadIdx.x; j < t && !earlier; j += 256) earlier = ids[j] == id;
-  if (__syncthreads_or(earlier)) return;
-  int turn = 0;
-  for (int p0 = 0; p0 < packs; p0 += 256) {
-    const int p = p0 + threadIdx.x;
-    float acc[8] = {};
-    if (p < packs) unpack8(dx[(size_t)t * packs + p], acc);
-    for (int j0 = t + 1; j0 < tokens; j0 += 256, turn ^= 1) {
-      const int j = j0 + threadIdx.x;
-      const bool same = j < tokens && ids[j] == id;
-      const uint32_t bits = __ballot_sync(~0u, same);
-      if (lane == 0) hit[turn][warp] = bits;
-      if (!__syncthreads_or(same)) continue;
-      if (p < packs)
-        for (int w = 0; w < 8; ++w)
-          for (uint32_t b = hit[turn][w]; b; b &= b - 1) {
-            float f[8];
-            unpack8(dx[(size_t)(j0 + w * 32 + __ffs(b) - 1) * packs + p], f);
+// out[id] = sum over the tokens with that id of dx, in fp32 in a fixed order, rounded once; all other rows are zero. Ids repeat (a padding id may
+// be half of a batch), so the work is cut by tokens and not by ids: the token positions are ordered by id, a CTA adds the rows of kIdRows
+// neighbours, and an id that reaches over several of them leaves fp32 sums that a third kernel adds. With a CTA per id, one row behind the
+// other, 2048 tokens of 4096 channels into a table of 16384 rows took 39 us for uniform ids, 1040 with half of them one id and 2060 with all
+// of them; now 39, 41 and 43, most of it the table's zeros (8192 tokens: 124, 4120 and 8160 us, now 78, 84 and 90; the framework's kernel with
+// its fills and copies 762, 624 and 471).
+constexpr int kIdRows = 16, kMaxIds = 8192, kPosBits = 13;
+static_assert(kMaxIds == 1 << kPosBits, "positions must fit");
+constexpr int kRankTokens = 32;   // of a CTA, four per warp
+
+// keys[rank] = id << 13 | position, ascending, ids outside the table as `vocab`: the rank of a token is the number of ids below its own, and of equal
+// ones ahead of it. Every CTA looks at all ids for its kRankTokens tokens (the work grows with the square of the tokens: 2048 hide behind the zeros, 8192 take 40 us). The CTAs behind
+// the first `ranking` write the table's zeros meanwhile.
+__global__ void __launch_bounds__(256) rankIdsKernel(const long long* ids, unsigned long long* keys, uint4* out, size_t outPacks, int tokens, int vocab, int ranking) {
+  extern __shared__ uint32_t id[];
+  if ((int)blockIdx.x >= ranking) {
+    const size_t step = (size_t)(gridDim.x - ranking) * blockDim.x;
+    for (size_t i = (size_t)(blockIdx.x - ranking) * blockDim.x + threadIdx.x; i < outPacks; i += step) out[i] = make_uint4(0, 0, 0, 0);
+    return;
+  }
+  for (int i = threadIdx.x; i < tokens; i += blockDim.x) {
+    const long long v = ids[i];
+    id[i] = v >= 0 && v < vocab ? (uint32_t)v : (uint32_t)vocab;
+  }
+  __syncthreads();
+  constexpr int N = kRankTokens / 8;
+  const int lane = threadIdx.x & 31, t0 = blockIdx.x * kRankTokens + threadIdx.x / 32 * N;
+  if (t0 >= tokens) return;
+  uint32_t mine[N], rank[N];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[i] += f[i];
-          }
+  for (int n = 0; n < N; ++n) {
+    mine[n] = t0 + n < tokens ? id[t0 + n] : 0;
+    rank[n] = 0;
+  }
+  auto count = [&](int j, const uint32_t (&below)[N]) {
+    const uint32_t v = id[j];
+#pragma unroll
+    for (int n = 0; n < N; ++n) rank[n] += v < below[n];
+  };
+  uint32_t withEqual[N];
+#pragma unroll
+  for (int n = 0; n < N; ++n) withEqual[n] = mine[n] + 1;
+  const int block = t0 / 32 * 32;   // of the tokens themselves (N divides 32)
+  int j = lane;
+#pragma unroll 4
+  for (; j < block; j += 32) count(j, withEqual);
+  if (j < tokens) {
+#pragma unroll
+    for (int n = 0; n < N; ++n) rank[n] += id[j] < mine[n] + (j < t0 + n);
+  }
+#pragma unroll 4
+  for (j += 32; j < tokens; j += 32) count(j, mine);
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const uint32_t r = __reduce_add_sync(~0u, rank[n]);
+    if (lane == n && t0 + n < tokens) keys[r] = (unsigned long long)mine[n] << kPosBits | (unsigned)(t0 + n);
+  }
+}
+
+// CTA (c, slice): positions [c * kIdRows, ...) of the order, 128 packs of channels at most. Sums of an id that begins and ends here go to `out`;
+// partial[c][0] takes what belongs to an id that began before, partial[c][1] the begin of one that goes on.
+__global__ void __launch_bounds__(128) embeddingSumKernel(const unsigned long long* keys, const uint4* dx, uint4* out, float4* partial, int tokens, int vocab, int packs) {
+  constexpr int U = 8;   // rows on their way
+  __shared__ unsigned long long key[kIdRows + 2];   // with the neighbours on both sides
+  const int first = blockIdx.x * kIdRows, rows = min(kIdRows, tokens - first);
+  for (int i = threadIdx.x; i < rows + 2; i += blockDim.x) {
+    const int at = first + i - 1;
+    key[i] = at >= 0 && at < tokens ? keys[at] : ~0ull;
+  }
+  __syncthreads();
+  const int p = blockIdx.y * blockDim.x + threadIdx.x;
+  if (p >= packs) return;
+  auto idOf = [&](int r) { return key[r + 1] >> kPosBits; };
+  bool began = idOf(-1) == idOf(0);   // before this CTA
+  float acc[8] = {};
+  for (int r0 = 0; r0 < rows; r0 += U) {
+    uint4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (r0 + u < rows) v[u] = dx[(size_t)(key[r0 + u + 1] & (kMaxIds - 1)) * packs + p];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = r0 + u;
+      if (r >= rows) break;
+      float f[8];
+      unpack8(v[u], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] += f[i];
+      const unsigned long long id = idOf(r);
+      const bool goesOn = idOf(r + 1) == id;
+      if (goesOn && r + 1 < rows) continue;
+      if (id < (unsigned long long)vocab) {
+        if (began || goesOn) {
+          float4* to = partial + (((size_t)blockIdx.x * 2 + (began ? 0 : 1)) * packs + p) * 2;
+          to[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+          to[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+        } else {
+          out[id * packs + p] = pack8(acc);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = 0.0f;
+      began = false;
     }
-    if (p < packs) out[(size_t)id * packs + p] = pack8(acc);
+  }
+}
+
+// CTA (c, slice): the id that begins in positions [c * kIdRows, ...) and goes on behind them, if there is one: 8 warps take its sums in
+// turn, 256 channels each, and their results are added in order.
+constexpr int kJoinQuads = 2;   // of a thread
+__global__ void __launch_bounds__(256) embeddingJoinKernel(const unsigned long long* keys, const float4* partial, uint2* out, int tokens, int vocab, int hidden) {
+  __shared__ float4 sums[7][kJoinQuads][32];
+  const int c = blockIdx.x, last = (c + 1) * kIdRows - 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;   // never the last chunk: last + 1 < tokens
+  const unsigned long long id = keys[last] >> kPosBits;
+  if (id >= (unsigned long long)vocab || keys[last + 1] >> kPosBits != id) return;
+  if (c > 0 && keys[c * kIdRows - 1] >> kPosBits == id) return;   // began before
+  int more = 0;   // chunks that it goes on into
+  for (int k = c + 1 + threadIdx.x, got = 256; got == 256; k += 256) more += got = __syncthreads_count(k * kIdRows < tokens && keys[k * kIdRows] >> kPosBits == id);
+  const int quads = hidden / 4, q0 = blockIdx.y * 32 * kJoinQuads + lane;
+  float4 acc[kJoinQuads];
+#pragma unroll
+  for (int k = 0; k < kJoinQuads; ++k) acc[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+  for (int i = warp; i <= more; i += 8) {
+    const float4* from = partial + ((size_t)(c + i) * 2 + (i == 0)) * quads + q0;
+#pragma unroll
+    for (int k = 0; k < kJoinQuads; ++k) {
+      if (q0 + k * 32 >= quads) break;
+      const float4 v = from[k * 32];
+      acc[k].x += v.x;
+      acc[k].y += v.y;
+      acc[k].z += v.z;
+      acc[k].w += v.w;
+    }
+  }
+  if (warp) {
+#pragma unroll
+    for (int k = 0; k < kJoinQuads; ++k) sums[warp - 1][k][lane] = acc[k];
+  }
+  __syncthreads();
+  if (warp) return;
+#pragma unroll
+  for (int k = 0; k < kJoinQuads; ++k) {
+    if (q0 + k * 32 >= quads) break;
+    for (int w = 0; w < 7; ++w) {
+      acc[k].x += sums[w][k][lane].x;
+      acc[k].y += sums[w][k][lane].y;
+      acc[k].z += sums[w][k][lane].z;
+      acc[k].w += sums[w][k][lane].w;
+    }
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(acc[k].x, acc[k].y), hi = __floats2bfloat162_rn(acc[k].z, acc[k].w);
+    out[id * quads + q0 + k * 32] = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
   }
 }
 
@@ -514,11 +633,25 @@ extern "C" ncclResult_t b200SwiGluBackward(void* gu, void* dact, int rows, int f
   return launched();
 }
 
-// Gradient of an embedding table [vocab][hidden]: rows of the ids that occur are written over, all others become zero.
-extern "C" ncclResult_t b200EmbeddingBackward(const long long* ids, const void* dx, void* out, int tokens, int vocab, int hidden, cudaStream_t stream) {
-  if (!ids || !dx || !out || tokens <= 0 || vocab <= 0 || hidden <= 0 || hidden % 8 || !aligned16({dx, out})) return ncclInvalidArgument;
-  if (cudaMemsetAsync(out, 0, (size_t)vocab * hidden * 2, stream) != cudaSuccess) { (void)cudaGetLastError(); return ncclUnhandledCudaError; }
-  embeddingBackwardKernel<<<tokens, 256, 0, stream>>>(ids, (const uint4*)dx, (uint4*)out, tokens, vocab, hidden / 8);
+// Floats that b200EmbeddingBackward needs for `work`, 0 for more tokens than it takes.
+extern "C" size_t b200EmbeddingBackwardWork(int tokens, int hidden) {
+  return tokens > 0 && tokens <= kMaxIds ? ((size_t)tokens * 2 + 3) / 4 * 4 + (size_t)(tokens + kIdRows - 1) / kIdRows * 2 * hidden : 0;
+}
+
+// Gradient of an embedding table [vocab][hidden]: rows of the ids that occur are written over, all others become zero. Ids outside the table are
+// left out.
+extern "C" ncclResult_t b200EmbeddingBackward(const long long* ids, const void* dx, void* out, float* work, int tokens, int vocab, int hidden, cudaStream_t stream) {
+  if (!ids || !dx || !out || !work || tokens <= 0 || tokens > kMaxIds || vocab <= 0 || hidden <= 0 || hidden % 8 || !aligned16({dx, out, work})) return ncclInvalidArgument;
+  unsigned long long* keys = (unsigned long long*)work;
+  float4* partial = (float4*)(work + ((size_t)tokens * 2 + 3) / 4 * 4);
+  const int packs = hidden / 8, chunks = (tokens + kIdRows - 1) / kIdRows, threads = std::min(128, (packs + 31) / 32 * 32);
+  const int ranking = (tokens + kRankTokens - 1) / kRankTokens;
+  const size_t outPacks = (size_t)vocab * packs;
+  const int zeroing = (int)std::min<size_t>((outPacks + 2047) / 2048, 1 << 30);   // neighbours write neighbouring pages at about the same time
+  rankIdsKernel<<<ranking + zeroing, 256, tokens * 4, stream>>>(ids, keys, (uint4*)out, outPacks, tokens, vocab, ranking);
+  embeddingSumKernel<<<dim3(chunks, (packs + threads - 1) / threads), threads, 0, stream>>>(keys, (const uint4*)dx, (uint4*)out, partial, tokens, vocab, packs);
+  if (chunks > 1)
+    embeddingJoinKernel<<<dim3(chunks - 1, (hidden / 4 + 32 * kJoinQuads - 1) / (32 * kJoinQuads)), 256, 0, stream>>>(keys, partial, (uint2*)out, tokens, vocab, hidden);
   return launched();
 }
 

@@ -265,3 +265,55 @@ def test_embedding_backward(shape, hidden, vocab):
     u.embedding_backward(tokens, gx, out)
     ref, spread = (torch.zeros(vocab, hidden, dtype=torch.float64, device="cuda").index_add_(0, tokens.view(-1), t.view(-1, hidden)) for t in (gx.double(), gx.double().abs()))
     _close(out.view(vocab, hidden), ref, spread)
+
+
+@gpu
+@pytest.mark.parametrize("tokens", [31, 32, 33, 64, 65, 1000, 8192])
+@pytest.mark.parametrize("ids", ["one", "two", "half", "runs"])
+def test_embedding_backward_of_repeated_ids(tokens, ids):
+    """Ids that reach over the rows one CTA adds, up to all of them; the first and last id of the table; the same bits again; time that does not grow with
+    the repetition."""
+    hidden, vocab = 1032, 600
+    u = _units(hidden=hidden, vocab=vocab)
+    g = torch.Generator().manual_seed(tokens)
+    tok = torch.randint(0, vocab, (1, tokens), generator=g)
+    if ids == "one":
+        tok[:] = 7
+    elif ids == "two":
+        tok[:] = torch.where(torch.arange(tokens) % 3 == 0, 0, vocab - 1)
+    elif ids == "half":
+        tok[0, torch.randperm(tokens, generator=g)[:tokens // 2]] = 300
+    else:
+        tok[0] = torch.arange(tokens) // 47 % vocab
+    tok = tok.cuda()
+    gx = _rand(1, tokens, hidden, seed=1)
+    out, again = (torch.full((vocab * hidden,), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    u.embedding_backward(tok, gx, out)
+    u.embedding_backward(tok, gx, again)
+    ref, spread = (torch.zeros(vocab, hidden, dtype=torch.float64, device="cuda").index_add_(0, tok.view(-1), t.view(-1, hidden)) for t in (gx.double(), gx.double().abs()))
+    _close(out.view(vocab, hidden), ref, spread)
+    assert torch.equal(out, again)
+    if tokens == 8192:
+        def ms(t):
+            at = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            u.embedding_backward(t, gx, out)
+            at[0].record()
+            for _ in range(5):
+                u.embedding_backward(t, gx, out)
+            at[1].record()
+            at[1].synchronize()
+            return at[0].elapsed_time(at[1])
+        # one CTA that adds all rows of an id took 30 times as long for one id as for uniform ones
+        assert ms(tok) <= 3 * ms(torch.randint(0, vocab, (1, tokens), generator=g).cuda()) + 0.2
+
+
+@gpu
+def test_embedding_backward_leaves_out_ids_behind_the_table():
+    u = _units(hidden=64, vocab=10)
+    ids = torch.tensor([3, -1, 10, 3, 1 << 40, -(1 << 62), 9] * 20, device="cuda")
+    gx = _rand(ids.numel(), 64, seed=1)
+    out = torch.full((640,), 7.0, dtype=torch.bfloat16, device="cuda")
+    u.embedding_backward(ids.view(1, -1), gx, out)
+    valid = (ids >= 0) & (ids < 10)
+    ref, spread = (torch.zeros(10, 64, dtype=torch.float64, device="cuda").index_add_(0, ids[valid], t[valid]) for t in (gx.double(), gx.double().abs()))
+    _close(out.view(10, 64), ref, spread)
