@@ -16,6 +16,9 @@ import ctypes
 
 import torch
 import torch.nn.functional as F
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
+from torch.utils._python_dispatch import _get_current_dispatch_mode_stack
 
 from .. import _lib
 from . import llama as M
@@ -35,13 +38,22 @@ _ENTRIES = {
 }
 
 
+def _watched():
+    """Whether something in the framework looks into, or changes, the single operations: the row kernels would pass it by. A default
+    device is a function mode too, but changes none of them."""
+    return (torch.is_autocast_enabled("cuda") or torch.is_anomaly_enabled() or torch.jit.is_tracing() or torch.compiler.is_compiling() or
+            bool(_get_current_dispatch_mode_stack()) or any(not isinstance(m, DeviceContext) for m in _get_current_function_mode_stack()) or
+            torch._C._autograd._top_saved_tensors_default_hooks(False) is not None or torch._C._functorch.peek_interpreter_stack() is not None)
+
+
 def applies(cfg, tokens, targets):
-    """Whether a step on a GPU takes this path: shapes that the kernels' 16-byte accesses fit, and no mode of the framework that
-    looks into, or changes, the single operations. Everything else goes through `llama` and autograd."""
+    """Whether a step on a GPU takes this path: shapes that the kernels' 16-byte accesses fit, gradients wanted, and nothing that watches the
+    operations (autocast, anomaly detection, dispatch and function modes, hooks for saved tensors, tracing, function transforms).
+    Everything else goes through `llama` and autograd."""
     h, d = cfg.hidden, cfg.head_dim
     return (h % 8 == 0 and h <= 16384 and d > 0 and d % 16 == 0 and d * cfg.heads == h and cfg.heads % cfg.kv_heads == 0 and cfg.ffn % 8 == 0 and
             cfg.vocab % 8 == 0 and tokens.dim() == 2 and tokens.numel() > 0 and targets.dtype == torch.int64 and targets.numel() == tokens.numel() and
-            torch.is_grad_enabled() and not torch.is_anomaly_enabled() and not torch.is_autocast_enabled("cuda"))
+            torch.is_grad_enabled() and not _watched())
 
 
 def embedding_applies(tokens):

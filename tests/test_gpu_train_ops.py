@@ -222,6 +222,28 @@ def test_what_stays_with_autograd():
         assert not llama_fused.applies(cfg, tok, tok)
 
 
+def test_modes_that_watch_operations_stay_with_autograd():
+    from torch.overrides import TorchFunctionMode
+    from torch.utils.flop_counter import FlopCounterMode
+    tok = torch.zeros(2, 8, dtype=torch.int64)
+    cfg = M.LlamaConfig(hidden=256, heads=4, kv_heads=2, ffn=512, vocab=1024)
+    ident = lambda t: t  # noqa: E731
+
+    class Functions(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    for mode in (FlopCounterMode(display=False), Functions(), torch.autograd.graph.saved_tensors_hooks(ident, ident)):
+        with mode:
+            assert not llama_fused.applies(cfg, tok, tok), mode
+    seen = []
+    torch.func.vmap(lambda x: seen.append(llama_fused.applies(cfg, tok, tok)) or x)(torch.zeros(2))
+    assert seen == [False]
+    with torch.device("cpu"):   # a default device changes no operation
+        assert llama_fused.applies(cfg, tok, tok)
+    assert llama_fused.applies(cfg, tok, tok)
+
+
 def test_gradient_buffers_are_waited_for_behind_the_recomputation():
     """On the CPU, with kernels that do nothing: what is called before the first write stands right in front of that product."""
     from torch.utils._python_dispatch import TorchDispatchMode
