@@ -31,8 +31,8 @@ def _align(n, a):
     return (n + a - 1) // a * a
 
 
-# elements of a unit from which one rank updates it in pieces: a piece's launch and event cost the host 15 us, its update at least as much
-# of the GPU's time
+# elements of a unit from which one rank updates it in pieces, each a quarter of that at least: a piece's launch and event cost the host 15 us,
+# the update of 2^22 elements takes 17 us of the GPU's time (28 bytes each at 6.7 TB/s)
 kEarlyUpdate = 1 << 24
 
 
@@ -295,6 +295,8 @@ class FSDPEngine:
                 done = [u.shard]
                 if self.n == 1 and u.numel >= kEarlyUpdate:
                     def ready(lo):
+                        if done[0] - lo < kEarlyUpdate // 4:
+                            return   # goes with the next piece, or with the rest
                         self._update_early(idx, lo, done[0])
                         done[0] = lo
                 else:

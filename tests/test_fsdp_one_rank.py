@@ -67,3 +67,33 @@ def test_pieces_of_a_unit_are_updated_like_the_whole():
     for a, b in zip(*got):
         assert a == b if isinstance(a, float) else torch.equal(a, b)
     comm.destroy()
+
+
+@pytest.mark.gpu
+def test_small_pieces_wait_for_the_next():
+    """wo and norm2 of this shape are a million elements, far below what is worth a launch of its own."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from nccl_b200 import Communicator, get_unique_id
+    from nccl_b200.models import llama as M
+    from nccl_b200.parallel import fsdp
+    torch.cuda.set_device(0)
+    comm = Communicator(1, 0, get_unique_id())
+    cfg = M.LlamaConfig(layers=2, hidden=1024, heads=8, kv_heads=2, ffn=4864, vocab=512)
+    eng = fsdp.FSDPEngine(comm, cfg, device="cuda", seed=1, init_on_device=True)
+    assert eng.units[1].numel >= fsdp.kEarlyUpdate
+    pieces, update = [], eng._update_early
+
+    def record(idx, lo, hi):
+        pieces.append((idx, lo, hi))
+        update(idx, lo, hi)
+
+    eng._update_early = record
+    tok = torch.randint(0, cfg.vocab, (1, 32))
+    eng.step(tok, tok)
+    w_down, w_gu = cfg.hidden * cfg.ffn, 2 * cfg.hidden * cfg.ffn
+    end = eng.units[1].shard
+    assert pieces == [(idx, lo, hi) for idx in (2, 1) for lo, hi in ((end - w_down, end), (end - w_down - w_gu, end - w_down))]
+    assert all(hi - lo >= 1 << 22 for _, lo, hi in pieces)
+    eng.close()
+    comm.destroy()
