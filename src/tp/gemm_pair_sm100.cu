@@ -206,8 +206,6 @@ tpGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 const void* tpGemmPairKernelFn(int width) {
   switch (width) {
-    case 128: return (const void*)tpGemmPairKernel<128>;
-    case 160: return (const void*)tpGemmPairKernel<160>;
     case 192: return (const void*)tpGemmPairKernel<192>;
     case 224: return (const void*)tpGemmPairKernel<224>;
     default: return (const void*)tpGemmPairKernel<256>;

@@ -186,8 +186,8 @@ static float expectedUs(const ncclTpContext* tp, const TpGemmArgs* a, const Gemm
   const int share = p.shares > 1 ? (steps * own + p.shares - 1) / p.shares : steps;   // K steps of a CTA
   float step;
   switch (p.width) {
-    case 128: step = p.pair ? 0.23f : 0.21f; break;
-    case 160: step = p.pair ? 0.25f : 0.255f; break;
+    case 128: step = 0.21f; break;
+    case 160: step = 0.255f; break;
     case 192: step = p.pair ? 0.26f : 0.31f; break;
     case 224: step = p.pair ? 0.315f : 0.38f; break;
     default: step = p.pair ? 0.35f : 0.385f; break;
@@ -207,7 +207,8 @@ static float expectedUs(const ncclTpContext* tp, const TpGemmArgs* a, const Gemm
 // last wave matters less and the widest tiles have the best rate (8192 x 8192 x 3584: pairs of 256 303 us, 224 312, 192 349).
 // Kernel times with 256 columns / the choice, us: 1152 x 2304 x 7168 40.6 / 31.8 (160 columns), 2048 x 2560 x 4096 46.1 / 35.4 (160),
 // 1280 x 4096 x 3584 38.4 / 31.9 (pairs of 192), 2560 x 3072 x 2048 25.6 / 23.7 (pairs of 224).
-// The other side of the line: 1920 x 4096 x 7168 82.3 with pairs of 256, 91.7 of 192; 3328 x 4096 x 1536 29.5 / 31.7.
+// The other side of the line: 1920 x 4096 x 7168 82.3 with pairs of 256, 91.7 of 192; 3328 x 4096 x 1536 29.5 / 31.7. Pairs of 160 were never
+// faster than both pairs of 192 and one CTA with 160 columns (16 shapes, 0.99 to 1.12 of the better one).
 // The width never changes the sums: where K is summed in shares it stays so, with an accumulator per share. Weights from memory: 128 x
 // 1024 x 2048 10.2 / 7.5 (128 columns, four CTAs), 128 x 4096 x 4096 17.5 / 14.3 (six shares on four CTAs), 128 x 8192 x 8192 29.7 / 29.3 (four on
 // two), 512 x 4096 x 1024 10.2 / 8.2 (two on one); 896 x 1536 x 3264 stays, 14.7 / 17.2 (three on one). Fewer shares would be faster by what their sums
@@ -217,7 +218,10 @@ static GemmPlan planGemm(const ncclTpContext* tp, const TpGemmArgs* a, bool pair
   GemmPlan best = basePlan(tp, a, pairs);
   for (int w : kTpWidths)
     if (w == paramTpWidth()) {
-      if (best.shares == 1) best.width = w;
+      if (best.shares == 1) {
+        best.width = w;
+        best.pair = best.pair && w >= kTpPairWidth;
+      }
       return best;
     }
   if (((a->M + 255) / 256 * (a->N / 256) + tp->smCount / 2 - 1) / (tp->smCount / 2) > 4) return best;
@@ -240,7 +244,7 @@ static GemmPlan planGemm(const ncclTpContext* tp, const TpGemmArgs* a, bool pair
   }
   for (int w : kTpWidths)
     for (bool pair : {false, true})
-      if (pairs || !pair) consider({pair, w});
+      if (!pair || (pairs && w >= kTpPairWidth)) consider({pair, w});
   return best;
 }
 
@@ -476,7 +480,7 @@ ncclResult_t ncclTpCreate(ncclComm_t comm, size_t maxRows, size_t maxCols, ncclT
     int clusters = 0;
     bool pairsFit = true;
     for (int width : kTpWidths)
-      pairsFit = pairsFit && cudaFuncSetAttribute(tpGemmPairKernelFn(width), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmPairSmemBytes()) == cudaSuccess;
+      if (width >= kTpPairWidth) pairsFit = pairsFit && cudaFuncSetAttribute(tpGemmPairKernelFn(width), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tpGemmPairSmemBytes()) == cudaSuccess;
     if (pairsFit && cudaOccupancyMaxActiveClusters(&clusters, tpGemmPairKernelFn(256), &cfg) == cudaSuccess)
       tp->pairClusters = std::min(clusters, tp->smCount / 2);
     else

@@ -14,6 +14,7 @@ constexpr int kTpMaxSplit = 8;     // largest cluster of CTAs that share the K b
 constexpr int kTpMaxOwnShares = 4; // of a CTA of the bf16 split kernel, on tiles of 128 columns
 constexpr int kTpMaxEarly = 4;     // sums of 32 columns behind the operand ring: four stages of operands stay
 constexpr int kTpWidths[] = {256, 224, 192, 160, 128};   // tile widths of plain bf16 GEMMs; the fused modes use the first
+constexpr int kTpPairWidth = 192;                        // the narrowest of CTA pairs
 
 struct TpGemmArgs {
   void* C;                        // bf16 output [M, ldc] (STORE / GATHER)
@@ -89,7 +90,7 @@ __device__ __forceinline__ TileCoord tileOf(const TpGemmArgs& a, int t, int bm =
 #endif
 
 const void* tpGemmKernelFn(int width);       // tiles of 128 x width (one of kTpWidths), W map with boxes of width rows
-const void* tpGemmPairKernelFn(int width);   // CTA-pair variant (cluster of two, tiles of 256 x width): same arguments, W map with boxes of width / 2 rows
+const void* tpGemmPairKernelFn(int width);   // CTA-pair variant (cluster of two, tiles of 256 x width from kTpPairWidth on): same arguments, W map with boxes of width / 2 rows
 const void* tpGemmSplitKernelFn(int width);  // plain C = A * W^T, one tile of 128 x width (256 or 128) per cluster of splitK CTAs, K in `shares` sums
 int tpGemmSplitPlan(TpGemmArgs* a, int width);   // from splitK and shares; returns `early`, and above kTpMaxEarly there is no such form
 size_t tpGemmSplitSmemBytes();
