@@ -656,7 +656,8 @@ extern "C" ncclResult_t b200EmbeddingBackward(const long long* ids, const void* 
 }
 
 // Mean cross entropy of logits [rows][vocab] (bf16, vocab a multiple of 8) over the rows whose target is not -100; logits become their
-// gradient. work: rows + 1 floats. *ok (device): whether every target is in range; the others are left out.
+// gradient. work: rows + 1 floats. *ok (device): whether every target is in range. Rows of targets that are not get no gradient and add
+// nothing to the loss, but count in its mean.
 extern "C" ncclResult_t b200CrossEntropy(void* logits, const long long* target, float* loss, float* work, void* ok, int rows, int vocab, cudaStream_t stream) {
   if (!logits || !target || !loss || !work || !ok || rows <= 0 || vocab <= 0 || vocab % 8 || !aligned16({logits})) return ncclInvalidArgument;
   countTargetsKernel<<<1, 1024, 0, stream>>>(target, rows, vocab, work + rows, (bool*)ok);

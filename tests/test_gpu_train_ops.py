@@ -138,6 +138,30 @@ def test_cross_entropy_without_a_row_that_counts():
 
 
 @gpu
+@pytest.mark.parametrize("bad", [[], [-1], [64], [1 << 40, -101, -(1 << 62)]])
+def test_cross_entropy_reports_targets_out_of_range(bad):
+    """The entry itself (its caller asserts on what it reports): rows of such targets get no gradient and add nothing to the loss, but count in its mean."""
+    import ctypes
+    u = _units()
+    rows, vocab = 8, 64
+    logits = _rand(rows, vocab, seed=1)
+    targets = torch.tensor([3, -100, 0, 63, 9, 10, 11, 12], device="cuda")
+    targets[5:5 + len(bad)] = torch.tensor(bad, dtype=torch.int64, device="cuda")
+    good = (targets >= 0) & (targets < vocab)
+    count = int((targets != -100).sum())
+    x = logits.double().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(x[good], targets[good], reduction="sum") / count
+    g, = torch.autograd.grad(ref, x)
+    loss, work, ok = torch.empty((), device="cuda"), torch.empty(rows + 1, device="cuda"), torch.empty((), dtype=torch.bool, device="cuda")
+    fn = u.lib.b200CrossEntropy
+    assert fn(*[ctypes.c_void_p(t.data_ptr()) for t in (logits, targets, loss, work, ok)], rows, vocab, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    assert bool(ok) == (not bad)
+    assert abs(float(loss) - float(ref)) <= 2e-6 * abs(float(ref)) + 1e-6
+    assert not logits[~good].any()
+    _close(logits, g, spread=2.0 ** 20 * 1e-5 * torch.softmax(x.detach(), -1) / count)
+
+
+@gpu
 def test_cross_entropy_of_infinite_and_nan_logits():
     u = _units()
     logits = _rand(4, 64, seed=1)
