@@ -3,8 +3,10 @@
 // results once, bf16 in memory and fp32 in between; as chains of framework operations they were 60 to 80 launches per layer with
 // an fp32 copy of most operands in memory.
 // Sizes in the comments are those of 2048 tokens of a layer with hidden 4096, 32 + 8 heads of 128, ffn 14336, or of a vocabulary of
-// 16384; all kernels are bound by memory or by the latency of one row. RMSNorm takes 9 us (12 to 14 with an addition), its backward 20, the
-// rotation 8 (10 back), SwiGLU 34 (57 back: 6.2 TB/s), the cross entropy with its gradient 61 (two exponentials per logit).
+// 16384; kernel times with cold caches. The SwiGLU backward is bound by memory (55 us, 6.4 TB/s), SwiGLU by memory and its exponential
+// (35 us, 5.1 TB/s, the SMs at 72 %), the cross entropy with its gradient by its two exponentials per logit (60 us, the SMs at 80 %; its bytes
+// would take 20). The small ones are bound by the latency of a row, two trips to memory with a reduction between them: RMSNorm takes 12 us
+// (16 with an addition), its backward 19 and 6 for the gains, the rotation 10 (12 back).
 // The reference has no model code; frameworks above it (FSDP, ZeRO) run this between its all-gather and reduce-scatter calls
 // (src/collectives.cc: ncclAllGather / ncclReduceScatter).
 #include <cuda_bf16.h>

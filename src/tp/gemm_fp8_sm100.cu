@@ -3,8 +3,8 @@
 // block (scaleW[K/128][N/128]); accumulation is fp32.
 //
 // The tensor cores cannot apply fp32 block scales themselves, so accumulation has two levels:
-//   level 1  tcgen05.mma kind::f8f6f4 (128x256x32) sums one 128-wide K block into a TMEM
-//            accumulator; two 256-column accumulators alternate block by block;
+//   level 1  tcgen05.mma kind::f8f6f4 (128xBNx32, BN = 256 or 128) sums one 128-wide K block into
+//            a TMEM accumulator; two accumulators alternate block by block;
 //   level 2  the epilogue warps read each finished block from TMEM (tcgen05.ld), multiply by
 //            scaleA[row] * scaleW[block] and add into fp32 registers, while the tensor cores
 //            already work on the next K block in the other accumulator.
@@ -16,9 +16,9 @@
 // shape).
 // Plain calls with few tiles take tiles of 128 columns, or a cluster of CTAs to a tile, each with its share of the K blocks, so that
 // more SMs work (the rule and its figures are in tp.cc).
-// Persistent CTAs of three warpgroups: warp 0 TMA producer (128x128-byte A tiles, 256x128-byte W tiles,
-// 128-byte swizzle, 4-stage ring), warp 1 MMA issuer, warps 4-11 epilogue (each warp owns 32 TMEM
-// lanes and one 128-column half of the tile: 128 fp32 accumulators per thread, for which the first warpgroup hands over its
+// Persistent CTAs of three warpgroups: warp 0 TMA producer (128x128-byte A tiles, BNx128-byte W tiles,
+// 128-byte swizzle, ring of four stages, six at 128 columns), warp 1 MMA issuer, warps 4-11 epilogue (each warp owns 32 TMEM
+// lanes and one half of the tile's columns: up to 128 fp32 accumulators per thread, for which the first warpgroup hands over its
 // registers).
 // The fused modes work as in the bf16 kernel (gemm_sm100.cu): REDUCE stores the scaled tile as bf16
 // into this rank's slot of the owning rank's staging buffer over NVLink (summed afterwards);

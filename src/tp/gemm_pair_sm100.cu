@@ -1,12 +1,13 @@
 // CTA-pair variant of the tensor-parallel bf16 GEMM for sm_100a: two CTAs on neighbouring SMs (a
-// cluster of two) work on one 256 x 256 output tile with tcgen05.mma.cta_group::2.
+// cluster of two) work on one 256 x BN output tile with tcgen05.mma.cta_group::2; BN is 256, and 224 or
+// 192 for plain GEMMs that leave SMs idle otherwise (tp.cc).
 //
 // Each CTA streams only its half of the operands per 64-wide K step: 128 rows of A (its half of the
-// tile's rows) and 128 rows of W (its half of the tile's columns), 32 KiB instead of the 48 KiB a
-// single CTA needs for a 128 x 256 tile, through a 6-stage ring. One thread of the even ("leader")
-// CTA issues 256 x 256 x 16 MMAs that read both CTAs' shared memory and write both CTAs' tensor
-// memory: each CTA ends up with its 128 rows x 256 columns of the accumulator and runs the same
-// epilogue as the one-CTA kernel.
+// tile's rows) and BN / 2 rows of W (its half of the tile's columns), at 256 columns 32 KiB instead of
+// the 48 KiB a single CTA needs for a 128 x 256 tile, through a ring of six stages. One
+// thread of the even ("leader") CTA issues 256 x BN x 16 MMAs that read both CTAs' shared memory and
+// write both CTAs' tensor memory: each CTA ends up with its 128 rows x BN columns of the accumulator
+// and runs the same epilogue as the one-CTA kernel.
 //
 // Synchronisation inside the pair:
 //   fullBar[s]   (leader's copy only) counts the TMA bytes of BOTH CTAs for ring stage s: the peer's

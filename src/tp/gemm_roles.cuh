@@ -71,7 +71,7 @@ __device__ __forceinline__ bool tpWaitBlock(const TpGemmArgs& a, int mb, volatil
   return false;
 }
 
-// Epilogue of one warp for its 32 rows x 256 columns of an accumulator: tBase is the tensor-memory
+// Epilogue of one warp for its 32 rows x W columns of an accumulator: tBase is the tensor-memory
 // address of the warp's first lane and the tile's first column, row0 the global row of that lane.
 // STORE / GATHER write C; REDUCE writes slot `rank` of the staging buffer of the rank that owns the rows
 // (over NVLink when that is a peer). Each lane owns one row of the accumulator, so storing straight
@@ -79,7 +79,7 @@ __device__ __forceinline__ bool tpWaitBlock(const TpGemmArgs& a, int mb, volatil
 // transposes 64 columns at a time through 4 KiB of shared memory (16-byte chunks XOR-swizzled by
 // row against bank conflicts) and writes 128 contiguous bytes per row, four rows per instruction:
 // whole lines for HBM and NVLink.
-// W is the width of the tile: the columns behind it, and those behind the last of C, are left out (both in steps of 32).
+// Columns behind the tile's W, and those behind the last of C, are left out (both in steps of 32).
 template <int W>
 __device__ __forceinline__ void tpStoreAccum(const TpGemmArgs& a, uint32_t tBase, int row0, int nBlk, int owner, uint8_t* wbuf, int lane) {
   using namespace sm100;

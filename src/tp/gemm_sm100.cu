@@ -2,11 +2,12 @@
 // accumulation in tensor memory, fused with the collective that follows or precedes it.
 //
 // One persistent CTA per SM, 192 threads in three roles:
-//   warp 0      TMA producer: streams 128x64 A tiles and 256x64 W tiles (128-byte swizzle) through
-//               a 4-stage shared-memory ring, one elected thread, mbarrier transaction counts.
-//   warp 1      MMA issuer: one elected thread issues tcgen05.mma (128x256x16, cta_group::1) into
-//               one of two 256-column TMEM accumulators; tcgen05.commit releases ring stages and
-//               publishes finished accumulators.
+//   warp 0      TMA producer: streams 128x64 A tiles and BNx64 W tiles (128-byte swizzle) through a
+//               shared-memory ring (four stages at 256 columns, six at 128), one elected thread,
+//               mbarrier transaction counts.
+//   warp 1      MMA issuer: one elected thread issues tcgen05.mma (128xBNx16, cta_group::1) into
+//               one of two TMEM accumulators; tcgen05.commit releases ring stages and publishes
+//               finished accumulators.
 //   warps 2-5   epilogue: tcgen05.ld the accumulator (each warp owns 32 TMEM lanes = 32 rows),
 //               then, depending on the mode,
 //                 STORE      convert to bf16 and store C;
@@ -23,8 +24,9 @@
 // No load uses cluster multicast; tensor-map (tiled) TMA loads read local memory only.
 // Every wait (mbarrier, flag, cross-GPU barrier) is bounded; on expiry the kernel records a status,
 // drains its outstanding TMA copies, frees its tensor memory and returns.
-// gemm_pair_sm100.cu is the variant on CTA pairs (256 x 256 tiles, tcgen05 cta_group::2), which the host
-// prefers when every rank's rows split into 256-row tiles; this kernel covers the remaining shapes.
+// Tiles are BN = 256 columns wide in the modes with a collective; plain GEMMs take the width that fills the SMs (tp.cc).
+// gemm_pair_sm100.cu is the variant on CTA pairs (tiles of 256 rows, tcgen05 cta_group::2), which the fused modes
+// take when every rank's rows split into such tiles; gemm_split_sm100.cu shares K among CTAs where tiles are few.
 // The reference has no GEMM kernels; the comparison point is its reduce-scatter / all-gather plus a
 // separate GEMM.
 #include "gemm_roles.cuh"
