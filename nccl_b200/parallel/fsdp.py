@@ -44,6 +44,8 @@ class FSDPEngine:
     def __init__(self, comm, cfg, device="cuda", seed=0, lr=1e-4, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.1, symmetric=True, init_on_device=False):
         self.comm, self.cfg, self.device = comm, cfg, torch.device(device)
         self.cuda = self.device.type == "cuda"
+        if self.cuda and self.device.index is None:
+            self.device = torch.device("cuda", torch.cuda.current_device())
         self.n, self.rank = comm.nranks, comm.rank
         self.lr, self.betas, self.eps, self.wd = lr, betas, eps, weight_decay
         self.step_count = 0
@@ -220,6 +222,12 @@ class FSDPEngine:
     # ------------------------------------------------------------------ one training step
     def step(self, tokens, targets):
         """tokens, targets: int64 [B, S] (host or device). Returns the loss of this rank as a 0-d tensor."""
+        if not self.cuda:
+            return self._step(tokens, targets)
+        with torch.cuda.device(self.device):   # kernels and events go to the current device's streams, whichever the caller has current
+            return self._step(tokens, targets)
+
+    def _step(self, tokens, targets):
         cfg, U = self.cfg, len(self.units)
         self.step_count += 1
         tokens = tokens.to(self.device, non_blocking=True)

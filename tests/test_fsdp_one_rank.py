@@ -97,3 +97,24 @@ def test_small_pieces_wait_for_the_next():
     assert all(hi - lo >= 1 << 22 for _, lo, hi in pieces)
     eng.close()
     comm.destroy()
+
+
+def test_a_step_runs_on_the_device_of_its_engine(monkeypatch):
+    """Kernels are launched into the current device's stream: a step under another current device would give them the wrong one. No GPU is
+    touched here."""
+    import contextlib
+
+    from nccl_b200.parallel.fsdp import FSDPEngine
+    entered = []
+
+    @contextlib.contextmanager
+    def device(d):
+        entered.append(d)
+        yield
+        entered.append("left")
+
+    monkeypatch.setattr(torch.cuda, "device", device)
+    eng = FSDPEngine.__new__(FSDPEngine)
+    eng.cuda, eng.device = True, torch.device("cuda", 1)
+    eng._step = lambda tokens, targets: entered.append("step") or "loss"
+    assert eng.step(None, None) == "loss" and entered == [torch.device("cuda", 1), "step", "left"]
