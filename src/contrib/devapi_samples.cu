@@ -147,15 +147,16 @@ __global__ void __launch_bounds__(kThreads) devApiArRmsNormKernel(ncclDevComm_t 
 }
 
 // One rank: x = partial + residual, residual <- x, out <- rmsnorm(x) * weight, as above without the sources to wait for.
-// Bound by memory on the SMs that the caller grants, so what counts is how much each of them has in flight: a producer warp
+// Bound on the SMs that the caller grants by what each of them moves through shared memory and has in flight: a producer warp
 // streams chunks of R neighbouring rows (partial and residual) into a ring of shared memory with bulk copies, groups of G
-// threads take one row each from there. 2048 rows of 8192 take 34 us a call on 64 CTAs; with a CTA to a row, its loads waiting for
-// the previous row's stores, they took 127. Values are added, squared and scaled in pairs, and the gains stay in registers from row to
-// row (40 % fewer instructions: 2048 rows of 4096 20.9 -> 19.1 us, 4096 of 8192 63.0 -> 61.8); 56 registers and 1024 threads spilled.
+// threads take one row each from there. 2048 rows of 8192 take 24 us a call on 64 CTAs (5.5 TB/s; the same on 96 and 148): 127 with a CTA
+// to a row whose loads wait for the previous row's stores, and 33 while the compiler read the rows word by word, four lanes to a bank (13
+// wavefronts for 16 bytes a lane instead of 4): hence addBf16 takes values, and the ring is visibly shared memory. Values are added, squared and scaled in pairs; the gains lie beside the ring, so that 768 threads have the registers they need.
 constexpr int kRowPacks = 8;          // 16-byte packs of a row per thread, at most
 constexpr int kRowStages = 16;        // chunks in the ring, at most
 constexpr size_t kRowRing = 200 << 10;
-constexpr int kRowThreads = kThreads + 32;
+constexpr int kRowsWide = 768;        // threads of the groups where rows are long and many, kThreads otherwise
+constexpr int kRowSmem = (227 << 10) - 1024;   // ring and gains; the rest is static
 constexpr int kStatusRing = 6;        // status word: a wait on the ring ran out
 
 // Pairs of values: bf16 is the upper half of fp32.
@@ -167,7 +168,7 @@ __device__ __forceinline__ uint64_t mulF32x2(uint64_t a, uint64_t b) {
 }
 // The exact sum rounded once, which is what fp32 gives too: where a sum of two bf16 numbers does not fit into fp32, the smaller one is
 // far below a tie of the larger.
-__device__ __forceinline__ uint4 addBf16(const uint4& a, const uint4& b) {
+__device__ __forceinline__ uint4 addBf16(uint4 a, uint4 b) {
   uint4 r;
   const __nv_bfloat162 *x = (const __nv_bfloat162*)&a, *y = (const __nv_bfloat162*)&b;
   __nv_bfloat162* z = (__nv_bfloat162*)&r;
@@ -182,26 +183,29 @@ struct RowArgs {
   char* out;
   const char* weight;
   float eps;
-  int tokens, hidden, chunkRows, stages;
+  int tokens, hidden, chunkShift, stages;
   int* status;
 };
 
-template <int G>
-__global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid_constant__ RowArgs a) {
+// FULL: every thread of a group has the same number of packs. W: threads of all groups
+template <int G, bool FULL, int W>
+__global__ void __launch_bounds__(W + 32, 1) rmsNormRowsKernel(const __grid_constant__ RowArgs a) {
   using namespace b200::sm100;
-  constexpr int kGroups = kThreads / G, kWarps = G / 32;
-  extern __shared__ uint8_t ringRaw[];
-  uint8_t* ring = (uint8_t*)(((uintptr_t)ringRaw + 127) & ~(uintptr_t)127);
-  __shared__ float red[2][kThreads / 32];
+  constexpr int kGroups = W / G, kWarps = G / 32;
+  // the gains, then the ring. Aligned here and not by arithmetic, behind which the compiler no longer knew that it reads shared memory:
+  // generic loads of 16 bytes took 13 wavefronts instead of 4
+  extern __shared__ __align__(128) uint8_t gains[];
+  __shared__ float red[2][W / 32];
   __shared__ uint64_t fullBar[kRowStages], emptyBar[kRowStages];
   __shared__ volatile int gaveUp;
-  const int R = a.chunkRows, chunks = (a.tokens + R - 1) / R;
+  const int shift = a.chunkShift, R = 1 << shift, chunks = (a.tokens + R - 1) >> shift, packs = a.hidden / 8;
   const size_t rowBytes = (size_t)a.hidden * 2;
+  uint8_t* ring = gains + ((rowBytes + 127) & ~(size_t)127);
   const uint32_t half = (uint32_t)(R * rowBytes);   // partial rows, then residual rows
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.stages; ++s) {
       mbarInit(smemAddr(&fullBar[s]), 1);
-      mbarInit(smemAddr(&emptyBar[s]), R);   // one arrival per row
+      mbarInit(smemAddr(&emptyBar[s]), R * kWarps);   // one arrival per row and warp
     }
     gaveUp = 0;
     mbarInitFence();
@@ -216,8 +220,8 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
     atomicExch(a.status, kStatusRing);
     return false;
   };
-  if (threadIdx.x >= kThreads) {
-    if (threadIdx.x == kThreads) {
+  if (threadIdx.x >= W) {
+    if (threadIdx.x == W) {
       int i = 0;
       for (int c = blockIdx.x; c < chunks && !gaveUp; c += gridDim.x, ++i) {
         const int s = i % a.stages;
@@ -235,41 +239,51 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
         for (int j = i > a.stages ? i - a.stages : 0; j < i; ++j) mbarWait(smemAddr(&fullBar[j % a.stages]), (j / a.stages) & 1, 1u << 20);
     }
   } else {
-    const int grp = threadIdx.x / G, tid = threadIdx.x % G;
-    const int packs = a.hidden / 8;
-    uint4 gain[kRowPacks];   // the same channels of every row
-#pragma unroll
-    for (int k = 0; k < kRowPacks; ++k)
-      if (tid + k * G < packs) gain[k] = *(const uint4*)(a.weight + (size_t)(tid + k * G) * 16);
+    // the gains, while the first rows travel
+    for (int pk = threadIdx.x; pk < packs; pk += W) *(uint4*)(gains + (size_t)pk * 16) = *(const uint4*)(a.weight + (size_t)pk * 16);
+    asm volatile("bar.sync 15, %0;" ::"n"(W) : "memory");
+    const int grp = threadIdx.x / G;
+    const int tid = threadIdx.x % G, mine = packs / G, lap = a.stages << shift;   // rows of a lap of the ring, whole steps of the group
+    auto has = [&](int k) { return FULL ? k < mine : tid + k * G < packs; };
+    int m = grp;   // this group's row, counted from the lap's first
+    uint32_t phase = 0;
     int parity = 0;
     // row n of this CTA: row n % R of its chunk n / R
     for (int n = grp;; n += kGroups, parity ^= 1) {
-      const int i = n / R, c = (int)blockIdx.x + i * (int)gridDim.x, r = n - i * R;
+      const int c = (int)blockIdx.x + (n >> shift) * (int)gridDim.x;
       if (c >= chunks) break;
-      const int t = c * R + r;
+      const int r = m & (R - 1), t = c * R + r;
       if (t >= a.tokens) break;
-      const int s = i % a.stages;
+      const int s = m >> shift;
       // a row that did not arrive is left alone: neither read, stored nor released; its group still meets at the barrier
-      const bool ok = wait(&fullBar[s], (i / a.stages) & 1);
-      const int rowPacks = ok ? packs : 0;
-      const uint8_t* part = ring + (size_t)s * 2 * half + r * rowBytes;
-      char* res = a.residual + t * rowBytes;
+      const bool ok = wait(&fullBar[s], phase);
+      if ((m += kGroups) >= lap) {
+        m -= lap;
+        phase ^= 1;
+      }
+      const uint8_t* part = ring + (size_t)s * 2 * half + r * rowBytes + tid * 16;
+      const size_t at = t * rowBytes + tid * 16;
+      char* res = a.residual + at;
       uint4 sum[kRowPacks];
       uint64_t squares = 0;   // two fp32 sums
+      if (ok) {
 #pragma unroll
-      for (int k = 0; k < kRowPacks; ++k) {
-        const int pk = tid + k * G;
-        if (pk < rowPacks) {
-          // the residual stream is kept in bf16: normalise exactly what is stored
-          sum[k] = addBf16(*(const uint4*)(part + (size_t)pk * 16), *(const uint4*)(part + half + (size_t)pk * 16));
-          *(uint4*)(res + (size_t)pk * 16) = sum[k];
-          const uint32_t u[4] = {sum[k].x, sum[k].y, sum[k].z, sum[k].w};
+        for (int k = 0; k < kRowPacks; ++k) {
+          if (has(k)) {
+            // the residual stream is kept in bf16: normalise exactly what is stored
+            const uint4 x = *(const uint4*)(part + k * G * 16), y = *(const uint4*)(part + half + k * G * 16);
+            sum[k] = addBf16(x, y);
+            *(uint4*)(res + k * G * 16) = sum[k];
+            const uint32_t u[4] = {sum[k].x, sum[k].y, sum[k].z, sum[k].w};
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint64_t x = unpackBf16x2(u[j]);
-            fmaF32x2(squares, x, x);
+            for (int j = 0; j < 4; ++j) {
+              const uint64_t x = unpackBf16x2(u[j]);
+              fmaF32x2(squares, x, x);
+            }
           }
         }
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) mbarArrive(smemAddr(&emptyBar[s]));   // the warp has read its part of the row
       }
       float ss = __uint_as_float((uint32_t)squares) + __uint_as_float((uint32_t)(squares >> 32));
 #pragma unroll
@@ -282,25 +296,24 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) ss += red[parity][grp * kWarps + w];
       }
-      if (tid == 0 && ok) mbarArrive(smemAddr(&emptyBar[s]));   // the whole group has read the row
+      if (!ok) continue;
       const float inv = rsqrtf(ss / (float)a.hidden + a.eps);
       const uint64_t inv2 = packF32x2(__float_as_uint(inv), __float_as_uint(inv));
-      char* out = a.out + t * rowBytes;
+      char* out = a.out + at;
+      const uint8_t* gain = gains + tid * 16;
 #pragma unroll
       for (int k = 0; k < kRowPacks; ++k) {
-        const int pk = tid + k * G;
-        if (pk < rowPacks) {
-          const uint32_t u[4] = {sum[k].x, sum[k].y, sum[k].z, sum[k].w};
-          uint32_t g[4] = {gain[k].x, gain[k].y, gain[k].z, gain[k].w}, o[4];
-          // keeps the gains packed: unpacked ahead of the loop over the rows they would not fit
-          asm volatile("" : "+r"(g[0]), "+r"(g[1]), "+r"(g[2]), "+r"(g[3]));
+        if (has(k)) {
+          const uint4 gk = *(const uint4*)(gain + k * G * 16);
+          const uint32_t u[4] = {sum[k].x, sum[k].y, sum[k].z, sum[k].w}, g[4] = {gk.x, gk.y, gk.z, gk.w};
+          uint32_t o[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const uint64_t y = mulF32x2(mulF32x2(unpackBf16x2(u[j]), inv2), unpackBf16x2(g[j]));
             const __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float((uint32_t)y), __uint_as_float((uint32_t)(y >> 32)));
             o[j] = *(const uint32_t*)&b;
           }
-          *(uint4*)(out + (size_t)pk * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+          *(uint4*)(out + k * G * 16) = make_uint4(o[0], o[1], o[2], o[3]);
         }
       }
     }
@@ -314,9 +327,9 @@ __global__ void __launch_bounds__(kRowThreads, 1) rmsNormRowsKernel(const __grid
 // when it has seen the one before: nothing orders the copies of two chunks, and a wait that skips a use would take a slot whose
 // copy of the lap before is still under way for loaded. Group g takes rows g, g + groups, ... of its CTA, so it sees every use of
 // the slots that it reads when a lap of the ring (stages x chunkRows rows) is a whole number of its steps. Both are kept to
-// multiples that see to it: 8192 channels get 4 stages where the ring would hold 6.
+// multiples that see to it: four groups get 4 stages of 8192 channels where the ring would hold 6.
 struct RowPlan {
-  int group, chunkRows, stages;
+  int group, threads, chunkRows, stages;
 };
 
 RowPlan rowPlan(int tokens, int hidden, int nCtas) {
@@ -325,30 +338,37 @@ RowPlan rowPlan(int tokens, int hidden, int nCtas) {
   // the fewest threads to a row that hold it, more where there are not enough rows for that many groups
   p.group = 32;
   while (p.group < kThreads && (p.group * kRowPacks < hidden / 8 || (long long)nCtas * (kThreads / p.group) > tokens)) p.group *= 2;
-  // chunks of about 8 KiB (a copy below that costs more to issue than to move), while every CTA still gets several; a power of
-  // two, like the number of groups
+  // Six rows under way in a CTA instead of four where that many fit the ring as well as four do and there are enough of them: 2048 x 8192 24.2 us
+  // for 25.5 with 512 threads, 3000 x 7168 30.5 for 33.0, 1000 x 8104 13.8 for 14.1. The other side of the line: 1024 x 5120 10.1 / 9.9, 700 x 6144
+  // 8.5 / 8.3, 256 x 8192 5.0 / 4.8.
+  p.threads = p.group == 128 && hidden > 6144 && tokens >= 12 * nCtas ? kRowsWide : kThreads;
+  // chunks of about 8 KiB (a copy below that costs more to issue than to move), while every CTA still gets several; a power of two
   const int rows = std::min((int)(8192 / rowBytes), tokens / (4 * nCtas));
   p.chunkRows = 1;
   while (2 * p.chunkRows <= rows) p.chunkRows *= 2;
-  const int step = std::max(1, kThreads / p.group / p.chunkRows);
+  int step = p.threads / p.group;
+  for (int r = p.chunkRows; r > 1 && step % 2 == 0; r /= 2) step /= 2;
   p.stages = (int)std::min<size_t>(kRowStages, kRowRing / (2 * p.chunkRows * rowBytes)) / step * step;
   return p;
 }
 
+template <int G, int W = kThreads> const void* rowsKernel(bool full) { return full ? (const void*)rmsNormRowsKernel<G, true, W> : (const void*)rmsNormRowsKernel<G, false, W>; }
+
 ncclResult_t launchRmsNormRows(RowArgs a, int nCtas, cudaStream_t stream) {
   const RowPlan p = rowPlan(a.tokens, a.hidden, nCtas);
-  a.chunkRows = p.chunkRows;
+  a.chunkShift = __builtin_ctz(p.chunkRows);
   a.stages = p.stages;
-  const size_t smem = 128 + (size_t)a.hidden * 4 * a.chunkRows * a.stages;
-  const void* fn = p.group == 32 ? (const void*)rmsNormRowsKernel<32> : p.group == 64 ? (const void*)rmsNormRowsKernel<64> : p.group == 128 ? (const void*)rmsNormRowsKernel<128> :
-                   p.group == 256 ? (const void*)rmsNormRowsKernel<256> : (const void*)rmsNormRowsKernel<512>;
+  const size_t smem = 128 + (size_t)a.hidden * 4 * p.chunkRows * p.stages + (size_t)a.hidden * 2;
+  const bool full = a.hidden / 8 % p.group == 0;
+  const void* fn = p.threads == kRowsWide ? rowsKernel<128, kRowsWide>(full) : p.group == 32 ? rowsKernel<32>(full) : p.group == 64 ? rowsKernel<64>(full) :
+                   p.group == 128 ? rowsKernel<128>(full) : p.group == 256 ? rowsKernel<256>(full) : rowsKernel<512>(full);
   // The limit belongs to the function, which threads with other shapes launch at the same time: every call sets the same value, the
   // largest ring, and never one below what another is about to launch with.
   void* args[1] = {&a};
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute pdl;
   cfg.gridDim = dim3(nCtas);
-  cfg.blockDim = dim3(kRowThreads);
+  cfg.blockDim = dim3(p.threads + 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   if (b200::devPlanePdl()) {
@@ -357,7 +377,7 @@ ncclResult_t launchRmsNormRows(RowArgs a, int nCtas, cudaStream_t stream) {
     cfg.attrs = &pdl;
     cfg.numAttrs = 1;
   }
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(128 + kRowRing)) == cudaSuccess &&
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowSmem) == cudaSuccess &&
       cudaLaunchKernelExC(&cfg, fn, args) == cudaSuccess)
     return ncclSuccess;
   (void)cudaGetLastError();   // the call reports it: later checks do not find it again
@@ -453,7 +473,7 @@ ncclResult_t b200DevApiArRmsNormPlan(int tokens, int hidden, int nCtas, int plan
   if (!plan || tokens < 0 || hidden < 8 || hidden % 8 || hidden > 8 * kThreads * 4 || nCtas < 1) return ncclInvalidArgument;
   const RowPlan p = rowPlan(tokens, hidden, nCtas);
   plan[0] = p.group;
-  plan[1] = kThreads;
+  plan[1] = p.threads;
   plan[2] = p.chunkRows;
   plan[3] = p.stages;
   return ncclSuccess;

@@ -41,6 +41,13 @@ def test_rows(hidden, tokens, ctas):
     comm.destroy()
 
 
+@pytest.mark.parametrize("hidden", [6144, 6152, 7168, 8104, 8184])
+@pytest.mark.parametrize("tokens,ctas", [(35, 3), (36, 3), (77, 5), (770, 64)])
+def test_long_rows(hidden, tokens, ctas):
+    """Both sides of the line behind which a CTA has six rows under way: rows longer than 6144, twelve to a CTA."""
+    test_rows(hidden, tokens, ctas)
+
+
 @pytest.mark.parametrize("tokens,hidden", [(5, 0), (5, -8), (0, 1024)])
 def test_empty_calls(tokens, hidden):
     """No rows, or rows without channels, are an empty call of the C entry point: nothing is divided by their size, nothing is
