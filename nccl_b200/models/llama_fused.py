@@ -7,7 +7,7 @@ buffers, with the backward written out:
     (src/contrib/train_ops.cu) in place of chains of framework operations;
   * wq | wk | wv and w_gate | w_up lie next to each other in the flat buffer and are one matrix each;
   * weight gradients are written where the reduce-scatter reads them, and the recomputation leaves out the last product,
-    whose result no gradient needs.
+    whose result no gradient needs; a layer whose activations were kept is not computed again.
 
 Between kernels everything is bf16 as before; sums, exponentials and rotations are held in fp32. The forward rounds where the
 operations of `llama` round, so that both give the same loss up to the order of sums; the backward rounds each result once.
@@ -147,19 +147,33 @@ class FusedUnits:
         q, k, v = (t.transpose(1, 2) for t in qkv.view(B, S, c.heads + 2 * c.kv_heads, c.head_dim).split((c.heads, c.kv_heads, c.kv_heads), dim=2))
         if backward:
             q, k, v = (t.detach().requires_grad_(True) for t in (q, k, v))
-        return x, h, rstd, (q, k, v), F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
+        with torch.set_grad_enabled(backward):
+            return x, h, rstd, (q, k, v), F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
 
-    def layer(self, x, add, flat, rope, shape):
-        """The layer of input x + add (add may be None), [B * S, hidden] with shape = (B, S): its input and its output, the latter as two terms
-        that the next unit's norm adds up."""
+    def activation_bytes(self, tokens):
+        """What `layer` hands over to its backward for so many tokens, beside its input."""
+        c = self.cfg
+        return tokens * (2 * (4 * c.hidden + (c.heads + 2 * c.kv_heads) * c.head_dim + 2 * c.ffn) + 4 * c.heads + 8)
+
+    def _to_product(self, x, add, p, rope, shape, backward):
+        """(x + add, (norm1's output and 1 / rms, q, k, v, attention's output, norm2's sum, output and 1 / rms, gate and up))."""
+        x, h1, rstd1, qkv, a = self._up_to_attention(x, add, p, rope, shape, backward)
+        o = a.detach().transpose(1, 2).reshape(x.shape)
+        x2, h2, rstd2 = self.norm(x, p["norm2"], add=torch.mm(o, p["wo"].t()), need_rstd=backward)
+        return x, (h1, rstd1, qkv, a, x2, h2, rstd2, torch.mm(h2, p["w_gu"].t()))
+
+    def layer(self, x, add, flat, rope, shape, keep=False):
+        """The layer of input x + add (add may be None), [B * S, hidden] with shape = (B, S): its input, its output as two terms that the next
+        unit's norm adds up, and with `keep` what `layer_backward` would compute again."""
         p = self._layer_views(flat)
-        x, _, _, _, a = self._up_to_attention(x, add, p, rope, shape, False)
-        y, h, _ = self.norm(x, p["norm2"], add=torch.mm(a.transpose(1, 2).reshape(x.shape), p["wo"].t()))
-        return x, y, torch.mm(self.swiglu(torch.mm(h, p["w_gu"].t())), p["w_down"].t())
+        x, acts = self._to_product(x, add, p, rope, shape, keep)
+        out = x, acts[4], torch.mm(self.swiglu(acts[7]), p["w_down"].t())
+        return out + (acts,) if keep else out
 
-    def layer_backward(self, x, flat, gflat, rope, shape, gy, ready=None, before=None):
+    def layer_backward(self, x, flat, gflat, rope, shape, gy, ready=None, before=None, kept=None):
         """Gradient of the layer's input; the weights' gradients go into gflat (laid out like flat). before() is called ahead of the first
-        write into gflat, ready(lo) is told that from element lo on the gradients are written and the weights are read no more."""
+        write into gflat, ready(lo) is told that from element lo on the gradients are written and the weights are read no more. `kept` comes
+        from `layer`, and is used up."""
         p, g = self._layer_views(flat), self._layer_views(gflat)
         begin = flat.data_ptr()
 
@@ -167,10 +181,9 @@ class FusedUnits:
             if ready:
                 ready((p[name].data_ptr() - begin) // flat.element_size())
 
-        _, h1, rstd1, qkv, a = self._up_to_attention(x, None, p, rope, shape, True)
+        h1, rstd1, qkv, a, x2, h2, rstd2, gu = kept or self._to_product(x, None, p, rope, shape, True)[1]
+        del kept
         o = a.detach().transpose(1, 2).reshape(x.shape)
-        x2, h2, rstd2 = self.norm(x, p["norm2"], add=torch.mm(o, p["wo"].t()), need_rstd=True)
-        gu = torch.mm(h2, p["w_gu"].t())
         act = torch.mm(gy, p["w_down"])
         self.swiglu_backward(gu, act)
         if before:

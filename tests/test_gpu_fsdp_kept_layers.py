@@ -1,0 +1,47 @@
+"""The sharded engine with the activations of none, some and all layers kept for the backward: the same gradients as computing them again."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape", [(1, 65), (2, 128)])
+def test_kept_layers(shape, monkeypatch):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from nccl_b200 import Communicator, get_unique_id
+    from nccl_b200.models import llama as M
+    from nccl_b200.parallel.fsdp import FSDPEngine
+    torch.cuda.set_device(0)
+    comm = Communicator(1, 0, get_unique_id())
+    cfg = M.LlamaConfig(layers=3, hidden=256, heads=4, kv_heads=2, ffn=512, vocab=1024)
+    g = torch.Generator().manual_seed(3)
+    tok, tgt = (torch.randint(0, cfg.vocab, shape, generator=g) for _ in range(2))
+    got = []
+    for layers in (0, 2, 3, None):
+        eng = FSDPEngine(comm, cfg, device="cuda", seed=1, lr=1e-3, eps=1.0, init_on_device=True)
+        used = []
+        again = eng.fused._to_product
+        monkeypatch.setattr(eng.fused, "_to_product", lambda *a: used.append(a[-1]) or again(*a))
+        if layers is None:   # by what is free: a small model has room for all
+            assert eng._layers_kept(tok.numel()) == cfg.layers
+            monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (0, 0))
+            monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda *a: {k: {"all": {"current": 0}} for k in ("reserved_bytes", "allocated_bytes")})
+            assert eng._layers_kept(tok.numel()) == 0   # nothing free: none
+            monkeypatch.undo()
+        else:
+            monkeypatch.setattr(eng, "_layers_kept", lambda tokens: layers)
+        losses = [eng.step(tok, tgt) for _ in range(2)]
+        torch.cuda.synchronize()
+        if layers is not None:   # forward passes with and without what the backward needs, then the layers computed again, for each step
+            assert used == ([False] * (3 - layers) + [True] * 3) * 2
+        got.append((torch.stack(losses), [u.m.clone() for u in eng.units]))
+        eng.close()
+    for losses, ms in got[1:]:
+        # the same operations on the same values; attention alone may pick another kernel where no gradient is wanted, and adds its gradients up
+        # in no fixed order: both within bf16's rounding of one of some 30 chained results (2**-9)
+        assert torch.allclose(losses, got[0][0], rtol=2 ** -9)
+        for a, b in zip(ms, got[0][1]):
+            assert float((a.double() - b.double()).norm() / b.double().norm()) < 3e-2
+    comm.destroy()
