@@ -663,29 +663,41 @@ __global__ void __launch_bounds__(kEpThreads, 1) epCombineKernel(const __grid_co
 // claims the rows of the output tensors and writes them straight from the input (the general kernel stores into a landing
 // zone and packs from there: written twice, read once more), combine reads the experts' rows where they lie. Both are bound
 // by memory: for 4096 tokens of 7168 bf16 channels and 8 of 32 experts dispatch went from 313 to 103 us and combine from 434 to
-// 81 us (5.1 and 6.5 TB/s).
+// 81 us (5.1 and 6.5 TB/s). Dispatch reads and writes 32 bytes at a time where tokens in and out are aligned to them, which the
+// queue of memory instructions held up (us with 16 / 32 bytes, launches of one after the other): 2000 tokens of 4096 to one row each
+// in fp8 8.9 / 7.0, 1000 of 7168 in bf16 to four experts 16.1 / 14.2, 8 of 7168 in fp8 to eight 5.4 / 5.0, one of 1024 3.7 / 3.6.
 constexpr int kLocTokens = 64;    // tokens of a CTA whose rows are claimed (or looked up) together
 constexpr int kLocMaxK = 16;
 
-// Payload of the tokens t0 + j * tStep, j < batch, to the rows sRow[j * R .. j * R + R) (-1: none). A work item is one 16-byte
-// store per row: 8 channels of bf16, or 16 channels of e4m3, whose group of 128 is then shared by 8 lanes. The items of the
-// batch are dealt to the threads without regard to token borders, and the loads of a round are issued before the previous
-// round is stored. `claim` fills sRow between the first loads and the first stores.
-template <bool FP8, typename Claim>
+// Payload of the tokens t0 + j * tStep, j < batch, to the rows sRow[j * R .. j * R + R) (-1: none). A work item is one store of
+// 16 bytes (WIDE: 32) per row: 8 (16) channels of bf16, or 16 (32) channels of e4m3, whose group of 128 is then shared by 8 (4) lanes.
+// The items of the batch are dealt to the threads without regard to token borders, and the loads of a round are issued before the
+// previous round is stored. `claim` fills sRow between the first loads and the first stores.
+template <bool FP8, bool WIDE, typename Claim>
 __device__ __forceinline__ void localPayload(const EpArgs& a, const __nv_bfloat16* x, int t0, int tStep, int batch, int R, const int* sRow, Claim claim) {
-  constexpr int U = 2;                      // items of a thread per round
-  constexpr int kIn = FP8 ? 2 : 1;          // 16-byte loads of an item
+  constexpr int U = WIDE && FP8 ? 1 : 2;    // items of a thread per round
+  constexpr int W = WIDE ? 2 : 1;           // 16-byte packs of a store
+  constexpr int kIn = FP8 ? 2 * W : W;      // and of an item's channels in bf16
+  constexpr int kLanes = 8 / W;             // of a group of 128 channels
   const int H = a.hidden, C = H / (8 * kIn);
-  const int total = batch * C;              // a multiple of 8: the lanes of a group are in or out together
+  const int total = batch * C;              // a multiple of kLanes: the lanes of a group are in or out together
   uint4 cur[U][kIn];
   auto load = [&](int first) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = first + u * kEpLocalThreads;
       const int j = i / C, c = i - j * C;
+      const __nv_bfloat16* from = x + (size_t)(t0 + j * tStep) * H + (size_t)c * kIn * 8;
 #pragma unroll
-      for (int q = 0; q < kIn; ++q)
-        cur[u][q] = i < total ? ldStream16(x + (size_t)(t0 + j * tStep) * H + (size_t)(c * kIn + q) * 8) : make_uint4(0, 0, 0, 0);
+      for (int q = 0; q < kIn; q += W) {
+        if (WIDE) {
+          const Pack32 p = i < total ? ldStream32(from + q * 8) : Pack32{};
+          cur[u][q] = p.lo;
+          cur[u][q + W - 1] = p.hi;
+        } else {
+          cur[u][q] = i < total ? ldStream16(from + q * 8) : make_uint4(0, 0, 0, 0);
+        }
+      }
     }
   };
   const size_t rowBytes = FP8 ? (size_t)H : (size_t)H * 2;
@@ -693,13 +705,13 @@ __device__ __forceinline__ void localPayload(const EpArgs& a, const __nv_bfloat1
   load(threadIdx.x);
   claim();
   for (int first = threadIdx.x; first - (int)(threadIdx.x & 31) < total; first += U * kEpLocalThreads) {
-    uint4 val[U];
+    uint4 val[U][W];
     float scale[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       scale[u] = 0.0f;
       if (FP8) {
-        float v[16];
+        float v[kIn * 8];
         float amax = 0.0f;
 #pragma unroll
         for (int q = 0; q < kIn; ++q) {
@@ -712,20 +724,19 @@ __device__ __forceinline__ void localPayload(const EpArgs& a, const __nv_bfloat1
           }
         }
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        for (int o = kLanes / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
         amax = fmaxf(amax, 1e-4f);
         scale[u] = amax * (1.0f / 448.0f);
         const float inv = 448.0f / amax;
-        uint32_t w[4];
+        auto e4m3x4 = [&](int i) {
+          return (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(v[i] * inv, v[i + 1] * inv), __NV_SATFINITE, __NV_E4M3) |
+                 ((uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(v[i + 2] * inv, v[i + 3] * inv), __NV_SATFINITE, __NV_E4M3) << 16);
+        };
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          w[i] = (uint32_t)__nv_cvt_float_to_fp8(v[4 * i] * inv, __NV_SATFINITE, __NV_E4M3) |
-                 ((uint32_t)__nv_cvt_float_to_fp8(v[4 * i + 1] * inv, __NV_SATFINITE, __NV_E4M3) << 8) |
-                 ((uint32_t)__nv_cvt_float_to_fp8(v[4 * i + 2] * inv, __NV_SATFINITE, __NV_E4M3) << 16) |
-                 ((uint32_t)__nv_cvt_float_to_fp8(v[4 * i + 3] * inv, __NV_SATFINITE, __NV_E4M3) << 24);
-        val[u] = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int w = 0; w < W; ++w) val[u][w] = make_uint4(e4m3x4(16 * w), e4m3x4(16 * w + 4), e4m3x4(16 * w + 8), e4m3x4(16 * w + 12));
       } else {
-        val[u] = cur[u][0];
+#pragma unroll
+        for (int w = 0; w < W; ++w) val[u][w] = cur[u][w];
       }
     }
     load(first + U * kEpLocalThreads);
@@ -737,14 +748,16 @@ __device__ __forceinline__ void localPayload(const EpArgs& a, const __nv_bfloat1
       for (int r = 0; r < R; ++r) {
         const int row = sRow[j * R + r];
         if (row < 0) continue;
-        st16(out + (size_t)row * rowBytes + (size_t)c * 16, val[u]);
-        if (FP8 && (c & 7) == 0) a.outScales[a.rank][(size_t)row * (H / 128) + (c >> 3)] = scale[u];
+        char* to = out + (size_t)row * rowBytes + (size_t)c * 16 * W;
+        if (WIDE) st32(to, {val[u][0], val[u][W - 1]});
+        else st16(to, val[u][0]);
+        if (FP8 && c % kLanes == 0) a.outScales[a.rank][(size_t)row * (H / 128) + c / kLanes] = scale[u];
       }
     }
   }
 }
 
-template <bool FP8>
+template <bool FP8, bool WIDE>
 __global__ void __launch_bounds__(kEpLocalThreads, 2) epDispatchLocalKernel(const __grid_constant__ EpArgs a) {
   pdlEnter();
   __shared__ int sRow[kLocTokens * kLocMaxK];
@@ -795,7 +808,7 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epDispatchLocalKernel(cons
     const bool has = (int)threadIdx.x < batch * K;
     const int64_t e0 = has ? idx[o0] : -1;
     const float w0 = has && rankMajor && a.outTopkW[me] && a.topkW[me] ? a.topkW[me][o0] : 0.0f;
-    localPayload<FP8>(a, a.x[me], t0, grid, batch, R, sRow, [&] {
+    localPayload<FP8, WIDE>(a, a.x[me], t0, grid, batch, R, sRow, [&] {
       __syncthreads();   // the previous batch is stored
       if (rankMajor) {
         for (int j = threadIdx.x; j < batch; j += kEpLocalThreads) sRow[j] = -1;
@@ -1007,7 +1020,10 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epCombineLocalKernel(const
 
 const void* epDispatchKernelFn() { return (const void*)epDispatchKernel; }
 const void* epCombineKernelFn() { return (const void*)epCombineKernel; }
-const void* epDispatchLocalKernelFn(int fp8) { return fp8 ? (const void*)epDispatchLocalKernel<true> : (const void*)epDispatchLocalKernel<false>; }
+const void* epDispatchLocalKernelFn(int fp8, bool wide) {
+  if (wide) return fp8 ? (const void*)epDispatchLocalKernel<true, true> : (const void*)epDispatchLocalKernel<false, true>;
+  return fp8 ? (const void*)epDispatchLocalKernel<true, false> : (const void*)epDispatchLocalKernel<false, false>;
+}
 const void* epCombineLocalKernelFn() { return (const void*)epCombineLocalKernel; }
 
 }  // namespace b200

@@ -76,7 +76,7 @@ const void* epDispatchKernelFn();
 const void* epCombineKernelFn();
 // A group of one rank, both halves in one call, expert-major or rank-major: no landing zones, no flags. kEpLocalThreads threads.
 constexpr int kEpLocalThreads = 512;
-const void* epDispatchLocalKernelFn(int fp8);
+const void* epDispatchLocalKernelFn(int fp8, bool wide);   // wide: tokens in and out are 32-byte aligned
 const void* epCombineLocalKernelFn();
 
 }  // namespace b200

@@ -414,7 +414,8 @@ ncclResult_t ncclEpDispatch(ncclEpHandle_t h, const ncclEpDispatchInputs_t* in, 
                 {outW, rows * K * sizeof(float)}, {counters, g->El * sizeof(int)}},
                {{a.x[me], T * g->H * 2}, {a.topkIdx[me], T * K * sizeof(int64_t)}, {a.topkW[me], T * K * sizeof(float)}})) {
     a.userCount = (int*)counters;
-    return launchEpLocal(g, epDispatchLocalKernelFn(fp8), &a, std::max(h->T, a.layout == EP_RANK_MAJOR ? (g->maxTokens + kEpLocalThreads - 1) / kEpLocalThreads : 1), stream);
+    const bool wide = !(((uintptr_t)a.x[me] | (uintptr_t)a.outTokens[me]) & 31);   // rows are whole multiples of 128 bytes
+    return launchEpLocal(g, epDispatchLocalKernelFn(fp8, wide), &a, std::max(h->T, a.layout == EP_RANK_MAJOR ? (g->maxTokens + kEpLocalThreads - 1) / kEpLocalThreads : 1), stream);
   }
   // the per-rank layouts count the tokens of every local expert with atomics while they unpack: start from zero
   if (a.layout != EP_EXPERT_MAJOR && !sendOnly) CUDACHECK(cudaMemsetAsync(h->expertCount, 0, (size_t)g->El * sizeof(int), stream));

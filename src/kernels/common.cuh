@@ -66,6 +66,20 @@ __device__ __forceinline__ uint4 ldStream16(const void* p) {
   asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
   return v;
 }
+// 32 bytes in one access: half of the instructions where rows are 32-byte aligned
+struct Pack32 {
+  uint4 lo, hi;
+};
+__device__ __forceinline__ Pack32 ldStream32(const void* p) {
+  Pack32 v;
+  asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v.lo.x), "=r"(v.lo.y), "=r"(v.lo.z), "=r"(v.lo.w), "=r"(v.hi.x), "=r"(v.hi.y), "=r"(v.hi.z), "=r"(v.hi.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st32(void* p, Pack32 v) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v.lo.x), "r"(v.lo.y), "r"(v.lo.z), "r"(v.lo.w), "r"(v.hi.x), "r"(v.hi.y),
+               "r"(v.hi.z), "r"(v.hi.w) : "memory");
+}
 __device__ __forceinline__ uint4 ldLocal16(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 __device__ __forceinline__ void st16(void* p, uint4 v) { *reinterpret_cast<uint4*>(p) = v; }
 

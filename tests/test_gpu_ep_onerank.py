@@ -161,3 +161,30 @@ def test_calls_in_a_row_leave_no_counts_behind(comm, layout):
         torch.testing.assert_close(out.float(), ref, rtol=2 ** -7, atol=1e-6)
     assert comm.async_error() == 0
     ep.destroy()
+
+
+@pytest.mark.parametrize("T,H,max_sms", [(1, 128, 0), (33, 384, 0), (200, 640, 1)])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_tokens_at_sixteen_bytes(comm, T, H, max_sms, fp8):
+    """Tokens that start on 16 bytes, but not on 32, give the bytes that aligned ones give, and nothing beside the rows is written."""
+    from nccl_b200.ops.ep import ExpertParallel
+    ep = ExpertParallel(comm, 8, T, H, max_sms=max_sms, layout="rank_major")
+    x, idx, w = _batch(T, 8, 2, H, 11, 0.1)
+    dt, off = (torch.uint8, 16) if fp8 else (torch.bfloat16, 8)
+    got = []
+    for at_in, at_out in ((0, 0), (8, 0), (0, off), (8, off)):
+        xs = torch.empty(T * H + 16, dtype=torch.bfloat16, device="cuda")[at_in:at_in + T * H].view(T, H).copy_(x)
+        buf = torch.full((T * H + 64,), 7, dtype=dt, device="cuda")
+        toks = buf[at_out:at_out + T * H].view(1, T, H)
+        assert xs.data_ptr() % 32 == 2 * at_in and toks.data_ptr() % 32 == (16 if at_out else 0)
+        scales = torch.zeros(1, T, H // 128, device="cuda") if fp8 else None
+        ep.dispatch(xs, idx, w, fp8=fp8, toks=toks, scales=scales)
+        torch.cuda.synchronize()
+        assert (buf[:at_out] == 7).all() and (buf[at_out + T * H:] == 7).all()
+        used = (idx >= 0).any(1)
+        got.append((toks[0][used].clone(), scales[0][used].clone() if fp8 else None))
+    for toks, scales in got[1:]:
+        assert torch.equal(toks, got[0][0]) and (not fp8 or torch.equal(scales, got[0][1]))
+    if not fp8:
+        assert torch.equal(got[0][0], x[(idx >= 0).any(1)])
+    ep.destroy()
