@@ -22,7 +22,9 @@ namespace {
 
 constexpr int kMaxRowThreads = 512;
 
-__device__ __forceinline__ void unpack8(const uint4& q, float* f) {
+// By value: bound to memory, a reference was read word by word, 16 bytes apart from lane to lane (2048 rows of 4096, caches flushed: the norm with an
+// addition 21.4 us, 19.4 by value, its backward 29.5 and 27.5; kernels that load every operand at once lost nothing).
+__device__ __forceinline__ void unpack8(uint4 q, float* f) {
   const __nv_bfloat162* p = (const __nv_bfloat162*)&q;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -266,10 +268,11 @@ __global__ void __launch_bounds__(256) swigluBackwardKernel(uint4* gu, uint4* da
   uint4* gp = gu + row * 2 * packs + p;
   uint4* up = gp + packs;
   uint4* dp = dact + row * packs + p;
+  const uint4 qg = *gp, qu = *up, qd = *dp;
   float g[8], u[8], d[8];
-  unpack8(*gp, g);
-  unpack8(*up, u);
-  unpack8(*dp, d);
+  unpack8(qg, g);
+  unpack8(qu, u);
+  unpack8(qd, d);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const float sig = 1.0f / (1.0f + expf(-g[i])), silu = g[i] * sig, dd = d[i];
