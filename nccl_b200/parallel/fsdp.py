@@ -37,6 +37,10 @@ def _align(n, a):
 kEarlyUpdate = 1 << 24
 
 
+# bytes that a program may have allocated since the last decision on kept layers (losses that it collects) without another one
+kDrift = 16 << 20
+
+
 class _Unit:
     pass
 
@@ -107,6 +111,7 @@ class FSDPEngine:
                 e.record()
         self.collectives = 0      # all-gathers + reduce-scatters issued (for reporting)
         self.kernels = 0          # AdamW launches
+        self._kept_for = None
 
     # ------------------------------------------------------------------ memory
     def _buffer(self, numel, dtype):
@@ -232,19 +237,27 @@ class FSDPEngine:
         """How many layers, counted from the last, keep their activations for the backward instead of computing them again there: as many as leave
         half of the memory that the framework's allocator can still get beyond what the step takes anyway (the logits, every
         layer's input, one layer's activations). Two layers of hidden 4096 and ffn 14336 with 2048 tokens: 420 MB. Under capture, and where the allocator does
-        not tell, none."""
+        not tell, none.
+
+        The driver is asked (60 us, and many milliseconds while other processes keep it busy) only when the allocator holds other memory than
+        at the last decision for as many tokens: while it does not, the step runs in the memory that it ran in before."""
         if torch.cuda.is_current_stream_capturing():
             return 0
         try:
             stats = torch.cuda.memory_stats_as_nested_dict(self.device)
-            cached = stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"]
-            room = torch.cuda.mem_get_info(self.device)[0] + cached
+            reserved, used = stats["reserved_bytes"]["all"]["current"], stats["allocated_bytes"]["all"]["current"]
+            decided = self._kept_for
+            if decided and decided[:2] == (tokens, reserved) and used <= decided[2] + kDrift:
+                return decided[3]
+            room = torch.cuda.mem_get_info(self.device)[0] + reserved - used
         except (RuntimeError, KeyError):
             return 0
         c, layers = self.cfg, len(self.units) - 2
         each = self.fused.activation_bytes(tokens)
         needed = each + 2 * tokens * (c.vocab + (layers + 8) * c.hidden + 2 * c.ffn)
-        return max(0, min(layers, (room // 2 - needed) // each))
+        kept = max(0, min(layers, (room // 2 - needed) // each))
+        self._kept_for = (tokens, reserved, used, kept)
+        return kept
 
     def _step(self, tokens, targets):
         cfg, U = self.cfg, len(self.units)

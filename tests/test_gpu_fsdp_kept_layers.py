@@ -30,15 +30,29 @@ def test_kept_layers(shape, monkeypatch):
             monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda *a: {k: {"all": {"current": 0}} for k in ("reserved_bytes", "allocated_bytes")})
             assert eng._layers_kept(tok.numel()) == 0   # nothing free: none
             monkeypatch.undo()
+            asked = []
+            real = torch.cuda.mem_get_info
+            monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: asked.append(1) or real(*a))
+            for _ in range(3):   # the second step finds what the first one left in the allocator, the third finds no change
+                eng.step(tok, tgt)
+            n = len(asked)
+            eng.step(tok, tgt)
+            assert 1 <= n <= 3 and len(asked) == n
+            held = torch.empty(1 << 26, dtype=torch.uint8, device="cuda")
+            eng.step(tok, tgt)
+            assert len(asked) == n + 1
+            del held
+            eng.close()
+            continue
         else:
             monkeypatch.setattr(eng, "_layers_kept", lambda tokens: layers)
         losses = [eng.step(tok, tgt) for _ in range(2)]
         torch.cuda.synchronize()
-        if layers is not None:   # forward passes with and without what the backward needs, then the layers computed again, for each step
-            assert used == ([False] * (3 - layers) + [True] * 3) * 2
+        # forward passes with and without what the backward needs, then the layers computed again, for each step
+        assert used == ([False] * (3 - layers) + [True] * layers + [True] * (3 - layers)) * 2
         got.append((torch.stack(losses), [u.m.clone() for u in eng.units]))
         eng.close()
-    for losses, ms in got[1:]:
+    for losses, ms in got[1:3]:
         # the same operations on the same values; attention alone may pick another kernel where no gradient is wanted, and adds its gradients up
         # in no fixed order: both within bf16's rounding of one of some 30 chained results (2**-9)
         assert torch.allclose(losses, got[0][0], rtol=2 ** -9)
