@@ -36,7 +36,16 @@ IRLIB := $(LIBDIR)/libnccl_device_c.a
 
 PERFLOOP := $(LIBDIR)/libperf_loop.so
 
-all: $(LIB) $(TOOLS) plugins examples ir $(PERFLOOP)
+# native host path of the Python wrappers, where the interpreter's headers are there (the wrappers do without it)
+PYTHON     ?= python3
+PYINCLUDE  := $(shell $(PYTHON) -c "import sysconfig; print(sysconfig.get_paths()['include'])" 2>/dev/null)
+FASTCALL   := $(if $(wildcard $(PYINCLUDE)/Python.h),$(LIBDIR)/_fastcall.so)
+
+all: $(LIB) $(TOOLS) plugins examples ir $(PERFLOOP) $(FASTCALL)
+
+$(LIBDIR)/_fastcall.so: bindings/python/fastcall.c
+	@mkdir -p $(LIBDIR)
+	$(CC) -O2 -Wall -fPIC -shared -fvisibility=hidden -I$(PYINCLUDE) $< -o $@
 
 # the loop of collective calls that the timing harness runs outside the interpreter (knows no library: entry points come in as addresses)
 $(PERFLOOP): tools/perf_loop.c

@@ -4,6 +4,9 @@ The library exports the NCCL host API (reference: src/nccl.h.in); everything in 
 reaches the data plane through these ctypes prototypes.
 """
 import ctypes
+import functools
+import importlib.machinery
+import importlib.util
 import os
 import subprocess
 import threading
@@ -152,6 +155,26 @@ def load(path=None):
                 build()
             _lib = declare(ctypes.CDLL(LIB_PATH, mode=ctypes.RTLD_GLOBAL))
         return _lib
+
+
+@functools.lru_cache(maxsize=None)
+def fastcall():
+    """The module that calls entry points outside ctypes (bindings/python/fastcall.c), or None where it was not built for this interpreter."""
+    path = os.path.join(_HERE, "lib", "_fastcall.so")
+    if not os.path.exists(path):
+        return None
+    loader = importlib.machinery.ExtensionFileLoader("_fastcall", path)
+    try:
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", path, loader=loader))
+        loader.exec_module(module)
+    except ImportError:
+        return None
+    return module
+
+
+def address(lib, name):
+    """Address of an entry point for `fastcall`; None for what is no loaded library."""
+    return ctypes.cast(getattr(lib, name), ctypes.c_void_p).value if isinstance(lib, ctypes.CDLL) else None
 
 
 class NcclError(RuntimeError):

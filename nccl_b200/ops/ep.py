@@ -119,6 +119,10 @@ class ExpertParallel:
         g = ctypes.c_void_p()
         _lib.check(L.ncclEpCreateGroup(ctypes.byref(g), comm.handle, ctypes.byref(cfg)), "ncclEpCreateGroup", L)
         self.group = g
+        self._lead = {"expert_major": (self.El, self.cap), "rank_major": (self.n, max_tokens), "flat": (self.cap,)}[layout]
+        fast = _lib.fastcall()
+        entries = [_lib.address(L, name) for name in ("b200EpDispatch", "b200EpCombine")]
+        self._fast = (fast.invoke, *entries) if fast and all(entries) else None
         self.handle = None
         self._keep = None
         self.recv_total = None
@@ -167,7 +171,7 @@ class ExpertParallel:
             h = ctypes.c_void_p()
             _lib.check(L.ncclEpCreateHandle(ctypes.byref(h), self.group, self.layout_code, ctypes.byref(idx_t), None, None, stream), "ncclEpCreateHandle", L)
             self.handle = h
-        lead = {"expert_major": (self.El, self.cap), "rank_major": (self.n, self.max_tokens), "flat": (self.cap,)}[self.layout]
+        lead = self._lead
         if toks is None:
             toks = torch.empty(*lead, self.H, dtype=torch.uint8 if fp8 else torch.bfloat16, device=x.device)
         if scales is None and fp8:
@@ -182,9 +186,14 @@ class ExpertParallel:
             if self.layout == "flat" or self.recv_total is None:   # nothing writes the rank-major one: it stays zero
                 self.recv_total = torch.zeros(1, dtype=torch.int32, device=x.device)
             recv = (self.recv_topk_idx.data_ptr(), self.recv_topk_weights.data_ptr(), self.recv_total.data_ptr() if self.layout == "flat" else None)
-        _lib.check(L.b200EpDispatch(self.handle, x.data_ptr(), *self._dims(x), topk_idx.data_ptr(), *self._dims(topk_idx), topk_weights.data_ptr(),
-                                    *self._dims(topk_weights), toks.data_ptr(), *self._dims(toks), scales.data_ptr() if fp8 else None, counts.data_ptr(),
-                                    *recv, int(send_only), stream), "ncclEpDispatch", L)
+        sp = scales.data_ptr() if fp8 else None
+        if self._fast:   # a shape stands for the four words of `_dims`
+            rc = self._fast[0](self._fast[1], self.handle, x.data_ptr(), x.shape, topk_idx.data_ptr(), topk_idx.shape, topk_weights.data_ptr(), topk_weights.shape,
+                               toks.data_ptr(), toks.shape, sp, counts.data_ptr(), *recv, int(send_only), stream)
+        else:
+            rc = L.b200EpDispatch(self.handle, x.data_ptr(), *self._dims(x), topk_idx.data_ptr(), *self._dims(topk_idx), topk_weights.data_ptr(),
+                                  *self._dims(topk_weights), toks.data_ptr(), *self._dims(toks), sp, counts.data_ptr(), *recv, int(send_only), stream)
+        _lib.check(rc, "ncclEpDispatch", L)
         self._keep = (x, topk_idx, topk_weights, toks, scales, counts)
         self.T = x.shape[0]
         return toks, scales, counts
@@ -192,6 +201,10 @@ class ExpertParallel:
     def combine(self, y, out=None, send_only=False):
         torch, L = self.torch, self.lib
         out = out if out is not None else torch.empty(self.T, self.H, dtype=torch.bfloat16, device=y.device)
-        _lib.check(L.b200EpCombine(self.handle, y.data_ptr(), *self._dims(y), out.data_ptr(), *self._dims(out), int(send_only), self._stream()), "ncclEpCombine", L)
+        if self._fast:
+            rc = self._fast[0](self._fast[2], self.handle, y.data_ptr(), y.shape, out.data_ptr(), out.shape, int(send_only), self._stream())
+        else:
+            rc = L.b200EpCombine(self.handle, y.data_ptr(), *self._dims(y), out.data_ptr(), *self._dims(out), int(send_only), self._stream())
+        _lib.check(rc, "ncclEpCombine", L)
         self._keep_c = (y, out)
         return out

@@ -7,6 +7,7 @@
     y  = tp.all_gather_gemm(xg, w)          # column-parallel layer: gathers the rows while multiplying
 """
 import ctypes
+import functools
 
 from .. import _lib
 from ..core import current_stream
@@ -33,6 +34,11 @@ class TensorParallel:
         _lib.check(L.ncclTpCreate(comm.handle, max_rows, max_cols, ctypes.byref(h)), "ncclTpCreate", L)
         self.handle = h
         self._gathered = {}
+        self._fp8_protos()
+        fast = _lib.fastcall()
+        for name in ("ncclTpGemm", "ncclTpGemmFp8", "ncclTpQuantizeFp8"):
+            entry = _lib.address(L, name) if fast else None
+            setattr(self, "_" + name, functools.partial(fast.invoke, entry) if entry else getattr(L, name))
 
     def destroy(self):
         if self.handle:
@@ -57,7 +63,7 @@ class TensorParallel:
         M, K = x.shape
         N = w.shape[0]
         out = out if out is not None else torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
-        _lib.check(self.lib.ncclTpGemm(self.handle, x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, self._stream(stream)), "ncclTpGemm", self.lib)
+        _lib.check(self._ncclTpGemm(self.handle, x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, self._stream(stream)), "ncclTpGemm", self.lib)
         return out
 
     def gemm_reduce_scatter(self, x, w, out=None, stream=None):
@@ -113,7 +119,7 @@ class TensorParallel:
             raise ValueError("x must be a contiguous bf16 matrix")
         q = q if q is not None else torch.empty(R, K, dtype=torch.float8_e4m3fn, device=x.device)
         scales = scales if scales is not None else torch.empty(K // 128, R // block_rows, dtype=torch.float32, device=x.device)
-        rc = self.lib.ncclTpQuantizeFp8(self.handle, x.data_ptr(), q.data_ptr(), scales.data_ptr(), R, K, block_rows, self._stream(stream))
+        rc = self._ncclTpQuantizeFp8(self.handle, x.data_ptr(), q.data_ptr(), scales.data_ptr(), R, K, block_rows, self._stream(stream))
         _lib.check(rc, "ncclTpQuantizeFp8", self.lib)
         return q, scales
 
@@ -123,7 +129,7 @@ class TensorParallel:
         M, K = xq.shape
         N = wq.shape[0]
         out = out if out is not None else torch.empty(M, N, dtype=torch.bfloat16, device=xq.device)
-        rc = self.lib.ncclTpGemmFp8(self.handle, xq.data_ptr(), xs.data_ptr(), wq.data_ptr(), ws.data_ptr(), out.data_ptr(), M, N, K, self._stream(stream))
+        rc = self._ncclTpGemmFp8(self.handle, xq.data_ptr(), xs.data_ptr(), wq.data_ptr(), ws.data_ptr(), out.data_ptr(), M, N, K, self._stream(stream))
         _lib.check(rc, "ncclTpGemmFp8", self.lib)
         return out
 

@@ -1,0 +1,103 @@
+"""The native host path of the wrappers (bindings/python/fastcall.c): what reaches an entry point is what ctypes hands over, and what the wrappers
+refuse stays refused."""
+import ctypes
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from mp_util import run_ranks  # noqa: E402
+from nccl_b200 import _lib, core  # noqa: E402
+
+P, I, Z = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
+needs_module = pytest.mark.skipif(_lib.fastcall() is None, reason="built without the interpreter's headers")
+
+
+def _recorder(types):
+    calls = []
+
+    def fn(*a):
+        calls.append(a)
+        return 7 if len(calls) > 1 else 0
+    cb = ctypes.CFUNCTYPE(I, *types)(fn)
+    return calls, cb, ctypes.cast(cb, P).value
+
+
+@needs_module
+def test_collectives():
+    fast = _lib.fastcall()
+    a, b = torch.zeros(3, 4, dtype=torch.bfloat16), torch.zeros(6)
+    types, handle = core._torch_types(), ctypes.c_void_p(0x1234)
+    for lead, n, t in ((0, 12, core.BF16), (1, 6, core.FP32), (2, 12, core.BF16), (3, 6, core.FP32)):
+        calls, keep, at = _recorder([P, P, Z, I, I, P, P])
+        assert fast.collective(at, types, None, a, b, lead, 1, -2, handle, None) == 0
+        assert fast.collective(at, types, None, a, b, lead, 3, 4, handle, 77) == 7
+        assert calls == [(a.data_ptr(), b.data_ptr(), n, t, -2, 0x1234, None), (a.data_ptr(), b.data_ptr(), n // 3, t, 4, 0x1234, 77)]
+    calls, keep, at = _recorder([P, P, Z, I, P, P])
+
+    class Stream:
+        cuda_stream = 1 << 40
+    assert fast.collective(at, types, None, None, b, 3, 1, None, None, Stream()) == 0
+    assert calls == [(None, b.data_ptr(), 6, core.FP32, None, 1 << 40)]
+
+
+@needs_module
+def test_refused():
+    fast, types = _lib.fastcall(), core._torch_types()
+    calls, keep, at = _recorder([P, P, Z, I, P, P])
+    ok = torch.zeros(4)
+    for bad, error in ((torch.zeros(4, 4).t(), ValueError), (torch.zeros(4, dtype=torch.complex64), KeyError)):
+        for pair in ((ok, bad), (bad, ok)):
+            with pytest.raises(error):
+                fast.collective(at, types, None, *pair, 0, 1, None, 0, None)
+    for other in (np.zeros(4, np.float32), [1, 2], object()):
+        assert fast.collective(at, types, None, ok, other, 0, 1, None, 0, None) is NotImplemented
+    for args in ((at, 1.5), (at, "x"), (at, *range(33)), (0, 1), ()):
+        with pytest.raises((TypeError, AttributeError)):
+            fast.invoke(*args)
+    with pytest.raises(TypeError):
+        fast.collective(at, types, None, None, ok, 0, 1, None, 0, None)   # nothing to count
+    assert not calls
+
+
+@needs_module
+@pytest.mark.parametrize("n", [1, 8, 9, 16, 17, 32])
+def test_words(n):
+    """Words on both sides of the forms that a call takes; shapes are four of them."""
+    calls, keep, at = _recorder([ctypes.c_uint64] * n)
+    args = [(1 << 64) - 1 - k if k % 3 else k - 5 for k in range(n)]
+    assert _lib.fastcall().invoke(at, *args) == 0
+    assert calls == [tuple(v % (1 << 64) for v in args)]
+    if n == 16:   # words behind the last are whatever the registers and the stack hold
+        calls, keep, at = _recorder([ctypes.c_uint64] * n)
+        _lib.fastcall().invoke(at, torch.Size((2, 3)), (4, 5, 6), (9,), torch.Size((1, 2, 3, 4)))
+        assert calls == [(2, 2, 3, 0, 3, 4, 5, 6, 1, 0, 0, 0, 4, 0, 0, 0)]
+
+
+def _rank(rank, nranks, uid):
+    import torch
+    from nccl_b200 import Communicator
+    comm = Communicator(nranks, rank, uid)
+    got = []
+    for native in (True, False):
+        if not native:
+            comm._entries = dict.fromkeys(("ncclAllReduce", "ncclBroadcast", "ncclReduceScatter", "ncclAllGather", "ncclAlltoAll"))
+        x = torch.arange(8, dtype=torch.float32) * (rank + 1)
+        out = [comm.all_reduce(x, torch.zeros(8)), comm.all_reduce(x.clone(), op="max"), comm.broadcast(x if rank == 1 else None, torch.zeros(8), 1),
+               comm.reduce_scatter(x, torch.zeros(4), op="avg"), comm.all_gather(x, torch.zeros(16)), comm.all_to_all(x, torch.zeros(8))]
+        got.append([t.tolist() for t in out])
+        with pytest.raises(ValueError):
+            comm.all_reduce(torch.zeros(4, 4).t())
+        with pytest.raises(TypeError):
+            comm.all_reduce([1, 2])
+        assert comm.all_reduce(np.ones(3, np.float32), np.zeros(3, np.float32)).tolist() == [nranks] * 3
+    comm.destroy()
+    return got
+
+
+def test_communicator_either_way():
+    got = run_ranks(_rank, 2, env={"NCCL_B200_HOST_ONLY": "1", "NCCL_SOCKET_IFNAME": "lo"}, timeout=300)
+    for rank in range(2):
+        native, through_ctypes = got[rank]
+        assert native == through_ctypes and native[0] == [3.0 * i for i in range(8)]
