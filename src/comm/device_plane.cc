@@ -141,7 +141,7 @@ static void preloadKernels(int dev) {
                          signalKernelFn(), waitSignalKernelFn()})
     touch(fn);
   for (int t = 0; t < ncclNumTypes; ++t) {
-    touch(scaleKernelFn((ncclDataType_t)t));
+    for (const void* src : {(const void*)nullptr, (const void*)1}) touch(scaleKernelFn((ncclDataType_t)t, src, nullptr));
     for (int op = RED_SUM; op <= RED_MIN; ++op) {
       touch(reduceKernelFn(KERNEL_REDUCE_P2P, (ncclDataType_t)t, op));
       touch(reduceKernelFn(KERNEL_REDUCE_NVLS, (ncclDataType_t)t, op));
@@ -415,7 +415,7 @@ static ncclResult_t scaleCopy(ncclComm* comm, ncclDataType_t type, const void* s
   const size_t perCta = 512 * 4 * 16;   // bytes that a CTA of the kernel moves in one tile
   int ctas = (int)std::min<size_t>((count * typeSize(type) + perCta - 1) / perCta, (size_t)comm->devPlane->smCount * 16);
   comm->devPlane->launches++;
-  return launchKernel(scaleKernelFn(type), dim3(std::max(ctas, 1)), dim3(512), 0, &sa, stream, false, devPlanePdl());
+  return launchKernel(scaleKernelFn(type, src, dst), dim3(std::max(ctas, 1)), dim3(512), 0, &sa, stream, false, devPlanePdl());
 }
 
 void sliceEven(size_t count, size_t es, int n, size_t* begin, size_t* cnt) {

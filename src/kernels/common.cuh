@@ -76,6 +76,12 @@ __device__ __forceinline__ Pack32 ldStream32(const void* p) {
                : "=r"(v.lo.x), "=r"(v.lo.y), "=r"(v.lo.z), "=r"(v.lo.w), "=r"(v.hi.x), "=r"(v.hi.y), "=r"(v.hi.z), "=r"(v.hi.w) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ Pack32 ldLocal32(const void* p) {
+  Pack32 v;
+  asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v.lo.x), "=r"(v.lo.y), "=r"(v.lo.z), "=r"(v.lo.w), "=r"(v.hi.x), "=r"(v.hi.y), "=r"(v.hi.z), "=r"(v.hi.w) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ void st32(void* p, Pack32 v) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v.lo.x), "r"(v.lo.y), "r"(v.lo.z), "r"(v.lo.w), "r"(v.hi.x), "r"(v.hi.y),
                "r"(v.hi.z), "r"(v.hi.w) : "memory");

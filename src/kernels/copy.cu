@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) reshardKernel(const __grid_con
 const void* reshardKernelFn() { return (const void*)reshardKernel; }
 
 // ------------------------------------------------------------------------- local copy and scale
-// How a byte range splits when dst is written in 16-byte packs and src may lie at any other alignment: `head` bytes before
+// How a byte range splits when dst is written in packs of 16 or 32 bytes and src may lie at any other alignment: `head` bytes before
 // the first pack, `packs` packs, the rest behind them. With shift != 0 a pack of dst straddles two aligned words of src and
 // is put together from both; head and packs are chosen so that neither word reaches outside the source range.
 //
@@ -544,51 +544,79 @@ struct PackSpan {
   size_t head, packs;
   int shift;
 };
+// B: bytes of a pack, 16 or 32
+template <int B>
 __device__ __forceinline__ PackSpan packSpan(const char* src, const char* dst, size_t bytes) {
   PackSpan s;
-  s.head = (16 - ((uintptr_t)dst & 15)) & 15;
-  s.shift = (int)(((uintptr_t)src + s.head) & 15);
-  if (s.shift > (int)s.head) s.head += 16;
-  const size_t last = s.shift ? 32 - s.shift : 16;   // bytes of src from a pack's first byte to the end of the last word read for it
-  s.packs = bytes >= s.head + last ? (bytes - s.head - last) / 16 + 1 : 0;
+  s.head = (B - ((uintptr_t)dst & (B - 1))) & (B - 1);
+  s.shift = (int)(((uintptr_t)src + s.head) & (B - 1));
+  if (s.shift > (int)s.head) s.head += B;
+  const size_t last = s.shift ? 2 * B - s.shift : B;   // bytes of src from a pack's first byte to the end of the last word read for it
+  s.packs = bytes >= s.head + last ? (bytes - s.head - last) / B + 1 : 0;
   if (s.packs == 0) s.head = 0;
   return s;
 }
-template <bool SHIFTED>
-__device__ __forceinline__ uint4 ldPack(const char* p, int shift) {
-  if (!SHIFTED) return ldStream16(p);
-  // neighbouring lanes share a word: the second load of a word finds it in L1
-  const uint4 a = ldLocal16(p - shift), b = ldLocal16(p - shift + 16);
-  uint32_t w0 = a.x, w1 = a.y, w2 = a.z, w3 = a.w, w4 = b.x, w5 = b.y, w6 = b.z, w7 = b.w;
-  if (shift & 8) { w0 = w2; w1 = w3; w2 = w4; w3 = w5; w4 = w6; w5 = w7; }
-  if (shift & 4) { w0 = w1; w1 = w2; w2 = w3; w3 = w4; w4 = w5; }
+// The 32 bytes at p, put together from the aligned words that hold them. Neighbouring lanes share a word: the second load of a word finds it
+// in L1.
+__device__ __forceinline__ Pack32 ldShifted32(const char* p, int shift) {
+  uint32_t w[16];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const Pack32 q = ldLocal32(p - shift + k * 32);
+    const uint32_t part[8] = {q.lo.x, q.lo.y, q.lo.z, q.lo.w, q.hi.x, q.hi.y, q.hi.z, q.hi.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[k * 8 + i] = part[i];
+  }
+#pragma unroll
+  for (int by = 4; by > 0; by /= 2)
+    if (shift & (by * 4)) {
+#pragma unroll
+      for (int i = 0; i + by < 16; ++i) w[i] = w[i + by];
+    }
   const int bits = (shift & 3) * 8;
-  return make_uint4(__funnelshift_r(w0, w1, bits), __funnelshift_r(w1, w2, bits), __funnelshift_r(w2, w3, bits), __funnelshift_r(w3, w4, bits));
+  uint32_t r[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) r[i] = __funnelshift_r(w[i], w[i + 1], bits);
+  return {make_uint4(r[0], r[1], r[2], r[3]), make_uint4(r[4], r[5], r[6], r[7])};
 }
 
-// dst[i] = f(src[i]) over `packs` 16-byte packs. A CTA moves contiguous tiles of U x blockDim packs (all loads of a tile
-// issued before its stores), and CTAs stride over tiles, so that each DRAM page is opened once and enough bytes are in
-// flight for HBM speed.
-template <int U, bool SHIFTED, typename F>
+// dst[i] = f(src[i]) over `packs` packs of 16 bytes, shifted ones of 32. A CTA moves contiguous tiles of 64 bytes per thread (all
+// loads of a tile issued before its stores), and CTAs stride over tiles, so that each DRAM page is opened once and enough bytes are
+// in flight for HBM speed.
+template <bool SHIFTED, typename F>
 __device__ __forceinline__ void streamPacks(const char* src, char* dst, size_t packs, int shift, F f) {
+  constexpr int B = SHIFTED ? 32 : 16, U = 64 / B;
   const size_t tilePacks = (size_t)U * blockDim.x;
-  const size_t fullTiles = packs / tilePacks;
-  for (size_t t = blockIdx.x; t < fullTiles; t += gridDim.x) {
-    const size_t base = t * tilePacks + threadIdx.x;
-    uint4 v[U];
+  const size_t fullTiles = packs / tilePacks, stride = (size_t)gridDim.x * blockDim.x;
+  const size_t rest = fullTiles * tilePacks + (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if constexpr (SHIFTED) {
+    auto store = [&](size_t i, const Pack32& v) { st32(dst + i * B, {f(v.lo), f(v.hi)}); };
+    for (size_t t = blockIdx.x; t < fullTiles; t += gridDim.x) {
+      const size_t base = t * tilePacks + threadIdx.x;
+      Pack32 v[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) v[u] = ldPack<SHIFTED>(src + (base + (size_t)u * blockDim.x) * 16, shift);
+      for (int u = 0; u < U; ++u) v[u] = ldShifted32(src + (base + (size_t)u * blockDim.x) * B, shift);
 #pragma unroll
-    for (int u = 0; u < U; ++u) st16(dst + (base + (size_t)u * blockDim.x) * 16, f(v[u]));
+      for (int u = 0; u < U; ++u) store(base + (size_t)u * blockDim.x, v[u]);
+    }
+    for (size_t i = rest; i < packs; i += stride) store(i, ldShifted32(src + i * B, shift));
+  } else {
+    for (size_t t = blockIdx.x; t < fullTiles; t += gridDim.x) {
+      const size_t base = t * tilePacks + threadIdx.x;
+      uint4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = ldStream16(src + (base + (size_t)u * blockDim.x) * B);
+#pragma unroll
+      for (int u = 0; u < U; ++u) st16(dst + (base + (size_t)u * blockDim.x) * B, f(v[u]));
+    }
+    for (size_t i = rest; i < packs; i += stride) st16(dst + i * B, f(ldStream16(src + i * B)));
   }
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = fullTiles * tilePacks + (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < packs; i += stride)
-    st16(dst + i * 16, f(ldPack<SHIFTED>(src + i * 16, shift)));
 }
 
 // dst = src * scalar, one 16-byte pack per access like the copy below. Bound by memory: 24 MiB of bf16 take 9 us, element by
 // element they took 25.
-template <typename T>
+// SHIFTED: src and dst lie differently to 16 bytes
+template <typename T, bool SHIFTED>
 __global__ void __launch_bounds__(512, 2) scaleKernel(ScaleArgs a) {
   pdlEnter();
   using A = typename Elem<T>::Acc;
@@ -603,7 +631,8 @@ __global__ void __launch_bounds__(512, 2) scaleKernel(ScaleArgs a) {
   }
   const char* src = (const char*)a.src;
   char* dst = (char*)a.dst;
-  const PackSpan sp = packSpan(src, dst, a.count * sizeof(T));
+  constexpr int B = SHIFTED ? 32 : 16;
+  const PackSpan sp = packSpan<B>(src, dst, a.count * sizeof(T));
   auto scalePack = [sa](uint4 v) {
     Pack16<T> p;
     p.v = v;
@@ -611,10 +640,9 @@ __global__ void __launch_bounds__(512, 2) scaleKernel(ScaleArgs a) {
     for (int i = 0; i < Pack16<T>::N; ++i) p.e[i] = Elem<T>::st(Elem<T>::ld(p.e[i]) * sa);
     return p.v;
   };
-  if (sp.shift) streamPacks<4, true>(src + sp.head, dst + sp.head, sp.packs, sp.shift, scalePack);
-  else streamPacks<4, false>(src + sp.head, dst + sp.head, sp.packs, 0, scalePack);
+  streamPacks<SHIFTED>(src + sp.head, dst + sp.head, sp.packs, sp.shift, scalePack);
   // elements before the first and behind the last pack
-  const size_t before = sp.head / sizeof(T), behind = before + sp.packs * Pack16<T>::N;
+  const size_t before = sp.head / sizeof(T), behind = before + sp.packs * (B / sizeof(T));
   const size_t loose = before + (a.count - behind);
   for (size_t i = tid; i < loose; i += stride) {
     const size_t e = i < before ? i : behind + (i - before);
@@ -622,22 +650,26 @@ __global__ void __launch_bounds__(512, 2) scaleKernel(ScaleArgs a) {
   }
 }
 
-const void* scaleKernelFn(ncclDataType_t type) {
+template <bool SHIFTED>
+static const void* scaleKernelOf(ncclDataType_t type) {
   switch (type) {
-    case ncclInt8: return (const void*)scaleKernel<int8_t>;
-    case ncclUint8: return (const void*)scaleKernel<uint8_t>;
-    case ncclInt32: return (const void*)scaleKernel<int32_t>;
-    case ncclUint32: return (const void*)scaleKernel<uint32_t>;
-    case ncclInt64: return (const void*)scaleKernel<int64_t>;
-    case ncclUint64: return (const void*)scaleKernel<uint64_t>;
-    case ncclFloat16: return (const void*)scaleKernel<__half>;
-    case ncclFloat32: return (const void*)scaleKernel<float>;
-    case ncclFloat64: return (const void*)scaleKernel<double>;
-    case ncclBfloat16: return (const void*)scaleKernel<__nv_bfloat16>;
-    case ncclFloat8e4m3: return (const void*)scaleKernel<F8E4>;
-    case ncclFloat8e5m2: return (const void*)scaleKernel<F8E5>;
+    case ncclInt8: return (const void*)scaleKernel<int8_t, SHIFTED>;
+    case ncclUint8: return (const void*)scaleKernel<uint8_t, SHIFTED>;
+    case ncclInt32: return (const void*)scaleKernel<int32_t, SHIFTED>;
+    case ncclUint32: return (const void*)scaleKernel<uint32_t, SHIFTED>;
+    case ncclInt64: return (const void*)scaleKernel<int64_t, SHIFTED>;
+    case ncclUint64: return (const void*)scaleKernel<uint64_t, SHIFTED>;
+    case ncclFloat16: return (const void*)scaleKernel<__half, SHIFTED>;
+    case ncclFloat32: return (const void*)scaleKernel<float, SHIFTED>;
+    case ncclFloat64: return (const void*)scaleKernel<double, SHIFTED>;
+    case ncclBfloat16: return (const void*)scaleKernel<__nv_bfloat16, SHIFTED>;
+    case ncclFloat8e4m3: return (const void*)scaleKernel<F8E4, SHIFTED>;
+    case ncclFloat8e5m2: return (const void*)scaleKernel<F8E5, SHIFTED>;
     default: return nullptr;
   }
+}
+const void* scaleKernelFn(ncclDataType_t type, const void* src, const void* dst) {
+  return ((uintptr_t)src ^ (uintptr_t)dst) & 15 ? scaleKernelOf<true>(type) : scaleKernelOf<false>(type);
 }
 
 // Local copy of `count` bytes between 16-byte aligned buffers: the data movement of a single-rank communicator
@@ -668,10 +700,12 @@ __global__ void __launch_bounds__(512) localCopyKernel(ScaleArgs a) {
   for (size_t j = packs * 16 + tid; j < bytes; j += stride) dst[j] = src[j];
 }
 // The same at any alignment. A kernel of its own: putting packs together takes registers that the aligned form needs for its second
-// CTA per SM (178 instead of 166 us for 512 MiB when both shared a kernel). 32 MiB at odd offsets take 13 us; byte by byte they
-// took 120. The shifted form spills 12 bytes at the 64 registers that two CTAs per SM leave it.
+// CTA per SM (178 instead of 166 us for 512 MiB when both shared a kernel). 32 MiB at odd offsets take 12.0 us like aligned ones; byte by byte they
+// took 120, in packs of 16 bytes 14.1: a word that two packs share is fetched twice, and with 32 bytes there are half as many accesses. Copies
+// (and the products above) between buffers of the same alignment gain nothing from 32 bytes: 64 MiB 18.4 us with 16, 21.3 with 32.
 template <bool SHIFTED>
 __global__ void __launch_bounds__(512, 2) localCopyUnalignedKernel(ScaleArgs a) {
+  constexpr int B = SHIFTED ? 32 : 16;
   pdlEnter();
   const char* src = (const char*)a.src;
   char* dst = (char*)a.dst;
@@ -680,10 +714,10 @@ __global__ void __launch_bounds__(512, 2) localCopyUnalignedKernel(ScaleArgs a) 
     for (size_t i = tid; i < a.count; i += stride) dst[i] = src[i];
     return;
   }
-  const PackSpan sp = packSpan(src, dst, a.count);
+  const PackSpan sp = packSpan<B>(src, dst, a.count);
   auto same = [](uint4 v) { return v; };
-  streamPacks<4, SHIFTED>(src + sp.head, dst + sp.head, sp.packs, sp.shift, same);
-  const size_t behind = sp.head + sp.packs * 16, loose = sp.head + (a.count - behind);
+  streamPacks<SHIFTED>(src + sp.head, dst + sp.head, sp.packs, sp.shift, same);
+  const size_t behind = sp.head + sp.packs * B, loose = sp.head + (a.count - behind);
   for (size_t i = tid; i < loose; i += stride) {
     const size_t j = i < sp.head ? i : behind + (i - sp.head);
     dst[j] = src[j];

@@ -38,6 +38,14 @@ def test_copy_at_any_alignment(comm, nbytes, soff, doff):
     assert (draw[:doff] == 77).all() and (draw[doff + nbytes:] == 77).all()
 
 
+@pytest.mark.parametrize("nbytes", [2049, 2111, 2112, 2113, 65536 + 31, 3 * 32768 + 77])
+def test_copy_at_every_shift(comm, nbytes):
+    """Packs of 32 bytes from two words each: every distance of source and destination, from both ends of a word."""
+    for shift in range(32):
+        for doff in (0, 1, 31):
+            test_copy_at_any_alignment(comm, nbytes, doff + shift, doff)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16", "float16", "float64", "int32", "int64"])
 @pytest.mark.parametrize("count,soff,doff", [(1, 0, 0), (7, 0, 0), (9, 1, 0), (40, 1, 1), (256, 1, 0), (257, 0, 1), (513, 1, 2), (1025, 3, 1), (2047, 0, 3), (16384, 0, 0), (16391, 3, 2), (100003, 1, 0)])
 def test_scale_at_any_element_offset(comm, dtype, count, soff, doff):
