@@ -662,8 +662,8 @@ __global__ void __launch_bounds__(kEpThreads, 1) epCombineKernel(const __grid_co
 // With one rank every row stays on this GPU and nobody has to be waited for. The local forms move each row once: dispatch
 // claims the rows of the output tensors and writes them straight from the input (the general kernel stores into a landing
 // zone and packs from there: written twice, read once more), combine reads the experts' rows where they lie. Both are bound
-// by memory: for 4096 tokens of 7168 bf16 channels and 8 of 32 experts dispatch went from 313 to 103 us and combine from 434 to
-// 81 us (5.1 and 6.5 TB/s). Dispatch reads and writes 32 bytes at a time where tokens in and out are aligned to them, which the
+// by memory: for 4096 tokens of 7168 bf16 channels and 8 of 32 experts dispatch went from 313 to 104 us and combine from 434 to
+// 87 us (5.1 and 6.1 TB/s; a fill of the bytes that dispatch writes runs at 3.8). Dispatch reads and writes 32 bytes at a time where tokens in and out are aligned to them, which the
 // queue of memory instructions held up (us with 16 / 32 bytes, launches of one after the other): 2000 tokens of 4096 to one row each
 // in fp8 8.9 / 7.0, 1000 of 7168 in bf16 to four experts 16.1 / 14.2, 8 of 7168 in fp8 to eight 5.4 / 5.0, one of 1024 3.7 / 3.6.
 constexpr int kLocTokens = 64;    // tokens of a CTA whose rows are claimed (or looked up) together
@@ -868,18 +868,21 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epDispatchLocalKernel(cons
 }
 
 // Items first, first + kEpLocalThreads, ... of a batch of tokens: KR rows of U items are fetched together, so that several loads
-// are in flight whatever the number of experts (one row per item ran at 1.8 TB/s). `store` takes token, channels and sums.
-template <int KR, typename Store>
+// are in flight whatever the number of experts (one row per item ran at 1.8 TB/s). An item is 8 channels (WIDE: 16). `store` takes token,
+// item and sums.
+template <int KR, bool WIDE, typename Store>
 __device__ __forceinline__ void localSums(const __nv_bfloat16* y, int H, int C, int nItems, int shift, int R, const int* sRow, const float* sW, Store store) {
-  constexpr int U = KR == 1 ? 4 : 8 / KR;
+  constexpr int W = WIDE ? 2 : 1, N = 8 * W;
+  constexpr int U = KR == 1 ? 4 / W : 8 / KR / W;
+  static_assert(U >= 1, "at least one item");
   for (int first = threadIdx.x; first < nItems; first += U * kEpLocalThreads) {
-    float acc[U][8];
+    float acc[U][N];
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int q = 0; q < 8; ++q) acc[u][q] = 0.0f;
+      for (int q = 0; q < N; ++q) acc[u][q] = 0.0f;
     for (int r0 = 0; r0 < R; r0 += KR) {
-      uint4 v[U][KR];
+      uint4 v[U][KR][W];
       float wk[U][KR];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -888,25 +891,35 @@ __device__ __forceinline__ void localSums(const __nv_bfloat16* y, int H, int C, 
 #pragma unroll
         for (int r = 0; r < KR; ++r) {
           const int row = i - shift < nItems && r0 + r < R ? sRow[j * R + r0 + r] : -1;
-          v[u][r] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+          for (int w = 0; w < W; ++w) v[u][r][w] = make_uint4(0, 0, 0, 0);
           wk[u][r] = 0.0f;
           if (row >= 0) {
             wk[u][r] = sW[j * R + r0 + r];
-            v[u][r] = ldStream16(y + (size_t)row * H + (size_t)c * 8);
+            const __nv_bfloat16* from = y + (size_t)row * H + (size_t)c * N;
+            if (WIDE) {
+              const Pack32 p = ldStream32(from);
+              v[u][r][0] = p.lo;
+              v[u][r][W - 1] = p.hi;
+            } else {
+              v[u][r][0] = ldStream16(from);
+            }
           }
         }
       }
 #pragma unroll
       for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int r = 0; r < KR; ++r) {
-          const __nv_bfloat162* p = (const __nv_bfloat162*)&v[u][r];
+        for (int r = 0; r < KR; ++r)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            acc[u][2 * q] += wk[u][r] * __bfloat162float(p[q].x);
-            acc[u][2 * q + 1] += wk[u][r] * __bfloat162float(p[q].y);
+          for (int w = 0; w < W; ++w) {
+            const __nv_bfloat162* p = (const __nv_bfloat162*)&v[u][r][w];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              acc[u][8 * w + 2 * q] += wk[u][r] * __bfloat162float(p[q].x);
+              acc[u][8 * w + 2 * q + 1] += wk[u][r] * __bfloat162float(p[q].y);
+            }
           }
-        }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -918,16 +931,22 @@ __device__ __forceinline__ void localSums(const __nv_bfloat16* y, int H, int C, 
 }
 
 // The same where row t of y is all that goes into token t, if it has an expert at all: the first rows travel while `lookup` fills sRow.
-template <typename Lookup, typename Store>
+template <bool WIDE, typename Lookup, typename Store>
 __device__ __forceinline__ void localRows(const __nv_bfloat16* y, int H, int C, int tb, int nItems, int shift, const int* sRow, Lookup lookup, Store store) {
-  constexpr int U = 4;
-  uint4 v[U];
+  constexpr int W = WIDE ? 2 : 1, U = 4 / W, N = 8 * W;
+  uint4 v[U][W];
   auto load = [&](int first) {
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = first + u * kEpLocalThreads;
-      v[u] = make_uint4(0, 0, 0, 0);
-      if (i < nItems) v[u] = ldStream16(y + (size_t)tb * H + (size_t)(i + shift) * 8);
+      const __nv_bfloat16* from = y + (size_t)tb * H + (size_t)(i + shift) * N;
+      if (WIDE) {
+        const Pack32 p = i < nItems ? ldStream32(from) : Pack32{};
+        v[u][0] = p.lo;
+        v[u][W - 1] = p.hi;
+      } else {
+        v[u][0] = i < nItems ? ldStream16(from) : make_uint4(0, 0, 0, 0);
+      }
     }
   };
   load(threadIdx.x);
@@ -938,13 +957,18 @@ __device__ __forceinline__ void localRows(const __nv_bfloat16* y, int H, int C, 
       const int i = first + u * kEpLocalThreads + shift;
       if (i - shift >= nItems) continue;
       const int j = i / C;
-      float acc[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-      if (sRow[j] >= 0) {
-        const __nv_bfloat162* p = (const __nv_bfloat162*)&v[u];
+      float acc[N];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          acc[2 * q] += __bfloat162float(p[q].x);
-          acc[2 * q + 1] += __bfloat162float(p[q].y);
+      for (int q = 0; q < N; ++q) acc[q] = 0.0f;
+      if (sRow[j] >= 0) {
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const __nv_bfloat162* p = (const __nv_bfloat162*)&v[u][w];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            acc[8 * w + 2 * q] += __bfloat162float(p[q].x);
+            acc[8 * w + 2 * q + 1] += __bfloat162float(p[q].y);
+          }
         }
       }
       store(j, i - j * C, acc);
@@ -953,8 +977,9 @@ __device__ __forceinline__ void localRows(const __nv_bfloat16* y, int H, int C, 
   }
 }
 
-// out[t] = sum over the token's selected experts of w * row, in fp32, in slot order. The (token, 8 channels) items are dealt to
+// out[t] = sum over the token's selected experts of w * row, in fp32, in slot order. The (token, 8 channels) items (WIDE: 16) are dealt to
 // the CTAs as contiguous ranges; where the rows lie and their weights is looked up once per token and CTA.
+template <bool WIDE>
 __global__ void __launch_bounds__(kEpLocalThreads, 2) epCombineLocalKernel(const __grid_constant__ EpArgs a) {
   pdlEnter();
   __shared__ int sRow[kLocTokens * kLocMaxK];
@@ -965,7 +990,8 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epCombineLocalKernel(const
   const int64_t* idx = a.topkIdx[me];
   const __nv_bfloat16* y = a.x[me];
   __nv_bfloat16* out = (__nv_bfloat16*)a.outTokens[me];
-  const int C = H / 8;
+  constexpr int W = WIDE ? 2 : 1;
+  const int C = H / (8 * W);
   const size_t items = (size_t)T * C;
   const size_t lo = items * blockIdx.x / gridDim.x, hi = items * (blockIdx.x + 1) / gridDim.x;
   if (lo >= hi) return;
@@ -999,22 +1025,27 @@ __global__ void __launch_bounds__(kEpLocalThreads, 2) epCombineLocalKernel(const
     const size_t first = (size_t)tb * C > lo ? (size_t)tb * C : lo;
     const size_t end = (size_t)(tb + batch) * C < hi ? (size_t)(tb + batch) * C : hi;
     const int nItems = (int)(end - first), shift = (int)(first - (size_t)tb * C);
-    auto store = [&](int j, int c, const float (&acc)[8]) {
-      uint4 o;
-      __nv_bfloat162* q = (__nv_bfloat162*)&o;
+    auto store = [&](int j, int c, const float (&acc)[8 * W]) {
+      uint4 o[W];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) q[k] = __floats2bfloat162_rn(acc[2 * k], acc[2 * k + 1]);
-      st16(out + (size_t)(tb + j) * H + (size_t)c * 8, o);
+      for (int w = 0; w < W; ++w) {
+        __nv_bfloat162* q = (__nv_bfloat162*)&o[w];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) q[k] = __floats2bfloat162_rn(acc[8 * w + 2 * k], acc[8 * w + 2 * k + 1]);
+      }
+      __nv_bfloat16* to = out + (size_t)(tb + j) * H + (size_t)c * 8 * W;
+      if (WIDE) st32(to, {o[0], o[W - 1]});
+      else st16(to, o[0]);
     };
     if (rankMajor) {   // the caller has weighted the rows
-      localRows(y, H, C, tb, nItems, shift, sRow, lookup, store);
+      localRows<WIDE>(y, H, C, tb, nItems, shift, sRow, lookup, store);
       continue;
     }
     lookup();
-    if (R == 1) localSums<1>(y, H, C, nItems, shift, R, sRow, sW, store);
-    else if (R == 2) localSums<2>(y, H, C, nItems, shift, R, sRow, sW, store);
-    else if (R <= 4) localSums<4>(y, H, C, nItems, shift, R, sRow, sW, store);
-    else localSums<8>(y, H, C, nItems, shift, R, sRow, sW, store);
+    if (R == 1) localSums<1, WIDE>(y, H, C, nItems, shift, R, sRow, sW, store);
+    else if (R == 2) localSums<2, WIDE>(y, H, C, nItems, shift, R, sRow, sW, store);
+    else if (WIDE || R <= 4) localSums<4, WIDE>(y, H, C, nItems, shift, R, sRow, sW, store);
+    else localSums<WIDE ? 4 : 8, WIDE>(y, H, C, nItems, shift, R, sRow, sW, store);
   }
 }
 
@@ -1024,6 +1055,6 @@ const void* epDispatchLocalKernelFn(int fp8, bool wide) {
   if (wide) return fp8 ? (const void*)epDispatchLocalKernel<true, true> : (const void*)epDispatchLocalKernel<false, true>;
   return fp8 ? (const void*)epDispatchLocalKernel<true, false> : (const void*)epDispatchLocalKernel<false, false>;
 }
-const void* epCombineLocalKernelFn() { return (const void*)epCombineLocalKernel; }
+const void* epCombineLocalKernelFn(bool wide) { return wide ? (const void*)epCombineLocalKernel<true> : (const void*)epCombineLocalKernel<false>; }
 
 }  // namespace b200

@@ -77,6 +77,6 @@ const void* epCombineKernelFn();
 // A group of one rank, both halves in one call, expert-major or rank-major: no landing zones, no flags. kEpLocalThreads threads.
 constexpr int kEpLocalThreads = 512;
 const void* epDispatchLocalKernelFn(int fp8, bool wide);   // wide: tokens in and out are 32-byte aligned
-const void* epCombineLocalKernelFn();
+const void* epCombineLocalKernelFn(bool wide);
 
 }  // namespace b200

@@ -134,6 +134,16 @@ static ncclResult_t launchEpLocal(ncclEpGroup* g, const void* fn, EpArgs* a, siz
   return launchKernel(fn, dim3((unsigned)std::max<size_t>(std::min(want, most), 1)), dim3(kEpLocalThreads), 0, a, stream, false, devPlanePdl());
 }
 
+// Whether combine's accesses are 32 bytes wide. A thread has 128 bytes under way either way: 8 rows of 16 or 4 of 32, so that more than four
+// rows take a second trip, which pays when they come from memory anyway. us with 16 / 32 bytes, 32 experts: rank-major 1000 x 7168 6.7 / 5.7, 64 x 2048
+// 2.35 / 2.22; one row 1000 x 4096 4.8 / 4.2; three 500 x 7168 8.6 / 6.6; four 16 x 7168 3.4 / 3.0, 500 x 7168 (28 MB) 9.2 / 9.2, 1000 x 7168 (57 MB) 13.6 / 15.0,
+// 4096 x 7168 (235 MB) 55 / 50; eight 64 x 7168 3.5 / 3.7, 1000 x 7168 (115 MB) 22.0 / 24.0, 2000 x 7168 (229 MB) 48.3 / 43.9, 4096 x 7168 101 / 87; six 4096 x 4096
+// (201 MB) 44.4 / 41.0.
+static bool combineWide(bool rankMajor, size_t T, int K, int H) {
+  const size_t rows = T * K * H * 2;
+  return rankMajor || K <= 3 || rows > (size_t)160 << 20 || (K == 4 && rows < (size_t)28 << 20);
+}
+
 B200_PARAM(EpBulk, "B200_EP_BULK", 1, "Expert-parallel dispatch hands the packed tokens to the bulk-copy engines (a ring of shared-memory stages per CTA) instead of storing them with the warps: 0 never, 1 for the expert-major layout, 2 for every layout")
 
 // Dynamic shared memory of the dispatch kernel: one packed token, or the ring of stages of the bulk form.
@@ -489,7 +499,8 @@ ncclResult_t ncclEpCombine(ncclEpHandle_t h, const ncclEpCombineInputs_t* in, co
                                                    {{inPlace ? nullptr : a.x[me], (a.layout == EP_EXPERT_MAJOR ? g->El * cap : cap) * rowBytes},
                                                     {a.topkIdx[me], T * h->K * sizeof(int64_t)}, {weights, T * h->K * sizeof(float)}})) {
     a.rowOf = h->rowOf;
-    return h->T ? launchEpLocal(g, epCombineLocalKernelFn(), &a, ((size_t)h->T * (g->H / 8) + kEpLocalThreads - 1) / kEpLocalThreads, stream) : ncclSuccess;
+    const bool wide = combineWide(a.layout == EP_RANK_MAJOR, T, h->K, g->H) && !(((uintptr_t)a.x[me] | (uintptr_t)a.outTokens[me]) & 31);
+    return h->T ? launchEpLocal(g, epCombineLocalKernelFn(wide), &a, ((size_t)h->T * (g->H / 8) + kEpLocalThreads - 1) / kEpLocalThreads, stream) : ncclSuccess;
   }
   NCCLCHECK(launchEp(epCombineKernelFn(), &a, ctas, 1, 0, stream, false));
   if (g->comm->devPlane) g->comm->devPlane->launches++;

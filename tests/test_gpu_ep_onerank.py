@@ -188,3 +188,32 @@ def test_tokens_at_sixteen_bytes(comm, T, H, max_sms, fp8):
     if not fp8:
         assert torch.equal(got[0][0], x[(idx >= 0).any(1)])
     ep.destroy()
+
+
+@pytest.mark.parametrize("layout", ["expert_major", "rank_major"])
+@pytest.mark.parametrize("T,K,H", [(1, 1, 128), (37, 3, 384), (65, 4, 640), (6000, 4, 4096), (2700, 8, 4096)])
+def test_results_at_sixteen_bytes(comm, T, K, H, layout):
+    """Combine with rows and results that start on 16 bytes, but not on 32, gives the bytes that aligned ones give: on each side of the lines
+    between accesses of 16 and 32 bytes."""
+    from nccl_b200.ops.ep import ExpertParallel
+    E = 16
+    ep = ExpertParallel(comm, E, T, H, layout=layout)
+    x, idx, w = _batch(T, E, K, H, 13, 0.1)
+    toks, _, _ = ep.dispatch(x, idx, w, fp8=False)
+    y = toks if layout == "expert_major" else torch.randn(1, T, H, device="cuda").bfloat16()
+    want = None
+    for at_in, at_out in ((0, 0), (8, 0), (0, 8), (8, 8)):
+        ys = torch.empty(y.numel() + 16, dtype=torch.bfloat16, device="cuda")[at_in:at_in + y.numel()].view(y.shape).copy_(y)
+        buf = torch.full((T * H + 32,), 7.0, dtype=torch.bfloat16, device="cuda")
+        out = ep.combine(ys, out=buf[at_out:at_out + T * H].view(T, H))
+        torch.cuda.synchronize()
+        assert (buf[:at_out] == 7).all() and (buf[at_out + T * H:] == 7).all()
+        want = out.clone() if want is None else want
+        assert torch.equal(out, want)
+    used = (idx >= 0).any(1)
+    if layout == "rank_major":
+        assert torch.equal(want, y[0] * used[:, None])
+    else:   # one bf16 rounding of an fp32 sum of at most eight products
+        ref = x.double() * (w.double() * (idx >= 0)).sum(1, keepdim=True)
+        assert ((want.double() - ref).abs() <= 2 ** -8 * ref.abs() + 2 ** -20 * x.double().abs() * w.double().sum(1, keepdim=True)).all()
+    ep.destroy()
