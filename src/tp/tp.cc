@@ -296,7 +296,7 @@ static ncclResult_t launchGemmFp8(ncclTpContext* tp, const void* A, const void* 
 }
 
 // Tile width, CTAs that share the K blocks of a tile (1: none), and grid of a plain fp8 GEMM: the least expected time. A K block takes
-// 0.53 us in a tile of 256 columns and 0.38 us in one of 128 (the round trip of the accumulator bounds both), a wave of tiles about
+// 0.50 us in a tile of 256 columns (0.53 where CTAs share it) and 0.38 us in one of 128 (the round trip of the accumulator bounds both), a wave of tiles about
 // 3.0 and 2.4 us besides (start, first operands, store), the exchange of a cluster 3.7 us (7 us for three CTAs and more on 256
 // columns, which are not used). Kernel times, whole 128 x 256 tiles / the choice: 128 x 1024 x 7168 33.8 / 12.0 us (128 columns, four
 // CTAs), 128 x 4096 x 4096 21.4 / 11.6 (the same), 512 x 2048 x 7168 33.9 / 17.6 (two CTAs), 1024 x 2048 x 7168 34.5 / 23.2 (256 columns,
@@ -315,7 +315,7 @@ static void planFp8(const ncclTpContext* tp, TpGemmArgs* a, int* width, int* gri
     for (int s = forced ? std::max(1, std::min(most, blocks)) : 1; s <= std::min(most, blocks); ++s) {
       if (s > 1 && !forced && tiles > tp->fp8Clusters[s]) break;
       const int waves = (tiles + tp->smCount - 1) / tp->smCount, share = (blocks + s - 1) / s;
-      const float us = waves * (w == 256 ? 3.0f + 0.53f * share : 2.4f + 0.38f * share) + (s > 1 ? 3.7f : 0.0f);
+      const float us = waves * (w == 256 ? 3.0f + (s > 1 ? 0.53f : 0.50f) * share : 2.4f + 0.38f * share) + (s > 1 ? 3.7f : 0.0f);
       if (*width && us > 0.97f * best) continue;   // what is simpler stays where the others are hardly faster
       best = us;
       *width = w;
