@@ -102,7 +102,9 @@ static int streamOf(PyObject* stream, PyObject* buf, const Buffer* b, PyObject* 
 
 // collective(address, types, current, send, recv, lead, divisor, extra, comm, stream): address(send, recv, count, type, [extra,] comm, stream)
 // with the count (over divisor) and type of recv if lead has bit 0, else of send, on the stream given or the current one of recv's device if lead
-// has bit 1, else of send's. types: codes by dtype; current: handle of a device's current stream. NotImplemented for buffers that are no tensors.
+// has bit 1, else of send's. Bit 2: the entry point takes `extra` (an operator, a root). Without the bit it does if an extra is given. types: codes by
+// dtype; current: handle of a device's current stream. NotImplemented for what ctypes has to see: buffers that are no tensors, no `extra` where one
+// is due.
 static PyObject* collective(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   (void)self;
   if (n != 10) return PyErr_Format(PyExc_TypeError, "collective takes 10 arguments, not %zd", n);
@@ -117,7 +119,11 @@ static PyObject* collective(PyObject* self, PyObject* const* a, Py_ssize_t n) {
     }
   }
   const long bits = PyLong_AsLong(a[5]);
-  const int lead = bits & 1, at = bits >> 1 & 1;
+  const int lead = bits & 1, at = bits >> 1 & 1, takesExtra = bits & 4 || a[7] != Py_None;
+  if (takesExtra && a[7] == Py_None && !PyErr_Occurred()) {
+    Py_INCREF(Py_NotImplemented);
+    return Py_NotImplemented;
+  }
   if (PyErr_Occurred() || handleOf(a[0], &fn) || handleOf(a[6], &divisor) || handleOf(a[7], &extra) || handleOf(a[8], &comm)) return NULL;
   if (streamOf(a[9], a[3 + at], &b[at], a[2], &stream)) return NULL;
   if (!fn || !divisor || b[lead].type < 0) {
@@ -127,7 +133,7 @@ static PyObject* collective(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   const size_t count = (size_t)(b[lead].count / divisor);
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  if (a[7] == Py_None)
+  if (!takesExtra)
     rc = ((int (*)(void*, void*, size_t, int, void*, void*))(uintptr_t)fn)((void*)(uintptr_t)b[0].ptr, (void*)(uintptr_t)b[1].ptr, count, b[lead].type,
                                                                            (void*)(uintptr_t)comm, (void*)(uintptr_t)stream);
   else

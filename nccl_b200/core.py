@@ -221,7 +221,7 @@ class Communicator:
     # ------------------------------------------------------------------ collectives
     def _native(self, name, send, recv, lead, divisor, extra, stream):
         """Whether the native host path took the call (it describes tensors as below, and raises what they raise); lead: 1 for the count and
-        type of recv, 2 for its stream."""
+        type of recv, 2 for its stream, 4 for an entry point that takes `extra`."""
         if isinstance(send, np.ndarray) or isinstance(recv, np.ndarray):
             return False
         fast = _fast()
@@ -241,7 +241,7 @@ class Communicator:
 
     def all_reduce(self, send, recv=None, op="sum", stream=None):
         recv = send if recv is None else recv
-        if self._native("ncclAllReduce", send, recv, 0, 1, self._op(op), stream):
+        if self._native("ncclAllReduce", send, recv, 4, 1, self._op(op), stream):
             return recv
         sp, n, dt, _ = describe(send)
         rp = describe(recv)[0]
@@ -273,7 +273,7 @@ class Communicator:
 
     def broadcast(self, send, recv, root, stream=None):
         ref = recv if recv is not None else send
-        if self._native("ncclBroadcast", send, ref, 3, 1, root, stream):
+        if self._native("ncclBroadcast", send, ref, 7, 1, root, stream):
             return recv
         sp = describe(send)[0]
         rp, n, dt, _ = describe(ref)
@@ -281,7 +281,7 @@ class Communicator:
         return recv
 
     def reduce_scatter(self, send, recv, op="sum", stream=None):
-        if self._native("ncclReduceScatter", send, recv, 1, 1, self._op(op), stream):
+        if self._native("ncclReduceScatter", send, recv, 5, 1, self._op(op), stream):
             return recv
         sp = describe(send)[0]
         rp, n, dt, _ = describe(recv)

@@ -101,3 +101,47 @@ def test_communicator_either_way():
     for rank in range(2):
         native, through_ctypes = got[rank]
         assert native == through_ctypes and native[0] == [3.0 * i for i in range(8)]
+
+
+@needs_module
+def test_no_integer_where_one_is_due():
+    """Whether an entry point takes an operator or a root is not told by the caller's value: None reaches none of them."""
+    fast, types = _lib.fastcall(), core._torch_types()
+    calls, keep, at = _recorder([P, P, Z, I, I, P, P])
+    a, b = torch.zeros(4), torch.zeros(4)
+    for lead in (4, 5, 7):
+        assert fast.collective(at, types, None, a, b, lead, 1, None, 0x1234, 0x77) is NotImplemented
+    assert not calls
+    assert fast.collective(at, types, None, a, b, 7, 1, 3, 0x1234, 0x77) == 0
+    assert calls == [(a.data_ptr(), b.data_ptr(), 4, core.FP32, 3, 0x1234, 0x77)]
+
+
+class _CallsOnly:
+    """A library of which the wrappers' methods see the entry points alone: each call is recorded."""
+
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        fn = ctypes.CFUNCTYPE(I, *_lib._PROTOS[name])(lambda *a: self.calls.append((name, *a)) or 0)
+        fn.argtypes = _lib._PROTOS[name]
+        setattr(self, name, fn)
+        return fn
+
+
+def _wrapper(monkeypatch):
+    """A communicator over recorded entry points that takes the native path where that is built."""
+    lib = _CallsOnly()
+    comm = core.Communicator(2, 0, None, lib=lib, _handle=ctypes.c_void_p(0x1234))
+    monkeypatch.setattr(_lib, "address", lambda lib, name: ctypes.cast(getattr(lib, name), P).value)
+    return lib, comm
+
+
+def test_broadcast_without_a_root(monkeypatch):
+    lib, comm = _wrapper(monkeypatch)
+    x, y = torch.zeros(4), torch.zeros(4)
+    with pytest.raises(ctypes.ArgumentError):
+        comm.broadcast(x, y, None, stream=0x77)
+    assert not lib.calls
+    comm.broadcast(x, y, 1, stream=0x77)
+    assert lib.calls == [("ncclBroadcast", x.data_ptr(), y.data_ptr(), 4, core.FP32, 1, 0x1234, 0x77)]
