@@ -87,7 +87,10 @@ static int streamOf(PyObject* stream, PyObject* buf, const Buffer* b, PyObject* 
       Py_INCREF(stream);
       return wordOf(stream, out);
     }
-    return wordOf(PyObject_GetAttr(stream, sCudaStream), out);
+    PyObject* handle = PyObject_GetAttr(stream, sCudaStream);
+    const int got = handle ? handleOf(handle, out) : -1;
+    Py_XDECREF(handle);
+    return got;
   }
   if (!b->cuda) return 0;
   PyObject* device = PyObject_GetAttr(buf, sDevice);
@@ -103,8 +106,8 @@ static int streamOf(PyObject* stream, PyObject* buf, const Buffer* b, PyObject* 
 // collective(address, types, current, send, recv, lead, divisor, extra, comm, stream): address(send, recv, count, type, [extra,] comm, stream)
 // with the count (over divisor) and type of recv if lead has bit 0, else of send, on the stream given or the current one of recv's device if lead
 // has bit 1, else of send's. Bit 2: the entry point takes `extra` (an operator, a root). Without the bit it does if an extra is given. types: codes by
-// dtype; current: handle of a device's current stream. NotImplemented for what ctypes has to see: buffers that are no tensors, no `extra` where one
-// is due.
+// dtype; current: handle of a device's current stream. NotImplemented for what ctypes has to see: buffers that are no tensors, an `extra` or a divisor
+// that is no int (ctypes takes whatever stands for one, and refuses the rest).
 static PyObject* collective(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   (void)self;
   if (n != 10) return PyErr_Format(PyExc_TypeError, "collective takes 10 arguments, not %zd", n);
@@ -120,7 +123,7 @@ static PyObject* collective(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   }
   const long bits = PyLong_AsLong(a[5]);
   const int lead = bits & 1, at = bits >> 1 & 1, takesExtra = bits & 4 || a[7] != Py_None;
-  if (takesExtra && a[7] == Py_None && !PyErr_Occurred()) {
+  if (((takesExtra && !PyLong_Check(a[7])) || !PyLong_Check(a[6])) && !PyErr_Occurred()) {
     Py_INCREF(Py_NotImplemented);
     return Py_NotImplemented;
   }
@@ -143,7 +146,8 @@ static PyObject* collective(PyObject* self, PyObject* const* a, Py_ssize_t n) {
   return PyLong_FromLong(rc);
 }
 
-// invoke(address, ...): an entry point whose parameters are integers and pointers. A tuple (a shape) stands for four of them: the number of
+// invoke(address, ...): an entry point whose parameters are integers and pointers. None is a null pointer wherever it stands: an integer of the
+// caller's comes here only as an int. A tuple (a shape) stands for four of them: the number of
 // dimensions and, for two or three dimensions, their sizes (zeros behind the last). System V x86-64: words are what such
 // parameters travel as, and words beyond the callee's last parameter are not looked at.
 enum { kWords = 32 };

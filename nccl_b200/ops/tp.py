@@ -119,7 +119,9 @@ class TensorParallel:
             raise ValueError("x must be a contiguous bf16 matrix")
         q = q if q is not None else torch.empty(R, K, dtype=torch.float8_e4m3fn, device=x.device)
         scales = scales if scales is not None else torch.empty(K // 128, R // block_rows, dtype=torch.float32, device=x.device)
-        rc = self._ncclTpQuantizeFp8(self.handle, x.data_ptr(), q.data_ptr(), scales.data_ptr(), R, K, block_rows, self._stream(stream))
+        # the native path knows ints; ctypes whatever stands for one
+        call = self._ncclTpQuantizeFp8 if type(block_rows) is int else self.lib.ncclTpQuantizeFp8
+        rc = call(self.handle, x.data_ptr(), q.data_ptr(), scales.data_ptr(), R, K, block_rows, self._stream(stream))
         _lib.check(rc, "ncclTpQuantizeFp8", self.lib)
         return q, scales
 

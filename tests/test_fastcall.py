@@ -1,6 +1,7 @@
 """The native host path of the wrappers (bindings/python/fastcall.c): what reaches an entry point is what ctypes hands over, and what the wrappers
 refuse stays refused."""
 import ctypes
+import functools
 
 import numpy as np
 import pytest
@@ -145,3 +146,47 @@ def test_broadcast_without_a_root(monkeypatch):
     assert not lib.calls
     comm.broadcast(x, y, 1, stream=0x77)
     assert lib.calls == [("ncclBroadcast", x.data_ptr(), y.data_ptr(), 4, core.FP32, 1, 0x1234, 0x77)]
+
+
+def test_integers_that_are_no_int(monkeypatch):
+    """What ctypes takes for an integer or a stream, either path takes; what it refuses, both refuse."""
+    lib, comm = _wrapper(monkeypatch)
+    x, y = torch.zeros(4), torch.zeros(4)
+
+    class Stream:
+        cuda_stream = P(0x77)
+    for root in (np.int64(1), np.uint8(1), torch.tensor(1), True):
+        comm.broadcast(x, y, root, stream=Stream())
+    Stream.cuda_stream = None
+    comm.broadcast(x, y, 1, stream=Stream())
+    at = ("ncclBroadcast", x.data_ptr(), y.data_ptr(), 4, core.FP32, 1, 0x1234)
+    assert lib.calls == [(*at, 0x77)] * 4 + [(*at, None)]
+    lib.calls.clear()
+    for root in (1.0, "1", object(), torch.zeros(2)):
+        with pytest.raises(ctypes.ArgumentError):
+            comm.broadcast(x, y, root)
+    comm.nranks = np.int64(2)
+    comm.all_to_all(x, y, stream=0x77)
+    assert lib.calls == [("ncclAlltoAll", x.data_ptr(), y.data_ptr(), 2, core.FP32, 0x1234, 0x77)]
+
+
+def test_block_rows(monkeypatch):
+    """The rows of a block of fp8 scales are the one integer that a caller hands to a call of words."""
+    from nccl_b200.ops.tp import TensorParallel
+    calls = []
+    types = [P, P, P, P, I, I, I, P]
+    fn = ctypes.CFUNCTYPE(I, *types)(lambda *a: calls.append(a) or 0)
+    fn.argtypes = types
+    fast = _lib.fastcall()
+    tp = TensorParallel.__new__(TensorParallel)
+    tp.lib, tp.handle, tp._fp8_ready = type("Lib", (), {"ncclTpQuantizeFp8": fn}), P(0x1234), True
+    tp._ncclTpQuantizeFp8 = functools.partial(fast.invoke, ctypes.cast(fn, P).value) if fast else fn
+    monkeypatch.setattr(tp, "_stream", lambda stream: 0x77, raising=False)
+    x = torch.zeros(256, 128, dtype=torch.bfloat16)
+    for rows in (128, np.int64(128), torch.tensor(128)):
+        q, scales = tp.quantize_fp8(x, rows)
+        assert tuple(scales.shape) == (1, 2) and calls.pop() == (0x1234, x.data_ptr(), q.data_ptr(), scales.data_ptr(), 256, 128, 128, 0x77)
+    for rows in (None, 128.0, "128"):
+        with pytest.raises(ctypes.ArgumentError):
+            tp.quantize_fp8(x, rows, q=q, scales=scales)
+    assert not calls
