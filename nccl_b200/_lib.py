@@ -157,12 +157,14 @@ def load(path=None):
         return _lib
 
 
-@functools.lru_cache(maxsize=None)
 def fastcall():
     """The module that calls entry points outside ctypes (bindings/python/fastcall.c), or None where it was not built for this interpreter."""
     path = os.path.join(_HERE, "lib", "_fastcall.so")
-    if not os.path.exists(path):
-        return None
+    return _fastcall_at(path) if os.path.exists(path) else None   # it may be built later than asked for: with the library, when that is loaded
+
+
+@functools.lru_cache(maxsize=None)
+def _fastcall_at(path):
     loader = importlib.machinery.ExtensionFileLoader("_fastcall", path)
     try:
         module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", path, loader=loader))

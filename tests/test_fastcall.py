@@ -2,6 +2,8 @@
 refuse stays refused."""
 import ctypes
 import functools
+import os
+import shutil
 
 import numpy as np
 import pytest
@@ -12,6 +14,7 @@ from mp_util import run_ranks  # noqa: E402
 from nccl_b200 import _lib, core  # noqa: E402
 
 P, I, Z = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
+_lib.load()   # builds library and module where they are not
 needs_module = pytest.mark.skipif(_lib.fastcall() is None, reason="built without the interpreter's headers")
 
 
@@ -80,7 +83,9 @@ def _rank(rank, nranks, uid):
     import torch
     from nccl_b200 import Communicator
     comm = Communicator(nranks, rank, uid)
-    got = []
+    got, took = [], []
+    real = comm._native
+    comm._native = lambda *a: took.append(real(*a)) or took[-1]
     for native in (True, False):
         if not native:
             comm._entries = dict.fromkeys(("ncclAllReduce", "ncclBroadcast", "ncclReduceScatter", "ncclAllGather", "ncclAlltoAll"))
@@ -88,15 +93,20 @@ def _rank(rank, nranks, uid):
         out = [comm.all_reduce(x, torch.zeros(8)), comm.all_reduce(x.clone(), op="max"), comm.broadcast(x if rank == 1 else None, torch.zeros(8), 1),
                comm.reduce_scatter(x, torch.zeros(4), op="avg"), comm.all_gather(x, torch.zeros(16)), comm.all_to_all(x, torch.zeros(8))]
         got.append([t.tolist() for t in out])
+        assert took == [native] * 6   # neither path stands in for the other
+        took.clear()
         with pytest.raises(ValueError):
             comm.all_reduce(torch.zeros(4, 4).t())
         with pytest.raises(TypeError):
             comm.all_reduce([1, 2])
         assert comm.all_reduce(np.ones(3, np.float32), np.zeros(3, np.float32)).tolist() == [nranks] * 3
+        assert not any(took)
+        took.clear()
     comm.destroy()
     return got
 
 
+@needs_module
 def test_communicator_either_way():
     got = run_ranks(_rank, 2, env={"NCCL_B200_HOST_ONLY": "1", "NCCL_SOCKET_IFNAME": "lo"}, timeout=300)
     for rank in range(2):
@@ -190,3 +200,14 @@ def test_block_rows(monkeypatch):
         with pytest.raises(ctypes.ArgumentError):
             tp.quantize_fp8(x, rows, q=q, scales=scales)
     assert not calls
+
+
+@needs_module
+def test_module_built_after_it_was_asked_for(monkeypatch, tmp_path):
+    """What is not there yet is looked for again: loading the library builds it."""
+    built = os.path.join(_lib._HERE, "lib", "_fastcall.so")
+    monkeypatch.setattr(_lib, "_HERE", str(tmp_path))
+    assert _lib.fastcall() is None
+    (tmp_path / "lib").mkdir()
+    shutil.copy(built, tmp_path / "lib")
+    assert _lib.fastcall() is not None
