@@ -255,8 +255,9 @@ __global__ void __launch_bounds__(W + 32, 1) rmsNormRowsKernel(const __grid_cons
       const int r = m & (R - 1), t = c * R + r;
       if (t >= a.tokens) break;
       const int s = m >> shift;
-      // a row that did not arrive is left alone: neither read, stored nor released; its group still meets at the barrier
-      const bool ok = wait(&fullBar[s], phase);
+      // a row that did not arrive is left alone: neither read, stored nor released; its group still meets at the barrier. The lanes of a warp
+      // vote: each of them polls and reads gaveUp for itself
+      const bool ok = __all_sync(0xffffffffu, wait(&fullBar[s], phase));
       if ((m += kGroups) >= lap) {
         m -= lap;
         phase ^= 1;

@@ -1,0 +1,20 @@
+"""Bounded waits of whole warps: whether one ran out is found by each lane for itself, so lanes may disagree, and what stands behind it (shuffles,
+warp barriers, tcgen05.ld) has to be reached by all of them or by none. The kernels vote. Shown on the source: a wait that runs out needs
+a copy or a product that never comes, which no test brings about."""
+import os
+import re
+
+SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "src")
+
+
+def _code(*parts):
+    with open(os.path.join(SRC, *parts)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def test_rows_of_the_norm():
+    code = _code("contrib", "devapi_samples.cu")
+    kernel = code[code.index("rmsNormRowsKernel(const"):code.index("struct RowPlan")]
+    waits = re.findall(r"[^\n]*\bwait\(&fullBar[^\n]*", kernel)
+    assert len(waits) == 1 and re.search(r"const bool ok = __all_sync\(0xffffffffu, wait\(&fullBar\[s\], phase\)\);", waits[0])
+
