@@ -295,12 +295,9 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       for (int kb = 0; kb < kBlocks && (kLeave || !bad); ++kb, ++kc) {
         const int buf = kc & 1;
         const uint32_t aph = (kc >> 1) & 1;
-        if (kLeave) {
-          if (!mbarWait(smemAddr(&accFull[buf]), aph)) { if (lane == 0) fail(WAIT_TILE, 4000 + buf); bad = true; break; }
-        } else {
-          bad = !mbarWait(smemAddr(&accFull[buf]), aph);
-          if (bad && lane == 0) fail(WAIT_TILE, 4000 + buf);
-        }
+        bad = !__all_sync(0xffffffffu, mbarWait(smemAddr(&accFull[buf]), aph));   // one answer for the warp, which loads together
+        if (bad && lane == 0) fail(WAIT_TILE, 4000 + buf);
+        if (kLeave && bad) break;
         tcFenceAfter();
         if (remoteRows && kb == 0) fetchScales(0);
         const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * kAccCols + c0;

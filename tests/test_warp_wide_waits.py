@@ -4,6 +4,8 @@ a copy or a product that never comes, which no test brings about."""
 import os
 import re
 
+import pytest
+
 SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "src")
 
 
@@ -18,3 +20,8 @@ def test_rows_of_the_norm():
     waits = re.findall(r"[^\n]*\bwait\(&fullBar[^\n]*", kernel)
     assert len(waits) == 1 and re.search(r"const bool ok = __all_sync\(0xffffffffu, wait\(&fullBar\[s\], phase\)\);", waits[0])
 
+
+@pytest.mark.parametrize("name", ["gemm_fp8_sm100.cu", "gemm_split_sm100.cu"])
+def test_accumulators(name):
+    waits = re.findall(r"[^\n]*\bmbarWait\(smemAddr\(&accFull[^\n]*", _code("tp", name))
+    assert waits and all(re.search(r"__all_sync\((0xffffffffu|~0u), mbarWait\(smemAddr\(&accFull", w) for w in waits)
