@@ -261,7 +261,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int wBlocksN = a.N / 128;
     uint32_t kc = 0;
     uint64_t acc[kChunks * 16];   // fp32 pairs
-    for (int t = tile0; t < nTiles; t += gemmCtas) {
+    for (int t = tile0; t < nTiles && !*abortFlag; t += gemmCtas) {
       const TileCoord tc = tileOf(a, t, BM, BN);
       const int row0 = tc.mBlk * BM + q * 32;
       const int row = row0 + lane;
@@ -295,7 +295,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       for (int kb = 0; kb < kBlocks && (kLeave || !bad); ++kb, ++kc) {
         const int buf = kc & 1;
         const uint32_t aph = (kc >> 1) & 1;
-        bad = !__all_sync(0xffffffffu, mbarWaitOr(smemAddr(&accFull[buf]), aph, abortFlag));   // one answer for the warp, which loads together
+        bad = !__all_sync(0xffffffffu, mbarWait(smemAddr(&accFull[buf]), aph));   // one answer for the warp, which loads together
         if (bad && lane == 0) fail(WAIT_TILE, 4000 + buf);
         if (kLeave && bad) break;
         tcFenceAfter();

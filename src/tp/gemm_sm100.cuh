@@ -39,15 +39,6 @@ __device__ __forceinline__ bool mbarWait(uint32_t bar, uint32_t parity, uint32_t
     if (mbarTry(bar, parity)) return true;
   return false;
 }
-// The same, given up as well when *gaveUp is set meanwhile. Where a whole warp waits, its lanes have to vote on the results. (A vote inside this
-// function cost the fp8 kernel 64 bytes of spills.)
-__device__ __forceinline__ bool mbarWaitOr(uint32_t bar, uint32_t parity, const volatile uint32_t* gaveUp) {
-  for (uint32_t i = 0; i < (1u << 24); ++i) {
-    if (mbarTry(bar, parity)) return true;
-    if (*gaveUp) return false;
-  }
-  return false;
-}
 
 // ---------------------------------------------------------------- TMA (tile mode, one CTA, no multicast)
 __device__ __forceinline__ void tmaLoad2d(uint32_t dstSmem, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
