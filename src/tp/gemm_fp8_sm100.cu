@@ -261,7 +261,7 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int wBlocksN = a.N / 128;
     uint32_t kc = 0;
     uint64_t acc[kChunks * 16];   // fp32 pairs
-    for (int t = tile0; t < nTiles && !*abortFlag; t += gemmCtas) {
+    for (int t = tile0; t < nTiles; t += gemmCtas) {
       const TileCoord tc = tileOf(a, t, BM, BN);
       const int row0 = tc.mBlk * BM + q * 32;
       const int row = row0 + lane;
@@ -271,7 +271,8 @@ tpGemmFp8Kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       // The scales of the next K block travel ahead of the accumulator that needs them.
       // In GATHER mode the scales of remote rows land together with the rows: the flag the TMA
       // producer waited for covers them, and accFull orders this warp after the producer.
-      bool bad = false;
+      bool bad = __any_sync(0xffffffffu, *abortFlag);
+      if (bad) break;
       // Rows gathered from a peer arrive during this kernel: their scales may be read only after
       // the tile's first accumulator is published (the producer saw the block's flag before it
       // issued the TMA loads that fed it), and never through the read-only cache path.

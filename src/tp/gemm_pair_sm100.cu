@@ -174,11 +174,11 @@ tpGemmPairKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int q = warp & 3;
     uint8_t* wbuf = epiBuf + (size_t)(warp - 2) * 4096;
     int it = 0;
-    for (int t = pairIdx; t < nTiles && !*abortFlag; t += nPairs, ++it) {
+    for (int t = pairIdx; t < nTiles && !__any_sync(0xffffffffu, *abortFlag); t += nPairs, ++it) {
       const TileCoord tc = tileOf(a, t, PM, BN);
       const int buf = it % kAccBufs;
       const uint32_t aph = (it / kAccBufs) & 1;
-      if (!mbarWait(smemAddr(&accFull[buf]), aph)) { if (lane == 0) fail(WAIT_TILE, 4000 + buf); break; }
+      if (!__all_sync(0xffffffffu, mbarWait(smemAddr(&accFull[buf]), aph))) { if (lane == 0) fail(WAIT_TILE, 4000 + buf); break; }
       tcFenceAfter();
       const int row0 = tc.mBlk * PM + (int)cr * 128 + q * 32;
       const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * 256;

@@ -170,11 +170,11 @@ tpGemmKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     // ---- epilogue warps: TMEM lanes [32q, 32q+32) belong to the warp with warp % 4 == q
     const int q = warp & 3;
     int it = 0;
-    for (int t = blockIdx.x; t < nTiles && !*abortFlag; t += gemmCtas, ++it) {
+    for (int t = blockIdx.x; t < nTiles && !__any_sync(0xffffffffu, *abortFlag); t += gemmCtas, ++it) {
       const TileCoord tc = tileOf(a, t, BM, BN);
       const int buf = it & 1;
       const uint32_t aph = (it >> 1) & 1;
-      if (!mbarWait(smemAddr(&accFull[buf]), aph)) { if (lane == 0) fail(WAIT_TILE, 4000 + buf); break; }
+      if (!__all_sync(0xffffffffu, mbarWait(smemAddr(&accFull[buf]), aph))) { if (lane == 0) fail(WAIT_TILE, 4000 + buf); break; }
       tcFenceAfter();
       const int row0 = tc.mBlk * BM + q * 32;   // first of this warp's 32 rows
       const uint32_t tBase = tmemBase + ((uint32_t)(q * 32) << 16) + buf * kAccCols;

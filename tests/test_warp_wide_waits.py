@@ -21,7 +21,14 @@ def test_rows_of_the_norm():
     assert len(waits) == 1 and re.search(r"const bool ok = __all_sync\(0xffffffffu, wait\(&fullBar\[s\], phase\)\);", waits[0])
 
 
-@pytest.mark.parametrize("name", ["gemm_fp8_sm100.cu", "gemm_split_sm100.cu"])
+@pytest.mark.parametrize("name", ["gemm_fp8_sm100.cu", "gemm_split_sm100.cu", "gemm_sm100.cu", "gemm_pair_sm100.cu"])
 def test_accumulators(name):
-    waits = re.findall(r"[^\n]*\bmbarWait\(smemAddr\(&accFull[^\n]*", _code("tp", name))
+    code = _code("tp", name)
+    waits = re.findall(r"[^\n]*\bmbarWait\(smemAddr\(&accFull[^\n]*", code)
     assert waits and all(re.search(r"__all_sync\((0xffffffffu|~0u), mbarWait\(smemAddr\(&accFull", w) for w in waits)
+    # the word that ends a kernel early, where whole warps go from tile to tile: the loops behind those of the single threads that load and multiply
+    loops = re.findall(r"for \(int t = [^\n]*", code)
+    assert len(loops) == (0 if "split" in name else 3)
+    for loop in loops[2:]:
+        body = code[code.rindex(loop):]
+        assert body[:body.index("accFull")].count("*abortFlag") == body[:body.index("accFull")].count("__any_sync(0xffffffffu, *abortFlag)") == 1
