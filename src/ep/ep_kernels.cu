@@ -663,9 +663,11 @@ __global__ void __launch_bounds__(kEpThreads, 1) epCombineKernel(const __grid_co
 // claims the rows of the output tensors and writes them straight from the input (the general kernel stores into a landing
 // zone and packs from there: written twice, read once more), combine reads the experts' rows where they lie. Both are bound
 // by memory: for 4096 tokens of 7168 bf16 channels and 8 of 32 experts dispatch went from 313 to 104 us and combine from 434 to
-// 87 us (5.1 and 6.1 TB/s; a fill of the bytes that dispatch writes runs at 3.8). Dispatch reads and writes 32 bytes at a time where tokens in and out are aligned to them, which the
-// queue of memory instructions held up (us with 16 / 32 bytes, launches of one after the other): 2000 tokens of 4096 to one row each
-// in fp8 8.9 / 7.0, 1000 of 7168 in bf16 to four experts 16.1 / 14.2, 8 of 7168 in fp8 to eight 5.4 / 5.0, one of 1024 3.7 / 3.6.
+// 87 us (5.1 and 6.1 TB/s, launches of one after the other; combine takes 100 there with 16 bytes per access, and behind a read of 256 MB 96 with 16
+// and 89 with 32). Dispatch writes eight rows there for each that it reads, and is held up by the queue of memory instructions; so it reads and
+// writes 32 bytes at a time where tokens in and out are aligned to them (us with 16 / 32 bytes, launches of one after the other): 2000 tokens
+// of 4096 to one row each in fp8 8.9 / 7.0, 1000 of 7168 in bf16 to four experts 16.1 / 14.2, 8 of 7168 in fp8 to eight 5.4 / 5.0, one of
+// 1024 3.7 / 3.6.
 constexpr int kLocTokens = 64;    // tokens of a CTA whose rows are claimed (or looked up) together
 constexpr int kLocMaxK = 16;
 

@@ -135,14 +135,17 @@ static ncclResult_t launchEpLocal(ncclEpGroup* g, const void* fn, EpArgs* a, siz
 }
 
 // Whether combine's accesses are 32 bytes wide. A thread has 128 bytes under way either way: 8 rows of 16 or 4 of 32, so that more than four
-// rows take a second trip, which pays when they come from memory anyway. us with 16 / 32 bytes, 32 experts: rank-major 1000 x 7168 6.7 / 5.7, 64 x 2048
-// 2.35 / 2.22; one row 1000 x 4096 4.8 / 4.2; three 500 x 7168 8.6 / 6.6; four 16 x 7168 3.4 / 3.0, 500 x 7168 (28 MB) 9.2 / 9.2, 1000 x 7168 (57 MB) 13.6 / 15.0,
-// 4096 x 7168 (235 MB) 55 / 50; eight 64 x 7168 3.5 / 3.7, 1000 x 7168 (115 MB) 22.0 / 24.0, 2000 x 7168 (229 MB) 48.3 / 43.9, 4096 x 7168 101 / 87; six 4096 x 4096
-// (201 MB) 44.4 / 41.0.
-static bool combineWide(bool rankMajor, size_t T, int K, int H) {
-  const size_t rows = T * K * H * 2;
-  return rankMajor || K <= 3 || rows > (size_t)160 << 20 || (K == 4 && rows < (size_t)28 << 20);
-}
+// rows take a second trip. That hides less of the caches' latency, and pays where the rows come from memory. us of dispatch and combine with
+// 16 / 32 bytes, 32 experts, of rows that dispatch has just written and of rows written before it:
+//   three  1000 x 7168 22.4 / 20.6 and 25.5 / 24.9;   four  64 x 7168 8.3 / 8.0 and 8.2 / 7.8, 500 (29 MB of rows) 16.8 / 15.7 and 20.0 / 20.3,
+//   1000 25.5 / 24.2 and 30.2 / 30.5, 2000 50.3 / 48.5 and 56.3 / 53.3, 4096 105.5 / 104.7 and 115 / 108: wide at every size;
+//   six  64 x 7168 8.9 / 9.4 and 8.8 / 9.0, 1000 x 4096 23.0 / 22.2 and 27.0 / 27.7, 4096 x 4096 (201 MB) 87.7 / 86.6 and 94.9 / 90.3;
+//   eight  64 x 4096 8.5 / 9.3 and 8.3 / 8.6, 1000 x 7168 (115 MB) 42.0 / 45.5 and 50.3 / 51.0, 1400 (161 MB) 60.5 / 64.4 and 69.8 / 69.7, 2000 (229 MB)
+//   88.9 / 91.8 and 99.5 / 95.7, 3500 (401 MB) 163.7 / 163.1 and 174 / 168, 4096 (470 MB) 195 / 193 and 206 / 197;   sixteen  4096 x 4096 (537 MB)
+//   207 / 211 and 218 / 215.
+// With more than four rows, up to 3 % is lost from 160 MB on where the caches still hold rows, and 2 to 5 % won where they do not. Entries
+// without an expert count as rows: the host does not see them.
+static bool combineWide(bool rankMajor, size_t T, int K, int H) { return rankMajor || K <= 4 || T * K * H * 2 > (size_t)160 << 20; }
 
 B200_PARAM(EpBulk, "B200_EP_BULK", 1, "Expert-parallel dispatch hands the packed tokens to the bulk-copy engines (a ring of shared-memory stages per CTA) instead of storing them with the warps: 0 never, 1 for the expert-major layout, 2 for every layout")
 
