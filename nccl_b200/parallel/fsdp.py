@@ -111,7 +111,7 @@ class FSDPEngine:
                 e.record()
         self.collectives = 0      # all-gathers + reduce-scatters issued (for reporting)
         self.kernels = 0          # AdamW launches
-        self._kept_for = None
+        self._kept_for = None     # (tokens, memory held and allowed), bytes in use, layers: the last decision of `_layers_kept`
 
     # ------------------------------------------------------------------ memory
     def _buffer(self, numel, dtype):
@@ -235,28 +235,30 @@ class FSDPEngine:
 
     def _layers_kept(self, tokens):
         """How many layers, counted from the last, keep their activations for the backward instead of computing them again there: as many as leave
-        half of the memory that the framework's allocator can still get beyond what the step takes anyway (the logits, every
-        layer's input, one layer's activations). Two layers of hidden 4096 and ffn 14336 with 2048 tokens: 420 MB. Under capture, and where the allocator does
+        half of the memory that the framework's allocator can still get (of what is free, and within the process's memory fraction) beyond what the
+        step takes anyway (the logits, every layer's input, one layer's activations). Two layers of hidden 4096 and ffn 14336 with 2048 tokens: 420 MB. Under capture, and where the allocator does
         not tell, none.
 
-        The driver is asked (60 us, and many milliseconds while other processes keep it busy) only when the allocator holds other memory than
-        at the last decision for as many tokens: while it does not, the step runs in the memory that it ran in before."""
+        The driver is asked (60 us, and many milliseconds while other processes keep it busy) only when the allocator holds or may hold other
+        memory than at the last decision for as many tokens: while it does not, the step runs in the memory that it ran in before."""
         if torch.cuda.is_current_stream_capturing():
             return 0
         try:
             stats = torch.cuda.memory_stats_as_nested_dict(self.device)
             reserved, used = stats["reserved_bytes"]["all"]["current"], stats["allocated_bytes"]["all"]["current"]
-            decided = self._kept_for
-            if decided and decided[:2] == (tokens, reserved) and used <= decided[2] + kDrift:
-                return decided[3]
-            room = torch.cuda.mem_get_info(self.device)[0] + reserved - used
+            fraction = torch.cuda.get_per_process_memory_fraction(self.device)
+            decided, now = self._kept_for, (tokens, reserved, fraction)
+            if decided and decided[0] == now and used <= decided[1] + kDrift:
+                return decided[2]
+            free, total = torch.cuda.mem_get_info(self.device)
+            room = min(free, max(0, int(fraction * total) - reserved)) + reserved - used
         except (RuntimeError, KeyError):
             return 0
         c, layers = self.cfg, len(self.units) - 2
         each = self.fused.activation_bytes(tokens)
         needed = each + 2 * tokens * (c.vocab + (layers + 8) * c.hidden + 2 * c.ffn)
         kept = max(0, min(layers, (room // 2 - needed) // each))
-        self._kept_for = (tokens, reserved, used, kept)
+        self._kept_for = (now, used, kept)
         return kept
 
     def _step(self, tokens, targets):

@@ -1,0 +1,61 @@
+"""How many layers of a step keep their activations: decided from what the allocator and the driver say, which these tests say for them (no GPU is
+touched)."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from nccl_b200.models import llama as M  # noqa: E402
+from nccl_b200.models.llama_fused import FusedUnits  # noqa: E402
+from nccl_b200.parallel.fsdp import FSDPEngine  # noqa: E402
+
+GB = 1 << 30
+CFG = M.LlamaConfig(layers=8, hidden=4096, heads=32, kv_heads=8, ffn=14336, vocab=128256)
+
+
+class Memory:
+    """One GPU's memory as torch.cuda tells of it."""
+
+    def __init__(self, monkeypatch, total=180 * GB, free=150 * GB, reserved=10 * GB, used=9 * GB, fraction=1.0):
+        self.total, self.free, self.reserved, self.used, self.fraction, self.asked = total, free, reserved, used, fraction, 0
+        monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+        monkeypatch.setattr(torch.cuda, "mem_get_info", self.info)
+        monkeypatch.setattr(torch.cuda, "get_per_process_memory_fraction", lambda device=None: self.fraction)
+        monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda device=None: {
+            "reserved_bytes": {"all": {"current": self.reserved}}, "allocated_bytes": {"all": {"current": self.used}}})
+
+    def info(self, device=None):
+        self.asked += 1
+        return self.free, self.total
+
+
+def _engine():
+    eng = FSDPEngine.__new__(FSDPEngine)
+    eng.cfg, eng.units, eng.device, eng._kept_for = CFG, [None] * (CFG.layers + 2), torch.device("cuda", 0), None
+    eng.fused = FusedUnits.__new__(FusedUnits)
+    eng.fused.cfg = CFG
+    return eng
+
+
+def test_memory_fraction(monkeypatch):
+    """Free memory beyond the process's share is none that a step can have."""
+    m, eng = Memory(monkeypatch), _engine()
+    each = eng.fused.activation_bytes(4096)
+    assert eng._layers_kept(4096) == CFG.layers
+    m.fraction = 10.5 / 180
+    assert eng._layers_kept(4096) == 0        # another share is another decision
+    for gb in (12, 15, 20, 30, 60):
+        m.fraction = gb / 180
+        kept = eng._layers_kept(4096)
+        assert kept * each <= (gb * GB - m.used) // 2
+    assert kept == CFG.layers
+
+
+def test_asked_once(monkeypatch):
+    m, eng = Memory(monkeypatch), _engine()
+    assert [eng._layers_kept(4096) for _ in range(3)] == [CFG.layers] * 3 and m.asked == 1
+    m.used += 8 << 20
+    eng._layers_kept(4096)
+    assert m.asked == 1
+    m.reserved += GB
+    eng._layers_kept(4096)
+    assert m.asked == 2
