@@ -45,9 +45,32 @@ class _Unit:
     pass
 
 
+class _Kept:
+    """Activations that the units from `first` on keep for the backward of one step; they are what can be done without when memory runs out."""
+
+    def __init__(self, first, units):
+        self.first, self.units, self.acts, self.ran_out = first, units, {}, False
+
+    def spare(self, fn):
+        """fn(), and if memory runs out in it once more without kept activations. fn may have started, but not changed anything."""
+        try:
+            return fn()
+        except torch.OutOfMemoryError:
+            if self.first == self.units:
+                raise
+        # behind the handler, which holds on to what the failed call had
+        self.ran_out, self.first = True, self.units
+        self.acts.clear()
+        return fn()
+
+
 class FSDPEngine:
-    def __init__(self, comm, cfg, device="cuda", seed=0, lr=1e-4, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.1, symmetric=True, init_on_device=False):
+    def __init__(self, comm, cfg, device="cuda", seed=0, lr=1e-4, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.1, symmetric=True, init_on_device=False,
+                 keep_layers=None):
+        """keep_layers: how many layers may keep their activations for the backward at most (0: all are computed again there); None: as many as
+        memory allows."""
         self.comm, self.cfg, self.device = comm, cfg, torch.device(device)
+        self.keep_layers = keep_layers
         self.cuda = self.device.type == "cuda"
         if self.cuda and self.device.index is None:
             self.device = torch.device("cuda", torch.cuda.current_device())
@@ -237,29 +260,35 @@ class FSDPEngine:
         """How many layers, counted from the last, keep their activations for the backward instead of computing them again there: as many as leave
         half of the memory that the framework's allocator can still get (of what is free, and within the process's memory fraction) beyond what the
         step takes anyway (the logits, every layer's input, one layer's activations). Two layers of hidden 4096 and ffn 14336 with 2048 tokens: 420 MB. Under capture, and where the allocator does
-        not tell, none.
+        not tell, none. At most `keep_layers`, which a step that ran out of memory halves.
 
         The driver is asked (60 us, and many milliseconds while other processes keep it busy) only when the allocator holds or may hold other
         memory than at the last decision for as many tokens: while it does not, the step runs in the memory that it ran in before."""
-        if torch.cuda.is_current_stream_capturing():
+        c, layers = self.cfg, len(self.units) - 2
+        most = layers if self.keep_layers is None else min(layers, self.keep_layers)
+        if most <= 0 or torch.cuda.is_current_stream_capturing():
             return 0
         try:
             stats = torch.cuda.memory_stats_as_nested_dict(self.device)
             reserved, used = stats["reserved_bytes"]["all"]["current"], stats["allocated_bytes"]["all"]["current"]
             fraction = torch.cuda.get_per_process_memory_fraction(self.device)
-            decided, now = self._kept_for, (tokens, reserved, fraction)
+            decided, now = self._kept_for, (tokens, most, reserved, fraction)
             if decided and decided[0] == now and used <= decided[1] + kDrift:
                 return decided[2]
             free, total = torch.cuda.mem_get_info(self.device)
             room = min(free, max(0, int(fraction * total) - reserved)) + reserved - used
         except (RuntimeError, KeyError):
             return 0
-        c, layers = self.cfg, len(self.units) - 2
         each = self.fused.activation_bytes(tokens)
-        needed = each + 2 * tokens * (c.vocab + (layers + 8) * c.hidden + 2 * c.ffn)
-        kept = max(0, min(layers, (room // 2 - needed) // each))
+        needed = self._backward_bytes(tokens) + 2 * tokens * (c.vocab + layers * c.hidden)
+        kept = max(0, min(most, (room // 2 - needed) // each))
         self._kept_for = (now, used, kept)
         return kept
+
+    def _backward_bytes(self, tokens):
+        """What the backward of a layer allocates, its activations among it."""
+        c = self.cfg
+        return self.fused.activation_bytes(tokens) + 2 * tokens * (8 * c.hidden + 2 * c.ffn)
 
     def _step(self, tokens, targets):
         cfg, U = self.cfg, len(self.units)
@@ -290,8 +319,8 @@ class FSDPEngine:
         def weights(idx, slot):
             return self._whole(idx, slot)[:self.units[idx].numel]
 
-        kept = [None] * U
-        first_kept = U - 1 - self._layers_kept(tokens.numel()) if fused else U
+        layers_kept = self._layers_kept(tokens.numel()) if fused else 0
+        kept = _Kept(U - 1 - layers_kept if layers_kept else U, U)
 
         # forward (the head is differentiated at once: its recompute would be wasted work)
         self._gather(0, 0)
@@ -301,8 +330,9 @@ class FSDPEngine:
             self._wait_gathered(idx % 2)
             with torch.no_grad():
                 if fused and idx:
-                    saved[idx], x, add, *acts = fused.layer(x, add, weights(idx, idx % 2), rope, shape, keep=idx >= first_kept)
-                    kept[idx] = acts[0] if acts else None
+                    saved[idx], x, add, *acts = kept.spare(lambda: fused.layer(x, add, weights(idx, idx % 2), rope, shape, keep=idx >= kept.first))
+                    if acts:
+                        kept.acts[idx] = acts[0]
                     del acts
                 else:
                     saved[idx] = x
@@ -314,8 +344,8 @@ class FSDPEngine:
         slot = idx % 2
         self._wait_gathered(slot)
         if fused:
-            loss, gx = fused.head(x, add, weights(idx, slot), self._grad_flat(idx, slot), targets.reshape(-1).contiguous(),
-                                  before=lambda: self._take_grads(idx, slot))
+            loss, gx = kept.spare(lambda: fused.head(x, add, weights(idx, slot), self._grad_flat(idx, slot), targets.reshape(-1).contiguous(),
+                                                     before=lambda: self._take_grads(idx, slot)))
             self._release(slot)
         else:
             vs = params(idx, slot, True)
@@ -329,6 +359,10 @@ class FSDPEngine:
             del grads, vs, xin
         self._reduce_and_update(idx, slot)
         del x, add
+        if kept.acts:   # a layer's backward updates weights on its way and cannot be begun again: whether its memory is there shows before the first
+            kept.spare(lambda: torch.empty(self._backward_bytes(tokens.numel()), dtype=torch.uint8, device=self.device) if kept.acts else None)
+        if kept.ran_out:
+            self.keep_layers = layers_kept // 2
         # backward through the layers and the embedding; the last layer's parameters are still gathered from the forward
         for idx in range(U - 2, -1, -1):
             slot = idx % 2
@@ -348,7 +382,7 @@ class FSDPEngine:
                         done[0] = lo
                 else:
                     ready = None
-                acts, kept[idx] = kept[idx], None
+                acts = kept.acts.pop(idx, None)
                 gx = fused.layer_backward(saved[idx], weights(idx, slot), self._grad_flat(idx, slot), rope, shape, gx, ready,
                                           before=lambda: self._take_grads(idx, slot), kept=acts)
                 del acts

@@ -6,7 +6,7 @@ torch = pytest.importorskip("torch")
 
 from nccl_b200.models import llama as M  # noqa: E402
 from nccl_b200.models.llama_fused import FusedUnits  # noqa: E402
-from nccl_b200.parallel.fsdp import FSDPEngine  # noqa: E402
+from nccl_b200.parallel.fsdp import FSDPEngine, _Kept  # noqa: E402
 
 GB = 1 << 30
 CFG = M.LlamaConfig(layers=8, hidden=4096, heads=32, kv_heads=8, ffn=14336, vocab=128256)
@@ -28,8 +28,9 @@ class Memory:
         return self.free, self.total
 
 
-def _engine():
+def _engine(keep_layers=None):
     eng = FSDPEngine.__new__(FSDPEngine)
+    eng.keep_layers = keep_layers
     eng.cfg, eng.units, eng.device, eng._kept_for = CFG, [None] * (CFG.layers + 2), torch.device("cuda", 0), None
     eng.fused = FusedUnits.__new__(FusedUnits)
     eng.fused.cfg = CFG
@@ -59,3 +60,35 @@ def test_asked_once(monkeypatch):
     m.reserved += GB
     eng._layers_kept(4096)
     assert m.asked == 2
+
+
+def test_at_most_as_many_as_the_caller_says(monkeypatch):
+    m = Memory(monkeypatch)
+    for most in (0, 1, 5, CFG.layers, 100, None):
+        eng = _engine(most)
+        assert eng._layers_kept(4096) == (CFG.layers if most is None else min(most, CFG.layers))
+    assert m.asked == 5                       # nothing to ask for none
+    eng.keep_layers = 3                       # and from then on
+    assert eng._layers_kept(4096) == 3
+
+
+def test_out_of_memory_costs_what_was_kept_only():
+    kept = _Kept(3, 6)
+    kept.acts[3] = kept.acts[4] = "activations"
+    tried = []
+
+    def fn():
+        tried.append((kept.first, dict(kept.acts)))
+        if kept.acts:
+            raise torch.OutOfMemoryError("no memory")
+        return "done"
+    assert kept.spare(fn) == "done" and kept.ran_out and len(tried) == 2 and tried[1] == (6, {})
+
+    def full():
+        tried.append(None)
+        raise torch.OutOfMemoryError("no memory at all")
+    with pytest.raises(torch.OutOfMemoryError):   # nothing is left to give up: once
+        kept.spare(full)
+    assert len(tried) == 3
+    with pytest.raises(ValueError):
+        _Kept(3, 6).spare(lambda: [].index(1))

@@ -59,3 +59,90 @@ def test_kept_layers(shape, monkeypatch):
         for a, b in zip(ms, got[0][1]):
             assert float((a.double() - b.double()).norm() / b.double().norm()) < 3e-2
     comm.destroy()
+
+
+@pytest.mark.parametrize("where", ["first layer kept", "last layer", "head", "backward", "declined"])
+def test_memory_that_runs_out(where, monkeypatch):
+    """A step that runs out of memory with activations kept is one that computes them again, and the next steps keep fewer."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from nccl_b200 import Communicator, get_unique_id
+    from nccl_b200.models import llama as M
+    from nccl_b200.parallel.fsdp import FSDPEngine
+    torch.cuda.set_device(0)
+    comm = Communicator(1, 0, get_unique_id())
+    cfg = M.LlamaConfig(layers=4, hidden=256, heads=4, kv_heads=2, ffn=512, vocab=1024)
+    g = torch.Generator().manual_seed(3)
+    tok, tgt = (torch.randint(0, cfg.vocab, (1, 65), generator=g) for _ in range(2))
+    eng = FSDPEngine(comm, cfg, device="cuda", seed=1, lr=1e-3, eps=1.0, init_on_device=True, keep_layers=0 if where == "declined" else None)
+    ref = FSDPEngine(comm, cfg, device="cuda", seed=1, lr=1e-3, eps=1.0, init_on_device=True, keep_layers=0)
+    used, failed = [], []
+    product, head, backward_bytes = eng.fused._to_product, eng.fused.head, eng._backward_bytes
+
+    def fail(now):
+        if now and not failed:
+            failed.append(1)
+            raise torch.OutOfMemoryError("no memory")
+
+    def counted(*a):
+        fail(a[-1] and where in ("first layer kept", "last layer") and len(used) == (0 if where == "first layer kept" else 3))
+        used.append(a[-1])
+        return product(*a)
+
+    def failing_head(*a, **kw):
+        fail(where == "head")
+        return head(*a, **kw)
+
+    def failing_bytes(tokens):   # of the check ahead of the backward, not of the decision ahead of the forward
+        if where == "backward" and len(used) == cfg.layers and not failed:
+            failed.append(1)
+            return 1 << 50
+        return backward_bytes(tokens)
+    monkeypatch.setattr(eng.fused, "_to_product", counted)
+    monkeypatch.setattr(eng.fused, "head", failing_head)
+    monkeypatch.setattr(eng, "_backward_bytes", failing_bytes)
+    losses = [eng.step(tok, tgt)]
+    first = {"first layer kept": [False] * 4, "last layer": [True] * 3 + [False], "head": [True] * 4, "backward": [True] * 4, "declined": [False] * 4}[where]
+    assert used == first + [True] * 4 and bool(failed) == (where != "declined")
+    assert eng.keep_layers == (0 if where == "declined" else 2)
+    used.clear()
+    losses.append(eng.step(tok, tgt))
+    assert used == ([False] * 4 + [True] * 4 if where == "declined" else [False] * 2 + [True] * 2 + [True] * 2)
+    want = [ref.step(tok, tgt) for _ in range(2)]
+    torch.cuda.synchronize()
+    # the bounds of the test above: attention may pick another kernel where no gradient is wanted
+    assert torch.allclose(torch.stack(losses), torch.stack(want), rtol=2 ** -9)
+    for a, b in zip(eng.units, ref.units):
+        assert float((a.m.double() - b.m.double()).norm() / b.m.double().norm()) < 3e-2
+    eng.close()
+    ref.close()
+    comm.destroy()
+
+
+def test_step_within_a_share_of_the_memory():
+    """A step of a model whose layers would keep more than the process may have."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from nccl_b200 import Communicator, get_unique_id
+    from nccl_b200.models import llama as M
+    from nccl_b200.parallel.fsdp import FSDPEngine
+    torch.cuda.set_device(0)
+    comm = Communicator(1, 0, get_unique_id())
+    cfg = M.LlamaConfig(layers=12, hidden=1024, heads=8, kv_heads=2, ffn=3584, vocab=1024)
+    eng = FSDPEngine(comm, cfg, device="cuda", seed=1, init_on_device=True)
+    tok = torch.randint(0, cfg.vocab, (1, 8192))
+    each, total = eng.fused.activation_bytes(tok.numel()), torch.cuda.mem_get_info()[1]
+    torch.cuda.empty_cache()
+    try:
+        for layers in (6, 12, 40):
+            torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + layers * each) / total)
+            loss = eng.step(tok, tok)
+            torch.cuda.synchronize()
+            assert torch.isfinite(loss) and torch.cuda.memory_reserved() <= (torch.cuda.get_per_process_memory_fraction() + 1e-6) * total
+            kept = eng._kept_for[2] if eng._kept_for else 0
+            assert kept < cfg.layers or layers > 12
+            torch.cuda.empty_cache()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    eng.close()
+    comm.destroy()
