@@ -16,6 +16,7 @@ import ctypes
 
 import torch
 import torch.nn.functional as F
+from torch.nn.attention import SDPBackend
 from torch.overrides import _get_current_function_mode_stack
 from torch.utils._device import DeviceContext
 from torch.utils._python_dispatch import _get_current_dispatch_mode_stack
@@ -138,16 +139,19 @@ class FusedUnits:
         h, qkv, f = c.hidden, (c.heads + 2 * c.kv_heads) * c.head_dim, c.ffn
         return M.views(flat, [("norm1", (h,)), ("wqkv", (qkv, h)), ("wo", (h, h)), ("norm2", (h,)), ("w_gu", (2 * f, h)), ("w_down", (h, f))])
 
-    def _up_to_attention(self, x, add, p, rope, shape, backward):
-        """(x + add, norm1's output and 1 / rms, q, k, v as attention takes them, its output [B, heads, S, head_dim])."""
+    def _up_to_attention(self, x, add, p, rope, shape, keep, backward):
+        """(x + add, norm1's output and 1 / rms, q, k, v as attention takes them, its output [B, heads, S, head_dim]). The output carries what
+        its backward takes if `backward`; with `keep`, which is for a later one, only if that is no more than `activation_bytes` counts."""
         c, (B, S) = self.cfg, shape
         x, h, rstd = self.norm(x, p["norm1"], add=add, need_rstd=backward)
         qkv = torch.mm(h, p["wqkv"].t())
         self.rope(qkv, rope, S)
         q, k, v = (t.transpose(1, 2) for t in qkv.view(B, S, c.heads + 2 * c.kv_heads, c.head_dim).split((c.heads, c.kv_heads, c.kv_heads), dim=2))
-        if backward:
-            q, k, v = (t.detach().requires_grad_(True) for t in (q, k, v))
         with torch.set_grad_enabled(backward):
+            if backward:
+                q, k, v = (t.detach().requires_grad_(True) for t in (q, k, v))
+                if keep and torch._fused_sdp_choice(q, k, v, is_causal=True, enable_gqa=True) == SDPBackend.MATH.value:
+                    q, k, v = (t.detach() for t in (q, k, v))   # single operations: S x S probabilities per head, and k and v for every head
             return x, h, rstd, (q, k, v), F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
 
     def activation_bytes(self, tokens):
@@ -155,20 +159,20 @@ class FusedUnits:
         c = self.cfg
         return tokens * (2 * (4 * c.hidden + (c.heads + 2 * c.kv_heads) * c.head_dim + 2 * c.ffn) + 4 * c.heads + 8)
 
-    def _to_product(self, x, add, p, rope, shape, backward):
+    def _to_product(self, x, add, p, rope, shape, keep, backward):
         """(x + add, (norm1's output and 1 / rms, q, k, v, attention's output, norm2's sum, output and 1 / rms, gate and up))."""
-        x, h1, rstd1, qkv, a = self._up_to_attention(x, add, p, rope, shape, backward)
+        x, h1, rstd1, qkv, a = self._up_to_attention(x, add, p, rope, shape, keep, backward)
         o = a.detach().transpose(1, 2).reshape(x.shape)
         x2, h2, rstd2 = self.norm(x, p["norm2"], add=torch.mm(o, p["wo"].t()), need_rstd=backward)
         return x, (h1, rstd1, qkv, a, x2, h2, rstd2, torch.mm(h2, p["w_gu"].t()))
 
     def layer(self, x, add, flat, rope, shape, keep=False):
         """The layer of input x + add (add may be None), [B * S, hidden] with shape = (B, S): its input, its output as two terms that the next
-        unit's norm adds up, and with `keep` what `layer_backward` would compute again."""
+        unit's norm adds up, and with `keep` what `layer_backward` would compute again (unless attention would save much more than that)."""
         p = self._layer_views(flat)
-        x, acts = self._to_product(x, add, p, rope, shape, keep)
+        x, acts = self._to_product(x, add, p, rope, shape, keep, keep)
         out = x, acts[4], torch.mm(self.swiglu(acts[7]), p["w_down"].t())
-        return out + (acts,) if keep else out
+        return out + (acts,) if keep and acts[3].requires_grad else out
 
     def layer_backward(self, x, flat, gflat, rope, shape, gy, ready=None, before=None, kept=None):
         """Gradient of the layer's input; the weights' gradients go into gflat (laid out like flat). before() is called ahead of the first
@@ -181,7 +185,7 @@ class FusedUnits:
             if ready:
                 ready((p[name].data_ptr() - begin) // flat.element_size())
 
-        h1, rstd1, qkv, a, x2, h2, rstd2, gu = kept or self._to_product(x, None, p, rope, shape, True)[1]
+        h1, rstd1, qkv, a, x2, h2, rstd2, gu = kept or self._to_product(x, None, p, rope, shape, False, True)[1]
         del kept
         o = a.detach().transpose(1, 2).reshape(x.shape)
         act = torch.mm(gy, p["w_down"])

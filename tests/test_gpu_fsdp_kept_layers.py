@@ -146,3 +146,42 @@ def test_step_within_a_share_of_the_memory():
         torch.cuda.set_per_process_memory_fraction(1.0)
     eng.close()
     comm.destroy()
+
+
+@pytest.mark.parametrize("fused_attention", [True, False])
+def test_attention_that_saves_probabilities(fused_attention, monkeypatch):
+    """Attention by single operations saves S x S values per head for its backward: layers that run it are computed again, and a step takes no more
+    memory than one that keeps none."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+    from nccl_b200 import Communicator, get_unique_id
+    from nccl_b200.models import llama as M
+    from nccl_b200.parallel.fsdp import FSDPEngine
+    torch.cuda.set_device(0)
+    comm = Communicator(1, 0, get_unique_id())
+    cfg = M.LlamaConfig(layers=4, hidden=512, heads=8, kv_heads=2, ffn=512, vocab=512)
+    g = torch.Generator().manual_seed(3)
+    tok, tgt = (torch.randint(0, cfg.vocab, (1, 1024), generator=g) for _ in range(2))
+    peaks, losses = [], []
+    for most in (0, None):
+        eng = FSDPEngine(comm, cfg, device="cuda", seed=1, lr=1e-3, init_on_device=True, keep_layers=most)
+        used, product = [], eng.fused._to_product
+        monkeypatch.setattr(eng.fused, "_to_product", lambda *a: used.append(a[-1]) or product(*a))
+        with sdpa_kernel([SDPBackend.FLASH_ATTENTION, SDPBackend.CUDNN_ATTENTION] if fused_attention else SDPBackend.MATH):
+            eng.step(tok, tgt)
+            torch.cuda.synchronize()
+            used.clear()
+            before = torch.cuda.memory_allocated()
+            torch.cuda.reset_peak_memory_stats()
+            losses.append(float(eng.step(tok, tgt)))
+            torch.cuda.synchronize()
+            peaks.append(torch.cuda.max_memory_allocated() - before)
+        again = 0 if most is None and fused_attention else cfg.layers
+        assert used == [most is None] * cfg.layers + [True] * again
+        eng.close()
+    assert abs(losses[1] - losses[0]) <= 2 ** -9 * losses[0]
+    if not fused_attention:
+        # a layer's 1 / rms, handed back at once: two words a token
+        assert peaks[1] <= peaks[0] + 2 * 4 * tok.numel()
+    comm.destroy()
