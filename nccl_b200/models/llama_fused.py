@@ -176,8 +176,8 @@ class FusedUnits:
 
     def layer_backward(self, x, flat, gflat, rope, shape, gy, ready=None, before=None, kept=None):
         """Gradient of the layer's input; the weights' gradients go into gflat (laid out like flat). before() is called ahead of the first
-        write into gflat, ready(lo) is told that from element lo on the gradients are written and the weights are read no more. `kept` comes
-        from `layer`, and is used up."""
+        write into gflat, ready(lo) is told that from element lo on the gradients are written and the weights are read no more. `kept` holds
+        what came from `layer` as the one element of a list, which is emptied: with no reference elsewhere it goes as it is used."""
         p, g = self._layer_views(flat), self._layer_views(gflat)
         begin = flat.data_ptr()
 
@@ -185,8 +185,7 @@ class FusedUnits:
             if ready:
                 ready((p[name].data_ptr() - begin) // flat.element_size())
 
-        h1, rstd1, qkv, a, x2, h2, rstd2, gu = kept or self._to_product(x, None, p, rope, shape, False, True)[1]
-        del kept
+        h1, rstd1, qkv, a, x2, h2, rstd2, gu = kept.pop() if kept else self._to_product(x, None, p, rope, shape, False, True)[1]
         o = a.detach().transpose(1, 2).reshape(x.shape)
         act = torch.mm(gy, p["w_down"])
         self.swiglu_backward(gu, act)

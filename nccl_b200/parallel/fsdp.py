@@ -382,7 +382,7 @@ class FSDPEngine:
                         done[0] = lo
                 else:
                     ready = None
-                acts = kept.acts.pop(idx, None)
+                acts = [kept.acts.pop(idx)] if idx in kept.acts else None   # no name of its own: the layer lets go of it bit by bit
                 gx = fused.layer_backward(saved[idx], weights(idx, slot), self._grad_flat(idx, slot), rope, shape, gx, ready,
                                           before=lambda: self._take_grads(idx, slot), kept=acts)
                 del acts

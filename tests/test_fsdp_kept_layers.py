@@ -92,3 +92,34 @@ def test_out_of_memory_costs_what_was_kept_only():
     assert len(tried) == 3
     with pytest.raises(ValueError):
         _Kept(3, 6).spare(lambda: [].index(1))
+
+
+def test_activations_go_as_they_are_used():
+    """On the CPU, with kernels that do nothing: by the gradient of the second norm, gate and up and that norm's output are gone, by the last product
+    all but the first norm's output, for a kept layer as for one that is computed again."""
+    import weakref
+
+    from nccl_b200 import _lib
+
+    class NoKernels(FusedUnits):
+        def _run(self, name, *args):
+            pass
+
+        def norm_backward(self, *a):
+            alive.append([r() is not None for r in refs])
+            return super().norm_backward(*a)
+
+    u = NoKernels(M.LlamaConfig(hidden=64, heads=4, kv_heads=2, ffn=128, vocab=64), _lib.load())
+    rope = M.rope_tables(u.cfg, 8, "cpu")
+    x, gy = (torch.zeros(16, 64, dtype=torch.bfloat16) for _ in range(2))
+    shapes = M.layer_shapes(u.cfg)
+    flat, gflat = (torch.zeros(M.numel(shapes), dtype=torch.bfloat16) for _ in range(2))
+    alive = []
+    with torch.no_grad():
+        x, y, add, acts = u.layer(x, None, flat, rope, (2, 8), keep=True)
+    h1, _, (q, _, _), a, x2, h2, _, gu = acts
+    refs = [weakref.ref(t) for t in (h1, q, a, x2, h2, gu)]
+    held = [acts]
+    del h1, q, _, a, x2, h2, gu, acts, y, add
+    u.layer_backward(x, flat, gflat, rope, (2, 8), gy, kept=held)
+    assert held == [] and alive == [[True, True, True, True, False, False], [True, False, False, True, False, False]]
