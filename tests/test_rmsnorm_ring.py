@@ -16,9 +16,9 @@ def test_a_group_meets_every_use_of_its_slots(lib, ctas):
     waited for the one before. Group g takes rows g, g + groups, ... of its CTA: it meets them all when a lap of the ring is a whole
     number of its steps, whatever order the copies land in. (No slot is used twice when a CTA's rows fit the ring.)"""
     for hidden in range(8, 16385, 8):
-        for tokens in (0, 1, ctas, 5 * ctas + 3, 17 * ctas, 32 * ctas + 1, 2048, 100003):
+        for tokens in (0, 1, ctas, 5 * ctas + 3, 12 * ctas - 1, 12 * ctas, 17 * ctas, 32 * ctas + 1, 2048, 100003):
             group, groups, rows, stages = _plan(lib, tokens, hidden, ctas)
             at = (tokens, hidden, ctas, group, rows, stages)
             assert group * 8 >= hidden // 8, at                       # 8 packs of 8 channels per thread hold a row
-            assert 1 <= stages <= 16 and rows >= 1 and stages * rows * hidden * 4 + 128 <= 227 * 1024 - 1024, at
+            assert 1 <= stages <= 16 and rows >= 1 and 128 + stages * rows * hidden * 4 + hidden * 2 <= 227 * 1024 - 1024, at   # ring and gains
             assert stages * rows % groups == 0, at
