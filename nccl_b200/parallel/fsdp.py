@@ -134,6 +134,7 @@ class FSDPEngine:
                 e.record()
         self.collectives = 0      # all-gathers + reduce-scatters issued (for reporting)
         self.kernels = 0          # AdamW launches
+        self.layers_kept = 0      # whose activations the last step kept for its backward (for reporting)
         self._kept_for = None     # (tokens, memory held and allowed), bytes in use, layers: the last decision of `_layers_kept`
 
     # ------------------------------------------------------------------ memory
@@ -363,6 +364,7 @@ class FSDPEngine:
             kept.spare(lambda: torch.empty(self._backward_bytes(tokens.numel()), dtype=torch.uint8, device=self.device) if kept.acts else None)
         if kept.ran_out:
             self.keep_layers = layers_kept // 2
+        self.layers_kept = len(kept.acts)
         # backward through the layers and the embedding; the last layer's parameters are still gathered from the forward
         for idx in range(U - 2, -1, -1):
             slot = idx % 2

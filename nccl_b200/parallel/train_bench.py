@@ -74,7 +74,7 @@ def main(argv=None):
                "warmup": a.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "dtype": "bf16", "data": "synthetic", "loss": loss,
                "collectives_per_step": (eng.collectives - c0) // a.steps, "h2d_bytes_per_step": 2 * tok.numel() * 8, "d2h_bytes_per_step": 4,
                "config": {"model": "llama3-8b-shaped" if not a.tiny and a.layers == 32 else "llama-%dL" % a.layers, "global_batch": a.batch * d.world,
-                          "seq_len": a.seq, "parallelism": "zero3-dp%d" % d.world, "activation_checkpointing": True, "layers_kept": eng._kept_for[2] if eng._kept_for else 0}}
+                          "seq_len": a.seq, "parallelism": "zero3-dp%d" % d.world, "activation_checkpointing": eng.layers_kept < cfg.layers, "layers_kept": eng.layers_kept}}
         eng.close()
     else:
         from nccl_b200.parallel.pipeline import PipelineStage

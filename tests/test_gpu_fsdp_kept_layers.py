@@ -103,11 +103,12 @@ def test_memory_that_runs_out(where, monkeypatch):
     monkeypatch.setattr(eng, "_backward_bytes", failing_bytes)
     losses = [eng.step(tok, tgt)]
     first = {"first layer kept": [False] * 4, "last layer": [True] * 3 + [False], "head": [True] * 4, "backward": [True] * 4, "declined": [False] * 4}[where]
-    assert used == first + [True] * 4 and bool(failed) == (where != "declined")
+    assert used == first + [True] * 4 and bool(failed) == (where != "declined") and eng.layers_kept == 0
     assert eng.keep_layers == (0 if where == "declined" else 2)
     used.clear()
     losses.append(eng.step(tok, tgt))
     assert used == ([False] * 4 + [True] * 4 if where == "declined" else [False] * 2 + [True] * 2 + [True] * 2)
+    assert eng.layers_kept == eng.keep_layers
     want = [ref.step(tok, tgt) for _ in range(2)]
     torch.cuda.synchronize()
     # the bounds of the test above: attention may pick another kernel where no gradient is wanted
