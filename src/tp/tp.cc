@@ -296,13 +296,14 @@ static ncclResult_t launchGemmFp8(ncclTpContext* tp, const void* A, const void* 
 }
 
 // Tile width, CTAs that share the K blocks of a tile (1: none), and grid of a plain fp8 GEMM: the least expected time. A K block takes
-// 0.50 us in a tile of 256 columns (0.53 where CTAs share it) and 0.38 us in one of 128 (the round trip of the accumulator bounds both), a wave of tiles about
-// 3.0 and 2.4 us besides (start, first operands, store), the exchange of a cluster 3.7 us (7 us for three CTAs and more on 256
-// columns, which are not used). Kernel times, whole 128 x 256 tiles / the choice: 128 x 1024 x 7168 33.8 / 12.0 us (128 columns, four
-// CTAs), 128 x 4096 x 4096 21.4 / 11.6 (the same), 512 x 2048 x 7168 33.9 / 17.6 (two CTAs), 1024 x 2048 x 7168 34.5 / 23.2 (256 columns,
-// two CTAs), 512 x 4096 x 1024 8.9 / 7.4 (128 columns, whole), 896 x 2560 x 3584 20.0 / 15.3 (the same). The other side of the line:
-// 2560 x 3072 x 2048 in 128 columns 32.3 / 24.6, 256 x 4096 x 1536 with two CTAs 9.1 / 8.6. Six and eight CTAs to a tile gained nothing over
-// four; widths of 160 to 224, whose warps meet two scales of W, lost 5 to 50 %.
+// 0.46 us in a tile of 256 columns, 0.54 at the clock of a long run (0.50 below; no choice changes between 0.46 and 0.56), about 0.53 where CTAs share
+// it and 0.38 us in one of 128 (the round trip of the accumulator bounds them), a wave of tiles about 3.0 and 2.4 us besides (start, first
+// operands, store), the exchange of a cluster 3.7 us (7 us for three CTAs and more on 256 columns, which are not used). Kernel times with
+// operands in L2, whole 128 x 256 tiles / the choice: 128 x 1024 x 7168 28.1 / 11.5 us (128 columns, four CTAs), 128 x 4096 x 4096 17.9 / 10.5
+// (the same), 512 x 2048 x 7168 28.6 / 17.4 (two CTAs), 1024 x 2048 x 7168 29.2 / 22.4 (256 columns, two CTAs), 512 x 4096 x 1024 8.1 / 6.9 (128
+// columns, whole), 896 x 2560 x 3584 17.1 / 15.0 (the same). The other side of the line: 2560 x 3072 x 2048 in 128 columns 32.0 / 22.2, 256 x 4096 x
+// 1536 with two CTAs to tiles of 256 columns 10.9 / 8.2. Six and eight CTAs to a tile gained nothing over four; widths of 160 to 224, whose warps meet
+// two scales of W, lost 5 to 50 %.
 static void planFp8(const ncclTpContext* tp, TpGemmArgs* a, int* width, int* grid) {
   const int blocks = a->K / 128;
   const int only = paramTpFp8Width() == 128 || paramTpFp8Width() == 256 ? (int)paramTpFp8Width() : 0;
