@@ -68,7 +68,7 @@ class FSDPEngine:
     def __init__(self, comm, cfg, device="cuda", seed=0, lr=1e-4, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.1, symmetric=True, init_on_device=False,
                  keep_layers=None):
         """keep_layers: how many layers may keep their activations for the backward at most (0: all are computed again there); None: as many as
-        memory allows."""
+        memory allows. What they take stays with the framework's allocator between steps (torch.cuda.empty_cache() gives it back)."""
         self.comm, self.cfg, self.device = comm, cfg, torch.device(device)
         self.keep_layers = keep_layers
         self.cuda = self.device.type == "cuda"
