@@ -183,6 +183,7 @@ def test_attention_that_saves_probabilities(fused_attention, monkeypatch):
         eng.close()
     assert abs(losses[1] - losses[0]) <= 2 ** -9 * losses[0]
     if not fused_attention:
-        # a layer's 1 / rms, handed back at once: two words a token
-        assert peaks[1] <= peaks[0] + 2 * 4 * tok.numel()
+        # a block may be up to 1 MiB larger than what it was taken for, by what the allocator had at hand; one layer that keeps its probabilities
+        # in bf16 takes 16 MiB
+        assert peaks[1] - peaks[0] < 2 * cfg.heads * tok.numel() ** 2
     comm.destroy()
